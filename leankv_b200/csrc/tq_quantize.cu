@@ -13,6 +13,7 @@
 // distance of a decision boundary.
 
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tq_layout.cuh"
@@ -22,13 +23,6 @@ namespace leankv {
 namespace {
 
 constexpr int kDim = LEANKV_TQ_DIM;
-constexpr int kTileVecs = 128;
-constexpr int kTileThreads = 256;
-constexpr size_t kTileSmemBytes = 2 * (size_t)kDim * 128 * sizeof(float);   // A and B panels
-
-__device__ __forceinline__ int packed_len_dev(int bits) {
-    return bits == 1 ? kDim / 8 : bits == 2 ? kDim / 4 : bits <= 4 ? kDim / 2 : kDim;
-}
 
 // Sum of squares of 64 values in fp64, ascending order.
 __device__ __forceinline__ double sumsq64(const float (&x)[64]) {
@@ -36,183 +30,6 @@ __device__ __forceinline__ double sumsq64(const float (&x)[64]) {
 #pragma unroll
     for (int i = 0; i < 64; ++i) s = fma((double)x[i], (double)x[i], s);
     return s;
-}
-
-struct TileParams {
-    const void* x;          // quantize: input vectors; dequantize: unused
-    int x_dtype;            // 0 fp16, 1 fp32
-    long long n_vec;
-    int bits;
-    const float* Pi;
-    const float* table;     // quantize: decision boundaries (2^bits-1); dequantize: centroids
-    uint8_t* indices;
-    float* norms;
-    void* out;              // dequantize output
-    int out_dtype;
-};
-
-// One CTA = 128 vectors x 128 coordinates, 8x8 register tile per thread, k ascending.
-// kQuantize: A[k][v] = u_v[k], B[k][j] = Pi[j][k]  -> y ; else A[k][v] = c[code_v[k]],
-// B[k][j] = Pi[k][j] -> x_hat (rotate_backward, leankv/turboquant/rotation.py:50-52).
-template <bool kQuantize>
-__global__ void __launch_bounds__(kTileThreads, 1) tq_tile_kernel(const TileParams p) {
-    extern __shared__ __align__(16) float smem[];
-    float* s_a = smem;                 // [k][128 vectors]
-    float* s_b = smem + kDim * 128;    // [k][128 coords]
-    __shared__ float s_norm[kTileVecs];
-    __shared__ float s_table[16];
-
-    const int tid = threadIdx.x;
-    const int bits = p.bits;
-    const int n_table = kQuantize ? (1 << bits) - 1 : (1 << bits);
-    if (tid < 16) s_table[tid] = tid < n_table ? p.table[tid] : __int_as_float(0x7f800000);
-
-    // B panel, loaded once per CTA (persistent over tiles).
-    for (int i = tid; i < kDim * kDim; i += kTileThreads) {
-        if (kQuantize) {
-            const int j = i & 127, k = i >> 7;   // lanes walk j: strided global read, conflict-free store
-            s_b[k * 128 + j] = p.Pi[j * kDim + k];
-        } else {
-            s_b[i] = p.Pi[i];
-        }
-    }
-
-    const int plen = packed_len_dev(bits);
-    const int vpb = kDim / plen;                  // codes per byte
-    const int bw = 8 / vpb;                       // bits per packed field
-    const long long n_tiles = (p.n_vec + kTileVecs - 1) / kTileVecs;
-
-    for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        const long long v0 = tile * kTileVecs;
-        __syncthreads();   // previous tile's readers of s_a are done; tables are visible
-        {
-            const int v = tid >> 1, hf = tid & 1;
-            const long long gv = v0 + v;
-            const bool ok = gv < p.n_vec;
-            if (kQuantize) {
-                float xr[64];
-                if (ok && p.x_dtype == 0) {
-                    const uint4* src = reinterpret_cast<const uint4*>(
-                        static_cast<const __half*>(p.x) + gv * kDim + hf * 64);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const uint4 w = __ldg(src + i);
-                        const float2 a = h2_to_f2(w.x), b = h2_to_f2(w.y), c = h2_to_f2(w.z),
-                                     d = h2_to_f2(w.w);
-                        xr[8 * i + 0] = a.x; xr[8 * i + 1] = a.y; xr[8 * i + 2] = b.x; xr[8 * i + 3] = b.y;
-                        xr[8 * i + 4] = c.x; xr[8 * i + 5] = c.y; xr[8 * i + 6] = d.x; xr[8 * i + 7] = d.y;
-                    }
-                } else if (ok) {
-                    const float4* src = reinterpret_cast<const float4*>(
-                        static_cast<const float*>(p.x) + gv * kDim + hf * 64);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const float4 w = __ldg(src + i);
-                        xr[4 * i + 0] = w.x; xr[4 * i + 1] = w.y; xr[4 * i + 2] = w.z; xr[4 * i + 3] = w.w;
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 64; ++i) xr[i] = 0.f;
-                }
-                const double mine = sumsq64(xr);
-                const double other = __shfl_xor_sync(0xffffffffu, mine, 1);
-                const double tot = hf == 0 ? mine + other : other + mine;
-                const float norm = (float)sqrt(tot);
-                const float denom = norm + 1e-10f;
-                if (hf == 0) s_norm[v] = norm;
-#pragma unroll
-                for (int i = 0; i < 64; ++i) s_a[(hf * 64 + i) * 128 + v] = xr[i] / denom;
-            } else {
-                const uint32_t mask = (1u << bw) - 1u;
-                const int bytes_half = plen / 2;
-                const uint8_t* src = p.indices + gv * plen + hf * bytes_half;
-                for (int bi = 0; bi < bytes_half; ++bi) {
-                    const uint32_t byte = ok ? src[bi] : 0u;
-                    for (int q = 0; q < vpb; ++q) {
-                        const int k = hf * 64 + bi * vpb + q;
-                        const int code = (byte >> (q * bw)) & mask;
-                        s_a[k * 128 + v] = ok ? s_table[code & 15] : 0.f;
-                    }
-                }
-                if (hf == 0) s_norm[v] = ok ? p.norms[gv] : 0.f;
-            }
-        }
-        __syncthreads();
-
-        const int tm = tid >> 4, tn = tid & 15;
-        float acc[8][8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-
-#pragma unroll 4
-        for (int k = 0; k < kDim; ++k) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&s_a[k * 128 + tm * 8]);
-            const float4 a1 = *reinterpret_cast<const float4*>(&s_a[k * 128 + tm * 8 + 4]);
-            const float4 b0 = *reinterpret_cast<const float4*>(&s_b[k * 128 + tn * 4]);
-            const float4 b1 = *reinterpret_cast<const float4*>(&s_b[k * 128 + 64 + tn * 4]);
-            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(b[j], a[i], acc[i][j]);
-        }
-
-        if (kQuantize) {
-            __syncthreads();   // everyone has finished reading s_a: reuse it for the codes
-            uint8_t* s_code = reinterpret_cast<uint8_t*>(s_a);   // [128 vectors][128 coords]
-            const int nb = n_table;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                uint32_t lo = 0, hi = 0;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    int c = 0;
-                    for (int q = 0; q < nb; ++q) c += (acc[i][j] > s_table[q]) ? 1 : 0;
-                    if (j < 4) lo |= (uint32_t)c << (8 * j);
-                    else hi |= (uint32_t)c << (8 * (j - 4));
-                }
-                const int v = tm * 8 + i;
-                *reinterpret_cast<uint32_t*>(&s_code[v * 128 + tn * 4]) = lo;
-                *reinterpret_cast<uint32_t*>(&s_code[v * 128 + 64 + tn * 4]) = hi;
-            }
-            __syncthreads();
-            const int total = kTileVecs * plen;
-            for (int o = tid; o < total; o += kTileThreads) {
-                const int v = o / plen, bi = o - v * plen;
-                if (v0 + v < p.n_vec) {
-                    uint32_t byte = 0;
-                    for (int q = 0; q < vpb; ++q) byte |= (uint32_t)s_code[v * 128 + bi * vpb + q] << (q * bw);
-                    p.indices[(v0 + v) * plen + bi] = (uint8_t)byte;
-                }
-            }
-            if (tid < kTileVecs && v0 + tid < p.n_vec) p.norms[v0 + tid] = s_norm[tid];
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int v = tm * 8 + i;
-                const long long gv = v0 + v;
-                if (gv >= p.n_vec) continue;
-                const float n = s_norm[v];
-                float r[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) r[j] = acc[i][j] * n;
-                if (p.out_dtype == 1) {
-                    float* o = static_cast<float*>(p.out) + gv * kDim;
-                    *reinterpret_cast<float4*>(o + tn * 4) = make_float4(r[0], r[1], r[2], r[3]);
-                    *reinterpret_cast<float4*>(o + 64 + tn * 4) = make_float4(r[4], r[5], r[6], r[7]);
-                } else {
-                    __half* o = static_cast<__half*>(p.out) + gv * kDim;
-                    __half2 h[4] = {__floats2half2_rn(r[0], r[1]), __floats2half2_rn(r[2], r[3]),
-                                    __floats2half2_rn(r[4], r[5]), __floats2half2_rn(r[6], r[7])};
-                    *reinterpret_cast<uint2*>(o + tn * 4) = *reinterpret_cast<uint2*>(&h[0]);
-                    *reinterpret_cast<uint2*>(o + 64 + tn * 4) = *reinterpret_cast<uint2*>(&h[2]);
-                }
-            }
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -357,6 +174,7 @@ __global__ void __launch_bounds__(128) tq_pool_append_kernel(const AppendParams 
 
 #include "tq_append_tc.cuh"
 #include "tq_append_t5.cuh"
+#include "tq_rows.cuh"
 
 // Coordinates decided by the exact chain / coordinates quantized by the tensor-core append, per device,
 // since the last reset (read by leankv_tq_band_stats).
@@ -421,26 +239,37 @@ int check_tq_common(long long n_vec, int dim, int bits) {
     return LEANKV_OK;
 }
 
-template <bool kQuantize>
-int launch_tile(const TileParams& p, void* stream) {
-    // The opt-in to 128 KiB of dynamic shared memory belongs to a device's copy of the function, so it is
-    // remembered per device ordinal (a process may quantize on several GPUs). Racing first calls all
-    // store the same value.
+// What a device is asked once: the kernel's opt-in to large shared memory, the status word's address. Racing first
+// calls store the same values.
+template <auto kKernel, typename... More>
+int launch_rows(RowsParams p, int per_cta, int threads, size_t smem, void* stream, More... more) {      // per_cta: vectors at least
     constexpr int kMaxDevices = 64;
-    static bool attr_done[kMaxDevices][2] = {};
+    static int* status[kMaxDevices] = {};
     int dev = 0;
     LEANKV_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDevices || !attr_done[dev][kQuantize]) {
-        LEANKV_CUDA_TRY(cudaFuncSetAttribute(tq_tile_kernel<kQuantize>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kTileSmemBytes));
-        if (dev >= 0 && dev < kMaxDevices) attr_done[dev][kQuantize] = true;
+    if (dev < 0 || dev >= kMaxDevices) return LEANKV_ELIMIT;
+    if (status[dev] == nullptr) {
+        void* word = nullptr;
+        LEANKV_CUDA_TRY(cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        LEANKV_CUDA_TRY(cudaGetSymbolAddress(&word, g_append_status));
+        status[dev] = static_cast<int*>(word);
     }
-    const long long n_tiles = (p.n_vec + kTileVecs - 1) / kTileVecs;
-    const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-    tq_tile_kernel<kQuantize><<<grid, kTileThreads, kTileSmemBytes, static_cast<cudaStream_t>(stream)>>>(p);
+    p.wide = aligned16(p.indices) ? 1 : 0;
+    p.status = status[dev];
+    const long long want = (p.n_vec + per_cta - 1) / per_cta;
+    const int grid = (int)(want < sm_count() ? want : sm_count());
+    kKernel<<<grid, threads, smem, static_cast<cudaStream_t>(stream)>>>(p, more...);
     LEANKV_CUDA_TRY(cudaGetLastError());
     return LEANKV_OK;
+}
+template <typename Raw>
+int launch_quantize(const RowsParams& p, int bits, void* stream) {
+    switch (bits) {
+        case 1: return launch_rows<tq_quantize_rows_kernel<1, Raw>>(p, kRowsTile, kRowsThreads, kRowsSmemBytes, stream);
+        case 2: return launch_rows<tq_quantize_rows_kernel<2, Raw>>(p, kRowsTile, kRowsThreads, kRowsSmemBytes, stream);
+        case 3: return launch_rows<tq_quantize_rows_kernel<3, Raw>>(p, kRowsTile, kRowsThreads, kRowsSmemBytes, stream);
+        default: return launch_rows<tq_quantize_rows_kernel<4, Raw>>(p, kRowsTile, kRowsThreads, kRowsSmemBytes, stream);
+    }
 }
 
 }  // namespace
@@ -463,16 +292,14 @@ extern "C" int leankv_tq_quantize(const void* x, int x_dtype, long long n_vec, i
     if (!x || !Pi || !decision_boundaries || !indices || !norms) return LEANKV_EINVAL;
     if (x_dtype != 0 && x_dtype != 1) return LEANKV_EINVAL;
     if (!aligned16(x) || !aligned16(Pi)) return LEANKV_EALIGN;
-    TileParams p{};
+    RowsParams p{};
     p.x = x;
-    p.x_dtype = x_dtype;
     p.n_vec = n_vec;
-    p.bits = bits;
     p.Pi = Pi;
     p.table = decision_boundaries;
     p.indices = indices;
     p.norms = norms;
-    return launch_tile<true>(p, stream);
+    return x_dtype == 0 ? launch_quantize<__half>(p, bits, stream) : launch_quantize<float>(p, bits, stream);
 }
 
 extern "C" int leankv_tq_dequantize(const uint8_t* indices, const float* norms, long long n_vec,
@@ -484,16 +311,15 @@ extern "C" int leankv_tq_dequantize(const uint8_t* indices, const float* norms, 
     if (!indices || !norms || !Pi || !centroids || !x_hat) return LEANKV_EINVAL;
     if (out_dtype != 0 && out_dtype != 1) return LEANKV_EINVAL;
     if (!aligned16(x_hat) || !aligned16(Pi)) return LEANKV_EALIGN;
-    TileParams p{};
+    RowsParams p{};
     p.n_vec = n_vec;
-    p.bits = bits;
     p.Pi = Pi;
     p.table = centroids;
     p.indices = const_cast<uint8_t*>(indices);
     p.norms = const_cast<float*>(norms);
     p.out = x_hat;
     p.out_dtype = out_dtype;
-    return launch_tile<false>(p, stream);
+    return launch_rows<tq_dequantize_rows_kernel>(p, 16, kDequantThreads, kDequantSmemBytes, stream, bits);
 }
 
 extern "C" size_t leankv_tq_pool_bytes(int n_pages, int n_kv_heads) {

@@ -6,7 +6,7 @@ import torch
 
 from conftest import rel_l2
 from gpu_util import RawPool, oracle_attention_from_pool
-from leankv_b200 import workloads
+from leankv_b200 import _native, workloads
 from leankv_b200.turboquant.cache import TurboQuantCache
 from leankv_b200.turboquant.paged_cache import PagedKVCache
 from leankv_b200.turboquant.quantizer import MSEQuantized, TurboQuantMSE, TurboQuantProd
@@ -576,3 +576,40 @@ def test_paged_cache_page_table_on_device_follows_the_reference_allocator():
     rc = cache._table_step(4000, 3)
     assert cache.page_table_status() & 1
     assert cache._seq_len_dev[:3].tolist() == lens          # no sequence grew
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 127, 128, 129, 2500, 148 * 128 + 1, 148 * 256 + 77])
+@pytest.mark.parametrize("bits", [1, 2, 3, 4])
+def test_quantize_and_dequantize_at_the_edges_of_their_tiles(n, bits):
+    """Tiles of 128 vectors, ranges in units of 16, more tiles than SMs; codes, norms and restored vectors are bits."""
+    quant = TurboQuantMSE(128, bits, _dev(), torch.float32, seed=11)
+    gen = torch.Generator().manual_seed(n + bits)
+    x = torch.randn(n, 128, generator=gen)
+    x[::7] *= 1e-3
+    x[5::31] = 0.0
+    x[1::3] *= 1e-14         # fp32 only: every coordinate next to the middle boundary
+    for xin in (x.half(), x):
+        q = quant.quantize(xin.to(_dev()))
+        codes, norms, _, _ = tq_exact.quantize(xin.float().numpy(), quant.Pi.cpu().numpy(),
+                                               quant.decision_boundaries.cpu().numpy())
+        per, width = {1: (8, 1), 2: (4, 2)}.get(bits, (2, 4))
+        packed = sum(codes.reshape(n, -1, per)[..., i].astype(np.uint8) << (width * i) for i in range(per))
+        assert np.array_equal(q.indices.cpu().numpy(), packed)
+        want_norms = torch.from_numpy(norms).to(xin.dtype)
+        assert torch.equal(q.norms.cpu(), want_norms)
+        out = quant.dequantize(q).cpu().numpy()
+        exact = tq_exact.dequantize(codes, want_norms.float().numpy(), quant.Pi.cpu().numpy(), quant.centroids.cpu().numpy())
+        assert np.array_equal(out, exact)
+
+    # indices that lie on no 4-byte boundary
+    buf = torch.zeros(packed.size + 1, dtype=torch.uint8, device=_dev())
+    nrm = torch.zeros(n, device=_dev())
+    Pi, _, bounds = quant._consts()
+    xd, lib = x.to(_dev()), _native.lib()
+    _native.check(lib.leankv_tq_quantize(xd.data_ptr(), 1, n, 128, bits, Pi.data_ptr(), bounds.data_ptr(),
+                                         buf.data_ptr() + 1, nrm.data_ptr(), _native.current_stream()), "quantize")
+    assert np.array_equal(buf[1:].cpu().numpy().reshape(packed.shape), packed)
+    back = torch.empty(n, 128, device=_dev())
+    _native.check(lib.leankv_tq_dequantize(buf.data_ptr() + 1, nrm.data_ptr(), n, 128, bits, Pi.data_ptr(),
+                                           quant._consts()[1].data_ptr(), back.data_ptr(), 1, _native.current_stream()), "dequantize")
+    assert np.array_equal(back.cpu().numpy(), exact)
