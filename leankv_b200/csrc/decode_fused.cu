@@ -33,12 +33,16 @@ struct PostParams {
     float* q_rot;             // [B][nq][128]
 };
 
-__global__ void __launch_bounds__(kDim) decode_qkv_post_kernel(const PostParams p) {
-    __shared__ float s_x[kDim];       // the head vector (after rotary embedding, fp16 values)
-    __shared__ float s_u[kDim];       // what gets rotated: x for q, x / (norm + 1e-10) for k and v
-    __shared__ double s_ss[2];
+// A CTA serves one head for kSeqs sequences at a time, its rotation column in registers. What bounds it is the chain of
+// one vector (the fp64 sum of 64 squares alone is 64 dependent steps), not any unit, so a batch takes four sequences
+// through the chain together: 32 sequences, 48 heads: 21.9 -> 12.6 us.
+template <int kSeqs>
+__global__ void __launch_bounds__(kDim, kSeqs > 1 ? 3 : 1) decode_qkv_post_kernel(const PostParams p) {
+    __shared__ float s_x[kSeqs][kDim];       // the head vectors (after rotary embedding, fp16 values)
+    __shared__ __align__(16) float s_u[kSeqs][kDim];   // what gets rotated: x for q, x / (norm + 1e-10) for k and v
+    __shared__ double s_ss[kSeqs][2];
     __shared__ float s_bounds[8];
-    __shared__ __align__(4) uint8_t s_code[kDim];
+    __shared__ __align__(4) uint8_t s_code[kSeqs][kDim];
 
     const int j = threadIdx.x;
     const int head = blockIdx.x;
@@ -53,108 +57,140 @@ __global__ void __launch_bounds__(kDim) decode_qkv_post_kernel(const PostParams 
     pdl_begin();
     if (j < 8) s_bounds[j] = j < 7 ? p.bounds[j] : __int_as_float(0x7f800000);
     const int row = (p.nq + 2 * p.nkv) * kDim;
+    const int which = kind - 1;
+    const int h = which == 0 ? head - p.nq : head - p.nq - p.nkv;
 
-    // One CTA serves its head for every gridDim.y-th sequence with the rotation column held in registers.
-    for (int b = blockIdx.y; b < p.B; b += gridDim.y) {
-        const int pos = p.pos[b];
-        const __half* src = p.qkv + (size_t)b * row + (size_t)head * kDim;
-        // where the new token goes: fetched now so that the page-table round trip (and, for V, the word
+    for (int b0 = blockIdx.y * kSeqs; b0 < p.B; b0 += gridDim.y * kSeqs) {
+        // where the new tokens go: fetched now so that the page-table round trip (and, for V, the word
         // shared with the pair token) overlaps the arithmetic instead of trailing it
-        const int which = kind - 1;
-        const int h = which == 0 ? head - p.nq : head - p.nq - p.nkv;
-        const int slot = pos & 15;
-        int page = -1;
-        uint32_t* words = nullptr;
-        uint32_t old_word = 0;
-        if (kind != 0) {
-            const int base = p.kv_indptr != nullptr ? p.kv_indptr[b] : 0;
-            page = p.page_indices[base + (pos >> 4)];
-            if (page >= 0 && page < p.n_pages) {
-                words = reinterpret_cast<uint32_t*>(p.pool + (((size_t)page * 2 + which) * p.nkv + h) * kChunkBytes);
-                if (which == 1 && j < 24) {
-                    const int g = j & 7, kk = j >> 3, pr = slot >> 1;
-                    old_word = words[kk * 64 + (pr < 4 ? 4 * g + pr : 32 + 4 * g + (pr - 4))];
+        int slot[kSeqs];
+        uint32_t* words[kSeqs];
+        uint32_t old_word[kSeqs];
+        float xf[kSeqs];
+#pragma unroll
+        for (int q = 0; q < kSeqs; ++q) {
+            const int b = min(b0 + q, p.B - 1);          // a sequence beyond the batch is computed and not stored
+            const int pos = p.pos[b];
+            const __half* src = p.qkv + (size_t)b * row + (size_t)head * kDim;
+            slot[q] = pos & 15;
+            words[q] = nullptr;
+            old_word[q] = 0;
+            if (kind != 0 && b0 + q < p.B) {
+                const int base = p.kv_indptr != nullptr ? p.kv_indptr[b] : 0;
+                const int page = p.page_indices[base + (pos >> 4)];
+                if (page >= 0 && page < p.n_pages) {
+                    words[q] = reinterpret_cast<uint32_t*>(p.pool + (((size_t)page * 2 + which) * p.nkv + h) * kChunkBytes);
+                    if (which == 1 && j < 24) {
+                        const int g = j & 7, kk = j >> 3, pr = slot[q] >> 1;
+                        old_word[q] = words[q][kk * 64 + (pr < 4 ? 4 * g + pr : 32 + 4 * g + (pr - 4))];
+                    }
                 }
             }
+            __half xv = src[j];
+            if (kind != 2) {
+                // rotate_half form: out[i] = x[i] cos - x[i+64] sin ; out[i+64] = x[i+64] cos + x[i] sin,
+                // cos/sin rounded to fp16, products and sum in fp16 (HF apply_rotary_pos_emb)
+                const int i = j & 63;
+                const float ang = (float)pos * p.inv_freq[i];
+                const __half c = __float2half_rn(cosf(ang)), s = __float2half_rn(sinf(ang));
+                const __half other = src[j ^ 64];
+                xv = j < 64 ? __hadd(__hmul(xv, c), __hmul(__hneg(other), s))
+                            : __hadd(__hmul(xv, c), __hmul(other, s));
+            }
+            xf[q] = __half2float(xv);
         }
-
-        __half xv = src[j];
-        if (kind != 2) {
-            // rotate_half form: out[i] = x[i] cos - x[i+64] sin ; out[i+64] = x[i+64] cos + x[i] sin,
-            // cos/sin rounded to fp16, products and sum in fp16 (HF apply_rotary_pos_emb)
-            const int i = j & 63;
-            const float ang = (float)pos * p.inv_freq[i];
-            const __half c = __float2half_rn(cosf(ang)), s = __float2half_rn(sinf(ang));
-            const __half other = src[j ^ 64];
-            xv = j < 64 ? __hadd(__hmul(xv, c), __hmul(__hneg(other), s))
-                        : __hadd(__hmul(xv, c), __hmul(other, s));
-        }
-        const float xf = __half2float(xv);
-        __syncthreads();                       // the previous sequence's readers of s_x / s_u / s_code are done
-        s_x[j] = xf;
+        __syncthreads();                       // the previous sequences' readers of s_x / s_u / s_code are done
+#pragma unroll
+        for (int q = 0; q < kSeqs; ++q) s_x[q][j] = xf[q];
         __syncthreads();
 
-        float norm = 0.f;
+        float norm[kSeqs];
         if (kind != 0) {
             // fp64 sums of squares of coordinates 0..63 and 64..127, ascending (one thread each)
-            if ((j & 63) == 0) {
+            if ((j & 63) < kSeqs) {
                 double ss = 0.0;
 #pragma unroll 8
                 for (int k = 0; k < 64; ++k) {
-                    const double v = (double)s_x[j + k];
+                    const double v = (double)s_x[j & 63][(j & 64) + k];
                     ss = fma(v, v, ss);
                 }
-                s_ss[j >> 6] = ss;
+                s_ss[j & 63][j >> 6] = ss;
             }
             __syncthreads();
-            norm = (float)sqrt(s_ss[0] + s_ss[1]);
-            s_u[j] = xf / (norm + 1e-10f);
+#pragma unroll
+            for (int q = 0; q < kSeqs; ++q) {
+                norm[q] = (float)sqrt(s_ss[q][0] + s_ss[q][1]);
+                s_u[q][j] = xf[q] / (norm[q] + 1e-10f);
+            }
         } else {
-            s_u[j] = xf;
+#pragma unroll
+            for (int q = 0; q < kSeqs; ++q) {
+                norm[q] = 0.f;
+                s_u[q][j] = xf[q];
+            }
         }
         __syncthreads();
 
         // y_j = sum_k Pi[j][k] u[k], k ascending
-        float y = 0.f;
+        float y[kSeqs];
 #pragma unroll
-        for (int k = 0; k < kDim; ++k) y = fmaf(pi_col[k], s_u[k], y);
+        for (int q = 0; q < kSeqs; ++q) y[q] = 0.f;
+#pragma unroll
+        for (int k = 0; k < kDim; k += 4) {
+#pragma unroll
+            for (int q = 0; q < kSeqs; ++q) {
+                const float4 u = *reinterpret_cast<const float4*>(&s_u[q][k]);
+                y[q] = fmaf(pi_col[k], u.x, y[q]);
+                y[q] = fmaf(pi_col[k + 1], u.y, y[q]);
+                y[q] = fmaf(pi_col[k + 2], u.z, y[q]);
+                y[q] = fmaf(pi_col[k + 3], u.w, y[q]);
+            }
+        }
         if (kind == 0) {
-            p.q_rot[((size_t)b * p.nq + head) * kDim + j] = y;
+#pragma unroll
+            for (int q = 0; q < kSeqs; ++q)
+                if (b0 + q < p.B) p.q_rot[((size_t)(b0 + q) * p.nq + head) * kDim + j] = y[q];
             continue;
         }
-        int code = 0;
 #pragma unroll
-        for (int q = 0; q < 7; ++q) code += (y > s_bounds[q]) ? 1 : 0;
-        s_code[j] = (uint8_t)code;
+        for (int q = 0; q < kSeqs; ++q) {
+            int code = 0;
+#pragma unroll
+            for (int i = 0; i < 7; ++i) code += (y[q] > s_bounds[i]) ? 1 : 0;
+            s_code[q][j] = (uint8_t)code;
+        }
         __syncthreads();
 
-        if (words == nullptr) continue;
-        uint8_t* chunk = reinterpret_cast<uint8_t*>(words);
-        if (j == 0) reinterpret_cast<__half*>(chunk + kNormOffsetBytes)[slot] = __float2half_rn(norm);
+#pragma unroll
+        for (int q = 0; q < kSeqs; ++q) {
+            if (words[q] == nullptr) continue;
+            uint8_t* chunk = reinterpret_cast<uint8_t*>(words[q]);
+            if (j == 0) reinterpret_cast<__half*>(chunk + kNormOffsetBytes)[slot[q]] = __float2half_rn(norm[q]);
 
-        // four codes per 32-bit shared-memory load; pack4 squeezes the low nibbles of 4 bytes into 16 bits
-        auto pack4 = [](uint32_t v) -> uint32_t {
-            const uint32_t t2 = (v | (v >> 4)) & 0x00FF00FFu;
-            return (t2 | (t2 >> 8)) & 0xFFFFu;
-        };
-        if (which == 0) {
-            if (j < 12) {                      // 4 units (quarters of the vector) x 3 words, this token only
-                const int t4 = j & 3, kk = j >> 2;
-                const uint32_t* c4 = reinterpret_cast<const uint32_t*>(&s_code[32 * t4]);
-                const uint32_t lo = c4[2 * kk] & 0x07070707u, hi = c4[2 * kk + 1] & 0x07070707u;
-                const uint32_t s_lo = ((c4[6] >> kk) & 0x01010101u) << 3, s_hi = ((c4[7] >> kk) & 0x01010101u) << 3;
-                words[kk * 64 + slot * 4 + t4] = pack4(lo) | (pack4(hi) << 16) | pack4(s_lo) | (pack4(s_hi) << 16);
-            }
-        } else {
-            if (j < 24) {                      // 8 units (16-coordinate groups) x 3 words, shared with the pair token
-                const int g = j & 7, kk = j >> 3;
-                const int pr = slot >> 1, par = slot & 1;
-                const int ui = pr < 4 ? 4 * g + pr : 32 + 4 * g + (pr - 4);
-                const uint32_t* ca = reinterpret_cast<const uint32_t*>(&s_code[16 * g]);
-                const uint32_t a4 = ca[kk] & 0x07070707u, as4 = (ca[3] >> kk) & 0x01010101u;
-                const uint32_t bits = par ? ((a4 << 4) | (as4 << 7)) : (a4 | (as4 << 3));
-                const uint32_t keep = par ? 0x0F0F0F0Fu : 0xF0F0F0F0u;   // the other token's nibbles
-                words[kk * 64 + ui] = bits | (old_word & keep);
+            // four codes per 32-bit shared-memory load; pack4 squeezes the low nibbles of 4 bytes into 16 bits
+            auto pack4 = [](uint32_t v) -> uint32_t {
+                const uint32_t t2 = (v | (v >> 4)) & 0x00FF00FFu;
+                return (t2 | (t2 >> 8)) & 0xFFFFu;
+            };
+            if (which == 0) {
+                if (j < 12) {                      // 4 units (quarters of the vector) x 3 words, this token only
+                    const int t4 = j & 3, kk = j >> 2;
+                    const uint32_t* c4 = reinterpret_cast<const uint32_t*>(&s_code[q][32 * t4]);
+                    const uint32_t lo = c4[2 * kk] & 0x07070707u, hi = c4[2 * kk + 1] & 0x07070707u;
+                    const uint32_t s_lo = ((c4[6] >> kk) & 0x01010101u) << 3, s_hi = ((c4[7] >> kk) & 0x01010101u) << 3;
+                    words[q][kk * 64 + slot[q] * 4 + t4] = pack4(lo) | (pack4(hi) << 16) | pack4(s_lo) | (pack4(s_hi) << 16);
+                }
+            } else {
+                if (j < 24) {                      // 8 units (16-coordinate groups) x 3 words, shared with the pair token
+                    const int g = j & 7, kk = j >> 3;
+                    const int pr = slot[q] >> 1, par = slot[q] & 1;
+                    const int ui = pr < 4 ? 4 * g + pr : 32 + 4 * g + (pr - 4);
+                    const uint32_t* ca = reinterpret_cast<const uint32_t*>(&s_code[q][16 * g]);
+                    const uint32_t a4 = ca[kk] & 0x07070707u, as4 = (ca[3] >> kk) & 0x01010101u;
+                    const uint32_t bits = par ? ((a4 << 4) | (as4 << 7)) : (a4 | (as4 << 3));
+                    const uint32_t keep = par ? 0x0F0F0F0Fu : 0xF0F0F0F0u;   // the other token's nibbles
+                    words[q][kk * 64 + ui] = bits | (old_word[q] & keep);
+                }
             }
         }
     }
@@ -188,11 +224,17 @@ static int post_launch(const void* qkv, int B, const float* inv_freq, const int3
     p.nq = n_q_heads;
     p.nkv = n_kv_heads;
     p.q_rot = q_rot;
-    // enough CTAs to fill the GPU a few times over, each reusing its rotation column for ~8 sequences
+    // One sequence alone keeps the kernel whose chain is its only work; a batch goes four at a time, over as many CTAs as are
+    // resident at once (two or three an SM), each of which walks the rest of its head's sequences with the same column.
     const int heads = n_q_heads + 2 * n_kv_heads;
-    const int gy = std::max(1, std::min(B, (B + 7) / 8));
-    LEANKV_CUDA_TRY(launch_kernel_ex(true, decode_qkv_post_kernel, dim3(heads, gy), dim3(kDim), 0,
-                                     static_cast<cudaStream_t>(stream), p));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (B == 1) {
+        LEANKV_CUDA_TRY(launch_kernel_ex(true, decode_qkv_post_kernel<1>, dim3(heads, 1), dim3(kDim), 0, st, p));
+    } else {
+        constexpr int kSeqs = 4;
+        const int gy = std::max(1, std::min((B + kSeqs - 1) / kSeqs, 3 * sm_count() / heads));
+        LEANKV_CUDA_TRY(launch_kernel_ex(true, decode_qkv_post_kernel<kSeqs>, dim3(heads, gy), dim3(kDim), 0, st, p));
+    }
     return LEANKV_OK;
 }
 
