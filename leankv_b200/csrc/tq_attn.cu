@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(128) tq_qrot_kernel(const __half* q, const flo
 #include "tq_attn_kernel.cuh"
 #include "tq_prefill_kernel.cuh"
 #include "tq_prefill_ws.cuh"
+#include "tq_prefill_tile.cuh"
 
 // ---- host side ---------------------------------------------------------------
 struct AttnPlan {
@@ -451,16 +452,45 @@ static long long prefill_rows_pages(long long first_pos, long long n) {
     return upto(first_pos + n) - upto(first_pos);
 }
 
-// The prefill attention's two products: tcgen05 with operands in shared memory (default), mma.sync
-// (LEANKV_PREFILL_MMA=sync), or the warp-specialised tcgen05 form with query and probabilities in tensor memory
-// (LEANKV_PREFILL_MMA=ws).
+// The prefill attention's kernel: expanded tiles (default), or the kernels that walk the pages themselves: tcgen05 with
+// operands in shared memory (LEANKV_PREFILL_MMA=t5), mma.sync (=sync), or the warp-specialised tcgen05 form with
+// query and probabilities in tensor memory (=ws).
 static int prefill_mode() {
     static int v = -1;
     if (v < 0) {
         const char* e = std::getenv("LEANKV_PREFILL_MMA");
-        v = (e != nullptr && e[0] == 's') ? 0 : (e != nullptr && e[0] == 'w') ? 2 : 1;
+        v = e == nullptr ? 3 : e[0] == 's' ? 0 : e[0] == 'w' ? 2 : e[0] == 't' ? 1 : 3;
     }
     return v;
+}
+
+// The expansion is scratch that grows with the context (17 MB per 4096 tokens and 8 kv heads); beyond this many tokens the
+// page-walking kernel, whose scratch does not, takes the call.
+constexpr long long kExpandMaxTokens = 65536;
+struct ExpandPlan {
+    int q_tiles, k_tiles, n_splits;
+    size_t off_images, off_records, off_opart, off_ml, total;
+};
+static bool expand_plan(int T, int start_pos, int Hq, int Hkv, ExpandPlan* pl) {
+    const long long n = (long long)start_pos + T;
+    if (prefill_mode() != 3 || n > kExpandMaxTokens || Hkv >= 65535) return false;
+    pl->q_tiles = (T + kPtTokens - 1) / kPtTokens;
+    pl->k_tiles = (int)((n + kPtKeys - 1) / kPtKeys);
+    // One CTA per SM: where the query tiles leave SMs idle the keys are cut into ranges of at least two tiles (each costs the
+    // two rotations again, about 4 us, against 0.8 us a tile).
+    const long long ctas = (long long)pl->q_tiles * Hkv;
+    long long s = sm_count() / ctas;
+    if (s > pl->k_tiles / 2) s = pl->k_tiles / 2;
+    if (s > kRotMaxSplits) s = kRotMaxSplits;
+    pl->n_splits = s < 1 ? 1 : (int)s;
+    const size_t n_vec = (size_t)T * Hq;
+    pl->off_images = 256;
+    pl->off_records = pl->off_images + 4 * (size_t)umma::kTileBytes;
+    pl->off_opart = pl->off_records + (size_t)Hkv * pl->k_tiles * (kPtK + kPtV);
+    const size_t parts = pl->n_splits > 1 ? (size_t)pl->n_splits : 0;
+    pl->off_ml = pl->off_opart + round_up(sizeof(float) * n_vec * kDim * parts, 256);
+    pl->total = pl->off_ml + round_up(sizeof(float) * n_vec * 2 * parts, 256);
+    return true;
 }
 
 struct TilePlan {
@@ -557,6 +587,8 @@ extern "C" size_t leankv_tq_prefill_attn_workspace_bytes(int T, int start_pos, i
     if (T <= 0 || T > 65535 || start_pos < 0 || (long long)start_pos + T > (1ll << 24) || n_q_heads <= 0 ||
         n_kv_heads <= 0 || prefill_rows_pages(start_pos, T) > 0x7fffffffll)
         return 0;
+    ExpandPlan ep;
+    if (expand_plan(T, start_pos, n_q_heads, n_kv_heads, &ep)) return ep.total;
     return make_tile_plan(T, start_pos, n_q_heads, n_kv_heads).total;
 }
 
@@ -577,11 +609,7 @@ extern "C" int leankv_tq_prefill_attn(const void* q, void* out, int T, int start
     if (workspace_bytes < leankv_tq_prefill_attn_workspace_bytes(T, start_pos, n_q_heads, n_kv_heads))
         return LEANKV_EWORKSPACE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const TilePlan tp = make_tile_plan(T, start_pos, n_q_heads, n_kv_heads);
     char* ws = static_cast<char*>(workspace);
-    float* qprime = reinterpret_cast<float*>(ws + tp.off_qprime);
-    float* o_part = reinterpret_cast<float*>(ws + tp.off_opart);
-    float* ml_part = reinterpret_cast<float*>(ws + tp.off_ml);
     const Lut& lut = get_lut(centroids);
     static std::atomic<unsigned long long> attr_done{0};          // bit per device ordinal (< 64)
     int dev = 0;
@@ -594,6 +622,8 @@ extern "C" int leankv_tq_prefill_attn(const void* q, void* out, int T, int start
                                              (int)kT5SmemBytes));
         LEANKV_CUDA_TRY(cudaFuncSetAttribute(tq_prefill_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)kWsSmemBytes));
+        LEANKV_CUDA_TRY(cudaFuncSetAttribute(tq_prefill_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kPtSmemBytes));
         LEANKV_CUDA_TRY(cudaFuncSetAttribute(tq_rot_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)kRotSmemBytes));
         LEANKV_CUDA_TRY(cudaFuncSetAttribute(tq_rot_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -602,6 +632,49 @@ extern "C" int leankv_tq_prefill_attn(const void* q, void* out, int T, int start
     }
     const int n_vec = T * n_q_heads;
     const int rot_grid = (n_vec + kRotRows - 1) / kRotRows;
+    ExpandPlan ep;
+    if (expand_plan(T, start_pos, n_q_heads, n_kv_heads, &ep)) {
+        ExpandParams e{};
+        e.pool = static_cast<const uint8_t*>(pool);
+        e.n_pages = n_pages;
+        e.H = n_kv_heads;
+        e.seq_pages = seq_pages;
+        e.n_tokens = start_pos + T;
+        e.n_tiles = ep.k_tiles;
+        e.tl0 = lut.tl0; e.tl1 = lut.tl1; e.th0 = lut.th0; e.th1 = lut.th1;
+        e.inv_alpha = 1.0f / lut.alpha;
+        e.Pi_k = Pi_k;
+        e.Pi_v = Pi_v;
+        e.records = reinterpret_cast<uint8_t*>(ws + ep.off_records);
+        e.images = reinterpret_cast<uint8_t*>(ws + ep.off_images);
+        e.status = reinterpret_cast<int*>(ws);
+        LEANKV_CUDA_TRY(launch_kernel(tq_expand_kernel, dim3(std::max(ep.k_tiles, 8), n_kv_heads + 1), dim3(256), 0, st, e));
+        TileAttnParams a{};
+        a.q = static_cast<const __half*>(q);
+        a.qscale = scale * kLog2e;
+        a.records = e.records;
+        a.images = e.images;
+        a.out = static_cast<__half*>(out);
+        a.o_part = reinterpret_cast<float*>(ws + ep.off_opart);
+        a.ml_part = reinterpret_cast<float*>(ws + ep.off_ml);
+        a.n_splits = ep.n_splits;
+        a.H = n_kv_heads;
+        a.T = T;
+        a.start_pos = start_pos;
+        a.n_tiles = ep.k_tiles;
+        a.status = e.status;
+        LEANKV_CUDA_TRY(launch_kernel(tq_prefill_tile_kernel, dim3(ep.q_tiles, n_kv_heads, ep.n_splits), dim3(kPtThreads),
+                                      kPtSmemBytes, st, a));
+        if (ep.n_splits > 1)
+            LEANKV_CUDA_TRY(launch_kernel(tq_rot_rows_kernel<false>, dim3(rot_grid), dim3(kRotThreads), kRotSmemBytes, st,
+                                          static_cast<const void*>(a.o_part), static_cast<const float*>(a.ml_part), ep.n_splits,
+                                          Pi_v, out, n_vec, e.status));
+        return LEANKV_OK;
+    }
+    const TilePlan tp = make_tile_plan(T, start_pos, n_q_heads, n_kv_heads);
+    float* qprime = reinterpret_cast<float*>(ws + tp.off_qprime);
+    float* o_part = reinterpret_cast<float*>(ws + tp.off_opart);
+    float* ml_part = reinterpret_cast<float*>(ws + tp.off_ml);
     LEANKV_CUDA_TRY(launch_kernel(tq_rot_rows_kernel<true>, dim3(rot_grid), dim3(kRotThreads), kRotSmemBytes, st, q,
                                   static_cast<const float*>(nullptr), 0, Pi_k, static_cast<void*>(qprime), n_vec,
                                   reinterpret_cast<int*>(ws)));

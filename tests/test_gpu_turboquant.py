@@ -613,3 +613,47 @@ def test_quantize_and_dequantize_at_the_edges_of_their_tiles(n, bits):
     _native.check(lib.leankv_tq_dequantize(buf.data_ptr() + 1, nrm.data_ptr(), n, 128, bits, Pi.data_ptr(),
                                            quant._consts()[1].data_ptr(), back.data_ptr(), 1, _native.current_stream()), "dequantize")
     assert np.array_equal(back.cpu().numpy(), exact)
+
+
+@pytest.mark.parametrize("H, start, T", [(1, 0, 1), (2, 0, 31), (2, 95, 33), (1, 127, 1), (1, 128, 129), (2, 0, 385), (8, 3000, 200),
+                                         (1, 5000, 40)])
+def test_prefill_attention_at_the_edges_of_its_tiles(H, start, T):
+    """Tiles of 32 queries and 128 keys, one tile and several, ranges of keys over several CTAs; scores up to the
+    hundreds, so that the running maximum moves late. Against 64-bit attention over the de-quantized codes."""
+    dev = _dev()
+    gen = torch.Generator().manual_seed(start + T)
+    n = start + T
+    pages = torch.randperm((n + 15) // 16 + 1, generator=gen).tolist()[:(n + 15) // 16]
+    rp = RawPool(len(pages) + 1, H, dev)
+    k = torch.randn(1, H, n, 128, generator=gen) * torch.linspace(0.2, 4.0, n).reshape(1, 1, n, 1)
+    v = torch.randn(1, H, n, 128, generator=gen)
+    rp.append(k.half().to(dev), v.half().to(dev), [0, len(pages)], pages, [0])
+    q = (torch.randn(T, 4 * H, 128, generator=gen) * 2).half().to(dev)
+    got = rp.prefill_attention(q, pages, start).double()
+    hats = []
+    for which, Pi in ((0, rp.Pi_k), (1, rp.Pi_v)):
+        idx, norms = rp.unpack(pages, n, which)
+        codes = torch.from_numpy(pool_layout.nibbles_to_codes(idx).astype(np.int64)).to(dev)
+        hats.append((rp.centroids.double()[codes] @ Pi.double()) * torch.from_numpy(norms).to(dev).double().unsqueeze(-1))
+    see = torch.arange(n, device=dev).reshape(1, n) <= start + torch.arange(T, device=dev).reshape(T, 1)
+    for h in range(4 * H):
+        s = (q[:, h].double() @ hats[0][h // 4].t()) * 128 ** -0.5
+        want = torch.softmax(s.masked_fill(~see, -float("inf")), -1) @ hats[1][h // 4]
+        off = (got[:, h] - want).norm(dim=-1) / want.norm(dim=-1)
+        assert off.max().item() < ATTN_TOL, (h, off.argmax().item(), off.max().item())
+
+
+def test_prefill_attention_that_walks_the_pages_passes_the_same_checks():
+    """Contexts beyond 65536 tokens take the kernel without scratch per token; LEANKV_PREFILL_MMA=t5 selects it at any."""
+    import os
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    env = dict(os.environ, LEANKV_PREFILL_MMA="t5")
+    r = subprocess.run([sys.executable, "-m", "pytest", os.path.join(ROOT, "tests", "test_gpu_turboquant.py"), "-m", "gpu", "-x", "-q",
+                        "-k", "prefill_attention_on_packed or prefill_attention_of_a_late or prefill_attention_at_the_edges"],
+                       env=env, capture_output=True, text=True, timeout=600, cwd=ROOT)
+    assert r.returncode == 0, (r.stdout[-2000:], r.stderr[-1000:])
+    assert "10 passed" in r.stdout
