@@ -587,8 +587,11 @@ extern "C" size_t leankv_tq_prefill_attn_workspace_bytes(int T, int start_pos, i
     if (T <= 0 || T > 65535 || start_pos < 0 || (long long)start_pos + T > (1ll << 24) || n_q_heads <= 0 ||
         n_kv_heads <= 0 || prefill_rows_pages(start_pos, T) > 0x7fffffffll)
         return 0;
+    // Never less than a decode call of as many rows takes (and its page-table rows): a caller may keep one workspace for both.
+    const size_t decode = leankv_tq_decode_attn_workspace_bytes(T, n_q_heads, n_kv_heads, (int)((start_pos + (long long)T + kPage - 1) / kPage)) +
+                          sizeof(int32_t) * (size_t)T;
     ExpandPlan ep;
-    if (expand_plan(T, start_pos, n_q_heads, n_kv_heads, &ep)) return ep.total;
+    if (expand_plan(T, start_pos, n_q_heads, n_kv_heads, &ep)) return std::max(ep.total, decode);
     return make_tile_plan(T, start_pos, n_q_heads, n_kv_heads).total;
 }
 
