@@ -392,6 +392,12 @@ int leankv_batch_qkv_post(const void* qkv, int B, const float* inv_freq, const i
                           float* q_rot, void* stream);
 /* out[r][i] = fp16(silu(gate_up[r][i])) * gate_up[r][inter + i]  (LlamaMLP's act_fn(gate) * up). */
 int leankv_silu_mul_f16(const void* gate_up, void* out, int rows, int inter, void* stream);
+/* The same of two matrices fp16 [rows][inter]; out may be either of them. */
+int leankv_silu_mul_pair_f16(const void* gate, const void* up, void* out, int rows, int inter, void* stream);
+/* A prompt chunk's projections, fp16 [T][n_q_heads + 2 n_kv_heads][128], apart: queries [T][n_q_heads][128] and keys
+ * [n_kv_heads][T][128] with the rotary embedding (rotate_half form; cos, sin: fp16 [T][128]), values [n_kv_heads][T][128]. */
+int leankv_rope_split_f16(const void* qkv, const void* cos, const void* sin, void* q, void* k, void* v, int T,
+                          int n_q_heads, int n_kv_heads, void* stream);
 /* Per sequence: tokens[b] = argmax(logits[b]) (lowest index on ties);
  * history[b][steps[b]] = tokens[b]; steps[b] += 1; pos[b] += 1. vocab % 8 == 0. */
 int leankv_batch_decode_end(const void* logits, int vocab, int B, long long* tokens,

@@ -308,8 +308,16 @@ __global__ void __launch_bounds__(kPtThreads, 1) tq_prefill_tile_kernel(const Ti
     umma::fence_after_sync();
 
     const bool whole = p.n_splits == 1;
+    // the copies in flight at the end of the copying thread's work land before the block can leave
+    auto landed = [&] {
+        for (int j = max(nk - 2, 0); j < nk; ++j) wait(kPtKFull, j);
+        for (int j = max(nv - 2, 0); j < nv; ++j) wait(kPtVFull, j);
+    };
     if (!ok) {
-        // fall through to the end
+        if (warp == 9 && lane == 0) {
+            umma::bar_wait(bar(kPtPiBar), 0);
+            landed();
+        }
     } else if (warp == 9) {
         // ---- copies ----
         if (lane == 0) {
@@ -329,12 +337,10 @@ __global__ void __launch_bounds__(kPtThreads, 1) tq_prefill_tile_kernel(const Ti
                 if (ok) {
                     mbar_expect_tx(bar(kPtPiBar), 2 * umma::kTileBytes);
                     bulk_g2s(smem_u32(s_k), p.images + 2 * umma::kTileBytes, 2 * umma::kTileBytes, bar(kPtPiBar));
+                    ok = umma::bar_wait(bar(kPtPiBar), 1);
                 }
             }
-            if (!ok) {                                       // give up only once the copies in flight have landed
-                for (int j = max(nk - 2, 0); j < nk; ++j) wait(kPtKFull, j);
-                for (int j = max(nv - 2, 0); j < nv; ++j) wait(kPtVFull, j);
-            }
+            landed();
         }
     } else if (warp == 8) {
         // ---- products ----

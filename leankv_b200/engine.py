@@ -547,16 +547,18 @@ class DecodeEngine(DecodeLoop):
             if collect is not None:
                 collect.setdefault(l, {})[name] = t
 
+        q = torch.empty(T, self.nq, 128, dtype=torch.float16, device=self.dev)
+        kv = torch.empty(2, 1, self.nkv, T, 128, dtype=torch.float16, device=self.dev)
+        d = None
         for l, lw in enumerate(self.w["layers"]):
-            x = _rmsnorm(h, lw["ln1"], cfg.rms_eps)
+            h, x = self._add_norm(h, d, lw["ln1"])
             for p in ("q_proj", "k_proj", "v_proj"):
                 note(l, p, x)
             qkv = x @ lw["wqkv_t"]
-            q = _rope(qkv[:, :self.nq * 128].reshape(T, self.nq, 128), cos, sin)
-            k = _rope(qkv[:, self.nq * 128:(self.nq + self.nkv) * 128].reshape(T, self.nkv, 128), cos, sin)
-            v = qkv[:, (self.nq + self.nkv) * 128:].reshape(T, self.nkv, 128)
-            kh = k.transpose(0, 1).contiguous().unsqueeze(0)     # [1, nkv, T, 128]
-            vh = v.transpose(0, 1).contiguous().unsqueeze(0)
+            kh, vh = kv[0], kv[1]                                # [1, nkv, T, 128]
+            _native.check(self.lib.leankv_rope_split_f16(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), q.data_ptr(),
+                                                         kh.data_ptr(), vh.data_ptr(), T, self.nq, self.nkv,
+                                                         self._st()), "rope_split")
             if write_cache:
                 rc = self.lib.leankv_tq_pool_append(kh.data_ptr(), vh.data_ptr(), 1, self.nkv, T,
                                                     self.Pi_k[l].data_ptr(), self.Pi_v[l].data_ptr(),
@@ -569,8 +571,7 @@ class DecodeEngine(DecodeLoop):
             else:
                 kh, vh = self._roundtrip(kh, l, 0), self._roundtrip(vh, l, 1)
             if attention == "packed":
-                qc = q.contiguous()
-                rc = self.lib.leankv_tq_prefill_attn(qc.data_ptr(), attn_out.data_ptr(), T, start_pos,
+                rc = self.lib.leankv_tq_prefill_attn(q.data_ptr(), attn_out.data_ptr(), T, start_pos,
                                                      self.nq, self.nkv, self.pools[l].data_ptr(),
                                                      self.max_pages, pages.data_ptr(),
                                                      self.Pi_k[l].data_ptr(), self.Pi_v[l].data_ptr(),
@@ -586,16 +587,28 @@ class DecodeEngine(DecodeLoop):
             note(l, "o_proj", a)
             o = a @ lw["wo_t"]
             self._allreduce(o)
-            h = h + o
-            x = _rmsnorm(h, lw["ln2"], cfg.rms_eps)
+            h, x = self._add_norm(h, o, lw["ln2"])
             note(l, "gate_proj", x)
             note(l, "up_proj", x)
-            m = F.silu(x @ lw["wgate_t"]) * (x @ lw["wup_t"])
+            m, up = x @ lw["wgate_t"], x @ lw["wup_t"]
+            _native.check(self.lib.leankv_silu_mul_pair_f16(m.data_ptr(), up.data_ptr(), m.data_ptr(), T, self.inter,
+                                                            self._st()), "silu_mul_pair")
             note(l, "down_proj", m)
             d = m @ lw["wdown_t"]
             self._allreduce(d)
-            h = h + d
-        return _rmsnorm(h[-1], self.w["final_norm"], cfg.rms_eps)
+        return _rmsnorm(h[-1] if d is None else h[-1] + d[-1], self.w["final_norm"], cfg.rms_eps)
+
+    def _add_norm(self, h, delta, w):
+        """(h + delta, its RMSNorm) of every row; h, which the prompt pass owns, is updated in place where the kernel takes
+        the call: rows of whole 16-byte pieces, up to 16384 numbers, and an aligned weight."""
+        n = self.cfg.hidden_size
+        if n % 8 or n > 16384 or w.data_ptr() % 16:
+            h = h if delta is None else h + delta
+            return h, _rmsnorm(h, w, self.cfg.rms_eps)
+        x = torch.empty_like(h)
+        _native.check(self.lib.leankv_rmsnorm_rows_f16(h.data_ptr(), _native.ptr(delta), w.data_ptr(), x.data_ptr(),
+                                                       h.shape[0], n, self.cfg.rms_eps, self._st()), "rmsnorm_rows")
+        return h, x
 
     @torch.no_grad()
     def dense_step_reference(self, token: int, pos: int) -> torch.Tensor:

@@ -364,3 +364,32 @@ def test_sharded_argmax_with_a_single_rank_exchanging_with_itself():
         assert int(history[call].item()) == 32768 + 1234
     assert not ex.timed_out()
     ex.close()
+
+
+@pytest.mark.parametrize("T,n_q,n_kv,inter", [(1, 4, 1, 8), (33, 8, 2, 1000), (257, 32, 8, 3584)])
+def test_prompt_pass_glue_kernels(T, n_q, n_kv, inter):
+    """Rotary embedding with the split into heads: the tensor operations' own roundings, so the same bits. silu(gate) * up:
+    one fp16 rounding of silu may fall the other way where fp32 evaluations differ, which moves the product by 2^-10."""
+    from leankv_b200 import _native
+    from leankv_b200.engine import _rope
+
+    lib, gen = _native.lib(), torch.Generator(device=_dev()).manual_seed(T)
+    heads = n_q + 2 * n_kv
+    qkv = (torch.randn(T, heads, 128, generator=gen, device=_dev()) * 3).half()
+    ang = torch.randn(T, 64, generator=gen, device=_dev()) * 100
+    cos, sin = (torch.cat([f(ang), f(ang)], -1).half() for f in (torch.cos, torch.sin))
+    q = torch.empty(T, n_q, 128, dtype=torch.float16, device=_dev())
+    k, v = (torch.empty(n_kv, T, 128, dtype=torch.float16, device=_dev()) for _ in range(2))
+    _native.check(lib.leankv_rope_split_f16(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), q.data_ptr(), k.data_ptr(),
+                                            v.data_ptr(), T, n_q, n_kv, None), "rope_split")
+    turned = _rope(qkv[:, :n_q + n_kv], cos.unsqueeze(1), sin.unsqueeze(1))
+    assert torch.equal(q, turned[:, :n_q]) and torch.equal(k, turned[:, n_q:].transpose(0, 1))
+    assert torch.equal(v, qkv[:, n_q + n_kv:].transpose(0, 1))
+
+    gate, up = ((torch.randn(T, inter, generator=gen, device=_dev()) * 4).half() for _ in range(2))
+    gate.view(-1)[:4] = torch.tensor([0.0, 65504.0, -65504.0, -30.0], dtype=torch.float16)
+    want = torch.nn.functional.silu(gate) * up
+    _native.check(lib.leankv_silu_mul_pair_f16(gate.data_ptr(), up.data_ptr(), gate.data_ptr(), T, inter, None), "silu_mul_pair")
+    finite = torch.isfinite(want)
+    assert torch.equal(finite, torch.isfinite(gate))
+    assert ((gate - want).double().abs() <= want.double().abs() * 2.0 ** -10 + 2.0 ** -24)[finite].all()
