@@ -657,3 +657,23 @@ def test_prefill_attention_that_walks_the_pages_passes_the_same_checks():
                        env=env, capture_output=True, text=True, timeout=600, cwd=ROOT)
     assert r.returncode == 0, (r.stdout[-2000:], r.stderr[-1000:])
     assert "10 passed" in r.stdout
+
+
+@pytest.mark.parametrize("batch", [1, 2, 33, 64])
+def test_page_table_step_takes_pages_in_order(batch):
+    """Pages come off the stack sequence by sequence, whatever the number of warps that write them."""
+    cache = PagedKVCache(num_layers=1, num_kv_heads=1, num_q_heads=4, max_pages=40 * batch, device=_dev())
+    cache._ensure_batch_size(batch)
+    free, pages, length = list(range(40 * batch)), [[] for _ in range(batch)], 0
+    for t_new in (5, 0, 11, 1, 500):
+        cache._table_step(t_new, batch)
+        length += t_new
+        for p in pages:
+            while len(p) < -(-length // 16):
+                p.append(free.pop())
+        n = len(pages[0])
+        assert cache._kv_indptr[:batch + 1].tolist() == [n * b for b in range(batch + 1)]
+        assert cache._kv_page_indices[:n * batch].tolist() == [i for p in pages for i in p]
+        assert cache._block_table[:batch, :n].tolist() == pages
+        assert cache._start_dev[:batch].tolist() == [length - t_new] * batch
+        assert int(cache._free_top) == len(free) and cache.page_table_status() == 0
