@@ -7,6 +7,7 @@ kernel reports an error, a ``RuntimeError`` is raised.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from ctypes import (POINTER, Structure, c_char_p, c_float, c_int, c_int32, c_longlong, c_size_t,
@@ -301,9 +302,22 @@ def ptr(t) -> int | None:
 
 
 def current_stream() -> int:
+    """The current device's current stream, as a raw handle: 0.2 us against 1.6 through a Stream object."""
     import torch
 
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+_NO_SWITCH = contextlib.nullcontext()
+
+
+def on_device(device):
+    """``torch.cuda.device(device)``, without its two switches (2.5 us) where that device is the current one already."""
+    import torch
+
+    if device.type == "cuda" and (device.index is None or device.index == torch._C._cuda_getDevice()):
+        return _NO_SWITCH
+    return torch.cuda.device(device)
 
 
 def require_cuda(t, name: str) -> None:

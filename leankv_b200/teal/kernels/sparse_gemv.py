@@ -15,15 +15,21 @@ from ... import _native
 _workspaces: dict[tuple[int, int], torch.Tensor] = {}
 
 
-def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
+def _workspace(device: torch.device, nbytes: int, stream: int) -> torch.Tensor:
     """Zero-initialised split-K scratch, one per (device, stream), grown on demand."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(),
-           _native.current_stream())
+    key = (device.index, stream)
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
         _workspaces[key] = ws
     return ws
+
+
+def _token(x: torch.Tensor, z: int) -> torch.Tensor:
+    """One token's ``z`` inputs in fp16, contiguous."""
+    if x.dtype == torch.float16 and x.numel() == z and x.is_contiguous():
+        return x
+    return x.reshape(1, z).to(torch.float16).contiguous()
 
 
 def _weight_as_rows(weight: torch.Tensor) -> tuple[int, int]:
@@ -49,20 +55,16 @@ def sparse_gemv(x: torch.Tensor, weight: torch.Tensor, threshold: float,
     _native.require_cuda(x, "x")
     _native.require_cuda(weight, "weight")
     n, z = _weight_as_rows(weight)
-    xin = x.reshape(1, z)
-    xh = xin if xin.dtype == torch.float16 else xin.to(torch.float16)
-    xh = xh.contiguous()
-    y = torch.empty(1, n, device=x.device, dtype=torch.float16)
+    xh = _token(x, z)
+    y = torch.empty(1, 1, n, device=x.device, dtype=torch.float16)
     lib = _native.lib()
-    with torch.cuda.device(x.device):
-        nbytes = lib.leankv_sparse_gemv_workspace_bytes(n, z)
-        ws = _workspace(x.device, nbytes)
-        rc = lib.leankv_sparse_gemv_f16(weight.data_ptr(), xh.data_ptr(), y.data_ptr(), n, z,
-                                        float(threshold), None, None, ws.data_ptr(), ws.numel(),
-                                        None, _native.current_stream())
+    with _native.on_device(x.device):
+        stream = _native.current_stream()
+        ws = _workspace(x.device, lib.leankv_sparse_gemv_workspace_bytes(n, z), stream)
+        rc = lib.leankv_sparse_gemv_f16(weight.data_ptr(), xh.data_ptr(), y.data_ptr(), n, z, float(threshold), None, None,
+                                        ws.data_ptr(), ws.numel(), None, stream)
     _native.check(rc, "leankv_sparse_gemv_f16")
-    out = y.reshape(1, 1, n)
-    return out if x.dtype == torch.float16 else out.to(x.dtype)
+    return y if x.dtype == torch.float16 else y.to(x.dtype)
 
 
 def sparse_swiglu(x: torch.Tensor, gate_weight: torch.Tensor, up_weight: torch.Tensor,
@@ -76,19 +78,16 @@ def sparse_swiglu(x: torch.Tensor, gate_weight: torch.Tensor, up_weight: torch.T
     n, z = _weight_as_rows(gate_weight)
     if _weight_as_rows(up_weight) != (n, z):
         raise ValueError("gate and up weights must have the same shape")
-    xh = x.reshape(1, z).to(torch.float16).contiguous()
-    y = torch.empty(1, n, device=x.device, dtype=torch.float16)
+    xh = _token(x, z)
+    y = torch.empty(1, 1, n, device=x.device, dtype=torch.float16)
     lib = _native.lib()
-    with torch.cuda.device(x.device):
-        nbytes = lib.leankv_sparse_swiglu_workspace_bytes(n, z)
-        ws = _workspace(x.device, nbytes)
-        rc = lib.leankv_sparse_swiglu_f16(gate_weight.data_ptr(), up_weight.data_ptr(),
-                                          xh.data_ptr(), y.data_ptr(), n, z, float(gate_threshold),
-                                          float(up_threshold), ws.data_ptr(), ws.numel(), None,
-                                          _native.current_stream())
+    with _native.on_device(x.device):
+        stream = _native.current_stream()
+        ws = _workspace(x.device, lib.leankv_sparse_swiglu_workspace_bytes(n, z), stream)
+        rc = lib.leankv_sparse_swiglu_f16(gate_weight.data_ptr(), up_weight.data_ptr(), xh.data_ptr(), y.data_ptr(), n, z,
+                                          float(gate_threshold), float(up_threshold), ws.data_ptr(), ws.numel(), None, stream)
     _native.check(rc, "leankv_sparse_swiglu_f16")
-    out = y.reshape(1, 1, n)
-    return out if x.dtype == torch.float16 else out.to(x.dtype)
+    return y if x.dtype == torch.float16 else y.to(x.dtype)
 
 
 def batched_sparse_gemm(x: torch.Tensor, weight: torch.Tensor, threshold: float,

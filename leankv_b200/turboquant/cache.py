@@ -148,7 +148,7 @@ class TurboQuantCache:
         b, h, t, _ = idx.shape
         out = torch.empty((b, h, t, self.head_dim), dtype=torch.float16, device=idx.device)
         Pi, cents, _ = quantizer._consts()
-        with torch.cuda.device(idx.device):
+        with _native.on_device(idx.device):
             rc = _native.lib().leankv_tq_dequantize(idx.data_ptr(), norms.data_ptr(), b * h * t,
                                                     self.head_dim, self.bits, Pi.data_ptr(),
                                                     cents.data_ptr(), out.data_ptr(), 0,

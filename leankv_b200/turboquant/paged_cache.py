@@ -82,18 +82,19 @@ class PagedKVCache:
         old_table = getattr(self, "_block_table", None)
         old_len = getattr(self, "_seq_len_dev", None)
         rows = max(batch_cap, 1)
-        self._batch_cap = batch_cap
+        self._batch_cap = rows
         self._pps_cap = self.max_pages                       # a single sequence may take the whole pool
-        self._block_table = torch.zeros(rows, self._pps_cap, dtype=i32, device=dev)
-        self._seq_len_dev = torch.zeros(rows, dtype=i32, device=dev)
-        self._kv_indptr = torch.zeros(rows + 1, dtype=i32, device=dev)
-        self._kv_last = torch.zeros(rows, dtype=i32, device=dev)
-        self._start_dev = torch.zeros(rows, dtype=i32, device=dev)
+        # one zeroed allocation, each array from a 16-byte boundary on
+        sizes = [rows * self._pps_cap, rows, rows + 1, rows, rows]
         if old_table is None:
+            sizes += [self.max_pages, 1]
+        views = torch.zeros(sum(-(-n // 4) * 4 for n in sizes), dtype=i32, device=dev).split([-(-n // 4) * 4 for n in sizes])
+        self._block_table = views[0][:sizes[0]].view(rows, self._pps_cap)
+        self._seq_len_dev, self._kv_indptr, self._kv_last, self._start_dev = (v[:n] for v, n in zip(views[1:5], sizes[1:5]))
+        if old_table is None:
+            self._kv_page_indices, self._status = views[5][:self.max_pages], views[6][:1]
             self._free_stack = torch.arange(self.max_pages, dtype=i32, device=dev)
             self._free_top = torch.full((1,), self.max_pages, dtype=i32, device=dev)
-            self._kv_page_indices = torch.zeros(self.max_pages, dtype=i32, device=dev)
-            self._status = torch.zeros(1, dtype=i32, device=dev)
         else:
             n = old_table.shape[0]
             self._block_table[:n] = old_table
@@ -109,7 +110,7 @@ class PagedKVCache:
 
     def _table_step(self, t_new: int, batch: int):
         """Advance every sequence by ``t_new`` tokens on the device and rebuild the flat arrays."""
-        with torch.cuda.device(self._device):
+        with _native.on_device(self._device):
             rc = _native.lib().leankv_paged_table_step(
                 t_new, batch, self._seq_len_dev.data_ptr(), self._block_table.data_ptr(), self._pps_cap,
                 self._free_stack.data_ptr(), self._free_top.data_ptr(), self._kv_indptr.data_ptr(),
@@ -191,7 +192,7 @@ class PagedKVCache:
         k = key_states.to(torch.float16).contiguous()
         v = value_states.to(torch.float16).contiguous()
         kq, vq = self.key_quantizers[layer_idx], self.val_quantizers[layer_idx]
-        with torch.cuda.device(self._device):
+        with _native.on_device(self._device):
             rc = _native.lib().leankv_tq_pool_append(
                 k.data_ptr(), v.data_ptr(), batch, self.num_kv_heads, t_new, kq._consts()[0].data_ptr(),
                 vq._consts()[0].data_ptr(), self._bounds.data_ptr(), self.kv_data[layer_idx].data_ptr(),
@@ -205,7 +206,7 @@ class PagedKVCache:
         pages = self._block_table[batch_idx, :max(math.ceil(t / PAGE), 1)]      # device view, no host list
         idx = torch.empty(self.num_kv_heads, t, 64, dtype=torch.uint8, device=self._device)
         norms = torch.empty(self.num_kv_heads, t, dtype=torch.float32, device=self._device)
-        with torch.cuda.device(self._device):
+        with _native.on_device(self._device):
             rc = _native.lib().leankv_tq_pool_unpack(
                 self.kv_data[layer_idx].data_ptr(), self.max_pages, self.num_kv_heads,
                 pages.data_ptr(), t, which, idx.data_ptr(), norms.data_ptr(), _native.current_stream())
@@ -241,7 +242,7 @@ class PagedKVCache:
         q = query.to(torch.float16).contiguous()
         out = torch.empty_like(q)
         lib = _native.lib()
-        with torch.cuda.device(self._device):
+        with _native.on_device(self._device):
             need = lib.leankv_tq_decode_attn_workspace_bytes(batch, self.num_q_heads, self.num_kv_heads,
                                                              max_pages_seq)
             if self._workspace is None or self._workspace.numel() < need:
@@ -266,7 +267,7 @@ class PagedKVCache:
         lib = _native.lib()
         out = torch.empty(batch, t_new, self.num_q_heads, self.head_dim, dtype=torch.float16, device=self._device)
         kq, vq = self.key_quantizers[layer_idx], self.val_quantizers[layer_idx]
-        with torch.cuda.device(self._device):
+        with _native.on_device(self._device):
             for b in range(batch):
                 n = self._seq_lengths[b]
                 start = n - t_new

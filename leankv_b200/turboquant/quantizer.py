@@ -127,7 +127,7 @@ class TurboQuantMSE(torch.nn.Module):
         indices = torch.empty((n, plen), dtype=torch.uint8, device=x.device)
         norms = torch.empty((n,), dtype=torch.float32, device=x.device)
         Pi, _, bounds = self._consts()
-        with torch.cuda.device(x.device):
+        with _native.on_device(x.device):
             rc = lib.leankv_tq_quantize(xk.data_ptr(), 0 if xk.dtype == torch.float16 else 1, n,
                                         self.dim, self.bits, Pi.data_ptr(), bounds.data_ptr(),
                                         indices.data_ptr(), norms.data_ptr(),
@@ -157,7 +157,7 @@ class TurboQuantMSE(torch.nn.Module):
         n = idx.shape[0]
         out = torch.empty((n, self.dim), dtype=torch.float32, device=idx.device)
         Pi, cents, _ = self._consts()
-        with torch.cuda.device(idx.device):
+        with _native.on_device(idx.device):
             rc = _native.lib().leankv_tq_dequantize(idx.data_ptr(), norms.data_ptr(), n, self.dim,
                                                     q.bits, Pi.data_ptr(), cents.data_ptr(),
                                                     out.data_ptr(), 1, _native.current_stream())

@@ -347,3 +347,20 @@ def test_weight_prefetch_budget_never_changes_a_result():
         assert r.returncode == 0, r.stderr[-2000:]
         out[name] = [ln for ln in r.stdout.splitlines() if ln.startswith("OUT")][-1].split()[1]
     assert out["off"] == out["default"] == out["all"]
+
+
+@pytest.mark.parametrize("form", ["plain", "column", "strided", "float32", "bfloat16"])
+def test_sparse_gemv_and_swiglu_take_every_form_of_the_token(form):
+    """The wrapper passes a contiguous fp16 token as it is and copies every other form: the same bits either way."""
+    n, z = 264, 100
+    c = workloads.swiglu_case(n, z, 0.4, seed=3, device=_dev())
+    w = [prepare_weight_for_sparse_gemv(t) for t in (c.w_gate, c.w_up)]
+    x = c.x.reshape(-1).to(torch.bfloat16).half()            # exact in every type
+    given = {"plain": x.reshape(1, 1, z), "column": x.reshape(z, 1), "strided": torch.stack([x, -x], -1)[:, 0].reshape(1, 1, z),
+             "float32": x.float().reshape(1, 1, z), "bfloat16": x.to(torch.bfloat16).reshape(1, 1, z)}[form]
+    for got, want in ((sparse_gemv(given, w[0], c.threshold), sparse_gemv(x.reshape(1, 1, z).clone(), w[0], c.threshold)),
+                      (sparse_swiglu(given, *w, c.threshold, c.threshold),
+                       sparse_swiglu(x.reshape(1, 1, z).clone(), *w, c.threshold, c.threshold))):
+        assert got.shape == (1, 1, n) and got.dtype == given.dtype and torch.equal(got, want.to(given.dtype))
+    with pytest.raises(RuntimeError):
+        sparse_gemv(x[:-1], w[0], c.threshold)
