@@ -37,7 +37,9 @@ extern "C" {
  *   group_rows > 0: rows g * group_rows .. belong to group g and multiply x + g * group_stride (no gain, no delta).
  *   epilogue: y = acc + bias (first bias_rows rows);  gated: y = silu(acc_gate) * acc_up;
  *             softcap > 0: y = softcap * tanh(y / softcap);
- *             residual != NULL: y = residual + scale * acc (y may be residual; x may not be y). */
+ *             residual != NULL: y = residual + scale * acc (y may be residual; x may not be y).
+ *   early_weights: the launch directly ahead on the stream does not write w (a decode step's weights); w may be read while
+ *     it drains. */
 typedef struct leankv_dense_gemv {
     const void* w;
     const float* x;
@@ -61,6 +63,7 @@ typedef struct leankv_dense_gemv {
     float* x_out;
     int group_rows, group_stride;
     float softcap;
+    int early_weights;
 } leankv_dense_gemv_t;
 
 int leankv_dense_gemv(const leankv_dense_gemv_t* args, void* stream);

@@ -147,7 +147,8 @@ class DenseGemv(Structure):
                 ("bias", c_void_p), ("bias_rows", c_int),
                 ("scale", c_void_p), ("residual", c_void_p),
                 ("gain_per_col", c_int), ("delta", c_void_p), ("post_gain", c_void_p), ("post_mult", c_float),
-                ("x_out", c_void_p), ("group_rows", c_int), ("group_stride", c_int), ("softcap", c_float)]
+                ("x_out", c_void_p), ("group_rows", c_int), ("group_stride", c_int), ("softcap", c_float),
+                ("early_weights", c_int)]
 
 
 class StreamNorm(Structure):

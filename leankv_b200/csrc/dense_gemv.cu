@@ -7,6 +7,14 @@
 // range, so a lane's share of x stays in registers for the whole range and the weight stream needs no
 // shared memory. Per-warp row sums go to shared memory once and are added in warp order at the end:
 // bit-reproducible.
+//
+// A decode step is a chain of these launches (25 of 33 for six Rorosun layers), each a few microseconds long, so the time is
+// what stands between the launch ahead's last store and the first product: the first rows' weights are in registers by then
+// (128 bytes a lane, asked for before the dependency wait), and every next group is asked for under the reduction of
+// the last. That takes up to 128 registers, so sixteen warps an SM: 250 us a step of 295 MB of weights (width 1024) and
+// 239 of 560 MB (width 2048), where thirty-two warps of 64 registers that loaded after the wait took 274 and 258. Tried and slower:
+// rows through shared memory by bulk copies, 100 KB an SM (290, 304); 80 or 96 registers (spills; 284, 255 and
+// 289, 251); the next launch's weights asked into L2 as well (279, 278).
 
 #include <algorithm>
 #include <type_traits>
@@ -87,9 +95,9 @@ __device__ __forceinline__ int row_of_lane(int lane) { return (lane * R) >> 5; }
 // (one slab). kStaged: the same in shared memory, any number of slabs. kGrouped: row groups with an input slice each.
 enum class Input { kPlain, kJoined, kStaged, kGrouped };
 template <typename T, int CH, Input IN>
-__global__ void __launch_bounds__(512, sizeof(T) == 2 ? 2 : 1) dense_gemv_kernel(const GemvParams p) {
+__global__ void __launch_bounds__(512, 1) dense_gemv_kernel(const GemvParams p) {
     constexpr bool STAGED = IN == Input::kStaged, JOINED = IN == Input::kJoined, GROUPED = IN == Input::kGrouped;
-    constexpr int R = 8 / CH;                        // rows in flight: R * CH 16-byte loads per lane (bf16)
+    constexpr int R = (sizeof(T) == 2 ? 8 : 4) / CH;      // rows in flight: 128 bytes a lane
     extern __shared__ __align__(16) float s_dyn[];
     float* s_part = STAGED ? s_dyn + p.x_smem : s_dyn;      // [rows of this CTA (x2 if gated)][warps]
     __shared__ float s_tmp[64];
@@ -112,6 +120,21 @@ __global__ void __launch_bounds__(512, sizeof(T) == 2 ? 2 : 1) dense_gemv_kernel
             asm volatile("prefetch.global.L2 [%0];" ::"l"(base + off));
         }
     }
+    // The first rows' weights into registers: ahead of the dependency wait where the caller says that the launch ahead does
+    // not write them, else beside the loads of x.
+    const int n_rows = (hi - lo) * mult;
+    Raw8<T> raw[R][CH];
+    auto load_rows = [&](int s, int v, int last) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int vr = min(v + r, last);
+            const size_t row = a.gated ? (size_t)(lo + (vr >> 1)) + (size_t)(vr & 1) * a.rows : (size_t)(lo + vr);
+#pragma unroll
+            for (int c = 0; c < CH; ++c)
+                load_w8(W + row * cols, s * slab_cols + (c * warps + warp) * 256 + lane * 8, cols, vec, raw[r][c]);
+        }
+    };
+    if (a.early_weights) load_rows(0, 0, n_rows - 1);
     // kJoined: the gains do not depend on the launch ahead
     float gn[CH][8], pg[CH][8];
     if constexpr (JOINED) {
@@ -123,6 +146,7 @@ __global__ void __launch_bounds__(512, sizeof(T) == 2 ? 2 : 1) dense_gemv_kernel
         }
     }
     pdl_begin();
+    if (!a.early_weights) load_rows(0, 0, n_rows - 1);
 
     float rs = 1.f;
     float xj[CH][8];                // kJoined: this thread's columns of x'
@@ -256,15 +280,6 @@ __global__ void __launch_bounds__(512, sizeof(T) == 2 ? 2 : 1) dense_gemv_kernel
             }
             const int v0 = (r0 - lo) * mult, v1 = (r1 - lo) * mult;
             for (int v = v0; v < v1; v += R) {
-                Raw8<T> raw[R][CH];
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int vr = min(v + r, v1 - 1);
-                    const size_t row = a.gated ? (size_t)(lo + (vr >> 1)) + (size_t)(vr & 1) * a.rows : (size_t)(lo + vr);
-#pragma unroll
-                    for (int c = 0; c < CH; ++c)
-                        load_w8(W + row * cols, s * slab_cols + (c * warps + warp) * 256 + lane * 8, cols, vec, raw[r][c]);
-                }
                 float acc[R];
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
@@ -277,6 +292,10 @@ __global__ void __launch_bounds__(512, sizeof(T) == 2 ? 2 : 1) dense_gemv_kernel
                         for (int i = 0; i < 8; ++i) acc[r] = fmaf(w[i], xs[c][i], acc[r]);
                     }
                 }
+                // the next rows, of this segment, the next one or the next slab, under the reduction
+                const int next = min(v + R, v1);
+                if (next < n_rows) load_rows(s, next, n_rows - 1);
+                else if (s + 1 < p.slabs) load_rows(s + 1, 0, n_rows - 1);
                 const float sum = warp_reduce_rows<R>(acc, lane);
                 const int vr = v + row_of_lane<R>(lane);
                 if ((lane & (32 / R - 1)) == 0 && vr < v1) {
@@ -310,7 +329,7 @@ __global__ void __launch_bounds__(512, sizeof(T) == 2 ? 2 : 1) dense_gemv_kernel
 
 template <typename T, int CH, Input IN>
 int launch_gemv(const GemvParams& p, int warps, cudaStream_t st) {
-    const int per_sm = std::max(1, (sizeof(T) == 2 ? 2 : 1) * kMaxWarps / warps);
+    const int per_sm = std::max(1, kMaxWarps / warps);
     const int mult = p.a.gated ? 2 : 1;
     int grid = std::min(sm_count() * std::min(per_sm, 8), (p.a.rows + 1) / 2);
     grid = std::max(grid, 1);

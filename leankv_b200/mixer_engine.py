@@ -189,7 +189,7 @@ class MixerDecodeEngine(DecodeLoop):
                 else:
                     sub.body.prepare_step(into, out, self._bufs)
         self._head_args = _native.DenseGemv(w=self.head.data_ptr(), y=self.logits.data_ptr(), dtype=dtype_code(self.dtype),
-                                            rows=V, cols=W, softcap=cfg.logit_softcap, **entry(self.final_norm))
+                                            rows=V, cols=W, softcap=cfg.logit_softcap, early_weights=1, **entry(self.final_norm))
 
     @classmethod
     def random_tensors(cls, cfg: MixerModelConfig, device, seed: int = 0, rank: int = 64) -> dict:

@@ -37,6 +37,11 @@ def matmul(a: torch.Tensor, w: torch.Tensor, exact_out: bool = True) -> torch.Te
     return torch.mm(a, w.t())
 
 
+def _step_gemv(**kw) -> _native.DenseGemv:
+    """A projection of a decode step: its weights are constants, so they may be read while the launch ahead drains."""
+    return _native.DenseGemv(early_weights=1, **kw)
+
+
 @dataclass(frozen=True)
 class WindowPoolSpec:
     heads: int
@@ -241,7 +246,7 @@ class ParallelMixer:
         (both mixers) -> branch output."""
         y, out = bufs["y"], bufs["out"]
         code, n0, N = dtype_code(self.seq.dtype), self.left.spec.qkv_width, self.right.spec.out_width
-        a = _native.DenseGemv(w=self.w_in.data_ptr(), y=y.data_ptr(), dtype=code, rows=self.in_width,
+        a = _step_gemv(w=self.w_in.data_ptr(), y=y.data_ptr(), dtype=code, rows=self.in_width,
                               cols=self.width, n_mix=len(self.mix_end),
                               prev=self.prev.data_ptr(), state=state.data_ptr(), bias=self.bias.data_ptr(),
                               bias_rows=n0, **entry)
@@ -254,7 +259,7 @@ class ParallelMixer:
                               w2=self.right.w2.data_ptr(), out=out.data_ptr(), right_off=self.left.spec.out_width,
                               left_scale=self.left_scale, right_scale=self.right_scale, state=state.data_ptr(),
                               max_pos=max_pos, ws=self._step_ws.data_ptr(), ws_bytes=self._step_ws.numel())
-        o = _native.DenseGemv(w=self.w_out.data_ptr(), x=out.data_ptr(), dtype=code, rows=self.width,
+        o = _step_gemv(w=self.w_out.data_ptr(), x=out.data_ptr(), dtype=code, rows=self.width,
                               cols=self.out_width, **exit)
         self._step_args = (a, s, o)
 
@@ -292,9 +297,9 @@ class GatedMLP:
     def prepare_step(self, entry: dict, exit: dict, bufs: dict) -> None:
         code, act = dtype_code(self.dtype), bufs["act"]
         self._step_args = (
-            _native.DenseGemv(w=self.w_gu.data_ptr(), y=act.data_ptr(), dtype=code, rows=self.inter, cols=self.width,
+            _step_gemv(w=self.w_gu.data_ptr(), y=act.data_ptr(), dtype=code, rows=self.inter, cols=self.width,
                               gated=1, **entry),
-            _native.DenseGemv(w=self.w_down.data_ptr(), x=act.data_ptr(), dtype=code, rows=self.width, cols=self.inter,
+            _step_gemv(w=self.w_down.data_ptr(), x=act.data_ptr(), dtype=code, rows=self.width, cols=self.inter,
                               **exit))
 
     def bind(self, seq: SequenceState) -> "GatedMLP":
@@ -473,10 +478,10 @@ class RotaryAttention(_CausalMixer):
         """Stream -> y (q | k | v | gate) -> out (gated heads) -> branch output."""
         s, code, y, out = self.spec, self.c.dtype, bufs["y"].data_ptr(), bufs["out"].data_ptr()
         self._step_args = (
-            _native.DenseGemv(w=self.w_in.data_ptr(), y=y, dtype=code, rows=self.in_width, cols=self.width, **entry),
+            _step_gemv(w=self.w_in.data_ptr(), y=y, dtype=code, rows=self.in_width, cols=self.width, **entry),
             self._step_block(state, max_pos, q=y, q_stride=s.dim, k_new=y + 4 * self.at_k, v_new=y + 4 * self.at_v,
                              rot_own=s.rot.dims, gate=y + 4 * self.at_g, out=out),
-            _native.DenseGemv(w=self.w_out.data_ptr(), x=out, dtype=code, rows=self.width, cols=self.out_width, **exit))
+            _step_gemv(w=self.w_out.data_ptr(), x=out, dtype=code, rows=self.width, cols=self.out_width, **exit))
 
 
 def _per_head_padded(w: torch.Tensor, heads: int, n: int) -> torch.Tensor:
@@ -577,7 +582,7 @@ class LatentAttention(_CausalMixer):
         s, code = self.spec, self.c.dtype
         H, d, r, n = s.heads, s.dim, s.rot_dim, s.kv_rank
         y, q, folded, latent, out = (bufs[b].data_ptr() for b in ("y", "q", "folded", "latent", "out"))
-        gemv = lambda w, **kw: _native.DenseGemv(w=w.data_ptr(), dtype=code, **kw)
+        gemv = lambda w, **kw: _step_gemv(w=w.data_ptr(), dtype=code, **kw)
         self._step_args = (
             gemv(self.w_down, y=y, rows=self.in_width, cols=self.width, **entry),
             gemv(self.w_q, x=y, y=q, rows=H * (d + r), cols=s.q_rank, gain=self.q_norm.data_ptr(), gain_per_col=1, eps=self.eps),

@@ -561,3 +561,18 @@ def test_command_line_and_trace_replay(tmp_path):
     la, lb = plain.forward(cfg, w, a), plain.forward(cfg, w, b)
     assert rel(read(0), la[[27, 4]]) < MODEL_TOL[F32] and rel(read(2), la[29:]) < MODEL_TOL[F32]
     assert rel(read(3), lb) < MODEL_TOL[F32]
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("rows,cols,gated", [(1, 8, 0), (37, 264, 1), (700, 520, 0), (300, 1024, 1), (64, 9000, 0)])
+def test_gemv_weights_read_ahead_of_the_dependency_wait(dtype, rows, cols, gated):
+    """The same bits whether the first rows' weights are asked for before or after the wait."""
+    w, x = rnd(rows * (1 + gated), cols, seed=1, std=cols ** -0.5).to(dtype).to(DEV), rnd(cols, seed=2).to(DEV)
+    gain = torch.tensor(1.3, device=DEV)
+    ys = [torch.full((rows,), 7.0, device=DEV) for _ in range(2)]
+    for early, y in enumerate(ys):
+        gemv(w=w, x=x, y=y, dtype=CODE[dtype], rows=rows, cols=cols, gated=gated, gain=gain, eps=1e-5, early_weights=early)
+    assert torch.equal(*ys)
+    v = w.double() @ (x.double() * 1.3 / (x.double().square().mean() + 1e-5).sqrt())
+    want = torch.nn.functional.silu(v[:rows]) * v[rows:] if gated else v
+    assert float((ys[0].double() - want).norm() / want.norm()) < 1e-5
