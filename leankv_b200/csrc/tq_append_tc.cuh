@@ -15,15 +15,22 @@
 // Every other coordinate is farther from all boundaries than the fast path's error, so its code is
 // the chain's code. The fp32 kernels above remain the definition; tests compare whole pools.
 //
-// A CTA of 4 warps quantizes tiles of 64 tokens (4 pages, one per warp) of one (sequence, head,
-// K|V); CTAs are persistent over a contiguous range of tiles and keep the fp16 copies of Pi in
+// A CTA of 8 warps quantizes tiles of 64 tokens (4 pages, two warps each: half the coordinates a warp) of one
+// (sequence, head, K|V); CTAs are persistent over a contiguous range of tiles and keep the fp16 copies of Pi in
 // shared memory, reloading them only when their range crosses from K to V.
+//
+// A prompt chunk is one tile a CTA, so its time is the chain of a tile's phases, none of which fills the issue slots: with one
+// warp a page 512 tokens (8 heads) took 40 000 cycles (staging Pi 7 800, norms and division 6 500, products 4 700, codes 9 400,
+// exact chains 8 800, packing 1 300): 24 us; with two 13.
 
-constexpr int kTcThreads = 128;
+constexpr int kTcThreads = 256;
 constexpr int kTcTokens = 64;
 constexpr int kPiStride = 136;            // halves per row (272 bytes): conflict-free 8 x 16-byte ldmatrix rows
 constexpr int kUStride = 136;             // floats per row of the unit-vector tile
-constexpr float kBand = 1e-4f;
+// Rows of Pi and unit vectors have norm 1, so sums over k of |Pi u| are at most 1: the chain's own rounding is at most
+// 128 x 2^-24 = 7.6e-6, the fast value's (splits and fp16's subnormals 1.2e-6, the dropped lo x lo 2.4e-7, 24 accumulations
+// of two units in the last place each 5.7e-6) 7.2e-6.
+constexpr float kBand = 2.5e-5f;
 constexpr int kCodeStride = 132;          // bytes per token row of the code tile: 4-byte reads of 8 tokens x 4 quarters hit 32 banks
 constexpr int kListCap = 64;              // queue of boundary-band coordinates: flushed whenever it holds a full warp's worth
 constexpr size_t kTcSmemBytes = 2 * (size_t)kDim * kPiStride * sizeof(__half) +
@@ -71,6 +78,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
     pdl_begin();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
+    const int pgw = warp >> 1, side = warp & 1;           // page of the tile, half of the coordinates
     if (tid < 8) s_bounds[tid] = tid < 7 ? p.bounds[tid] : __int_as_float(0x7f800000);
 
     const long long tile_lo = (long long)blockIdx.x * tp.n_tiles / gridDim.x;
@@ -105,16 +113,17 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
         const int pos_end = pos0 + p.T_new;
         const __half* src = (which == 0 ? p.k : p.v) + ((size_t)b * p.H + h) * (size_t)p.T_new * kDim;
 
-        // ---- norms and unit vectors: two threads per token, 64 coordinates each ----
+        // ---- norms and unit vectors: four threads per token, 32 coordinates each. The norm is the contract's: the squares of
+        // each half one after another, so the second thread of a half goes on from the first one's sum ----
         {
-            const int row = tid >> 1, hf = tid & 1;
+            const int row = tid >> 2, qr = tid & 3;
             const int pos = ord0 * 16 + row;
             const bool ok = pos >= pos0 && pos < pos_end;
-            float xr[64];
+            float xr[32];
             if (ok) {
-                const uint4* s4 = reinterpret_cast<const uint4*>(src + (size_t)(pos - pos0) * kDim + hf * 64);
+                const uint4* s4 = reinterpret_cast<const uint4*>(src + (size_t)(pos - pos0) * kDim + qr * 32);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 4; ++i) {
                     const uint4 w = __ldg(s4 + i);
                     const float2 a = h2_to_f2(w.x), bb = h2_to_f2(w.y), c = h2_to_f2(w.z), d = h2_to_f2(w.w);
                     xr[8 * i + 0] = a.x; xr[8 * i + 1] = a.y; xr[8 * i + 2] = bb.x; xr[8 * i + 3] = bb.y;
@@ -122,38 +131,46 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
                 }
             } else {
 #pragma unroll
-                for (int i = 0; i < 64; ++i) xr[i] = 0.f;
+                for (int i = 0; i < 32; ++i) xr[i] = 0.f;
             }
-            const double mine = sumsq64(xr);
-            const double other = __shfl_xor_sync(0xffffffffu, mine, 1);
-            const double tot = hf == 0 ? mine + other : other + mine;
+            double sum = 0.0;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) sum = fma((double)xr[i], (double)xr[i], sum);
+            const double before = __shfl_up_sync(0xffffffffu, sum, 1);
+            if (qr & 1) {
+                sum = before;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) sum = fma((double)xr[i], (double)xr[i], sum);
+            }
+            const int l0 = lane & ~3;
+            const double tot = __shfl_sync(0xffffffffu, sum, l0 + 1) + __shfl_sync(0xffffffffu, sum, l0 + 3);
             const float norm = (float)sqrt(tot);
             const float denom = norm + 1e-10f;
-            if (hf == 0) s_norm[row] = norm;
-            float4* dst = reinterpret_cast<float4*>(&s_u[row * kUStride + hf * 64]);
+            if (qr == 0) s_norm[row] = norm;
+            float4* dst = reinterpret_cast<float4*>(&s_u[row * kUStride + qr * 32]);
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
+            for (int i = 0; i < 8; ++i)
                 dst[i] = make_float4(xr[4 * i] / denom, xr[4 * i + 1] / denom, xr[4 * i + 2] / denom, xr[4 * i + 3] / denom);
         }
         __syncthreads();
 
         // ---- this warp's page ----
-        const int page_ord = ord0 + warp;
+        const int page_ord = ord0 + pgw;
         const int first = max(pos0, page_ord * 16), last = min(pos_end, page_ord * 16 + 16);
         const int nt_valid = last - first;                    // tokens of this launch in the page
-        if (nt_valid <= 0) continue;                          // warp-uniform; CTA-wide syncs are at the loop top
+        if (nt_valid <= 0) continue;                          // the same in both warps of the page; CTA-wide syncs are at the loop top
         const int slot0 = first - page_ord * 16;
         const int page = p.kv_page_indices[p.kv_indptr[b] + page_ord];
         const bool page_ok = page >= 0 && page < p.n_pages;
 
         // ---- fast rotation on tensor cores: rows = the page's 16 token slots, columns = coordinates ----
-        float acc[16][4];
+        float acc[8][4];                                      // columns 64 side + 8 n ..
 #pragma unroll
-        for (int n = 0; n < 16; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-        const float* u_lo_row = &s_u[(16 * warp + g) * kUStride];
+        for (int n = 0; n < 8; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+        const float* u_lo_row = &s_u[(16 * pgw + g) * kUStride];
         const float* u_hi_row = u_lo_row + 8 * kUStride;
         const uint32_t pi_addr = (uint32_t)__cvta_generic_to_shared((lane < 16 ? s_pih : s_pil)) +
-                                 (uint32_t)(((lane & 7) * kPiStride + ((lane >> 3) & 1) * 8) * sizeof(__half));
+                                 (uint32_t)(((64 * side + (lane & 7)) * kPiStride + ((lane >> 3) & 1) * 8) * sizeof(__half));
 #pragma unroll 1
         for (int ks = 0; ks < 8; ++ks) {
             uint32_t ah[4], al[4];
@@ -168,7 +185,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
                 split_h2(v3.x, v3.y, ah[3], al[3]);
             }
 #pragma unroll
-            for (int n = 0; n < 16; ++n) {
+            for (int n = 0; n < 8; ++n) {
                 uint32_t bh0, bh1, bl0, bl1;
                 ldmatrix_x4(bh0, bh1, bl0, bl1, pi_addr + (uint32_t)((n * 8 * kPiStride + ks * 16) * sizeof(__half)));
                 mma_f16_16816(acc[n], al, bh0, bh1);
@@ -179,53 +196,57 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
 
         // ---- codes; coordinates close to a boundary are queued for the sequential fp32 chain ----
         const float b1 = s_bounds[4], b2 = s_bounds[5], b3 = s_bounds[6];       // 0 < b1 < b2 < b3 (s_bounds[3] = 0)
-        uint8_t* code_rows = s_code + (size_t)(16 * warp) * kCodeStride;
+        uint8_t* code_rows = s_code + (size_t)(16 * pgw) * kCodeStride;
         // exact value of one coordinate: y = fma chain over k ascending, from the fp32 unit vector
         auto exact_code = [&](int slot, int coord) -> int {
             const float4* pr = reinterpret_cast<const float4*>(Pi + (size_t)coord * kDim);
-            const float4* ur = reinterpret_cast<const float4*>(&s_u[(16 * warp + slot) * kUStride]);
-            float4 pv[kDim / 4];
-#pragma unroll
-            for (int k4 = 0; k4 < kDim / 4; ++k4) pv[k4] = __ldg(pr + k4);      // one round trip for the whole row
+            const float4* ur = reinterpret_cast<const float4*>(&s_u[(16 * pgw + slot) * kUStride]);
             float ye = 0.f;
 #pragma unroll
-            for (int k4 = 0; k4 < kDim / 4; ++k4) {
-                const float4 uv = ur[k4];
-                ye = fmaf(pv[k4].x, uv.x, ye);
-                ye = fmaf(pv[k4].y, uv.y, ye);
-                ye = fmaf(pv[k4].z, uv.z, ye);
-                ye = fmaf(pv[k4].w, uv.w, ye);
+            for (int part = 0; part < 2; ++part) {                               // two round trips for the row
+                float4 pv[kDim / 8];
+#pragma unroll
+                for (int k4 = 0; k4 < kDim / 8; ++k4) pv[k4] = __ldg(pr + part * (kDim / 8) + k4);
+#pragma unroll
+                for (int k4 = 0; k4 < kDim / 8; ++k4) {
+                    const float4 uv = ur[part * (kDim / 8) + k4];
+                    ye = fmaf(pv[k4].x, uv.x, ye);
+                    ye = fmaf(pv[k4].y, uv.y, ye);
+                    ye = fmaf(pv[k4].z, uv.z, ye);
+                    ye = fmaf(pv[k4].w, uv.w, ye);
+                }
             }
             int code = 0;
 #pragma unroll
             for (int q = 0; q < 7; ++q) code += (ye > s_bounds[q]) ? 1 : 0;
             return code;
         };
-        uint32_t near_lo = 0, near_hi = 0;                     // bit 4n + i: value (n, i) of this lane is in the band
+        uint32_t near = 0;                                     // bit 4n + i: value (n, i) of this lane is in the band
 #pragma unroll
-        for (int n = 0; n < 16; ++n) {
+        for (int n = 0; n < 8; ++n) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int slot = g + (i >> 1) * 8;
-                const int coord = n * 8 + 2 * t + (i & 1);
-                const float y = acc[n][i];
-                const float ay = fabsf(y);
-                const int mag = (ay > b1 ? 1 : 0) + (ay > b2 ? 1 : 0) + (ay > b3 ? 1 : 0);
-                const int code = y > 0.f ? 4 + mag : 3 - mag;
-                const bool near = ay <= kBand || fabsf(ay - b1) <= kBand || fabsf(ay - b2) <= kBand ||
-                                  fabsf(ay - b3) <= kBand;
-                code_rows[slot * kCodeStride + coord] = (uint8_t)code;
-                if (near && slot >= slot0 && slot < slot0 + nt_valid) {
-                    if (n < 8) near_lo |= 1u << (4 * n + i);
-                    else near_hi |= 1u << (4 * (n - 8) + i);
+            for (int r = 0; r < 2; ++r) {
+                const int slot = g + 8 * r;
+                const bool mine = slot >= slot0 && slot < slot0 + nt_valid;
+                int code[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const float y = acc[n][2 * r + c];
+                    const float ay = fabsf(y);
+                    const int mag = (ay > b1 ? 1 : 0) + (ay > b2 ? 1 : 0) + (ay > b3 ? 1 : 0);
+                    code[c] = y > 0.f ? 4 + mag : 3 - mag;
+                    const float gap = fminf(fminf(ay, fabsf(ay - b1)), fminf(fabsf(ay - b2), fabsf(ay - b3)));
+                    if (gap <= kBand && mine) near |= 1u << (4 * n + 2 * r + c);
                 }
+                *reinterpret_cast<uint16_t*>(&code_rows[slot * kCodeStride + 64 * side + n * 8 + 2 * t]) =
+                    (uint16_t)(code[0] | (code[1] << 8));
             }
         }
-        n_coords += (unsigned long long)nt_valid * 4;          // per lane: 128 coordinates / 32 lanes
-        n_exact += __popc(near_lo) + __popc(near_hi);
+        n_coords += (unsigned long long)nt_valid * 2;          // per lane: 64 coordinates / 32 lanes
+        n_exact += __popc(near);
         // The band coordinates of all lanes are compacted into a queue; whenever it holds 32 of them every
         // lane runs one exact chain. (A page of all-zero vectors puts all 2048 coordinates in the band.)
-        if (__any_sync(0xffffffffu, (near_lo | near_hi) != 0u)) {
+        if (const unsigned any = __reduce_or_sync(0xffffffffu, near)) {
             int cnt = 0;                                       // warp-uniform
             auto flush = [&](int n_take) {
                 __syncwarp();
@@ -240,13 +261,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
                 cnt = rest;
             };
 #pragma unroll 1
-            for (int idx = 0; idx < 64; ++idx) {
-                const bool flag = ((idx < 32 ? near_lo >> idx : near_hi >> (idx - 32)) & 1u) != 0u;
+            for (unsigned left = any; left != 0u; left &= left - 1u) {
+                const int idx = __ffs(left) - 1;
+                const bool flag = ((near >> idx) & 1u) != 0u;
                 const unsigned m = __ballot_sync(0xffffffffu, flag);
-                if (m == 0u) continue;
                 if (flag) {
                     const int n = idx >> 2, i = idx & 3;
-                    const int slot = g + (i >> 1) * 8, coord = n * 8 + 2 * t + (i & 1);
+                    const int slot = g + (i >> 1) * 8, coord = 64 * side + n * 8 + 2 * t + (i & 1);
                     s_list[warp][cnt + __popc(m & ((1u << lane) - 1u))] = (uint16_t)((slot << 7) | coord);
                 }
                 cnt += __popc(m);
@@ -254,20 +275,20 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
             }
             if (cnt > 0) flush(cnt);
         }
-        __syncwarp();
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + pgw) : "memory");       // both halves' codes are there
         if (!page_ok) continue;                                // invalid table entry: write nothing
 
         // ---- pack this page's chunk (same words as tq_pool_append_kernel), four codes per shared-memory read ----
         uint8_t* chunk = p.pool + (((size_t)page * 2 + which) * p.H + h) * kChunkBytes;
         uint32_t* words = reinterpret_cast<uint32_t*>(chunk);
         __half* norms = reinterpret_cast<__half*>(chunk + kNormOffsetBytes);
-        if (lane >= slot0 && lane < slot0 + nt_valid) norms[lane] = __float2half_rn(s_norm[16 * warp + lane]);
+        if (side == 0 && lane >= slot0 && lane < slot0 + nt_valid) norms[lane] = __float2half_rn(s_norm[16 * pgw + lane]);
         // squeezes the low nibbles of 4 bytes into 16 bits
         auto pack4 = [](uint32_t v) -> uint32_t {
             const uint32_t t2 = (v | (v >> 4)) & 0x00FF00FFu;
             return (t2 | (t2 >> 8)) & 0xFFFFu;
         };
-        for (int w = lane; w < kChunkWords; w += 32) {
+        for (int w = lane + 32 * side; w < kChunkWords; w += 64) {
             const int kk = w >> 6, ui = w & 63;
             if (which == 0) {
                 // unit (slot, quarter t4): codes e = coordinates 32 t4 + e; word kk holds codes 8kk..8kk+7 as
