@@ -177,6 +177,13 @@ int leankv_tq_pool_append(const void* k, const void* v, int B, int n_kv_heads, i
                           void* pool, int n_pages,
                           const int32_t* kv_indptr, const int32_t* kv_page_indices,
                           const int32_t* start_pos, void* stream);
+/* The same of a part of larger tensors: tokens 128 elements apart, sequences and heads as many elements apart as given
+ * (multiples of 8). */
+int leankv_tq_pool_append_strided(const void* k, const void* v, int B, int n_kv_heads, int T_new,
+                                  long long k_seq, long long k_head, long long v_seq, long long v_head,
+                                  const float* Pi_k, const float* Pi_v, const float* decision_boundaries,
+                                  void* pool, int n_pages, const int32_t* kv_indptr, const int32_t* kv_page_indices,
+                                  const int32_t* start_pos, void* stream);
 
 /* Appends of 16 or more tokens per sequence (prompt processing, where the reference quantizes the
  * flushed tokens with one dense fp32 matmul, cache.py:136-142 / quantizer.py:119-129) run the
@@ -270,6 +277,13 @@ int leankv_tq_prefill_attn(const void* q, void* out, int T, int start_pos, int n
                            const void* pool, int n_pages, const int32_t* seq_pages, const float* Pi_k,
                            const float* Pi_v, const float* centroids, float scale, void* workspace,
                            size_t workspace_bytes, void* stream);
+/* The same with tokens and heads of q as many elements apart as given (multiples of 8); LEANKV_EUNSUPPORTED where the
+ * page-walking kernels take the call (contexts beyond 65536 tokens) and q is not [T][n_q_heads][128]. */
+int leankv_tq_prefill_attn_strided(const void* q, long long q_token, long long q_head, void* out, int T, int start_pos,
+                                   int n_q_heads, int n_kv_heads, const void* pool, int n_pages,
+                                   const int32_t* seq_pages, const float* Pi_k, const float* Pi_v,
+                                   const float* centroids, float scale, void* workspace, size_t workspace_bytes,
+                                   void* stream);
 
 /* ------------------------------------------------------------------------- *
  * Glue kernels of a batch-1 decode step (no reference counterpart: the reference leaves

@@ -93,6 +93,12 @@ SIGNATURES = {
     "leankv_decode_qkv_post": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "leankv_tq_decode_attn_status": (c_int, [c_void_p, POINTER(c_int)]),
+    "leankv_tq_pool_append_strided": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
+                                              c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
+                                              c_void_p, c_void_p]),
+    "leankv_tq_prefill_attn_strided": (c_int, [c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_int, c_int, c_int,
+                                               c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p,
+                                               c_size_t, c_void_p]),
     "leankv_tq_prefill_attn_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "leankv_tq_prefill_attn": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_size_t,
@@ -252,6 +258,8 @@ MIXER_SIGNATURES = {
     "leankv_causal_step": (c_int, [POINTER(CausalAttn), POINTER(CausalStep), c_void_p]),
 }
 _COMMON = ("leankv_strerror", "leankv_last_cuda_error", "leankv_abi_version")     # capi.cu, in both libraries
+
+EUNSUPPORTED = -5
 
 _lib = None
 _mixers = None

@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) tq_pool_append_t5_kernel(const 
         const int pos0 = p.start_pos[b];
         const int ord0 = pos0 / 16 + kT5Pages * grp;          // first page ordinal of this tile
         const int pos_end = pos0 + p.T_new;
-        const __half* src = (which == 0 ? p.k : p.v) + ((size_t)b * p.H + h) * (size_t)p.T_new * kDim;
+        const __half* src = append_source(p, which, b, h);
 
         // ---- norms and unit vectors: two threads per token, 64 coordinates each ----
         {

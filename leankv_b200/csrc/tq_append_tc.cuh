@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
         const int pos0 = p.start_pos[b];
         const int ord0 = pos0 / 16 + 4 * grp;                 // first page ordinal of this tile
         const int pos_end = pos0 + p.T_new;
-        const __half* src = (which == 0 ? p.k : p.v) + ((size_t)b * p.H + h) * (size_t)p.T_new * kDim;
+        const __half* src = append_source(p, which, b, h);
 
         // ---- norms and unit vectors: four threads per token, 32 coordinates each. The norm is the contract's: the squares of
         // each half one after another, so the second thread of a half goes on from the first one's sum ----

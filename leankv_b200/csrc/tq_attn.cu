@@ -618,11 +618,11 @@ extern "C" size_t leankv_tq_prefill_attn_workspace_bytes(int T, int start_pos, i
     return make_tile_plan(T, start_pos, n_q_heads, n_kv_heads).total;
 }
 
-extern "C" int leankv_tq_prefill_attn(const void* q, void* out, int T, int start_pos, int n_q_heads,
-                                      int n_kv_heads, const void* pool, int n_pages,
-                                      const int32_t* seq_pages, const float* Pi_k, const float* Pi_v,
-                                      const float* centroids, float scale, void* workspace,
-                                      size_t workspace_bytes, void* stream) {
+extern "C" int leankv_tq_prefill_attn_strided(const void* q, long long q_token, long long q_head, void* out, int T,
+                                              int start_pos, int n_q_heads, int n_kv_heads, const void* pool, int n_pages,
+                                              const int32_t* seq_pages, const float* Pi_k, const float* Pi_v,
+                                              const float* centroids, float scale, void* workspace,
+                                              size_t workspace_bytes, void* stream) {
     if (T < 0 || start_pos < 0 || n_q_heads <= 0 || n_kv_heads <= 0 || n_pages <= 0) return LEANKV_EINVAL;
     if (T == 0) return LEANKV_OK;
     if (!q || !out || !pool || !seq_pages || !workspace || !Pi_k || !Pi_v || !centroids) return LEANKV_EINVAL;
@@ -630,7 +630,7 @@ extern "C" int leankv_tq_prefill_attn(const void* q, void* out, int T, int start
     if (T > 65535 || (long long)start_pos + T > (1ll << 24)) return LEANKV_ELIMIT;
     if (prefill_rows_pages(start_pos, T) > 0x7fffffffll) return LEANKV_ELIMIT;     // page-table offsets are int32
     if (!aligned16(workspace) || !aligned16(q) || !aligned16(out) || !aligned16(pool) || !aligned16(Pi_k) ||
-        !aligned16(Pi_v))
+        !aligned16(Pi_v) || q_token % 8 != 0 || q_head % 8 != 0)
         return LEANKV_EALIGN;
     if (workspace_bytes < leankv_tq_prefill_attn_workspace_bytes(T, start_pos, n_q_heads, n_kv_heads))
         return LEANKV_EWORKSPACE;
@@ -677,6 +677,8 @@ extern "C" int leankv_tq_prefill_attn(const void* q, void* out, int T, int start
         LEANKV_CUDA_TRY(launch_kernel(tq_expand_kernel, dim3(std::max(ep.k_tiles, 8), n_kv_heads + 1), dim3(256), 0, st, e));
         TileAttnParams a{};
         a.q = static_cast<const __half*>(q);
+        a.q_token = q_token;
+        a.q_head = q_head;
         a.qscale = scale * kLog2e;
         a.records = e.records;
         a.images = e.images;
@@ -697,6 +699,7 @@ extern "C" int leankv_tq_prefill_attn(const void* q, void* out, int T, int start
                                           Pi_v, out, n_vec, e.status));
         return LEANKV_OK;
     }
+    if (q_head != kDim || q_token != (long long)n_q_heads * kDim) return LEANKV_EUNSUPPORTED;
     const TilePlan tp = make_tile_plan(T, start_pos, n_q_heads, n_kv_heads);
     float* qprime = reinterpret_cast<float*>(ws + tp.off_qprime);
     float* o_part = reinterpret_cast<float*>(ws + tp.off_opart);
@@ -736,6 +739,15 @@ extern "C" int leankv_tq_prefill_attn(const void* q, void* out, int T, int start
                                   static_cast<const void*>(o_part), static_cast<const float*>(ml_part), tp.n_splits,
                                   Pi_v, out, n_vec, reinterpret_cast<int*>(ws)));
     return LEANKV_OK;
+}
+
+extern "C" int leankv_tq_prefill_attn(const void* q, void* out, int T, int start_pos, int n_q_heads,
+                                      int n_kv_heads, const void* pool, int n_pages,
+                                      const int32_t* seq_pages, const float* Pi_k, const float* Pi_v,
+                                      const float* centroids, float scale, void* workspace,
+                                      size_t workspace_bytes, void* stream) {
+    return leankv_tq_prefill_attn_strided(q, (long long)n_q_heads * kDim, kDim, out, T, start_pos, n_q_heads, n_kv_heads, pool,
+                                          n_pages, seq_pages, Pi_k, Pi_v, centroids, scale, workspace, workspace_bytes, stream);
 }
 
 extern "C" int leankv_tq_decode_attn_status(const void* workspace, int* status) {

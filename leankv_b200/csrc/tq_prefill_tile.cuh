@@ -152,7 +152,8 @@ __global__ void __launch_bounds__(256) tq_expand_kernel(const ExpandParams p) {
 }
 
 struct TileAttnParams {
-    const __half* q;           // [T][Hq][128]
+    const __half* q;
+    long long q_token, q_head; // elements from a token / a head of q to the next
     float qscale;              // softmax scale * log2(e)
     const uint8_t* records;
     const uint8_t* images;
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(kPtThreads, 1) tq_prefill_tile_kernel(const Ti
             const int r = 8 * (2 * warp + (i & 1)) + (lane & 7), k8 = 4 * (i >> 1) + (lane >> 3);
             const int tok = tok0 + (r >> 2);
             uint4 v = make_uint4(0, 0, 0, 0);
-            if (tok < p.T) v = __ldg(reinterpret_cast<const uint4*>(p.q + ((size_t)tok * Hq + kvh * kGroup + (r & 3)) * kDim) + k8);
+            if (tok < p.T) v = __ldg(reinterpret_cast<const uint4*>(p.q + tok * p.q_token + (kvh * kGroup + (r & 3)) * p.q_head) + k8);
             *reinterpret_cast<uint4*>(s_qh + umma::offset(r, k8)) = v;
         }
     }

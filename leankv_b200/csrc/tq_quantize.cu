@@ -40,6 +40,7 @@ struct AppendParams {
     const __half* k;
     const __half* v;
     int B, H, T_new;
+    long long k_seq, k_head, v_seq, v_head;      // elements from a sequence / a head to the next; tokens are 128 apart
     const float* Pi_k;
     const float* Pi_v;
     const float* bounds;
@@ -49,6 +50,9 @@ struct AppendParams {
     const int32_t* kv_page_indices;
     const int32_t* start_pos;
 };
+__device__ __forceinline__ const __half* append_source(const AppendParams& p, int which, int b, int h) {
+    return which == 0 ? p.k + b * p.k_seq + h * p.k_head : p.v + b * p.v_seq + h * p.v_head;
+}
 
 template <int kTok>   // register accumulators per thread: 1 (single-token decode) or 16
 __global__ void __launch_bounds__(128) tq_pool_append_kernel(const AppendParams p) {
@@ -73,7 +77,7 @@ __global__ void __launch_bounds__(128) tq_pool_append_kernel(const AppendParams 
 
     if (tid < 8) s_bounds[tid] = tid < 7 ? p.bounds[tid] : __int_as_float(0x7f800000);
 
-    const __half* src = (which == 0 ? p.k : p.v) + (((size_t)b * p.H + h) * p.T_new + (first - pos0)) * kDim;
+    const __half* src = append_source(p, which, b, h) + (size_t)(first - pos0) * kDim;
     const float* Pi = which == 0 ? p.Pi_k : p.Pi_v;
 
     // norms and unit vectors: two threads per token, 64 coordinates each
@@ -327,7 +331,8 @@ extern "C" size_t leankv_tq_pool_bytes(int n_pages, int n_kv_heads) {
     return (size_t)n_pages * 2 * n_kv_heads * kChunkBytes;
 }
 
-extern "C" int leankv_tq_pool_append(const void* k, const void* v, int B, int n_kv_heads, int T_new,
+extern "C" int leankv_tq_pool_append_strided(const void* k, const void* v, int B, int n_kv_heads, int T_new, long long k_seq,
+                                             long long k_head, long long v_seq, long long v_head,
                                      const float* Pi_k, const float* Pi_v,
                                      const float* decision_boundaries, void* pool, int n_pages,
                                      const int32_t* kv_indptr, const int32_t* kv_page_indices,
@@ -339,8 +344,10 @@ extern "C" int leankv_tq_pool_append(const void* k, const void* v, int B, int n_
         return LEANKV_EINVAL;
     if (!aligned16(k) || !aligned16(v) || !aligned16(Pi_k) || !aligned16(Pi_v) || !aligned16(pool))
         return LEANKV_EALIGN;
+    if (k_seq % 8 != 0 || k_head % 8 != 0 || v_seq % 8 != 0 || v_head % 8 != 0) return LEANKV_EALIGN;
     if ((long long)B * n_kv_heads > 0x7fffffffLL) return LEANKV_ELIMIT;
     AppendParams p{};
+    p.k_seq = k_seq; p.k_head = k_head; p.v_seq = v_seq; p.v_head = v_head;
     p.k = static_cast<const __half*>(k);
     p.v = static_cast<const __half*>(v);
     p.B = B;
@@ -400,6 +407,16 @@ extern "C" int leankv_tq_pool_append(const void* k, const void* v, int B, int n_
     else
         LEANKV_CUDA_TRY(launch_kernel(tq_pool_append_kernel<16>, grid, dim3(128), 0, static_cast<cudaStream_t>(stream), p));
     return LEANKV_OK;
+}
+
+extern "C" int leankv_tq_pool_append(const void* k, const void* v, int B, int n_kv_heads, int T_new,
+                                     const float* Pi_k, const float* Pi_v,
+                                     const float* decision_boundaries, void* pool, int n_pages,
+                                     const int32_t* kv_indptr, const int32_t* kv_page_indices,
+                                     const int32_t* start_pos, void* stream) {
+    const long long head = (long long)T_new * kDim, seq = head * n_kv_heads;
+    return leankv_tq_pool_append_strided(k, v, B, n_kv_heads, T_new, seq, head, seq, head, Pi_k, Pi_v, decision_boundaries, pool,
+                                         n_pages, kv_indptr, kv_page_indices, start_pos, stream);
 }
 
 extern "C" int leankv_tq_pool_unpack(const void* pool, int n_pages, int n_kv_heads,

@@ -30,6 +30,22 @@ from .quantizer import TurboQuantMSE
 PAGE = _native.TQ_PAGE_TOKENS
 
 
+def _whole_pieces(t: torch.Tensor) -> bool:
+    """fp16 with contiguous vectors, each from a 16-byte boundary on: what the kernels read in place."""
+    return (t.dtype == torch.float16 and t.stride(-1) == 1 and t.data_ptr() % 16 == 0
+            and all(s % 8 == 0 for s in t.stride()[:-1]))
+
+
+def _rows(t: torch.Tensor) -> torch.Tensor:
+    """``[B, H, T, D]`` as the append kernels read it: sequences and heads anywhere, tokens one after another."""
+    return t if _whole_pieces(t) and t.stride(2) == t.shape[3] else t.to(torch.float16).contiguous()
+
+
+def _steps(t: torch.Tensor) -> tuple[int, int]:
+    """Elements from a sequence and from a head to the next; 0 where there is one only (its stride means nothing)."""
+    return tuple(t.stride(d) if t.shape[d] > 1 else 0 for d in (0, 1))
+
+
 class PagedKVCache:
     """Page pool of 3-bit TurboQuant KV + fused paged decode attention."""
 
@@ -189,12 +205,12 @@ class PagedKVCache:
                 self._seq_lengths[b] += t_new
         indptr, flat, _ = self._device_meta(batch)
         start = self._start_dev          # written by the table step, shared by all layers
-        k = key_states.to(torch.float16).contiguous()
-        v = value_states.to(torch.float16).contiguous()
+        k, v = _rows(key_states), _rows(value_states)
         kq, vq = self.key_quantizers[layer_idx], self.val_quantizers[layer_idx]
         with _native.on_device(self._device):
-            rc = _native.lib().leankv_tq_pool_append(
-                k.data_ptr(), v.data_ptr(), batch, self.num_kv_heads, t_new, kq._consts()[0].data_ptr(),
+            rc = _native.lib().leankv_tq_pool_append_strided(
+                k.data_ptr(), v.data_ptr(), batch, self.num_kv_heads, t_new, *_steps(k), *_steps(v),
+                kq._consts()[0].data_ptr(),
                 vq._consts()[0].data_ptr(), self._bounds.data_ptr(), self.kv_data[layer_idx].data_ptr(),
                 self.max_pages, indptr.data_ptr(), flat.data_ptr(), start.data_ptr(),
                 _native.current_stream())
@@ -276,14 +292,22 @@ class PagedKVCache:
                 need = lib.leankv_tq_prefill_attn_workspace_bytes(t_new, start, self.num_q_heads, self.num_kv_heads)
                 if self._prefill_ws is None or self._prefill_ws.numel() < need:
                     self._prefill_ws = torch.zeros(need, dtype=torch.uint8, device=self._device)
-                q = query[b].transpose(0, 1).to(torch.float16).contiguous()          # [T, Hq, D]
+                q = query[b]                                                         # [Hq, T, D]
+                if not _whole_pieces(q):
+                    q = q.to(torch.float16, copy=True, memory_format=torch.contiguous_format)
+                # the token stride of a single token is never used: what the packed order would have
+                token = q.stride(1) if t_new > 1 else self.num_q_heads * self.head_dim
                 pages = self._block_table[b, :math.ceil(n / PAGE)]
-                rc = lib.leankv_tq_prefill_attn(
-                    q.data_ptr(), out[b].data_ptr(), t_new, start, self.num_q_heads, self.num_kv_heads,
-                    self.kv_data[layer_idx].data_ptr(), self.max_pages, pages.data_ptr(),
+                attend = lambda q, token: lib.leankv_tq_prefill_attn_strided(
+                    q.data_ptr(), token, q.stride(0), out[b].data_ptr(), t_new, start, self.num_q_heads,
+                    self.num_kv_heads, self.kv_data[layer_idx].data_ptr(), self.max_pages, pages.data_ptr(),
                     kq._consts()[0].data_ptr(), vq._consts()[0].data_ptr(), self._centroids_host.data_ptr(),
                     1.0 / math.sqrt(self.head_dim), self._prefill_ws.data_ptr(), self._prefill_ws.numel(),
                     _native.current_stream())
+                rc = attend(q, token)
+                if rc == _native.EUNSUPPORTED:      # the kernel for the longest contexts reads [T, Hq, D]
+                    q = q.transpose(0, 1).contiguous().transpose(0, 1)
+                    rc = attend(q, self.num_q_heads * self.head_dim)
                 _native.check(rc, "leankv_tq_prefill_attn")
         out = out.transpose(1, 2)
         return out if query.dtype == torch.float16 else out.to(query.dtype)

@@ -677,3 +677,51 @@ def test_page_table_step_takes_pages_in_order(batch):
         assert cache._block_table[:batch, :n].tolist() == pages
         assert cache._start_dev[:batch].tolist() == [length - t_new] * batch
         assert int(cache._free_top) == len(free) and cache.page_table_status() == 0
+
+
+@pytest.mark.parametrize("form", ["slice", "token_major", "odd_stride", "unaligned", "float32", "expanded"])
+@pytest.mark.parametrize("t_new", [1, 5, 16, 70])
+def test_paged_cache_reads_parts_of_larger_tensors(form, t_new):
+    """Keys, values and queries in every layout a caller may hand over give the bits of contiguous fp16 ones."""
+    g, b, dev = 2, 2, _dev()
+    gen = torch.Generator().manual_seed(t_new)
+
+    def given(heads):
+        plain = torch.randn(b, heads, t_new, 128, generator=gen).half().to(dev)
+        if form == "expanded":
+            plain = plain[:1].expand(b, -1, -1, -1)
+        wide = {"slice": (b, heads + 1, t_new + 7, 128), "token_major": (b, t_new, heads, 128), "odd_stride": (b, heads, t_new, 131),
+                "unaligned": (b * heads * t_new * 128 + 4,)}.get(form)
+        if wide is None:
+            return plain.float() if form == "float32" else plain, plain.contiguous()
+        t = torch.zeros(wide, dtype=torch.float16, device=dev)
+        t = {"slice": lambda: t[:, 1:, 3:3 + t_new], "token_major": lambda: t.transpose(1, 2), "odd_stride": lambda: t[..., 1:129],
+             "unaligned": lambda: t[4:].view(b, heads, t_new, 128)}[form]()
+        t.copy_(plain)
+        return t, plain
+
+    caches = [PagedKVCache(num_layers=1, num_kv_heads=g, num_q_heads=4 * g, max_pages=32, device=dev) for _ in range(2)]
+    (k, k0), (v, v0), (q, q0) = given(g), given(g), given(4 * g)
+    if form == "unaligned":                # contiguous keys are read where they are: refused, as before
+        with pytest.raises(RuntimeError):
+            PagedKVCache(num_layers=1, num_kv_heads=g, num_q_heads=4 * g, max_pages=32, device=dev).append(0, k, v)
+        k, v = k0, v0
+    for cache, args in zip(caches, ((k, v), (k0, v0))):
+        cache.append(0, *args)
+    assert torch.equal(caches[0].kv_data, caches[1].kv_data)
+    got, want = caches[0].prefill_attention(0, q), caches[1].prefill_attention(0, q0)
+    assert got.dtype == q.dtype and torch.equal(got.half(), want)
+
+
+def test_prefill_attention_beyond_the_expanded_contexts_takes_strided_queries():
+    """Past 65536 tokens the page-walking kernel reads packed queries; the wrapper packs them."""
+    dev, n = _dev(), 65536 + 20
+    gen = torch.Generator(device=dev).manual_seed(1)
+    cache = PagedKVCache(num_layers=1, num_kv_heads=1, num_q_heads=4, max_pages=n // 16 + 2, device=dev)
+    k = torch.randn(1, 1, n, 128, generator=gen, device=dev).half()
+    cache.append(0, k, k)
+    q = torch.randn(1, 4, 3, 128, generator=gen, device=dev).half()
+    want = cache.prefill_attention(0, q.transpose(1, 2).contiguous().transpose(1, 2))
+    assert torch.equal(cache.prefill_attention(0, q), want)
+    one = cache.prefill_attention(0, q[:, :, 2:])
+    assert rel_l2(one.cpu(), want[:, :, 2:].cpu()) < 1e-3
