@@ -184,9 +184,9 @@ extern "C" int leankv_place_rows(const leankv_place_rows_t* a, void* stream) {
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (a->dtype == LEANKV_DT_BF16)
-        LEANKV_CUDA_TRY(launch_kernel(place_rows_kernel<bf16>, dim3(a->rows), dim3(kPlaceThreads), 0, st, *a));
+        LEANKV_CUDA_TRY(launch_early(place_rows_kernel<bf16>, dim3(a->rows), dim3(kPlaceThreads), 0, st, *a));
     else
-        LEANKV_CUDA_TRY(launch_kernel(place_rows_kernel<float>, dim3(a->rows), dim3(kPlaceThreads), 0, st, *a));
+        LEANKV_CUDA_TRY(launch_early(place_rows_kernel<float>, dim3(a->rows), dim3(kPlaceThreads), 0, st, *a));
     return LEANKV_OK;
 }
 

@@ -288,7 +288,7 @@ extern "C" int leankv_rmsnorm_f16(void* x, const void* delta, const void* weight
     if (n % 8 != 0 || !aligned16(x) || !aligned16(weight) || !aligned16(y) || (delta && !aligned16(delta)))
         return LEANKV_EALIGN;
     if (n > kNormThreads * 8 * kNormVecs) return LEANKV_ELIMIT;
-    LEANKV_CUDA_TRY(launch_kernel(rmsnorm_kernel, dim3(1), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(rmsnorm_kernel, dim3(1), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream),
                                   static_cast<__half*>(x), static_cast<const __half*>(delta),
                                   static_cast<const __half*>(weight), static_cast<__half*>(y), n, eps));
     return LEANKV_OK;
@@ -298,7 +298,7 @@ extern "C" int leankv_decode_begin(const void* embed_table, const long long* tok
                                    int hidden, int vocab, int32_t* state, void* stream) {
     if (!embed_table || !token || !h || !state || hidden <= 0 || vocab <= 0) return LEANKV_EINVAL;
     if (hidden % 8 != 0 || !aligned16(embed_table) || !aligned16(h)) return LEANKV_EALIGN;
-    LEANKV_CUDA_TRY(launch_kernel(decode_begin_kernel<__half, __half>, dim3(1), dim3(256), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(decode_begin_kernel<__half, __half>, dim3(1), dim3(256), 0, static_cast<cudaStream_t>(stream),
                                   static_cast<const __half*>(embed_table), token, static_cast<__half*>(h),
                                   hidden, vocab, state));
     return LEANKV_OK;
@@ -310,7 +310,7 @@ extern "C" int leankv_rope_f16(const void* qkv, const float* inv_freq, const int
     if (!qkv || !inv_freq || !state || !q_out || !k_out || n_q_heads <= 0 || n_kv_heads <= 0)
         return LEANKV_EINVAL;
     if (head_dim != 128) return LEANKV_EUNSUPPORTED;
-    LEANKV_CUDA_TRY(launch_kernel(rope_kernel, dim3(n_q_heads + n_kv_heads), dim3(64), 0,
+    LEANKV_CUDA_TRY(launch_early(rope_kernel, dim3(n_q_heads + n_kv_heads), dim3(64), 0,
                                   static_cast<cudaStream_t>(stream), static_cast<const __half*>(qkv), inv_freq,
                                   state, static_cast<__half*>(q_out), static_cast<__half*>(k_out), n_q_heads,
                                   n_kv_heads));
@@ -321,7 +321,7 @@ extern "C" int leankv_decode_end(const void* logits, int vocab, long long* token
                                  int history_cap, int32_t* state, void* stream) {
     if (!logits || !token || !history || !state || vocab <= 0 || history_cap < 0) return LEANKV_EINVAL;
     if (!aligned16(logits)) return LEANKV_EALIGN;
-    LEANKV_CUDA_TRY(launch_kernel(decode_end_kernel<__half>, dim3(1), dim3(1024), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<__half>, dim3(1), dim3(1024), 0, static_cast<cudaStream_t>(stream),
                                   static_cast<const __half*>(logits), vocab, token, history, history_cap,
                                   state + kPos, state + kStep, static_cast<int*>(nullptr)));
     return LEANKV_OK;
@@ -367,7 +367,7 @@ extern "C" int leankv_rmsnorm_rows_f16(void* x, const void* delta, const void* w
     if (n % 8 != 0 || !aligned16(x) || !aligned16(weight) || !aligned16(y) || (delta && !aligned16(delta)))
         return LEANKV_EALIGN;
     if (n > kNormThreads * 8 * kNormVecs) return LEANKV_ELIMIT;
-    LEANKV_CUDA_TRY(launch_kernel(rmsnorm_kernel, dim3(rows), dim3(kNormThreads), 0,
+    LEANKV_CUDA_TRY(launch_early(rmsnorm_kernel, dim3(rows), dim3(kNormThreads), 0,
                                   static_cast<cudaStream_t>(stream), static_cast<__half*>(x),
                                   static_cast<const __half*>(delta), static_cast<const __half*>(weight),
                                   static_cast<__half*>(y), n, eps));
@@ -382,7 +382,7 @@ extern "C" int leankv_batch_decode_begin(const void* embed_table, const long lon
         !kv_last_page_len || hidden <= 0 || vocab <= 0 || B <= 0 || max_pages_per_seq <= 0)
         return LEANKV_EINVAL;
     if (hidden % 8 != 0 || !aligned16(embed_table) || !aligned16(h)) return LEANKV_EALIGN;
-    LEANKV_CUDA_TRY(launch_kernel(batch_begin_kernel, dim3(B), dim3(256), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(batch_begin_kernel, dim3(B), dim3(256), 0, static_cast<cudaStream_t>(stream),
                                   static_cast<const __half*>(embed_table), tokens, static_cast<__half*>(h), hidden,
                                   vocab, B, pos, block_table, max_pages_per_seq, kv_indptr, kv_page_indices,
                                   kv_last_page_len));
@@ -392,7 +392,7 @@ extern "C" int leankv_batch_decode_begin(const void* embed_table, const long lon
 static int launch_silu_mul(const void* gate, const void* up, size_t ld, void* out, int rows, int inter, void* stream) {
     const long long total = (long long)rows * (inter / 8);
     const int grid = (int)std::min<long long>((total + 255) / 256, (long long)sm_count() * 8);
-    LEANKV_CUDA_TRY(launch_kernel(silu_mul_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(silu_mul_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream),
                                   static_cast<const __half*>(gate), static_cast<const __half*>(up), ld,
                                   static_cast<__half*>(out), inter, rows));
     return LEANKV_OK;
@@ -417,7 +417,7 @@ extern "C" int leankv_rope_split_f16(const void* qkv, const void* cos, const voi
         return LEANKV_EALIGN;
     const long long blocks = ((long long)T * ((long long)n_q_heads + 2ll * n_kv_heads) + 31) / 32;
     if (blocks > 0x7fffffffll) return LEANKV_ELIMIT;
-    LEANKV_CUDA_TRY(launch_kernel(rope_split_kernel, dim3((unsigned)blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(rope_split_kernel, dim3((unsigned)blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
                                   static_cast<const __half*>(qkv), static_cast<const __half*>(cos),
                                   static_cast<const __half*>(sin), static_cast<__half*>(q), static_cast<__half*>(k),
                                   static_cast<__half*>(v), T, n_q_heads, n_kv_heads));
@@ -430,7 +430,7 @@ extern "C" int leankv_batch_decode_end(const void* logits, int vocab, int B, lon
     if (!logits || !tokens || !history || !pos || !steps || vocab <= 0 || B <= 0 || history_cap < 0)
         return LEANKV_EINVAL;
     if (!aligned16(logits) || vocab % 8 != 0) return LEANKV_EALIGN;
-    LEANKV_CUDA_TRY(launch_kernel(decode_end_kernel<__half>, dim3(B), dim3(1024), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<__half>, dim3(B), dim3(1024), 0, static_cast<cudaStream_t>(stream),
                                   static_cast<const __half*>(logits), vocab, tokens, history, history_cap, pos,
                                   steps, static_cast<int*>(nullptr)));
     return LEANKV_OK;
@@ -532,7 +532,7 @@ extern "C" int leankv_paged_table_step(int t_new, int B, int32_t* seq_len, int32
         !kv_indptr || !kv_page_indices || !kv_last_page_len || !start_pos || !status)
         return LEANKV_EINVAL;
     if (B > kTableThreads) return LEANKV_ELIMIT;
-    LEANKV_CUDA_TRY(launch_kernel(paged_table_step_kernel, dim3(1), dim3(kTableThreads), 0,
+    LEANKV_CUDA_TRY(launch_early(paged_table_step_kernel, dim3(1), dim3(kTableThreads), 0,
                                   static_cast<cudaStream_t>(stream), t_new, B, seq_len, block_table, max_pages_per_seq,
                                   free_stack, free_top, kv_indptr, kv_page_indices, kv_last_page_len, start_pos,
                                   status));

@@ -241,16 +241,16 @@ int launch_stream_norm(const leankv_stream_norm_t* a, cudaStream_t st) {
                (!a->gain_per_col || aligned16(a->gain));
     for (int i = 0; i < a->n_mix; ++i) vec = vec && aligned16(a->mu[i]);
     if (!vec) {
-        LEANKV_CUDA_TRY(launch_kernel(stream_norm_kernel<T, D>, dim3(a->rows), dim3(kRowThreads), 0, st, *a));
+        LEANKV_CUDA_TRY(launch_early(stream_norm_kernel<T, D>, dim3(a->rows), dim3(kRowThreads), 0, st, *a));
         return LEANKV_OK;
     }
     const int per = a->n_mix > 0 && a->rows >= sm_count() * 8 ? 4 : 1;
     const dim3 grid((a->rows + per - 1) / per), block(kRowThreads);
     const int nv = (a->width + kRowThreads * 4 - 1) / (kRowThreads * 4);
-    if (nv <= 1) LEANKV_CUDA_TRY(launch_kernel(stream_norm_vec_kernel<T, D, 1>, grid, block, 0, st, *a, per));
-    else if (nv <= 2) LEANKV_CUDA_TRY(launch_kernel(stream_norm_vec_kernel<T, D, 2>, grid, block, 0, st, *a, per));
-    else if (nv <= 4) LEANKV_CUDA_TRY(launch_kernel(stream_norm_vec_kernel<T, D, 4>, grid, block, 0, st, *a, per));
-    else LEANKV_CUDA_TRY(launch_kernel(stream_norm_vec_kernel<T, D, 8>, grid, block, 0, st, *a, per));
+    if (nv <= 1) LEANKV_CUDA_TRY(launch_early(stream_norm_vec_kernel<T, D, 1>, grid, block, 0, st, *a, per));
+    else if (nv <= 2) LEANKV_CUDA_TRY(launch_early(stream_norm_vec_kernel<T, D, 2>, grid, block, 0, st, *a, per));
+    else if (nv <= 4) LEANKV_CUDA_TRY(launch_early(stream_norm_vec_kernel<T, D, 4>, grid, block, 0, st, *a, per));
+    else LEANKV_CUDA_TRY(launch_early(stream_norm_vec_kernel<T, D, 8>, grid, block, 0, st, *a, per));
     return LEANKV_OK;
 }
 
@@ -267,10 +267,10 @@ extern "C" int leankv_embed_begin(const void* table, int dtype, const long long*
     if (!known(dtype)) return LEANKV_EUNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dtype == LEANKV_DT_BF16)
-        LEANKV_CUDA_TRY(launch_kernel(decode_begin_kernel<bf16, float>, dim3(1), dim3(256), 0, st,
+        LEANKV_CUDA_TRY(launch_early(decode_begin_kernel<bf16, float>, dim3(1), dim3(256), 0, st,
                                       static_cast<const bf16*>(table), token, x, width, vocab, state));
     else
-        LEANKV_CUDA_TRY(launch_kernel(decode_begin_kernel<float, float>, dim3(1), dim3(256), 0, st,
+        LEANKV_CUDA_TRY(launch_early(decode_begin_kernel<float, float>, dim3(1), dim3(256), 0, st,
                                       static_cast<const float*>(table), token, x, width, vocab, state));
     return LEANKV_OK;
 }
@@ -279,7 +279,7 @@ extern "C" int leankv_greedy_end(const float* logits, int vocab, long long* toke
                                  int history_cap, int32_t* state, void* stream) {
     if (!logits || !token || !history || !state || vocab <= 0 || history_cap < 0) return LEANKV_EINVAL;
     if (!aligned16(logits)) return LEANKV_EALIGN;
-    LEANKV_CUDA_TRY(launch_kernel(decode_end_kernel<float>, dim3(1), dim3(1024), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<float>, dim3(1), dim3(1024), 0, static_cast<cudaStream_t>(stream),
                                   logits, vocab, token, history, history_cap, state + kPos, state + kStep,
                                   state + kParity));
     return LEANKV_OK;
@@ -312,7 +312,7 @@ extern "C" int leankv_silu_mul(const void* gate_up, void* out, int dtype, int ro
     const int grid = (int)std::min<long long>((total + 255) / 256, (long long)sm_count() * 16);
     auto go = [&](auto tag) -> int {
         using T = decltype(tag);
-        LEANKV_CUDA_TRY(launch_kernel(vec ? silu_mul_vec_kernel<T> : silu_mul_rows_kernel<T>, dim3(grid), dim3(256), 0,
+        LEANKV_CUDA_TRY(launch_early(vec ? silu_mul_vec_kernel<T> : silu_mul_rows_kernel<T>, dim3(grid), dim3(256), 0,
                                       st, static_cast<const T*>(gate_up), static_cast<T*>(out), inter, total));
         return LEANKV_OK;
     };
@@ -327,7 +327,7 @@ extern "C" int leankv_tanh_split(const float* in, void* out, int dtype, int rows
     const int grid = (int)std::min<long long>((total + 255) / 256, (long long)sm_count() * 8);
     auto go = [&](auto tag) -> int {
         using T = decltype(tag);
-        LEANKV_CUDA_TRY(launch_kernel(tanh_split_kernel<T>, dim3(grid), dim3(256), 0, st, in, static_cast<T*>(out), n,
+        LEANKV_CUDA_TRY(launch_early(tanh_split_kernel<T>, dim3(grid), dim3(256), 0, st, in, static_cast<T*>(out), n,
                                       total));
         return LEANKV_OK;
     };
@@ -337,6 +337,6 @@ extern "C" int leankv_tanh_split(const float* in, void* out, int dtype, int rows
 extern "C" int leankv_softcap(float* x, long long n, float cap, void* stream) {
     if (!x || n <= 0 || !(cap > 0.f)) return LEANKV_EINVAL;
     const int grid = (int)std::min<long long>((n + 255) / 256, (long long)sm_count() * 8);
-    LEANKV_CUDA_TRY(launch_kernel(softcap_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream), x, n, cap));
+    LEANKV_CUDA_TRY(launch_early(softcap_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream), x, n, cap));
     return LEANKV_OK;
 }

@@ -292,16 +292,16 @@ int scan(const leankv_time_mix_t& a, const void* r, const void* k, const void* v
     if (p.n_pieces > 1) {
         p.S_out = pieces;
         p.decay = decay;
-        LEANKV_CUDA_TRY(launch_kernel(time_mix_scan_kernel<T, L, false>, dim3(a.heads, cb, p.n_pieces - 1), block, 0, st,
+        LEANKV_CUDA_TRY(launch_early(time_mix_scan_kernel<T, L, false>, dim3(a.heads, cb, p.n_pieces - 1), block, 0, st,
                                       p, vec));
         const long long total = (long long)state_floats(a.heads, a.dim);
-        LEANKV_CUDA_TRY(launch_kernel(time_mix_carry_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, st,
+        LEANKV_CUDA_TRY(launch_early(time_mix_carry_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, st,
                                       static_cast<const float*>(a.S), pieces, static_cast<const float*>(decay), a.heads,
                                       a.dim, p.n_pieces));
         p.S_in = pieces;
     }
     p.S_out = a.S;
-    LEANKV_CUDA_TRY(launch_kernel(time_mix_scan_kernel<T, L, true>, dim3(a.heads, cb, p.n_pieces), block, 0, st, p, vec));
+    LEANKV_CUDA_TRY(launch_early(time_mix_scan_kernel<T, L, true>, dim3(a.heads, cb, p.n_pieces), block, 0, st, p, vec));
     return LEANKV_OK;
 }
 
@@ -318,7 +318,7 @@ int rows_all(const leankv_time_mix_t& a, const void* r, const void* k, const voi
     while (lanes < 32 && lanes * 8 < a.dim) lanes *= 2;
     const long long groups = (long long)rows * a.heads, threads = groups * lanes;
     const bool vec = a.dim % 8 == 0 && out_ld % 8 == 0 && aligned16(ws) && aligned16(g) && aligned16(out);
-    LEANKV_CUDA_TRY(launch_kernel(time_mix_out_kernel<T>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st,
+    LEANKV_CUDA_TRY(launch_early(time_mix_out_kernel<T>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st,
                                   static_cast<const float*>(ws), static_cast<const T*>(g), a.norm, a.eps,
                                   static_cast<T*>(out), out_ld, out_scale, groups, a.heads, a.dim, lanes, vec));
     return LEANKV_OK;

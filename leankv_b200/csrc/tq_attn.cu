@@ -674,7 +674,7 @@ extern "C" int leankv_tq_prefill_attn_strided(const void* q, long long q_token, 
         e.records = reinterpret_cast<uint8_t*>(ws + ep.off_records);
         e.images = reinterpret_cast<uint8_t*>(ws + ep.off_images);
         e.status = reinterpret_cast<int*>(ws);
-        LEANKV_CUDA_TRY(launch_kernel(tq_expand_kernel, dim3(std::max(ep.k_tiles, 8), n_kv_heads + 1), dim3(256), 0, st, e));
+        LEANKV_CUDA_TRY(launch_early(tq_expand_kernel, dim3(std::max(ep.k_tiles, 8), n_kv_heads + 1), dim3(256), 0, st, e));
         TileAttnParams a{};
         a.q = static_cast<const __half*>(q);
         a.q_token = q_token;

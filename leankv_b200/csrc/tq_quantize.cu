@@ -396,16 +396,16 @@ extern "C" int leankv_tq_pool_append_strided(const void* k, const void* v, int B
         }
         const long long slots = 2LL * sm_count();
         const int grid_tc = (int)(tp.n_tiles < slots ? tp.n_tiles : slots);
-        LEANKV_CUDA_TRY(launch_kernel(tq_pool_append_tc_kernel, dim3(grid_tc), dim3(kTcThreads), kTcSmemBytes,
+        LEANKV_CUDA_TRY(launch_early(tq_pool_append_tc_kernel, dim3(grid_tc), dim3(kTcThreads), kTcSmemBytes,
                                       static_cast<cudaStream_t>(stream), tp));
         return LEANKV_OK;
     }
     if (groups > 65535) return LEANKV_ELIMIT;
     dim3 grid(B * n_kv_heads, groups, 2);
     if (T_new == 1)
-        LEANKV_CUDA_TRY(launch_kernel(tq_pool_append_kernel<1>, grid, dim3(128), 0, static_cast<cudaStream_t>(stream), p));
+        LEANKV_CUDA_TRY(launch_early(tq_pool_append_kernel<1>, grid, dim3(128), 0, static_cast<cudaStream_t>(stream), p));
     else
-        LEANKV_CUDA_TRY(launch_kernel(tq_pool_append_kernel<16>, grid, dim3(128), 0, static_cast<cudaStream_t>(stream), p));
+        LEANKV_CUDA_TRY(launch_early(tq_pool_append_kernel<16>, grid, dim3(128), 0, static_cast<cudaStream_t>(stream), p));
     return LEANKV_OK;
 }
 

@@ -172,7 +172,7 @@ int append(const leankv_window_pool_t& a, const float* qkv, int ld, const float*
     const bool vec = a.dim % 4 == 0 && a.vdim % 4 == 0 && ld % 4 == 0 && nv <= 12 && aligned16(qkv) && aligned16(bias) &&
                      aligned16(a.q_norm) && aligned16(a.k_norm) && aligned16(q);
     auto go = [&](auto kernel) -> int {
-        LEANKV_CUDA_TRY(launch_kernel(kernel, dim3(rows), dim3(kAppendThreads), 0, st, a, qkv, ld, bias,
+        LEANKV_CUDA_TRY(launch_early(kernel, dim3(rows), dim3(kAppendThreads), 0, st, a, qkv, ld, bias,
                                       static_cast<T*>(q), start));
         return LEANKV_OK;
     };
@@ -183,7 +183,7 @@ int append(const leankv_window_pool_t& a, const float* qkv, int ld, const float*
     if (rc) return rc;
     const int b0 = start / a.pool, b1 = std::min((start + rows) / a.pool, a.max_blocks);
     if (b1 > b0)
-        LEANKV_CUDA_TRY(launch_kernel(window_pool_blocks_kernel<T>, dim3(b1 - b0), dim3(256), 0, st, a, b0));
+        LEANKV_CUDA_TRY(launch_early(window_pool_blocks_kernel<T>, dim3(b1 - b0), dim3(256), 0, st, a, b0));
     return LEANKV_OK;
 }
 
