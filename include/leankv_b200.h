@@ -187,7 +187,7 @@ int leankv_tq_pool_append_strided(const void* k, const void* v, int B, int n_kv_
 
 /* Appends of 16 or more tokens per sequence (prompt processing, where the reference quantizes the
  * flushed tokens with one dense fp32 matmul, cache.py:136-142 / quantizer.py:119-129) run the
- * rotation on tensor cores and re-derive every coordinate that lands within 1e-4 of a decision
+ * rotation on tensor cores and re-derive every coordinate that lands within 2.5e-5 of a decision
  * boundary with the sequential fp32 chain, so the codes are those of the definition above.
  * stats[0] = coordinates re-derived, stats[1] = coordinates quantized on the current device since
  * the last reset (synchronous copy; reset != 0 clears the counters). */
@@ -261,13 +261,14 @@ int leankv_tq_decode_attn_status(const void* workspace, int* status /* host */);
  * keys and values only, and never to an fp16 copy. Replaces, for prompt chunks, cache.update +
  * eager attention (leankv/turboquant/cache.py:136-142, transformers modeling_mistral.py:96-117).
  * q, out: [T][n_q_heads][128] fp16. seq_pages (device): the sequence's page ids in order, at least
- * (start_pos + T + 15) / 16 of them. Three launches: the query rotation (tcgen05 tensor cores, fp16
- * high/low split of Pi_K), the attention kernel (one CTA per 32 query tokens, kv head and page range: a
- * page is de-quantized once per 32 tokens into fp16 operand tiles; scores and the value sum on tensor cores
- * with the query as fp16 high + low halves and fp32 accumulation: tcgen05.mma with the accumulators in
- * tensor memory by default; LEANKV_PREFILL_MMA=sync in the environment selects an mma.sync form, =ws a
- * warp-specialised tcgen05 form with query and probabilities as tensor-memory operands), and the merge of
- * the page ranges with the inverse value rotation. The result agrees with decode steps at the same
+ * (start_pos + T + 15) / 16 of them. Up to 65536 tokens of context: one launch writes the centroids of all pages as operand
+ * tiles into the workspace, the attention kernel (one CTA per 32 query tokens, kv head and range of keys) takes 128 keys
+ * at a time by bulk copies, rotates the query in front and the values behind; where the keys are cut into ranges a
+ * third launch merges them. Beyond that three launches whose scratch does not grow with the context: the query rotation,
+ * an attention kernel that de-quantizes every page once per 32 tokens, and the merge with the inverse value rotation.
+ * Scores and the value sum are on tcgen05 tensor cores with the query as fp16 high + low halves and fp32 accumulation;
+ * LEANKV_PREFILL_MMA=t5 in the environment selects the page-walking kernel at every length, =sync an mma.sync form of it,
+ * =ws a warp-specialised one. The result agrees with decode steps at the same
  * positions to fp16 rounding (rel-L2 < 5e-4 in the tests). The workspace's first word is the status word
  * and must be zero before the first use (bit 0: a bounded wait ran out, bit 1: a page id out of range;
  * with bit 0, bits 4..6 say which wait: page copy, score MMAs, value MMAs); the rest needs no preparation

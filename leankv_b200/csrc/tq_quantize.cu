@@ -223,8 +223,8 @@ __global__ void tq_pool_unpack_kernel(const UnpackParams p) {
 
 // LEANKV_TQ_APPEND selects the kernel of multi-token appends: "fp32" = the fp32 kernel (the definition the
 // tensor-core paths are tested against), default / "mma" = fast rotation on mma.sync (64-token tiles, two CTAs
-// per SM), "t5" = fast rotation on tcgen05 (128-token tiles, one CTA per SM: measured slower, 1.49 ms against
-// 1.09 ms for a million vectors, because its norm / code / pack phases have no second CTA to overlap with).
+// per SM), "t5" = fast rotation on tcgen05 (128-token tiles, one CTA per SM: measured slower, 1.49 ms
+// for a million vectors against 0.64 ms, because its norm / code / pack phases have no second CTA to overlap with).
 // All three write the same bits.
 int tc_append_mode() {
     static int state = -1;
