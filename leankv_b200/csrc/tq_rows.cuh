@@ -37,6 +37,10 @@ constexpr int kRowsThreads = kRowsIn + kRowsOut + 32 + kRowsExact;
 constexpr int kRowsStagers = kRowsThreads - kRowsIn;         // the others stage the rotation while the first input is on its way
 constexpr uint32_t kRowsTmemCols = 256;
 constexpr int kRowsQueue = 512;                              // coordinates of a tile that may be listed for the exact chain
+// Norms are kept for 16 tiles. Input writes those of tile j once the products of j - 2 are complete, and these were issued
+// once every result thread had read the accumulators of j - 4; it does that before it waits for the list of j - 8 to be
+// cleared. So an exact warp may still read norms of tile j - 8 (not of j - 9, whose list the results of j - 5 waited for).
+constexpr int kRowsNorms = 16;
 constexpr int kRowsStageWords = 9;                           // words of a result row in shared memory (8 and one of padding)
 constexpr size_t kRowsSmemBytes = 6 * (size_t)umma::kTileBytes + (size_t)(kRowsOut / 32) * 32 * kRowsStageWords * 4 +
                                   4 * (size_t)kRowsQueue * sizeof(uint16_t);
@@ -244,7 +248,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) tq_quantize_rows_kernel(const
     __shared__ int s_listed[4];
     __shared__ float s_top[4];
     __shared__ float s_bounds[16];
-    __shared__ float s_norm[8][kRowsTile];      // of the last tiles: input is at most two ahead of the results, those four of the chains
+    __shared__ float s_norm[kRowsNorms][kRowsTile];
+    auto norms = [&](int j) { return s_norm[j & (kRowsNorms - 1)]; };
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     RowsFrame f = rows_begin(s_bar, &s_tmem);
@@ -272,7 +277,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) tq_quantize_rows_kernel(const
 #pragma unroll
     for (int q = 0; q < kBounds; ++q) b[q] = s_bounds[q];
     auto correction = [&](int j, int r, int coord, uint32_t word) -> uint32_t {
-        const float denom = s_norm[j & 7][r] + 1e-10f, inv = 1.0f / denom;
+        const float denom = norms(j)[r] + 1e-10f, inv = 1.0f / denom;
         auto over = [&](float x) { return kHalf ? divided(x, denom, inv) : x / denom; };
         const float4* pr = reinterpret_cast<const float4*>(p.Pi + (size_t)coord * kDim);
         const long long at = (first_vec(j) + r) * kDim;
@@ -363,7 +368,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) tq_quantize_rows_kernel(const
                 }
             }
             if (hf == 0) {
-                s_norm[j & 7][row] = norm;
+                norms(j)[row] = norm;
                 const long long gv = first_vec(j) + row;
                 if (gv < p.n_vec) p.norms[gv] = norm;
             }
@@ -447,7 +452,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) tq_quantize_rows_kernel(const
                 }
             }
             // a zero vector's fast values are exact
-            if (v0 + row >= p.n_vec || s_norm[j & 7][row] == 0.f) near[0] = near[1] = 0;
+            if (v0 + row >= p.n_vec || norms(j)[row] == 0.f) near[0] = near[1] = 0;
             // ---- what lies near a boundary goes to the exact warps, or, where the list or the indices' alignment does
             // not allow it, is done here ----
             const int slot = j & 3;

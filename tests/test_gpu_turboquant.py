@@ -615,6 +615,32 @@ def test_quantize_and_dequantize_at_the_edges_of_their_tiles(n, bits):
     assert np.array_equal(back.cpu().numpy(), exact)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("bits", [1, 2, 3, 4])
+def test_quantize_with_long_lists_of_undecided_coordinates(bits, dtype):
+    """Ten tiles and more a CTA, so that every ring of the kernel turns over, and some 380 coordinates a tile that only the
+    exact chain decides (now and then more than a list holds): rows whose rotated coordinates lie on a decision boundary, each
+    scaled differently, so that a neighbour's norm would give other codes. Codes and norms are bits."""
+    quant = TurboQuantMSE(128, bits, _dev(), torch.float32, seed=11)
+    n = torch.cuda.get_device_properties(_dev()).multi_processor_count * 128 * 10 + 77
+    gen = torch.Generator().manual_seed(bits)
+    x = torch.randn(n, 128, generator=gen)
+    on = torch.rand(n, generator=gen) < 3.2 / 128
+    bounds = quant.decision_boundaries.cpu()
+    edge = bounds[bounds.numel() // 2 + 1].item() if bits > 1 else 0.0
+    y = torch.full((int(on.sum()), 128), edge) * (1 - 2 * torch.randint(0, 2, (int(on.sum()), 128), generator=gen))
+    y[:, :8] = ((1 - 120 * edge ** 2) / 8) ** 0.5
+    x[on] = y @ quant.Pi.cpu()
+    x = (x * 2.0 ** (9 * torch.rand(n, 1, generator=gen) - 6)).to(dtype)
+    codes, norms, _, _ = tq_exact.quantize(x.float().numpy(), quant.Pi.cpu().numpy(), bounds.numpy())
+    per, width = {1: (8, 1), 2: (4, 2)}.get(bits, (2, 4))
+    packed = sum(codes.reshape(n, -1, per)[..., i].astype(np.uint8) << (width * i) for i in range(per))
+    for _ in range(3):
+        q = quant.quantize(x.to(_dev()))
+        assert np.array_equal(q.indices.cpu().numpy(), packed)
+        assert torch.equal(q.norms.cpu(), torch.from_numpy(norms).to(dtype))
+
+
 @pytest.mark.parametrize("H, start, T", [(1, 0, 1), (2, 0, 31), (2, 95, 33), (1, 127, 1), (1, 128, 129), (2, 0, 385), (8, 3000, 200),
                                          (1, 5000, 40)])
 def test_prefill_attention_at_the_edges_of_its_tiles(H, start, T):

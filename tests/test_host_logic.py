@@ -339,3 +339,51 @@ def test_argument_validation_of_the_prefill_attention_and_sharded_argmax_entry_p
     assert end(x, logits=None) == -1
     x.recv[1] = None
     assert end(x) == -1                            # a peer's area is missing
+
+
+def _quantize_reach(n_tiles):
+    """The largest distance, over all interleavings, from a tile whose norms the input role of the row-wise quantize kernel
+    writes back to one whose norms are still read. The roles as the kernel has them, with two accumulators and four
+    lists: input waits for the products two tiles back; products for the input of their tile and for the accumulators
+    two tiles back to be read; results read a tile's accumulators, then wait for the list four tiles back to be cleared and
+    read the tile's norms while they write its list; three exact warps take the lists in turn and read the norms."""
+    start = (0, 0, 0, 0, 0, (0, 1, 2), (False,) * 3)      # inputs, products, accumulators read, lists, and the chains'
+    seen, todo, reach = {start}, [start], 0               # tiles and whether they are in them
+    while todo:
+        state = todo.pop()
+        inputs, writing, products, taken, listed, tile, inside = state
+        cleared = {t for t in range(n_tiles) if t < tile[t % 3]}
+        if writing:
+            reading = [t for t, i in zip(tile, inside) if i] + ([listed] if taken > listed else [])
+            reach = max([reach] + [inputs - t for t in reading])
+        new = []
+        if writing:
+            new.append((inputs + 1, 0, products, taken, listed, tile, inside))
+        elif inputs < n_tiles and (inputs < 2 or products > inputs - 2):
+            new.append((inputs, 1, products, taken, listed, tile, inside))
+        if products < inputs and (products < 2 or taken > products - 2):
+            new.append((inputs, writing, products + 1, taken, listed, tile, inside))
+        if taken == listed and taken < products:
+            new.append((inputs, writing, products, taken + 1, listed, tile, inside))
+        if taken > listed and (listed < 4 or listed - 4 in cleared):
+            new.append((inputs, writing, products, taken, listed + 1, tile, inside))
+        for w in range(3):
+            if inside[w]:
+                new.append((inputs, writing, products, taken, listed, tile[:w] + (tile[w] + 3,) + tile[w + 1:],
+                            inside[:w] + (False,) + inside[w + 1:]))
+            elif tile[w] < listed:
+                new.append((inputs, writing, products, taken, listed, tile, inside[:w] + (True,) + inside[w + 1:]))
+        for s in new:
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
+    return reach
+
+
+def test_quantize_keeps_norms_as_long_as_they_are_read():
+    source = open(os.path.join(ROOT, "leankv_b200", "csrc", "tq_rows.cuh")).read()
+    depth = re.findall(r"__shared__ float s_norm\[(\w+)\]\[kRowsTile\];", source)[0]      # the quantize kernel comes first
+    depth = int(re.search(rf"constexpr int {depth} = (\d+);", source).group(1)) if not depth.isdigit() else int(depth)
+    reach = _quantize_reach(16)
+    assert reach == _quantize_reach(20) == 8
+    assert depth > reach and depth & (depth - 1) == 0
