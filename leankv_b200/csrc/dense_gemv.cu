@@ -94,10 +94,13 @@ __device__ __forceinline__ int row_of_lane(int lane) { return (lane * R) >> 5; }
 // kJoined: a branch joins the stream first, or there is a gain per column; every thread prepares its columns in registers
 // (one slab). kStaged: the same in shared memory, any number of slabs. kGrouped: row groups with an input slice each.
 enum class Input { kPlain, kJoined, kStaged, kGrouped };
-template <typename T, int CH, Input IN>
-__global__ void __launch_bounds__(512, 1) dense_gemv_kernel(const GemvParams p) {
+// kAhead: the weights of the next rows are in registers before they are needed, sixteen warps an SM. Otherwise rows are asked for
+// when it is their turn, by twice as many warps (bf16) or twice as many rows a warp (fp32): more bytes in flight, for
+// ranges so long that their start does not count (see launch_gemv).
+template <typename T, int CH, Input IN, bool kAhead>
+__global__ void __launch_bounds__(512, !kAhead && sizeof(T) == 2 ? 2 : 1) dense_gemv_kernel(const GemvParams p) {
     constexpr bool STAGED = IN == Input::kStaged, JOINED = IN == Input::kJoined, GROUPED = IN == Input::kGrouped;
-    constexpr int R = (sizeof(T) == 2 ? 8 : 4) / CH;      // rows in flight: 128 bytes a lane
+    constexpr int R = (sizeof(T) == 4 && kAhead ? 4 : 8) / CH;      // rows in flight: 128 bytes a lane (256 in fp32 without kAhead)
     extern __shared__ __align__(16) float s_dyn[];
     float* s_part = STAGED ? s_dyn + p.x_smem : s_dyn;      // [rows of this CTA (x2 if gated)][warps]
     __shared__ float s_tmp[64];
@@ -134,7 +137,7 @@ __global__ void __launch_bounds__(512, 1) dense_gemv_kernel(const GemvParams p) 
                 load_w8(W + row * cols, s * slab_cols + (c * warps + warp) * 256 + lane * 8, cols, vec, raw[r][c]);
         }
     };
-    if (a.early_weights) load_rows(0, 0, n_rows - 1);
+    if (kAhead && a.early_weights) load_rows(0, 0, n_rows - 1);
     // kJoined: the gains do not depend on the launch ahead
     float gn[CH][8], pg[CH][8];
     if constexpr (JOINED) {
@@ -146,7 +149,7 @@ __global__ void __launch_bounds__(512, 1) dense_gemv_kernel(const GemvParams p) 
         }
     }
     pdl_begin();
-    if (!a.early_weights) load_rows(0, 0, n_rows - 1);
+    if (kAhead && !a.early_weights) load_rows(0, 0, n_rows - 1);
 
     float rs = 1.f;
     float xj[CH][8];                // kJoined: this thread's columns of x'
@@ -280,6 +283,7 @@ __global__ void __launch_bounds__(512, 1) dense_gemv_kernel(const GemvParams p) 
             }
             const int v0 = (r0 - lo) * mult, v1 = (r1 - lo) * mult;
             for (int v = v0; v < v1; v += R) {
+                if (!kAhead) load_rows(s, v, v1 - 1);
                 float acc[R];
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
@@ -294,8 +298,8 @@ __global__ void __launch_bounds__(512, 1) dense_gemv_kernel(const GemvParams p) 
                 }
                 // the next rows, of this segment, the next one or the next slab, under the reduction
                 const int next = min(v + R, v1);
-                if (next < n_rows) load_rows(s, next, n_rows - 1);
-                else if (s + 1 < p.slabs) load_rows(s + 1, 0, n_rows - 1);
+                if (kAhead && next < n_rows) load_rows(s, next, n_rows - 1);
+                else if (kAhead && s + 1 < p.slabs) load_rows(s + 1, 0, n_rows - 1);
                 const float sum = warp_reduce_rows<R>(acc, lane);
                 const int vr = v + row_of_lane<R>(lane);
                 if ((lane & (32 / R - 1)) == 0 && vr < v1) {
@@ -327,9 +331,9 @@ __global__ void __launch_bounds__(512, 1) dense_gemv_kernel(const GemvParams p) 
     }
 }
 
-template <typename T, int CH, Input IN>
-int launch_gemv(const GemvParams& p, int warps, cudaStream_t st) {
-    const int per_sm = std::max(1, kMaxWarps / warps);
+template <typename T, int CH, Input IN, bool kAhead>
+int launch_gemv_as(const GemvParams& p, int warps, cudaStream_t st) {
+    const int per_sm = std::max(1, (!kAhead && sizeof(T) == 2 ? 2 : 1) * kMaxWarps / warps);
     const int mult = p.a.gated ? 2 : 1;
     int grid = std::min(sm_count() * std::min(per_sm, 8), (p.a.rows + 1) / 2);
     grid = std::max(grid, 1);
@@ -337,10 +341,25 @@ int launch_gemv(const GemvParams& p, int warps, cudaStream_t st) {
     while (smem_for(grid) > (size_t)kSmemPartials / 2 && grid < p.a.rows) grid = std::min(p.a.rows, grid * 2);
     const size_t smem = smem_for(grid) + (size_t)p.x_smem * sizeof(float);
     if (smem > 48 * 1024)
-        LEANKV_CUDA_TRY(cudaFuncSetAttribute(dense_gemv_kernel<T, CH, IN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        LEANKV_CUDA_TRY(cudaFuncSetAttribute(dense_gemv_kernel<T, CH, IN, kAhead>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              kSmemPartials + kMaxStaged * (int)sizeof(float)));
-    LEANKV_CUDA_TRY(launch_kernel_ex(true, dense_gemv_kernel<T, CH, IN>, dim3(grid), dim3(warps * 32), smem, st, p));
+    LEANKV_CUDA_TRY(launch_kernel_ex(true, dense_gemv_kernel<T, CH, IN, kAhead>, dim3(grid), dim3(warps * 32), smem, st, p));
     return LEANKV_OK;
+}
+
+// Which of the two kernels: by the rounds of 4 KB a warp that an SM's share of the weights takes, and by the warps that
+// fit beside one another (CTAs of `warps` warps, at most eight). Weights from HBM, us with kAhead and early weights /
+// without kAhead: bf16 32768 x 2048 (14 rounds) 24.4 / 22.4, 65536 x 2048 (28) 47.3 / 42.5, 32768 x 1024 (7) 13.1 / 13.8,
+// 5632 x 2048 gated (5) 10.2 / 10.6, 4096 x 1024 (1) 3.4 / 5.2; eleven warps, bf16 2048 x 5632 (3.5) 7.0 / 6.3; eight warps,
+// fp32 16384 x 128 (1.8) 5.6 / 5.2, bf16 16384 x 128 (0.9) 4.1 / 4.9.
+template <typename T, int CH, Input IN>
+int launch_gemv(const GemvParams& p, int warps, cudaStream_t st) {
+    const int resident = std::min(std::max(1, kMaxWarps / warps), 8) * warps;
+    const double bytes = (double)p.a.rows * (p.a.gated ? 2 : 1) * p.a.cols * sizeof(T);
+    const double rounds = bytes / sm_count() / (4096.0 * resident);
+    const bool thin = resident < (sizeof(T) == 2 ? 12 : 9);
+    return rounds >= 10.0 || (thin && rounds > 1.5) ? launch_gemv_as<T, CH, IN, false>(p, warps, st)
+                                                    : launch_gemv_as<T, CH, IN, true>(p, warps, st);
 }
 
 }  // namespace

@@ -576,3 +576,54 @@ def test_gemv_weights_read_ahead_of_the_dependency_wait(dtype, rows, cols, gated
     v = w.double() @ (x.double() * 1.3 / (x.double().square().mean() + 1e-5).sqrt())
     want = torch.nn.functional.silu(v[:rows]) * v[rows:] if gated else v
     assert float((ys[0].double() - want).norm() / want.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("form,rows,cols", [
+    # one round of an SM's warps: the next rows' weights ahead of their turn
+    ("plain", 301, 520), ("mixed", 301, 520), ("joined", 301, 520), ("staged", 37, 9000), ("grouped", 330, 264),
+    # many rounds of few resident warps (fp32, bf16), and a long range: rows as their turn comes
+    ("plain", 7203, 250), ("joined", 7203, 250), ("grouped", 7200, 250), ("mixed", 2001, 2816), ("joined", 2001, 2816),
+    ("grouped", 2010, 2816), ("staged", 701, 8400), ("plain", 24001, 2048)])
+def test_gemv_behind_the_launch_that_writes_its_input(dtype, form, rows, cols):
+    """Every kind of input, through both kernels: weights may be asked for before the launch ahead is done, its output may not.
+    The same bits with and without, against 64-bit sums."""
+    w = rnd(rows, cols, seed=1, std=cols ** -0.5).to(DEV).to(dtype)
+    src, mat = rnd(64, seed=2).to(DEV), rnd(cols, 64, seed=3, std=0.2).to(DEV)
+    gain, post = rnd(cols, seed=4, mean=0.7, std=0.2).to(DEV), rnd(cols, seed=5, mean=0.7, std=0.2).to(DEV)
+    one, mu = torch.tensor(1.3, device=DEV), rnd(2, cols, seed=6).to(DEV)
+    state = torch.zeros(8, dtype=torch.int32, device=DEV)
+    base, cut = rnd(cols, seed=7).to(DEV), rows // 3
+    outs = []
+    for early in (0, 1):
+        x, y, xo = (torch.full((n,), 7.0, device=DEV) for n in (cols, rows, cols))
+        prev = rnd(2, cols, seed=8).to(DEV)
+        kw = dict(w=w, y=y, dtype=CODE[dtype], rows=rows, cols=cols, early_weights=early)
+        if form == "plain":
+            kw.update(x=x, gain=one, eps=1e-5)
+        elif form == "mixed":
+            kw.update(x=x, gain=one, eps=1e-5, n_mix=2, prev=prev, state=state)
+        elif form == "grouped":
+            kw.update(x=x, group_rows=rows // 3, group_stride=0)
+        else:
+            kw.update(x=base, gain=gain, gain_per_col=1, eps=1e-5, delta=x, post_gain=post, post_mult=0.6, x_out=xo)
+        a = _native.DenseGemv(**{k: v.data_ptr() if torch.is_tensor(v) else v for k, v in kw.items()})
+        if form == "mixed":
+            a.mix_end[0], a.mix_end[1], a.mu[0], a.mu[1] = cut, rows, mu[0].data_ptr(), mu[1].data_ptr()
+        gemv(w=mat, x=src, y=x, dtype=CODE[F32], rows=cols, cols=64)
+        ok(_native.mixers().leankv_dense_gemv(ctypes.byref(a), stream()))
+        outs.append((y, xo, prev))
+    for got, want in zip(*outs):
+        assert torch.equal(got, want)
+    x = (mat.double() @ src.double())
+    if form in ("joined", "staged"):
+        norm = lambda v, g: v * g.double() / (v.square().mean() + 1e-5).sqrt()
+        x = norm(base.double() + 0.6 * norm(x, post), gain)
+    elif form != "grouped":
+        x = x * 1.3 / (x.square().mean() + 1e-5).sqrt()
+    want = w.double() @ x
+    if form == "mixed":
+        before = rnd(2, cols, seed=8).to(DEV)[0].double()
+        mixed = [x + (before - x) * mu[i].double() for i in range(2)]
+        want = torch.cat([w[:cut].double() @ mixed[0], w[cut:].double() @ mixed[1]])
+    assert rel(outs[0][0].cpu(), want.cpu()) < 1e-5
