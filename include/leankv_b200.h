@@ -192,8 +192,9 @@ int leankv_tq_pool_append_strided(const void* k, const void* v, int B, int n_kv_
  * stats[0] = coordinates re-derived, stats[1] = coordinates quantized on the current device since
  * the last reset (synchronous copy; reset != 0 clears the counters). */
 int leankv_tq_band_stats(unsigned long long* stats /* host, 2 */, int reset);
-/* *status = 0 unless a bounded wait for the tensor cores inside a multi-token append has ever run out on the
- * current device (the pages written by that launch are then incomplete). Synchronous copy. */
+/* *status = 0 unless a bounded wait inside leankv_tq_quantize or a multi-token append has ever run out on the current
+ * device. The pages written by that append are then incomplete; of a quantize call the norms of every vector that may lack
+ * codes are NaN. Synchronous copy on the legacy stream: wait for the launching stream first. */
 int leankv_tq_append_status(int* status /* host */);
 
 /* Pool -> reference format for pages of one sequence: codes as nibble-packed uint8

@@ -183,8 +183,8 @@ __global__ void __launch_bounds__(128) tq_pool_append_kernel(const AppendParams 
 // Coordinates decided by the exact chain / coordinates quantized by the tensor-core append, per device,
 // since the last reset (read by leankv_tq_band_stats).
 __device__ unsigned long long g_band_stats[2];
-// Non-zero once a bounded wait for the tensor cores inside the tcgen05 append has run out (per device, sticky;
-// read by leankv_tq_append_status).
+// Non-zero once a bounded wait inside the quantize kernel or the tcgen05 append has run out (per device, sticky; read by
+// leankv_tq_append_status).
 __device__ int g_append_status;
 
 struct UnpackParams {

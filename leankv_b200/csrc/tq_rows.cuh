@@ -166,14 +166,16 @@ __device__ __forceinline__ RowsFrame rows_begin(uint64_t* s_bar, uint32_t* s_tme
     }
     return f;
 }
-__device__ __forceinline__ void rows_end(const RowsFrame& f, bool ok, int* status) {
+// The end, which every thread reaches: whether a wait of this CTA ran out.
+__device__ __forceinline__ bool rows_end(const RowsFrame& f, bool ok, int* status) {
     if (!ok) atomicOr(status, 1);
     umma::fence_before_sync();
-    __syncthreads();
+    const bool failed = __syncthreads_or(!ok) != 0;
     if ((threadIdx.x >> 5) == kRowsIn / 32) {
         umma::fence_after_sync();
         umma::tmem_free_n(f.tmem, kRowsTmemCols);
     }
+    return failed;
 }
 // The issuing warp: `products(buffer)` issues a tile's MMAs from one elected lane.
 template <typename Products>
@@ -506,7 +508,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1) tq_quantize_rows_kernel(const
             umma::bar_arrive(f.bars.listed + 8 * slot);
         }
     }
-    rows_end(f, ok, p.status);
+    if (rows_end(f, ok, p.status)) {
+        // codes are missing: no vector of this CTA may pass for one that was quantized
+        for (int j = 0; j < n_mine; ++j)
+            if (tid < kRowsTile && first_vec(j) + tid < p.n_vec) p.norms[first_vec(j) + tid] = __int_as_float(0x7fffffff);
+    }
 }
 
 constexpr int kChainWarps = 8, kUnpackThreads = 128;

@@ -36,6 +36,7 @@ from . import _native
 from .decode_loop import DecodeLoop
 from .teal.sparse_fns import compute_threshold_for_sparsity
 from .turboquant.codebook import get_codebook_tensors
+from .turboquant.quantizer import kernel_status
 from .turboquant.rotation import generate_rotation_matrix
 
 PROJ_NAMES = ["q_proj", "k_proj", "v_proj", "o_proj", "gate_proj", "up_proj", "down_proj"]
@@ -510,6 +511,10 @@ class DecodeEngine(DecodeLoop):
             raise RuntimeError(f"prefill attention reported status {st.value} "
                                "(1 = a bounded wait ran out, 2 = page id outside the pool)")
 
+    def _check_quantize_status(self) -> None:
+        if kernel_status(self.dev) != 0:
+            raise RuntimeError("a bounded wait inside a quantize or append kernel ran out: codes are missing")
+
     def _dense_forward(self, ids: torch.Tensor, write_cache: bool, collect: Optional[dict] = None,
                        page_indices: Optional[torch.Tensor] = None, start_pos: int = 0,
                        attention: str = "dense"):
@@ -685,6 +690,7 @@ class DecodeEngine(DecodeLoop):
         collect: dict = {}
         with torch.cuda.device(self.dev):
             self._dense_forward(ids, write_cache=False, collect=collect)
+            self._check_quantize_status()
         thresholds = {}
         for l, acts in collect.items():
             thresholds[l] = {}
@@ -723,6 +729,7 @@ class DecodeEngine(DecodeLoop):
                                         attention=attention)
             if attention == "packed":
                 self._check_prefill_status()
+            self._check_quantize_status()
             logits = x @ self.w["lm_head_t"]
             tok = torch.argmax(logits.float()).reshape(1)
             self.token.copy_(tok)

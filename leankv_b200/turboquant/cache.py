@@ -16,7 +16,7 @@ from __future__ import annotations
 import torch
 
 from .. import _native
-from .quantizer import MSEQuantized, TurboQuantMSE
+from .quantizer import MSEQuantized, TurboQuantMSE, kernel_status
 
 
 class _ColdStore:
@@ -164,6 +164,10 @@ class TurboQuantCache:
         cold_k = self._dequant_cold(self.key_quantizers[layer_idx], self._cold_k[layer_idx])
         cold_v = self._dequant_cold(self.val_quantizers[layer_idx], self._cold_v[layer_idx])
         return torch.cat([cold_k, hot_k], dim=2), torch.cat([cold_v, hot_v], dim=2)
+
+    def kernel_status(self) -> int:
+        """0, or 1 once a bounded wait inside a quantize kernel of this device has run out."""
+        return kernel_status(self._device)
 
     # ── what HF generation calls ────────────────────────────────────────
 

@@ -25,7 +25,7 @@ import math
 import torch
 
 from .. import _native
-from .quantizer import TurboQuantMSE
+from .quantizer import TurboQuantMSE, kernel_status
 
 PAGE = _native.TQ_PAGE_TOKENS
 
@@ -313,10 +313,10 @@ class PagedKVCache:
         return out if query.dtype == torch.float16 else out.to(query.dtype)
 
     def kernel_status(self) -> int:
-        """Status words of the attention kernels' bounded waits, decode and prefill OR-ed (0 = clean)."""
+        """Status words of the bounded waits OR-ed: decode and prefill attention, append (0 = clean)."""
         import ctypes
 
-        status = 0
+        status = kernel_status(self._device)
         for ws in (self._workspace, self._prefill_ws):
             if ws is None:
                 continue

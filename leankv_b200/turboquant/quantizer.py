@@ -9,6 +9,7 @@ fields per byte for 3- and 4-bit codes (low nibble = even coordinate,
 
 from __future__ import annotations
 
+import ctypes
 import math
 from typing import NamedTuple
 
@@ -72,6 +73,16 @@ def _unpack_indices(packed: torch.Tensor, bits: int, d: int) -> torch.Tensor:
     shifts = torch.arange(per_byte, device=packed.device, dtype=torch.int32) * width
     fields = (packed.to(torch.int32).unsqueeze(-1) >> shifts) & ((1 << width) - 1)
     return fields.reshape(*packed.shape[:-1], -1)[..., :d].long()
+
+
+def kernel_status(device: torch.device) -> int:
+    """Status of the quantize and append kernels on ``device`` since it was first used: 0, or 1 once a bounded wait inside
+    one has run out, so that codes are missing (quantize then also returns NaN norms). Waits for the current stream."""
+    status = ctypes.c_int(0)
+    with _native.on_device(device):
+        torch.cuda.current_stream().synchronize()
+        _native.check(_native.lib().leankv_tq_append_status(ctypes.byref(status)), "leankv_tq_append_status")
+    return status.value
 
 
 class TurboQuantMSE(torch.nn.Module):
@@ -167,6 +178,10 @@ class TurboQuantMSE(torch.nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """Quantize then dequantize."""
         return self.dequantize(self.quantize(x))
+
+    def kernel_status(self) -> int:
+        """See :func:`kernel_status`, of the device that the buffers are on."""
+        return kernel_status(self.Pi.device)
 
 
 class TurboQuantProd(torch.nn.Module):

@@ -387,3 +387,35 @@ def test_quantize_keeps_norms_as_long_as_they_are_read():
     reach = _quantize_reach(16)
     assert reach == _quantize_reach(20) == 8
     assert depth > reach and depth & (depth - 1) == 0
+
+
+class _StatusLibrary:
+    """A kernel library whose quantize and append kernels have reported ``value``."""
+
+    def __init__(self, value):
+        self.value = value
+
+    def leankv_tq_append_status(self, status):
+        status._obj.value = self.value
+        return 0
+
+
+@pytest.mark.parametrize("value", [0, 1])
+def test_a_wait_that_ran_out_while_quantizing_is_reported(monkeypatch, value):
+    """What a user asks (quantizer, both caches) and where the engines ask by themselves."""
+    import contextlib
+    from types import SimpleNamespace
+
+    from leankv_b200.engine import DecodeEngine
+    from leankv_b200.turboquant.cache import TurboQuantCache
+    from leankv_b200.turboquant.paged_cache import PagedKVCache
+
+    monkeypatch.setattr(_native, "lib", lambda: _StatusLibrary(value))
+    monkeypatch.setattr(_native, "on_device", lambda device: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: SimpleNamespace(synchronize=lambda: None))
+    dev = torch.device("cpu")
+    assert quantizer.TurboQuantMSE(128, 3, dev).kernel_status() == value
+    assert TurboQuantCache(num_layers=1, device=dev).kernel_status() == value
+    assert PagedKVCache(num_layers=1, num_kv_heads=1, num_q_heads=4, max_pages=4, device=dev).kernel_status() == value
+    with pytest.raises(RuntimeError, match="codes are missing") if value else contextlib.nullcontext():
+        DecodeEngine._check_quantize_status(SimpleNamespace(dev=dev))
