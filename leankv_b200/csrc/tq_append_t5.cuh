@@ -2,7 +2,7 @@
 // inside namespace leankv::{anonymous}, after tq_append_tc.cuh whose contract and band logic it shares).
 //
 // Same two-step scheme as tq_pool_append_tc_kernel — a fast rotation y ~ Pi_hi u_hi + Pi_hi u_lo + Pi_lo u_hi
-// with fp32 accumulation decides every code that is farther than kBand from all decision boundaries, the
+// with fp32 accumulation decides every code that is farther than the band from all decision boundaries, the
 // sequential fp32 chain decides the rest — but the fast rotation is three tcgen05.mma products per k-step on a
 // tile of 128 tokens: the unit vectors' fp16 halves and Pi's are written to shared memory in the blocked K-major
 // layout of umma.cuh, one thread issues the 24 MMAs (M = N = 128, K = 16), the accumulator (128 tokens x 128
@@ -31,6 +31,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) tq_pool_append_t5_kernel(const 
     __shared__ float s_norm[kT5Tokens];
     __shared__ uint16_t s_list[kT5Threads / 32][kListCap];      // per warp: (token row << 7 | coordinate) awaiting the exact chain
     __shared__ float s_bounds[8];
+    __shared__ float s_top[kT5Threads / 32];
 
     const AppendParams& p = tp.a;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -47,6 +48,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) tq_pool_append_t5_kernel(const 
     const long long tile_hi = ((long long)blockIdx.x + 1) * tp.n_tiles / gridDim.x;
     const long long per_which = (long long)p.B * p.H * tp.groups;
     int loaded_which = -1;
+    float band = 0.f;
     unsigned long long n_exact = 0, n_coords = 0;
     uint32_t phase = 0;
     bool failed = false;
@@ -62,7 +64,8 @@ __global__ void __launch_bounds__(kT5Threads, 1) tq_pool_append_t5_kernel(const 
         umma::fence_before_sync();
         __syncthreads();                 // the previous tile's readers of the code tile, TMEM and operands are done
         umma::fence_after_sync();
-        if (which != loaded_which) {
+        const bool staged = which != loaded_which;
+        if (staged) {
             // B[k][n] = Pi[n][k]: rows of Pi as they are, split into fp16 halves
 #pragma unroll 4
             for (int i = tid; i < kDim * (kDim / 8); i += kT5Threads) {
@@ -124,6 +127,14 @@ __global__ void __launch_bounds__(kT5Threads, 1) tq_pool_append_t5_kernel(const 
         umma::fence_before_sync();
         __syncthreads();
         umma::fence_after_sync();
+
+        if (staged) {
+            HalfRow row;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                row.add(*reinterpret_cast<const uint4*>(s_bh + umma::offset(tid >> 1, 8 * (tid & 1) + i)));
+            band = band_for<kT5Threads / 32>(row.total(), s_top);
+        }
 
         // ---- fast rotation: y[token][j] = sum_k u[token][k] Pi[j][k], 24 MMAs from one thread ----
         if (tid == 0) {
@@ -190,9 +201,8 @@ __global__ void __launch_bounds__(kT5Threads, 1) tq_pool_append_t5_kernel(const 
                 const float ay = fabsf(y);
                 const int mag = (ay > b1 ? 1 : 0) + (ay > b2 ? 1 : 0) + (ay > b3 ? 1 : 0);
                 const uint32_t code = (uint32_t)(y > 0.f ? 4 + mag : 3 - mag);
-                const bool nr = ay <= kBand || fabsf(ay - b1) <= kBand || fabsf(ay - b2) <= kBand ||
-                                fabsf(ay - b3) <= kBand;
-                if (nr && row_ok) near[c] |= 1u << i;
+                const float gap = fminf(fminf(ay, fabsf(ay - b1)), fminf(fabsf(ay - b2), fabsf(ay - b3)));
+                if (!(gap > band) && row_ok) near[c] |= 1u << i;
                 if ((i & 3) == 0) packed[i >> 2] = code;
                 else packed[i >> 2] |= code << (8 * (i & 3));
             }

@@ -6,10 +6,8 @@
 // that chain, so the rotation is done twice over:
 //   1. fast: u and Pi are split into fp16 high and low parts (x = hi + lo, |lo| <= 2^-11 |hi|) and
 //      y ~ Pi_hi u_hi + Pi_hi u_lo + Pi_lo u_hi on m16n8k16 MMAs with fp32 accumulation. The result
-//      differs from the chain's value by far less than kBand (the dropped lo x lo term, the
-//      remainder of the two-part split, fp16 subnormal rounding of the low parts and the
-//      accumulation error of 24 MMAs sum to a few 1e-6 for |y| <= 1);
-//   2. exact: a coordinate whose fast value lies within kBand of a decision boundary (a few per
+//      differs from the chain's value by less than the band: kBand, widened where rows of Pi are longer than 1;
+//   2. exact: a coordinate whose fast value lies within the band around a decision boundary (one per
 //      thousand) is recomputed with the sequential chain from the fp32 unit vector kept in shared
 //      memory, and that value decides the code.
 // Every other coordinate is farther from all boundaries than the fast path's error, so its code is
@@ -27,10 +25,41 @@ constexpr int kTcThreads = 256;
 constexpr int kTcTokens = 64;
 constexpr int kPiStride = 136;            // halves per row (272 bytes): conflict-free 8 x 16-byte ldmatrix rows
 constexpr int kUStride = 136;             // floats per row of the unit-vector tile
-// Rows of Pi and unit vectors have norm 1, so sums over k of |Pi u| are at most 1: the chain's own rounding is at most
+// Where rows of Pi and unit vectors have norm 1, sums over k of |Pi u| are at most 1: the chain's own rounding is at most
 // 128 x 2^-24 = 7.6e-6, the fast value's (splits and fp16's subnormals 1.2e-6, the dropped lo x lo 2.4e-7, 24 accumulations
-// of two units in the last place each 5.7e-6) 7.2e-6.
+// of two units in the last place each 5.7e-6) 7.2e-6. All of these grow with the norm of a row of Pi, so the band does too:
+// band_for takes the squared norm of half a row's high parts from each thread (two neighbours share a row) and
+// returns kBand times the longest row's norm, at least kBand; infinite, and so every coordinate exact, where a sum of squares
+// is beyond fp16 (norms above 256 to 724, by how even the row is) or no number. s_top: a number a warp. It runs whenever Pi is staged: 12.1 -> 12.45 us for
+// 512 tokens of 8 heads, nothing where a CTA has several tiles (16 sequences of 2048 tokens: 329 -> 326).
 constexpr float kBand = 2.5e-5f;
+struct HalfRow {
+    __half2 sum[2] = {__floats2half2_rn(0.f, 0.f), __floats2half2_rn(0.f, 0.f)};
+    __device__ __forceinline__ void add(const uint4& w) {       // each sum is rounded sixteen times: 1 % at most
+        const __half2* h = reinterpret_cast<const __half2*>(&w);
+        sum[0] = __hfma2(h[0], h[0], sum[0]);
+        sum[1] = __hfma2(h[1], h[1], sum[1]);
+        sum[0] = __hfma2(h[2], h[2], sum[0]);
+        sum[1] = __hfma2(h[3], h[3], sum[1]);
+    }
+    __device__ __forceinline__ float total() const {
+        const float2 a = __half22float2(sum[0]), b = __half22float2(sum[1]);
+        return (a.x + a.y) + (b.x + b.y);
+    }
+};
+template <int kWarps>
+__device__ __forceinline__ float band_for(float half_row, float* s_top) {
+    const float row = half_row + __shfl_xor_sync(0xffffffffu, half_row, 1);
+    // bits of numbers that are not negative order as the numbers do, and a NaN above all of them
+    const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(row) & 0x7fffffffu);
+    if ((threadIdx.x & 31) == 0) s_top[threadIdx.x >> 5] = __uint_as_float(top);
+    __syncthreads();
+    unsigned all = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) all = max(all, __float_as_uint(s_top[w]));
+    const float norm = 1.01f * sqrtf(__uint_as_float(all));           // half of that 1 %, and the low parts' 2^-11
+    return norm < 1e30f ? kBand * fmaxf(norm, 1.f) : __int_as_float(0x7f800000);
+}
 constexpr int kCodeStride = 132;          // bytes per token row of the code tile: 4-byte reads of 8 tokens x 4 quarters hit 32 banks
 constexpr int kListCap = 64;              // queue of boundary-band coordinates: flushed whenever it holds a full warp's worth
 constexpr size_t kTcSmemBytes = 2 * (size_t)kDim * kPiStride * sizeof(__half) +
@@ -73,6 +102,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
     __shared__ float s_norm[kTcTokens];
     __shared__ uint16_t s_list[kTcThreads / 32][kListCap];      // per warp: (slot << 7 | coordinate) awaiting the exact chain
     __shared__ float s_bounds[8];
+    __shared__ float s_top[kTcThreads / 32];
 
     const AppendParams& p = tp.a;
     pdl_begin();
@@ -85,6 +115,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
     const long long tile_hi = ((long long)blockIdx.x + 1) * tp.n_tiles / gridDim.x;
     const long long per_which = (long long)p.B * p.H * tp.groups;
     int loaded_which = -1;
+    float band = 0.f;
     unsigned long long n_exact = 0, n_coords = 0;
 
     for (long long tile = tile_lo; tile < tile_hi; ++tile) {
@@ -96,7 +127,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
         const float* Pi = which == 0 ? p.Pi_k : p.Pi_v;
 
         __syncthreads();                 // the previous tile's readers of s_u / s_pi* are done
-        if (which != loaded_which) {
+        const bool staged = which != loaded_which;
+        if (staged) {
             for (int i = tid; i < kDim * kDim / 2; i += kTcThreads) {
                 const int j = i >> 6, k2 = (i & 63) * 2;
                 const float2 v = __ldg(reinterpret_cast<const float2*>(Pi + j * kDim + k2));
@@ -153,12 +185,19 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
                 dst[i] = make_float4(xr[4 * i] / denom, xr[4 * i + 1] / denom, xr[4 * i + 2] / denom, xr[4 * i + 3] / denom);
         }
         __syncthreads();
+        if (staged) {
+            const uint4* half = reinterpret_cast<const uint4*>(s_pih + (tid >> 1) * kPiStride + 64 * (tid & 1));
+            HalfRow row;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) row.add(half[i ^ (4 * (tid & 1))]);       // eight threads' reads in 32 banks
+            band = band_for<kTcThreads / 32>(row.total(), s_top);
+        }
 
         // ---- this warp's page ----
         const int page_ord = ord0 + pgw;
         const int first = max(pos0, page_ord * 16), last = min(pos_end, page_ord * 16 + 16);
         const int nt_valid = last - first;                    // tokens of this launch in the page
-        if (nt_valid <= 0) continue;                          // the same in both warps of the page; CTA-wide syncs are at the loop top
+        if (nt_valid <= 0) continue;                          // the same in both warps of the page; CTA-wide syncs are above
         const int slot0 = first - page_ord * 16;
         const int page = p.kv_page_indices[p.kv_indptr[b] + page_ord];
         const bool page_ok = page >= 0 && page < p.n_pages;
@@ -236,7 +275,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
                     const int mag = (ay > b1 ? 1 : 0) + (ay > b2 ? 1 : 0) + (ay > b3 ? 1 : 0);
                     code[c] = y > 0.f ? 4 + mag : 3 - mag;
                     const float gap = fminf(fminf(ay, fabsf(ay - b1)), fminf(fabsf(ay - b2), fabsf(ay - b3)));
-                    if (gap <= kBand && mine) near |= 1u << (4 * n + 2 * r + c);
+                    if (!(gap > band) && mine) near |= 1u << (4 * n + 2 * r + c);
                 }
                 *reinterpret_cast<uint16_t*>(&code_rows[slot * kCodeStride + 64 * side + n * 8 + 2 * t]) =
                     (uint16_t)(code[0] | (code[1] << 8));

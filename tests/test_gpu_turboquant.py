@@ -751,3 +751,43 @@ def test_prefill_attention_beyond_the_expanded_contexts_takes_strided_queries():
     assert torch.equal(cache.prefill_attention(0, q), want)
     one = cache.prefill_attention(0, q[:, :, 2:])
     assert rel_l2(one.cpu(), want[:, :, 2:].cpu()) < 1e-3
+
+
+@pytest.mark.parametrize("scale", [1.0, 100.0, 3000.0, 1e6])
+def test_append_with_longer_rows_of_the_rotation(scale):
+    """The band around the boundaries grows with the rows of Pi (somewhere above 256 every coordinate takes the exact chain; from
+    1e5 or so on the rows have no fp16 parts). One vector in twenty has 120 coordinates next to a boundary; the last holds a NaN."""
+    dev, H, T = _dev(), 2, 1000
+    rp = RawPool(T // 16 + 2, H, dev)
+    gen = torch.Generator().manual_seed(3)
+    edge = rp.bounds[4].item()
+    rp.bounds = rp.bounds * scale
+    given = []
+    for which, Pi in ((0, rp.Pi_k), (1, rp.Pi_v)):
+        x = torch.randn(H * T, 128, generator=gen)
+        on = torch.rand(H * T, generator=gen) < 0.05
+        y = edge * (1.0 - 2.0 * torch.randint(0, 2, (int(on.sum()), 128), generator=gen))
+        y[:, :8] = ((1 - 120 * edge ** 2) / 8) ** 0.5
+        x[on] = y @ Pi.cpu()
+        x[-1, 5] = float("nan")
+        given.append(x.half().reshape(1, H, T, 128))
+        Pi.mul_(scale)
+    rp.append(given[0].to(dev), given[1].to(dev), [0, T // 16 + 2], list(range(T // 16 + 2)), [3])
+    for which, Pi in ((0, rp.Pi_k), (1, rp.Pi_v)):
+        codes, norms, _, _ = tq_exact.quantize(given[which].float().numpy().reshape(-1, 128), Pi.cpu().numpy(), rp.bounds.cpu().numpy())
+        idx, got = rp.unpack(list(range(T // 16 + 2)), T + 3, which)
+        assert np.array_equal(pool_layout.nibbles_to_codes(idx[:, 3:]).reshape(-1, 128), codes)
+        assert np.array_equal(got[:, 3:].reshape(-1), torch.from_numpy(norms).half().float().numpy(), equal_nan=True)
+
+
+def test_append_on_the_other_tensor_cores_passes_the_same_checks():
+    import os
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    r = subprocess.run([sys.executable, "-m", "pytest", os.path.join(ROOT, "tests", "test_gpu_turboquant.py"), "-m", "gpu", "-x", "-q",
+                        "-k", "longer_rows"], env=dict(os.environ, LEANKV_TQ_APPEND="t5"), capture_output=True, text=True,
+                       timeout=600, cwd=ROOT)
+    assert r.returncode == 0 and "passed" in r.stdout, (r.stdout[-2000:], r.stderr[-1000:])
