@@ -329,6 +329,20 @@ def on_device(device):
     return torch.cuda.device(device)
 
 
+def grown_workspace(ws, need: int, device):
+    """A zeroed attention workspace of at least ``need`` bytes: ``ws`` itself where it is long enough, else a new one that
+    begins with the status word of ``ws``, so that a wait that ran out in an earlier chunk is still reported."""
+    import torch
+
+    if ws is not None and ws.numel() >= need:
+        return ws
+    new = torch.zeros(need, dtype=torch.uint8, device=device)
+    # not under capture: a replay would read memory that is gone by then
+    if ws is not None and not (ws.is_cuda and torch.cuda.is_current_stream_capturing()):
+        new[:4] = ws[:4]
+    return new
+
+
 def require_cuda(t, name: str) -> None:
     if not t.is_cuda:
         raise RuntimeError(

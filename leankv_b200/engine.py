@@ -536,8 +536,7 @@ class DecodeEngine(DecodeLoop):
             raise ValueError("the dense route handles whole prompts only")
         if attention == "packed":
             need = self.lib.leankv_tq_prefill_attn_workspace_bytes(T, start_pos, self.nq, self.nkv)
-            if self._prefill_ws is None or self._prefill_ws.numel() < need:
-                self._prefill_ws = torch.zeros(need, dtype=torch.uint8, device=self.dev)
+            self._prefill_ws = _native.grown_workspace(self._prefill_ws, need, self.dev)
             attn_out = torch.empty(T, self.nq, 128, dtype=torch.float16, device=self.dev)
         pos = torch.arange(start_pos, start_pos + T, device=self.dev).float()
         ang = torch.outer(pos, self.inv_freq)

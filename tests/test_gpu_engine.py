@@ -393,3 +393,24 @@ def test_prompt_pass_glue_kernels(T, n_q, n_kv, inter):
     finite = torch.isfinite(want)
     assert torch.equal(finite, torch.isfinite(gate))
     assert ((gate - want).double().abs() <= want.double().abs() * 2.0 ** -10 + 2.0 ** -24)[finite].all()
+
+
+def test_a_prompt_whose_first_chunk_failed_is_refused():
+    """The status word is read once, after the last chunk: a chunk that needs a longer workspace may not drop it."""
+    cfg = DecoderConfig(vocab_size=512, hidden_size=512, intermediate_size=1024, num_layers=1, num_q_heads=8, num_kv_heads=2)
+    eng = DecodeEngine.random_init(cfg, _dev(), seed=3, max_seq_len=3000)
+    eng.prefill(list(range(300)), chunk=100)
+    eng._prefill_ws = eng._prefill_ws[:1 << 16].clone()          # a short one, as behind a short prompt
+    forward, chunks = eng._dense_forward, []
+
+    def failing(ids, **kw):
+        out = forward(ids, **kw)
+        chunks.append(eng._prefill_ws)
+        if len(chunks) == 1:
+            eng._prefill_ws[:4].view(torch.int32).fill_(2)       # as if a page id had been outside the pool
+        return out
+
+    eng._dense_forward = failing
+    with pytest.raises(RuntimeError, match="status 2"):
+        eng.prefill([t % 512 for t in range(2900)], chunk=100)
+    assert len(chunks) == 29

@@ -791,3 +791,22 @@ def test_append_on_the_other_tensor_cores_passes_the_same_checks():
                         "-k", "longer_rows"], env=dict(os.environ, LEANKV_TQ_APPEND="t5"), capture_output=True, text=True,
                        timeout=600, cwd=ROOT)
     assert r.returncode == 0 and "passed" in r.stdout, (r.stdout[-2000:], r.stderr[-1000:])
+
+
+@pytest.mark.parametrize("call", ["prefill_attention", "decode_attention"])
+def test_a_failure_in_an_earlier_chunk_is_reported_after_the_workspace_grew(call):
+    dev = _dev()
+    cache = PagedKVCache(num_layers=1, num_kv_heads=2, num_q_heads=8, max_pages=4200, device=dev)
+    k = torch.randn(1, 2, 64000, 128, device=dev).half()
+    q = torch.randn(1, 8, 20, 128, device=dev).half()
+    name = {"prefill_attention": "_prefill_ws", "decode_attention": "_workspace"}[call]
+    attend = lambda: getattr(cache, call)(0, q if call == "prefill_attention" else q[:, :, 0])
+    for step, n in enumerate((40, 64000)):
+        cache.append(0, k[:, :, :n], k[:, :, :n])
+        attend()
+        if step == 0:
+            assert cache.kernel_status() == 0
+            before = getattr(cache, name)
+            before[:4].view(torch.int32).fill_(2)           # as if a page id had been outside the pool
+            setattr(cache, name, before[:len(before) // 2])      # too short for the next call
+    assert getattr(cache, name).numel() > len(before) // 2 and cache.kernel_status() == 2

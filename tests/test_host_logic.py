@@ -419,3 +419,12 @@ def test_a_wait_that_ran_out_while_quantizing_is_reported(monkeypatch, value):
     assert PagedKVCache(num_layers=1, num_kv_heads=1, num_q_heads=4, max_pages=4, device=dev).kernel_status() == value
     with pytest.raises(RuntimeError, match="codes are missing") if value else contextlib.nullcontext():
         DecodeEngine._check_quantize_status(SimpleNamespace(dev=dev))
+
+
+def test_a_longer_workspace_begins_with_the_status_of_the_one_it_replaces():
+    ws = _native.grown_workspace(None, 256, torch.device("cpu"))
+    assert ws.numel() == 256 and not ws.any()
+    ws[:4], ws[4:] = torch.tensor([2, 0, 0, 0], dtype=torch.uint8), 9
+    assert _native.grown_workspace(ws, 100, ws.device) is ws
+    new = _native.grown_workspace(ws, 257, ws.device)
+    assert new.numel() >= 257 and new[0] == 2 and not new[1:].any()
