@@ -428,3 +428,17 @@ def test_a_longer_workspace_begins_with_the_status_of_the_one_it_replaces():
     assert _native.grown_workspace(ws, 100, ws.device) is ws
     new = _native.grown_workspace(ws, 257, ws.device)
     assert new.numel() >= 257 and new[0] == 2 and not new[1:].any()
+
+
+def test_a_prompt_in_chunks_does_not_replace_its_workspace_at_each():
+    """512-token chunks of 65536 tokens, 8 kv heads: a handful of buffers, together a few times the last need."""
+    lib, dev = _native.lib(), torch.device("meta")
+    needs = [lib.leankv_tq_prefill_attn_workspace_bytes(512, start, 32, 8) for start in range(0, 65536, 512)]
+    ws, sizes = None, []
+    for need in needs:
+        new = _native.grown_workspace(ws, need, dev)
+        assert new.numel() >= need
+        if new is not ws:
+            ws = new
+            sizes.append(ws.numel())
+    assert len(sizes) <= 12 and sizes[-1] <= 1.5 * max(needs) + 256 and sum(sizes) <= 4.5 * max(needs)
