@@ -329,21 +329,24 @@ def on_device(device):
     return torch.cuda.device(device)
 
 
-def grown_workspace(ws, need: int, device):
-    """A zeroed attention workspace of at least ``need`` bytes: ``ws`` itself where it is long enough, else a new one that
-    begins with the status word of ``ws``, so that a wait that ran out in an earlier chunk is still reported. It is half as
-    long again at least: a prompt in chunks asks for a little more each time, and every exact size would be
-    allocated, cleared and left with the allocator (8 kv heads, 512-token chunks to 65536 tokens: 17 GB in 128 buffers)."""
+def grown_workspace(ws, need: int, device, cleared: bool = True):
+    """An attention workspace of at least ``need`` bytes: ``ws`` itself where it is long enough, else a new one that begins
+    with the status word of ``ws``, so that a wait that ran out in an earlier chunk is still reported. The rest is zero, or
+    with ``cleared=False`` (all that prompt attention asks for) anything. It is half as long again at least: a prompt in chunks
+    asks for a little more each time, and every exact size would be allocated and left with the allocator (8 kv heads,
+    512-token chunks to 65536 tokens: 17 GB in 128 buffers)."""
     import torch
 
     if ws is not None and ws.numel() >= need:
         return ws
     if ws is not None:
         need = max(need, ws.numel() * 3 // 2 // 256 * 256)
-    new = torch.zeros(need, dtype=torch.uint8, device=device)
+    new = (torch.zeros if cleared else torch.empty)(need, dtype=torch.uint8, device=device)
     # not under capture: a replay would read memory that is gone by then
     if ws is not None and not (ws.is_cuda and torch.cuda.is_current_stream_capturing()):
-        new[:4] = ws[:4]
+        new[:4].copy_(ws[:4])
+    elif not cleared:
+        new[:4].zero_()
     return new
 
 

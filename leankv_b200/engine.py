@@ -536,7 +536,7 @@ class DecodeEngine(DecodeLoop):
             raise ValueError("the dense route handles whole prompts only")
         if attention == "packed":
             need = self.lib.leankv_tq_prefill_attn_workspace_bytes(T, start_pos, self.nq, self.nkv)
-            self._prefill_ws = _native.grown_workspace(self._prefill_ws, need, self.dev)
+            self._prefill_ws = _native.grown_workspace(self._prefill_ws, need, self.dev, cleared=False)
             attn_out = torch.empty(T, self.nq, 128, dtype=torch.float16, device=self.dev)
         pos = torch.arange(start_pos, start_pos + T, device=self.dev).float()
         ang = torch.outer(pos, self.inv_freq)

@@ -289,7 +289,7 @@ class PagedKVCache:
                 if start < 0:
                     raise RuntimeError("prefill_attention: the chunk has not been appended to this sequence")
                 need = lib.leankv_tq_prefill_attn_workspace_bytes(t_new, start, self.num_q_heads, self.num_kv_heads)
-                self._prefill_ws = _native.grown_workspace(self._prefill_ws, need, self._device)
+                self._prefill_ws = _native.grown_workspace(self._prefill_ws, need, self._device, cleared=False)
                 q = query[b]                                                         # [Hq, T, D]
                 if not _whole_pieces(q):
                     q = q.to(torch.float16, copy=True, memory_format=torch.contiguous_format)

@@ -428,6 +428,9 @@ def test_a_longer_workspace_begins_with_the_status_of_the_one_it_replaces():
     assert _native.grown_workspace(ws, 100, ws.device) is ws
     new = _native.grown_workspace(ws, 257, ws.device)
     assert new.numel() >= 257 and new[0] == 2 and not new[1:].any()
+    for old, word in ((None, 0), (ws, 2)):              # prompt attention needs no more than the word
+        new = _native.grown_workspace(old, 300, ws.device, cleared=False)
+        assert new.numel() >= 300 and new[0] == word and not new[1:4].any()
 
 
 def test_a_prompt_in_chunks_does_not_replace_its_workspace_at_each():
