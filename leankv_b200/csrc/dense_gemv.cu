@@ -348,18 +348,20 @@ int launch_gemv_as(const GemvParams& p, int warps, cudaStream_t st) {
 }
 
 // Which of the two kernels: by the rounds of 4 KB a warp that an SM's share of the weights takes, and by the warps that
-// fit beside one another (CTAs of `warps` warps, at most eight). Weights from HBM, us with kAhead and early weights /
-// without kAhead: bf16 32768 x 2048 (14 rounds) 24.4 / 22.4, 65536 x 2048 (28) 47.3 / 42.5, 32768 x 1024 (7) 13.1 / 13.8,
-// 5632 x 2048 gated (5) 10.2 / 10.6, 4096 x 1024 (1) 3.4 / 5.2; eleven warps, bf16 2048 x 5632 (3.5) 7.0 / 6.3; eight warps,
-// fp32 16384 x 128 (1.8) 5.6 / 5.2, bf16 16384 x 128 (0.9) 4.1 / 4.9.
+// fit beside one another (CTAs of `warps` warps, at most eight). Weights from HBM, launches of one size one after another, us
+// with kAhead / without: bf16 32768 x 2048 (14 rounds) 25.2 / 22.4, 65536 x 2048 (28) 47.9 / 42.5, 32768 x 1024 (7) 13.6 /
+// 13.8, 4096 x 1024 (1) 3.8 / 5.2; eleven warps, bf16 2048 x 5632 (3.5) 7.4 / 6.3; eight warps, fp32 16384 x 128 (1.8) 5.9 / 5.2,
+// bf16 16384 x 128 (0.9) 4.6 / 4.9. With early weights a long range stays with kAhead: behind the other launches of a decode
+// step its first rows are there when these end, and a 32768 x 2048 head that starts as they drain cost the step 0.6 us more.
 template <typename T, int CH, Input IN>
 int launch_gemv(const GemvParams& p, int warps, cudaStream_t st) {
     const int resident = std::min(std::max(1, kMaxWarps / warps), 8) * warps;
     const double bytes = (double)p.a.rows * (p.a.gated ? 2 : 1) * p.a.cols * sizeof(T);
     const double rounds = bytes / sm_count() / (4096.0 * resident);
     const bool thin = resident < (sizeof(T) == 2 ? 12 : 9);
-    return rounds >= 10.0 || (thin && rounds > 1.5) ? launch_gemv_as<T, CH, IN, false>(p, warps, st)
-                                                    : launch_gemv_as<T, CH, IN, true>(p, warps, st);
+    const bool deep = rounds >= 10.0 && !p.a.early_weights;
+    return deep || (thin && rounds > 1.5) ? launch_gemv_as<T, CH, IN, false>(p, warps, st)
+                                          : launch_gemv_as<T, CH, IN, true>(p, warps, st);
 }
 
 }  // namespace
