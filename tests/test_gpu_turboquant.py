@@ -681,8 +681,8 @@ def test_prefill_attention_that_walks_the_pages_passes_the_same_checks():
     r = subprocess.run([sys.executable, "-m", "pytest", os.path.join(ROOT, "tests", "test_gpu_turboquant.py"), "-m", "gpu", "-x", "-q",
                         "-k", "prefill_attention_on_packed or prefill_attention_of_a_late or prefill_attention_at_the_edges"],
                        env=env, capture_output=True, text=True, timeout=600, cwd=ROOT)
-    assert r.returncode == 0, (r.stdout[-2000:], r.stderr[-1000:])
-    assert "10 passed" in r.stdout
+    assert r.returncode == 0, (r.stdout[-2000:], r.stderr[-1000:])      # 5 where nothing was selected
+    assert "passed" in r.stdout and "skipped" not in r.stdout
 
 
 @pytest.mark.parametrize("batch", [1, 2, 33, 64])
@@ -810,3 +810,41 @@ def test_a_failure_in_an_earlier_chunk_is_reported_after_the_workspace_grew(call
             before[:4].view(torch.int32).fill_(2)           # as if a page id had been outside the pool
             setattr(cache, name, before[:len(before) // 2])      # too short for the next call
     assert getattr(cache, name).numel() > len(before) // 2 and cache.kernel_status() == 2
+
+
+def test_early_launches_captured_behind_fills_copies_and_other_streams():
+    """Kernels that may start while the launch ahead drains, in a graph where a fill, a copy or another stream's kernel is
+    ahead of them: the pages and outputs of the same calls made one by one."""
+    dev, gen = _dev(), torch.Generator().manual_seed(5)
+    given = [torch.randn(2, 2, t, 128, generator=gen).half().to(dev) for t in (70, 3, 1, 33)]
+    q = torch.randn(2, 8, 128, generator=gen).half().to(dev)
+    side = torch.cuda.Stream()
+
+    def calls(cache):
+        kept = []
+        for layer, src in enumerate(given):
+            k = torch.empty_like(src)
+            k.zero_()
+            k.copy_(src)
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                kept.append((k, src * 2))
+            if layer % 2:
+                torch.cuda.current_stream().wait_stream(side)
+            cache.append(layer, k, k)
+            torch.cuda.current_stream().wait_stream(side)
+        return kept, cache.decode_attention(0, q), cache.prefill_attention(0, q.unsqueeze(2))
+
+    caches = [PagedKVCache(num_layers=4, num_kv_heads=2, num_q_heads=8, max_pages=64, device=dev) for _ in range(2)]
+    for cache in caches:
+        cache._ensure_batch_size(2)
+        cache._workspace, cache._prefill_ws = (torch.zeros(1 << 21, dtype=torch.uint8, device=dev) for _ in range(2))
+    want = calls(caches[0])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = calls(caches[1])
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(caches[0].kv_data, caches[1].kv_data) and caches[1].kernel_status() == 0
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
