@@ -28,8 +28,8 @@ int sm_count();
 // Whether launches carry the programmatic-stream-serialization attribute (default on; the
 // environment variable LEANKV_PDL=0 turns it off).
 bool pdl_enabled();
-// LEANKV_PDL: 0 = never, 1 = every kernel may start early, 2 (default) = only the bandwidth-bound
-// GEMV kernels may (their ramp-up is what is worth hiding; small latency-bound kernels run best alone).
+// LEANKV_PDL: 0 = never, 1 = every kernel may start early, 2 (default) = those whose launch says so: kernels that read
+// constants ahead of the dependency wait (GEMVs, decode attention, the post kernel) and those of launch_early.
 int pdl_mode();
 
 // Launch `kernel` on `st`, allowing it to overlap its start-up with the tail of the previous

@@ -487,8 +487,11 @@ static int prefill_mode() {
     return v;
 }
 
-// The expansion is scratch that grows with the context (17 MB per 4096 tokens and 8 kv heads); beyond this many tokens the
-// page-walking kernel, whose scratch does not, takes the call.
+// The expansion is scratch that grows with the context (17 MB per 4096 tokens and 8 kv heads, 272 MB at this line); beyond it
+// the page-walking kernel, whose scratch does not, takes the call. The line is a choice of memory, not of time: at 65 536 tokens and
+// 8 kv heads 1 / 16 / 512 / 2048 queries take 161 / 173 / 754 / 3028 us on expanded tiles and 396 / 411 / 1598 / 6296 on pages (its
+// scratch for that many queries: 0.1 / 2.3 / 73 / 292 MB). From 64 tokens of context up no count of queries is slower on
+// tiles (64 tokens, one query: 13.0 / 22.2).
 constexpr long long kExpandMaxTokens = 65536;
 struct ExpandPlan {
     int q_tiles, k_tiles, n_splits;

@@ -6,7 +6,7 @@
 // looked up once: tq_expand_kernel writes the centroids of 128 tokens at a time (fp16, as they are: norms stay
 // apart) in the very layout the tensor cores read, keys [token][coordinate] and values [coordinate][token], so that
 // the attention kernel fetches a tile with one bulk copy. The expansion is scratch of one layer's call, 520 bytes a token
-// and kv head; it is written and read through L2 (4096 tokens, 8 heads: 17 MB, 4 us).
+// and kv head; it is written and read through L2 (4096 tokens, 8 heads: 17 MB, 8 us with cold caches).
 //
 // tq_prefill_tile_kernel: a CTA takes 32 query tokens of one kv head = 128 rows (token, GQA head) and a range of
 // 128-key tiles. Both rotations are part of it:

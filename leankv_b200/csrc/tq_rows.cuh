@@ -27,7 +27,7 @@
 //
 // 65 544 vectors, fp16 in, fp32 out: quantize 155.5 -> 28.9 us (4.7 us for every 148 tiles, 10 us before the first result:
 // staging and the first vectors' norms), de-quantize 77.4 -> 44.8 us (0.73 of the multiply-add rate). 16 vectors: 50.2 ->
-// 12.8 and 22.0 -> 10.1 us. fp32 in, 65 544: 159.4 -> 40.7 us.
+// 13.0 and 22.0 -> 10.1 us. fp32 in, 65 544: 159.4 -> 40.9 us.
 
 constexpr int kRowsTile = umma::kRows;                       // vectors of a tile
 constexpr int kRowsIn = 256, kRowsOut = 256;                 // threads of the two roles; then the issuing warp
