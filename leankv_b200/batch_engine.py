@@ -198,7 +198,6 @@ class BatchDecodeEngine(DecodeEngine):
                 last.append(x)
             if attention == "packed":
                 self._check_prefill_status()
-            self._check_quantize_status()
             logits = torch.stack(last) @ self.w["lm_head_t"]
             tok = torch.argmax(logits.float(), dim=-1)
             self.tokens.copy_(tok)

@@ -536,7 +536,8 @@ class DecodeEngine(DecodeLoop):
             raise ValueError("the dense route handles whole prompts only")
         if attention == "packed":
             need = self.lib.leankv_tq_prefill_attn_workspace_bytes(T, start_pos, self.nq, self.nkv)
-            self._prefill_ws = _native.grown_workspace(self._prefill_ws, need, self.dev, cleared=False)
+            if self._prefill_ws is None or self._prefill_ws.numel() < need:
+                self._prefill_ws = _native.grown_workspace(self._prefill_ws, need, self.dev, cleared=False)
             attn_out = torch.empty(T, self.nq, 128, dtype=torch.float16, device=self.dev)
         pos = torch.arange(start_pos, start_pos + T, device=self.dev).float()
         ang = torch.outer(pos, self.inv_freq)
@@ -728,7 +729,6 @@ class DecodeEngine(DecodeLoop):
                                         attention=attention)
             if attention == "packed":
                 self._check_prefill_status()
-            self._check_quantize_status()
             logits = x @ self.w["lm_head_t"]
             tok = torch.argmax(logits.float()).reshape(1)
             self.token.copy_(tok)

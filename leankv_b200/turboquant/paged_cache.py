@@ -261,7 +261,8 @@ class PagedKVCache:
         with _native.on_device(self._device):
             need = lib.leankv_tq_decode_attn_workspace_bytes(batch, self.num_q_heads, self.num_kv_heads,
                                                              max_pages_seq)
-            self._workspace = _native.grown_workspace(self._workspace, max(need, 1 << 20), self._device)
+            if self._workspace is None or self._workspace.numel() < need:
+                self._workspace = _native.grown_workspace(self._workspace, max(need, 1 << 20), self._device)
             kq, vq = self.key_quantizers[layer_idx], self.val_quantizers[layer_idx]
             rc = lib.leankv_tq_decode_attn(
                 q.data_ptr(), out.data_ptr(), batch, self.num_q_heads, self.num_kv_heads,
@@ -289,7 +290,8 @@ class PagedKVCache:
                 if start < 0:
                     raise RuntimeError("prefill_attention: the chunk has not been appended to this sequence")
                 need = lib.leankv_tq_prefill_attn_workspace_bytes(t_new, start, self.num_q_heads, self.num_kv_heads)
-                self._prefill_ws = _native.grown_workspace(self._prefill_ws, need, self._device, cleared=False)
+                if self._prefill_ws is None or self._prefill_ws.numel() < need:
+                    self._prefill_ws = _native.grown_workspace(self._prefill_ws, need, self._device, cleared=False)
                 q = query[b]                                                         # [Hq, T, D]
                 if not _whole_pieces(q):
                     q = q.to(torch.float16, copy=True, memory_format=torch.contiguous_format)
