@@ -340,15 +340,14 @@ __global__ void __launch_bounds__(kThreads, kSwiglu ? 3 : 4) sparse_gemv_kernel(
         float* mine = p.partials + ((size_t)blockIdx.y * kArrays) * npad + col;
         mine[0] = sum;
         if (kSwiglu) mine[npad] = sum2;
-        __threadfence();
         __syncthreads();
         if (tid == 0) {
-            const int prev = atomicAdd(&p.counters[slice], 1);
+            int prev;
+            asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(prev) : "l"(p.counters + slice) : "memory");
             s_last = (prev == p.k_splits - 1);
         }
         __syncthreads();
         if (!s_last) return;
-        __threadfence();
         // Final merge, spread over the whole CTA so that it costs a couple of L2 round trips
         // instead of k_splits: warp w sums splits w, w+8, ... (ascending) for all 256 columns,
         // then the 8 warp sums are added in warp order. The order is fixed, so the result is too.
