@@ -8,9 +8,14 @@
 // memory, and its 8 warps stream the listed weight rows round-robin, 8 independent
 // 16-byte loads in flight per lane. Split-K partials go to a workspace; the last CTA to
 // arrive for a column slice sums them in split order, so the result does not depend on
-// arrival order and no floating-point atomics are used.
+// arrival order and no floating-point atomics are used. The sums are handed over by one acq_rel atomic behind a
+// CTA barrier: with a __threadfence by every thread on both sides, as it was, a layer's four launches took 2.5 us
+// more (7B shape; 4096 x 14336 at 40 % 14.4 instead of 14.1).
 //
-// The same kernel also serves: per-segment thresholds (fused q/k/v), bias, residual add, the fused
+// Small matrices go through sparse_gemv_cluster_kernel, where the splits of a slice are one thread-block cluster and
+// meet in distributed shared memory (see there).
+//
+// The first kernel also serves: per-segment thresholds (fused q/k/v), bias, residual add, the fused
 // gate/up SwiGLU (template flag), RMSNorm of the input row fused into the prologue, and the
 // tensor-parallel form in which the finishing CTA sums the ranks' partial products over peer
 // memory before it writes y.
@@ -18,6 +23,8 @@
 // Arithmetic follows the reference's B=1 path (leankv/teal/kernels/sparse_gemv.py:71-87:
 // fp16 operands widened to fp32, fp32 sums) and the mask of leankv/teal/sparse_fns.py:36
 // (strict '>' against the threshold rounded to fp16).
+
+#include <algorithm>
 
 #include "common.cuh"
 
@@ -32,6 +39,7 @@ constexpr int kMaxRowsPerSplit = kWarps * 32 * kLaneSlots;  // 1024
 constexpr int kMaxSplits = 128;
 constexpr int kMaxSplitsNarrow = 40;   // = kWarps x the merge's load batch: the last CTA sums a slice in one round trip
 constexpr int kCtasPerSm = 4;
+constexpr int kClusterCtas = 8;        // of a column slice, in the cluster kernel
 constexpr size_t kCounterAreaBytes = 16384;   // counters of up to 4096 column slices (N <= 1 048 576)
 
 struct GemvParams {
@@ -81,7 +89,7 @@ struct GemvPlan {
 // How many weight rows of its range a CTA asks into L2 ahead of the dependency wait: LEANKV_GEMV_PREFETCH_KB
 // kilobytes per CTA (default 32; 0 = off), at most LEANKV_GEMV_PREFETCH_PCT per cent of the range (default 25).
 // Measured on the Mistral-7B-shape decode step: off 427.2 tok/s, 16 KB 435.5, 32 KB 437.6 (25 %: 438.1), 48 KB 434.0.
-static int prefetch_rows(int rows_per_split, int arrays) {
+static int prefetch_rows(int rows_per_split, int arrays, int cols) {
     static int kb = -1, pct = -1;
     if (kb < 0) {
         const char* e = std::getenv("LEANKV_GEMV_PREFETCH_KB");
@@ -89,9 +97,9 @@ static int prefetch_rows(int rows_per_split, int arrays) {
         const char* f = std::getenv("LEANKV_GEMV_PREFETCH_PCT");
         pct = f != nullptr ? std::max(0, std::min(100, std::atoi(f))) : 25;
     }
-    const int by_bytes = kb * 1024 / (kColsPerCta * 2 * arrays);
+    const int by_bytes = kb * 1024 / (cols * 2 * arrays);
     const int by_share = (int)((long long)rows_per_split * pct / 100);
-    return std::min(std::min(by_bytes, by_share), kThreads / arrays);
+    return std::min(by_bytes, by_share);
 }
 
 GemvPlan make_plan(int N, int Z, int arrays) {
@@ -131,6 +139,69 @@ __device__ __forceinline__ void fma8(float (&acc)[8], const uint4& w, float xv) 
     acc[5] = fmaf(c.y, xv, acc[5]);
     acc[6] = fmaf(d.x, xv, acc[6]);
     acc[7] = fmaf(d.y, xv, acc[7]);
+}
+
+template <bool kSwiglu>
+__device__ __forceinline__ void finish_column(const GemvParams& p, int col, float sum, float sum2) {
+    if (kSwiglu) {
+        // Rounding points of the two-GEMV + act_fn(gate)*up path: fp16 gate, fp16 up,
+        // silu evaluated in fp32 and rounded, fp16 product.
+        const __half g16 = __float2half_rn(sum);
+        const __half u16 = __float2half_rn(sum2);
+        const float gf = __half2float(g16);
+        const __half s16 = __float2half_rn(gf / (1.0f + expf(-gf)));
+        p.y[col] = __hmul(s16, u16);
+    } else {
+        __half r = __float2half_rn(sum);
+        if (p.bias != nullptr) r = __hadd(r, p.bias[col]);
+        if (p.residual != nullptr) r = __hadd(p.residual[col], r);
+        p.y[col] = r;
+    }
+}
+
+__device__ float sum_over_ranks(const GemvParams& p, int col, int npad, float sum) {
+    // Sum of the ranks' partial products, inside this kernel: every thread of the CTA that holds
+    // a finished 256-column tile sends its column's fp32 value, tagged with the step's epoch, to
+    // every rank's receive area (one 64-bit store each, NVLink for the peers), then polls its
+    // column's words here until each carries this epoch, and adds them in rank order, so every
+    // rank ends up with the same bits. Epochs only grow, so nothing is ever reset. A poll that
+    // runs out sets the status word, which also turns all later polls off (the result is then
+    // meaningless, but no kernel hangs).
+    const unsigned int ep = (unsigned int)*reinterpret_cast<const volatile int*>(p.xepoch);
+    const unsigned long long word = ((unsigned long long)ep << 32) | (unsigned long long)__float_as_uint(sum);
+    // every rank starts with a different destination so that the ranks' stores do not all converge on
+    // one GPU's links at the same moment
+    for (int i = 0; i < p.xw; ++i) {
+        int r = p.xrank + i;
+        r = r >= p.xw ? r - p.xw : r;
+        st_relaxed_sys_u64(p.xrecv[r] + (size_t)p.xrank * npad + col, word);
+    }
+    const bool live = *reinterpret_cast<volatile int*>(p.xstatus) == 0;
+    // first look at every source at once (independent loads), then poll whatever is still missing
+    unsigned long long v[LEANKV_MAX_RANKS];
+    const unsigned long long* src0 = p.xrecv[p.xrank] + col;
+#pragma unroll
+    for (int r = 0; r < LEANKV_MAX_RANKS; ++r)
+        v[r] = r < p.xw ? ld_relaxed_sys_u64(src0 + (size_t)r * npad) : 0ull;
+    float tot = 0.f;
+    bool ok = live;
+#pragma unroll
+    for (int r = 0; r < LEANKV_MAX_RANKS; ++r) {
+        if (r < p.xw) {
+            if (live) {
+                int it = 0;
+                while ((unsigned int)(v[r] >> 32) != ep && it < p.xlimit) {
+                    __nanosleep(20);
+                    v[r] = ld_relaxed_sys_u64(src0 + (size_t)r * npad);
+                    ++it;
+                }
+                ok = ok && (unsigned int)(v[r] >> 32) == ep;
+            }
+            tot += __uint_as_float((unsigned int)v[r]);
+        }
+    }
+    if (!ok && live) atomicOr(p.xstatus, 1);
+    return tot;
 }
 
 template <bool kSwiglu>
@@ -405,66 +476,266 @@ __global__ void __launch_bounds__(kThreads, kSwiglu ? 3 : 4) sparse_gemv_kernel(
         if (tid == 0) p.counters[slice] = 0;   // leave the workspace ready for the next launch
     }
 
-    if (!kSwiglu && p.xw > 0) {
-        // Sum of the ranks' partial products, inside this kernel: every thread of the CTA that holds
-        // a finished 256-column tile sends its column's fp32 value, tagged with the step's epoch, to
-        // every rank's receive area (one 64-bit store each, NVLink for the peers), then polls its
-        // column's words here until each carries this epoch, and adds them in rank order, so every
-        // rank ends up with the same bits. Epochs only grow, so nothing is ever reset. A poll that
-        // runs out sets the status word, which also turns all later polls off (the result is then
-        // meaningless, but no kernel hangs).
-        const unsigned int ep = (unsigned int)*reinterpret_cast<const volatile int*>(p.xepoch);
-        const unsigned long long word = ((unsigned long long)ep << 32) | (unsigned long long)__float_as_uint(sum);
-        // every rank starts with a different destination so that the ranks' stores do not all converge on
-        // one GPU's links at the same moment
-        for (int i = 0; i < p.xw; ++i) {
-            int r = p.xrank + i;
-            r = r >= p.xw ? r - p.xw : r;
-            st_relaxed_sys_u64(p.xrecv[r] + (size_t)p.xrank * npad + col, word);
+    if (!kSwiglu && p.xw > 0) sum = sum_over_ranks(p, col, npad, sum);
+    if (col < p.N) finish_column<kSwiglu>(p, col, sum, sum2);
+}
+
+// One thread-block cluster a column slice: its CTAs take a share of the input channels each, and the split sums meet in the
+// first CTA's shared memory, added in rank order.
+//
+// What bounds a small matrix is the chain of one launch, and most of it was the merge through the workspace: store, arrive
+// at an atomic, read back, a trip to L2 each. Here it is one store into a neighbour and a cluster barrier. Weights from HBM, 40 % of
+// the channels off, launches one behind the other, us through the workspace / here: 512 x 512 4.1 / 3.0, 1024 x 4096 5.7 / 4.6,
+// 2048 x 4096 7.1 / 5.2, 4096 x 4096 8.0 / 7.0; gate and up together 1792 x 4096 8.8 / 6.0, 3584 x 1024 6.7 / 4.5,
+// 4096 x 4096 10.7 / 9.2. A slice of 64 or 128 columns keeps a cluster to the eight CTAs that every device places.
+template <bool kSwiglu, int kCols, int kT>
+__global__ void __launch_bounds__(kT, kT == 512 ? 2 : kSwiglu ? 3 : 4) sparse_gemv_cluster_kernel(const __grid_constant__ GemvParams p) {
+    constexpr int kArrays = kSwiglu ? 2 : 1, kNumWarps = kT / 32;
+    constexpr int kUnroll = kSwiglu ? (kT == 512 ? 3 : 4) : 8;
+    constexpr int kLanes = kCols / 8;              // lanes on a row, 16 bytes each
+    constexpr int kGroups = 32 / kLanes;           // rows a warp reads at once
+    constexpr int kStep = kNumWarps * kGroups;
+    constexpr int kChunkRows = kSwiglu ? 1024 : 2048;       // input channels listed at a time
+    constexpr int kSlots = kChunkRows / kT;
+
+    __shared__ uint16_t s_row[kChunkRows];
+    __shared__ float s_x[kChunkRows];
+    __shared__ float s_x2[kSwiglu ? kChunkRows : 1];
+    __shared__ __align__(16) float s_red[kNumWarps][kArrays][kCols];
+    __shared__ float s_part[kClusterCtas][kArrays][kCols];      // first CTA: the sums of every CTA
+    __shared__ float s_ss[kNumWarps];
+    __shared__ int s_wcount[kNumWarps];
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int slice = blockIdx.x, rank = blockIdx.y;
+    const int z0 = rank * p.rows_per_split, z1 = min(p.Z, z0 + p.rows_per_split);
+    if (p.k_splits > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    if (p.prefetch_rows > 0) {                     // the first rows into L2 ahead of the dependency wait, as above
+        constexpr int kLines = kCols / 64;
+        const int nr = min(p.prefetch_rows, z1 - z0);
+        for (int t = tid; t < nr * kArrays * kLines; t += kT) {
+            const int line = t % kLines, r = t / kLines / kArrays, col = slice * kCols + line * 64;
+            const __half* base = kSwiglu && (t / kLines & 1) ? p.Wt2 : p.Wt;
+            if (col < p.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(base + (size_t)(z0 + r) * p.N + col));
         }
-        const bool live = *reinterpret_cast<volatile int*>(p.xstatus) == 0;
-        // first look at every source at once (independent loads), then poll whatever is still missing
-        unsigned long long v[LEANKV_MAX_RANKS];
-        const unsigned long long* src0 = p.xrecv[p.xrank] + col;
+    }
+    pdl_begin();
+
+    float thr = p.thr[0];
+    if (!kSwiglu) {
+        int s = 0;
+        while (s + 1 < p.n_segments && slice * kCols >= p.seg_end[s]) ++s;
+        thr = p.thr[s];
+    }
+    const __half thr_h = __float2half_rn(thr), thr2_h = __float2half_rn(kSwiglu ? p.thr_up : thr);
+
+    const int col0 = slice * kCols + (lane % kLanes) * 8, group = lane / kLanes;
+    const bool col_ok = col0 < p.N;                // N % 8 == 0: a lane's 8 columns are all in or all out
+    const size_t ldw = (size_t)p.N;
+    float acc[8], acc2[8];
 #pragma unroll
-        for (int r = 0; r < LEANKV_MAX_RANKS; ++r)
-            v[r] = r < p.xw ? ld_relaxed_sys_u64(src0 + (size_t)r * npad) : 0ull;
-        float tot = 0.f;
-        bool ok = live;
+    for (int j = 0; j < 8; ++j) acc[j] = acc2[j] = 0.f;
+    float rnorm = 0.f;
+    int counted = 0;
+    for (int c0 = z0; c0 < z1; c0 += kChunkRows) {
+        const int nrows = min(kChunkRows, z1 - c0);
+        const int per_warp = (nrows + kNumWarps - 1) / kNumWarps, w0 = warp * per_warp, w1 = min(nrows, w0 + per_warp);
+        __half x[kSlots], nw[kSlots];
 #pragma unroll
-        for (int r = 0; r < LEANKV_MAX_RANKS; ++r) {
-            if (r < p.xw) {
-                if (live) {
-                    int it = 0;
-                    while ((unsigned int)(v[r] >> 32) != ep && it < p.xlimit) {
-                        __nanosleep(20);
-                        v[r] = ld_relaxed_sys_u64(src0 + (size_t)r * npad);
-                        ++it;
-                    }
-                    ok = ok && (unsigned int)(v[r] >> 32) == ep;
-                }
-                tot += __uint_as_float((unsigned int)v[r]);
+        for (int s = 0; s < kSlots; ++s) {
+            const int r = w0 + s * 32 + lane;
+            x[s] = nw[s] = __float2half_rn(0.f);
+            if (r < w1) {
+                x[s] = p.x[c0 + r];
+                if (p.norm_w != nullptr) nw[s] = p.norm_w[c0 + r];
             }
         }
-        if (!ok && live) atomicOr(p.xstatus, 1);
-        sum = tot;
-    }
+        if (c0 != z0) {
+            __syncthreads();                       // the list of the last rows has been read
+        } else if (p.norm_w != nullptr) {          // RMSNorm of the whole row, in every CTA the same sum
+            float ss = 0.f;
+            const uint4* hv = reinterpret_cast<const uint4*>(p.x);
+#pragma unroll 4
+            for (int i = tid; i < (p.Z >> 3); i += kT) {
+                const uint4 a = hv[i];
+                const float2 f0 = h2_to_f2(a.x), f1 = h2_to_f2(a.y), f2 = h2_to_f2(a.z), f3 = h2_to_f2(a.w);
+                ss = fmaf(f0.x, f0.x, ss); ss = fmaf(f0.y, f0.y, ss);
+                ss = fmaf(f1.x, f1.x, ss); ss = fmaf(f1.y, f1.y, ss);
+                ss = fmaf(f2.x, f2.x, ss); ss = fmaf(f2.y, f2.y, ss);
+                ss = fmaf(f3.x, f3.x, ss); ss = fmaf(f3.y, f3.y, ss);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (lane == 0) s_ss[warp] = ss;
+            __syncthreads();
+            float tot = 0.f;
+#pragma unroll
+            for (int w = 0; w < kNumWarps; ++w) tot += s_ss[w];
+            rnorm = rsqrtf(tot / (float)p.Z + p.norm_eps);
+        }
+        // ---- threshold test + ordered compaction ----
+        unsigned live = 0;
+        int wtotal = 0;
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s) {
+            if (s * 32 >= per_warp) break;
+            const int r = w0 + s * 32 + lane;
+            if (p.norm_w != nullptr) x[s] = __hmul(nw[s], __float2half_rn(__half2float(x[s]) * rnorm));
+            const __half m = __habs(x[s]);
+            const bool a = r < w1 && (__hgt(m, thr_h) || (kSwiglu && __hgt(m, thr2_h)));
+            live |= (unsigned)a << s;
+            wtotal += __popc(__ballot_sync(0xffffffffu, a));
+        }
+        if (lane == 0) s_wcount[warp] = wtotal;
+        __syncthreads();
+        int at = 0, total = 0;
+#pragma unroll
+        for (int w = 0; w < kNumWarps; ++w) {
+            const int c = s_wcount[w];
+            if (w < warp) at += c;
+            total += c;
+        }
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s) {
+            if (s * 32 >= per_warp) break;
+            const bool a = (live >> s) & 1;
+            const unsigned b = __ballot_sync(0xffffffffu, a);
+            if (a) {
+                const int e = at + __popc(b & ((1u << lane) - 1u));
+                const __half m = __habs(x[s]);
+                const float f = __half2float(x[s]);
+                s_row[e] = (uint16_t)(w0 + s * 32 + lane);
+                s_x[e] = !kSwiglu || __hgt(m, thr_h) ? f : 0.f;
+                if (kSwiglu) s_x2[e] = __hgt(m, thr2_h) ? f : 0.f;
+            }
+            at += __popc(b);
+        }
+        counted += total;
+        __syncthreads();
 
-    if (col >= p.N) return;
-    if (kSwiglu) {
-        // Rounding points of the two-GEMV + act_fn(gate)*up path: fp16 gate, fp16 up,
-        // silu evaluated in fp32 and rounded, fp16 product.
-        const __half g16 = __float2half_rn(sum);
-        const __half u16 = __float2half_rn(sum2);
-        const float gf = __half2float(g16);
-        const __half s16 = __float2half_rn(gf / (1.0f + expf(-gf)));
-        p.y[col] = __hmul(s16, u16);
-    } else {
-        __half r = __float2half_rn(sum);
-        if (p.bias != nullptr) r = __hadd(r, p.bias[col]);
-        if (p.residual != nullptr) r = __hadd(p.residual[col], r);
-        p.y[col] = r;
+        // ---- stream the active weight rows ----
+        if (col_ok) {
+            const __half* wbase = p.Wt + (size_t)c0 * ldw + col0;
+            const __half* wbase2 = kSwiglu ? p.Wt2 + (size_t)c0 * ldw + col0 : nullptr;
+            for (int e0 = warp * kGroups + group; e0 < total; e0 += kStep * kUnroll) {
+                uint4 w[kUnroll], w2[kSwiglu ? kUnroll : 1];
+                float xs[kUnroll], xs2[kSwiglu ? kUnroll : 1];
+#pragma unroll
+                for (int u = 0; u < kUnroll; ++u) {
+                    const int e = e0 + u * kStep;
+                    w[u] = make_uint4(0, 0, 0, 0);
+                    xs[u] = 0.f;
+                    if (kSwiglu) {
+                        w2[u] = make_uint4(0, 0, 0, 0);
+                        xs2[u] = 0.f;
+                    }
+                    if (e < total) {
+                        const size_t off = (size_t)s_row[e] * ldw;
+                        w[u] = ld_stream_16(wbase + off);
+                        xs[u] = s_x[e];
+                        if (kSwiglu) {
+                            w2[u] = ld_stream_16(wbase2 + off);
+                            xs2[u] = s_x2[e];
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kUnroll; ++u) {
+                    fma8(acc, w[u], xs[u]);
+                    if (kSwiglu) fma8(acc2, w2[u], xs2[u]);
+                }
+            }
+        }
     }
+    if (p.active_elems != nullptr && tid == 0)
+        atomicAdd(p.active_elems, (unsigned long long)counted * min(kCols, p.N - slice * kCols) * kArrays);
+
+    // ---- sums over the lane groups of a warp (halving: a lane keeps ever fewer of its columns), the warps, the CTAs ----
+    const auto put = [&](float (&v)[8], int arr) {
+        int c = (lane % kLanes) * 8;
+        const bool up = (lane & 16) != 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float send = up ? v[i] : v[i + 4], keep = up ? v[i + 4] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+        }
+        c += up ? 4 : 0;
+        if (kGroups == 4) {
+            const bool up8 = (lane & 8) != 0;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float send = up8 ? v[i] : v[i + 2], keep = up8 ? v[i + 2] : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+            }
+            c += up8 ? 2 : 0;
+        }
+#pragma unroll
+        for (int i = 0; i < 8 / kGroups; ++i) s_red[warp][arr][c + i] = v[i];
+    };
+    put(acc, 0);
+    if (kSwiglu) put(acc2, kArrays - 1);
+    __syncthreads();
+    if (p.k_splits > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");       // every CTA of the cluster runs
+    for (int i = tid; i < kArrays * kCols; i += kT) {
+        const int arr = i / kCols, c = i - arr * kCols;
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < kNumWarps; ++w) t += s_red[w][arr][c];
+        uint32_t to;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, 0;"
+                     : "=r"(to) : "r"((uint32_t)__cvta_generic_to_shared(&s_part[rank][arr][c])));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to), "f"(t) : "memory");
+    }
+    if (p.k_splits > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+        __syncthreads();
+    }
+    if (rank != 0 || tid >= kCols) return;
+    float sum = 0.f, sum2 = 0.f;
+    for (int r = 0; r < p.k_splits; ++r) {
+        sum += s_part[r][0][tid];
+        if (kSwiglu) sum2 += s_part[r][kArrays - 1][tid];
+    }
+    const int col = slice * kCols + tid;
+    if (!kSwiglu && p.xw > 0) sum = sum_over_ranks(p, col, (p.N + kColsPerCta - 1) / kColsPerCta * kColsPerCta, sum);
+    if (col < p.N) finish_column<kSwiglu>(p, col, sum, sum2);
+}
+
+// Which matrices: those whose bytes take less time than a launch's chain. One array: up to 17 M elements (us before / here: 8192
+// x 2048 7.9 / 7.1, 14336 x 1024 7.5 / 6.9, but 6144 x 4096 8.3 / 8.3, 3584 x 7168 8.9 / 9.6); two: up to 40 M in all (8192 x 2048
+// 10.1 / 9.1, but 14336 x 2048 14.2 / 14.4). A narrow matrix with very many rows is spread over too few SMs (one array 1024 x
+// 14336 8.8 / 9.1, 1024 x 7168 6.4 / 6.4, but 2048 x 7168 8.1 / 7.3). Clusters of eight fit up to 256 CTAs of 512 threads (two an
+// SM); 16 CTAs a cluster found room for few clusters at once (4096 x 4096: 41 us).
+struct ClusterPlan {
+    int cols, ctas, threads;       // ctas: of a cluster; 0: not for these sizes
+};
+
+ClusterPlan cluster_plan(int N, int Z, int arrays) {
+    const long long elems = (long long)N * Z * arrays;
+    const bool long_narrow = arrays == 1 && Z > 6144 && N < 1536;
+    if (elems > (arrays == 1 ? 17000000 : 40000000) || N > 32768 || Z > 8192 || long_narrow) return {0, 0, 0};
+    const int cols = N <= 2048 ? 64 : 128, slices = (N + cols - 1) / cols;
+    const int ctas = std::min(std::min(kClusterCtas, 256 / slices), std::max(1, Z / 64));
+    // few rows a CTA: eight warps list and add faster than sixteen (512 x 512 3.0 / 3.3, 1024 x 2048 3.5 / 4.6; 4096 x 4096 7.0 / 7.1)
+    const bool light = N <= 2048 ? Z * arrays < 4096 : N <= 4096 && arrays == 1;
+    return {cols, ctas, light ? 256 : 512};
+}
+
+template <bool kSwiglu>
+cudaError_t launch_clusters(GemvParams& p, const ClusterPlan& pl, cudaStream_t st) {
+    constexpr int kArrays = kSwiglu ? 2 : 1;
+    p.n_slices = (p.N + pl.cols - 1) / pl.cols;
+    p.k_splits = pl.ctas;
+    p.rows_per_split = (p.Z + pl.ctas - 1) / pl.ctas;
+    p.prefetch_rows = prefetch_rows(p.rows_per_split, kArrays, pl.cols);
+    const auto go = [&](auto kernel) {
+        return launch_cluster_kernel_ex(true, dim3(1, pl.ctas, 1), kernel, dim3(p.n_slices, pl.ctas), dim3(pl.threads), 0, st, p);
+    };
+    if (pl.cols == 64)
+        return pl.threads == 256 ? go(sparse_gemv_cluster_kernel<kSwiglu, 64, 256>) : go(sparse_gemv_cluster_kernel<kSwiglu, 64, 512>);
+    return pl.threads == 256 ? go(sparse_gemv_cluster_kernel<kSwiglu, 128, 256>) : go(sparse_gemv_cluster_kernel<kSwiglu, 128, 512>);
 }
 
 int check_common(const void* Wt, const void* x, const void* y, int N, int Z) {
@@ -527,7 +798,7 @@ int launch_gemv(const void* Wt, const void* x, void* y, int N, int Z, const lean
     p.n_slices = pl.n_slices;
     p.k_splits = pl.k_splits;
     p.rows_per_split = pl.rows_per_split;
-    p.prefetch_rows = prefetch_rows(pl.rows_per_split, 1);
+    p.prefetch_rows = std::min(prefetch_rows(pl.rows_per_split, 1, kColsPerCta), kThreads / 1);
     p.n_segments = segs->n_segments;
     for (int s = 0; s < LEANKV_MAX_SEGMENTS; ++s) {
         p.seg_end[s] = s < segs->n_segments ? segs->seg_end[s] : N;
@@ -552,6 +823,11 @@ int launch_gemv(const void* Wt, const void* x, void* y, int N, int Z, const lean
             p.xrecv[r] = static_cast<unsigned long long*>(xchg->recv[r]) +
                          (size_t)slot * xchg->world * xchg->max_cols;
         }
+    }
+    const ClusterPlan cl = cluster_plan(N, Z, 1);
+    if (cl.ctas > 0) {
+        LEANKV_CUDA_TRY(launch_clusters<false>(p, cl, static_cast<cudaStream_t>(stream)));
+        return LEANKV_OK;
     }
     dim3 grid(pl.n_slices, pl.k_splits);
     LEANKV_CUDA_TRY(launch_kernel_ex(true, sparse_gemv_kernel<false>, grid, dim3(kThreads), 0,
@@ -654,7 +930,7 @@ static int launch_swiglu(const void* Wt_gate, const void* Wt_up, const void* x, 
     p.n_slices = pl.n_slices;
     p.k_splits = pl.k_splits;
     p.rows_per_split = pl.rows_per_split;
-    p.prefetch_rows = prefetch_rows(pl.rows_per_split, 2);
+    p.prefetch_rows = std::min(prefetch_rows(pl.rows_per_split, 2, kColsPerCta), kThreads / 2);
     p.n_segments = 1;
     for (int s = 0; s < LEANKV_MAX_SEGMENTS; ++s) {
         p.seg_end[s] = N;
@@ -663,6 +939,11 @@ static int launch_swiglu(const void* Wt_gate, const void* Wt_up, const void* x, 
     p.thr_up = t_up;
     p.norm_w = static_cast<const __half*>(norm_w);
     p.norm_eps = norm_eps;
+    const ClusterPlan cl = cluster_plan(N, Z, 2);
+    if (cl.ctas > 0) {
+        LEANKV_CUDA_TRY(launch_clusters<true>(p, cl, static_cast<cudaStream_t>(stream)));
+        return LEANKV_OK;
+    }
     dim3 grid(pl.n_slices, pl.k_splits);
     LEANKV_CUDA_TRY(launch_kernel_ex(true, sparse_gemv_kernel<true>, grid, dim3(kThreads), 0,
                                   static_cast<cudaStream_t>(stream), p));
@@ -745,7 +1026,7 @@ extern "C" int leankv_sparse_gemv_f16_static(const void* Wt, const void* x, void
     void* scratch = g_static_scratch_addr[dev];
     // The array keeps whatever the previous call left. Only the arrival counters must start at zero
     // (partials are fully overwritten before they are read), so those are cleared on the stream.
-    if (pl.k_splits > 1)
+    if (pl.k_splits > 1 && cluster_plan(N, Z, 1).ctas == 0)
         LEANKV_CUDA_TRY(cudaMemsetAsync(scratch, 0, pl.counter_bytes, static_cast<cudaStream_t>(stream)));
 
     leankv_segments_t segs{};

@@ -364,3 +364,30 @@ def test_sparse_gemv_and_swiglu_take_every_form_of_the_token(form):
         assert got.shape == (1, 1, n) and got.dtype == given.dtype and torch.equal(got, want.to(given.dtype))
     with pytest.raises(RuntimeError):
         sparse_gemv(x[:-1], w[0], c.threshold)
+
+
+@pytest.mark.parametrize("n,z", [(8, 1), (64, 63), (72, 129), (2048, 64), (2048, 8192), (2056, 2047), (1536, 6145), (4096, 4150),
+                                 (4104, 512), (32768, 130), (520, 2051)])
+@pytest.mark.parametrize("sparsity", [0.0, 0.5, 1.0])
+def test_cluster_kernel_edges(n, z, sparsity):
+    """Slices of 64 and 128 columns, one to eight CTAs a slice, ragged columns and channels, several lists a CTA and empty
+    ones: against float64. The sums are fp32 (z terms: below 1e-5 of the result), so the fp16 rounding of the output, 2^-11 a
+    value, bounds the difference; silu * up rounds three times."""
+    gen = torch.Generator(device="cpu").manual_seed(n + z)
+    ws = [(torch.randn(z, n, generator=gen) * 0.02).half().to(_dev()) for _ in range(2)]
+    x = torch.randn(z, generator=gen).half().to(_dev())
+    k = int(sparsity * z)
+    t = float(x.abs().float().kthvalue(k).values) if k else -1.0
+    live = torch.where(x.abs().float() > t, x, torch.zeros_like(x)).double()
+    y, active = _raw_gemv(ws[0], x, t)
+    want = live @ ws[0].double()
+    assert active == int((x.abs().float() > t).sum()) * n
+    assert (y.double() - want).norm() <= 2 ** -11 * want.norm() + 1e-6
+    lib, out = _native.lib(), torch.empty(n, dtype=torch.float16, device=_dev())
+    area = torch.zeros(max(lib.leankv_sparse_swiglu_workspace_bytes(n, z), 256), dtype=torch.uint8, device=_dev())
+    _native.check(lib.leankv_sparse_swiglu_f16(ws[0].data_ptr(), ws[1].data_ptr(), x.data_ptr(), out.data_ptr(), n, z, t, t / 2,
+                                               area.data_ptr(), area.numel(), None, torch.cuda.current_stream().cuda_stream),
+                  "sparse swiglu")
+    up = torch.where(x.abs().float() > torch.tensor(t / 2).half().float(), x, torch.zeros_like(x)).double() @ ws[1].double()
+    want = torch.nn.functional.silu(want) * up
+    assert (out.double() - want).norm() <= 4 * 2 ** -11 * want.norm() + 1e-6
