@@ -191,7 +191,7 @@ class MixerStep(Structure):
     _fields_ = [("y", c_void_p), ("qkv_off", c_int), ("rkvg_off", c_int), ("w1_off", c_int), ("rank", c_int),
                 ("w2", c_void_p), ("out", c_void_p), ("right_off", c_int),
                 ("left_scale", c_float), ("right_scale", c_float), ("state", c_void_p), ("max_pos", c_int),
-                ("ws", c_void_p), ("ws_bytes", c_size_t)]
+                ("ws", c_void_p), ("ws_bytes", c_size_t), ("early_state", c_int)]
 
 
 class CausalAttn(Structure):

@@ -258,7 +258,8 @@ class ParallelMixer:
         s = _native.MixerStep(y=y.data_ptr(), qkv_off=0, rkvg_off=n0, w1_off=n0 + 4 * N, rank=self.right.rank,
                               w2=self.right.w2.data_ptr(), out=out.data_ptr(), right_off=self.left.spec.out_width,
                               left_scale=self.left_scale, right_scale=self.right_scale, state=state.data_ptr(),
-                              max_pos=max_pos, ws=self._step_ws.data_ptr(), ws_bytes=self._step_ws.numel())
+                              max_pos=max_pos, ws=self._step_ws.data_ptr(), ws_bytes=self._step_ws.numel(),
+                              early_state=1)          # behind the input projections
         o = _step_gemv(w=self.w_out.data_ptr(), x=out.data_ptr(), dtype=code, rows=self.width,
                               cols=self.out_width, **exit)
         self._step_args = (a, s, o)

@@ -243,6 +243,19 @@ def test_window_pool_prompt_portions_and_steps_agree_with_plain(dtype, shape):
     assert rel(feed(steps, qkv, [1] * T), want) < tol(dtype)
 
 
+@pytest.mark.parametrize("shape", [(8, 2, 128, 128, 255, 16), (16, 4, 128, 128, 270, 16), (16, 16, 16, 32, 260, 8),
+                                   (16, 2, 64, 48, 250, 300), (5, 1, 112, 16, 262, 7), (7, 7, 128, 128, 40, 3)])
+@pytest.mark.parametrize("normed,talk", [(True, True), (False, True), (True, False)])
+def test_step_on_tensor_cores_around_whole_tiles(shape, normed, talk):
+    """A CTA's share of the keys grows from 16 to 17 (255 .. 274 visible keys over 16 CTAs), the window moves past its first
+    token, blocks become visible and complete: against float64. The bound is the tests' own for bf16 keys and values."""
+    T = 300
+    win = Window(BF16, *shape, chunk=T, limit=T, normed=normed, talk=talk)
+    qkv = win.qkv(T)
+    got = feed(win, qkv, [252] + [1] * (T - 252))
+    assert rel(got[252:], win.expected(qkv)[252:]) < 3e-2
+
+
 @pytest.mark.parametrize("normed,talk", [(False, True), (True, False), (False, False)])
 def test_window_pool_without_norm_or_mixing(normed, talk):
     win = Window(F32, 4, 2, 16, 24, 10, 3, chunk=60, limit=60, normed=normed, talk=talk)
