@@ -12,9 +12,11 @@ it, is part of a branch's first GEMV: {norm, every input projection}, {mixers}, 
 from __future__ import annotations
 
 import ctypes
+from array import array
 from dataclasses import dataclass
 from typing import Optional, Sequence
 
+import numpy as np
 import torch
 
 from . import _native
@@ -85,6 +87,16 @@ class MixerModelConfig:
         mult, cap = c.get("residual_mult"), c.get("logit_softcap")
         return cls(c["architecture"], int(c["vocab"]), int(c["width"]), float(c["norm"]["eps"]), tuple(c["layers"]),
                    (start, stop, times), 1.0 if mult is None else float(mult), float(cap or 0.0))
+
+
+def _whole_numbers(tokens: Sequence[int]) -> np.ndarray:
+    """Token ids as int64; a list of Python numbers without a look at each one's type."""
+    try:
+        return np.frombuffer(array("q", list(tokens)), dtype=np.int64)
+    except OverflowError:
+        raise ValueError("token outside the vocabulary") from None
+    except TypeError:                      # floating-point numbers and whatever else a tensor takes
+        return torch.as_tensor(list(tokens), dtype=torch.int64).numpy()
 
 
 class _Sublayer:
@@ -375,27 +387,40 @@ class MixerDecodeEngine(DecodeLoop):
         n = len(tokens)
         if n < 1 or self.pos + n > self.max_seq_len:
             raise ValueError(f"{n} tokens at position {self.pos} do not fit {self.max_seq_len}")
-        if min(tokens) < 0 or max(tokens) >= self.cfg.vocab_size:
+        host = _whole_numbers(tokens)
+        if host.min() < 0 or host.max() >= self.cfg.vocab_size:
             raise ValueError("token outside the vocabulary")
         if any(not 0 <= w < n for w in want):
             raise ValueError("wanted place outside the portion")
-        out = torch.empty(len(want), self.cfg.vocab_size, dtype=torch.float32, device=self.dev)
         with torch.cuda.device(self.dev):
             if n == 1:
+                out = torch.empty(len(want), self.cfg.vocab_size, dtype=torch.float32, device=self.dev)
                 self.token.fill_(int(tokens[0]))
                 self.step()
                 if len(want):
                     out[:] = self.logits
                 return out
-            ids = torch.as_tensor(list(tokens), dtype=torch.int64, device=self.dev)
-            for s0 in range(0, n, self.max_chunk):
-                x = self._portion(ids[s0:s0 + self.max_chunk])
-                rows = [k for k, w in enumerate(want) if s0 <= w < s0 + x.shape[0]]
-                if rows:
-                    at = torch.tensor([want[k] - s0 for k in rows], device=self.dev)
-                    out[torch.tensor(rows, device=self.dev)] = self._logits_of(x[at])
-            if len(want):
-                self.check_status()
+            # Tokens, wanted places and their rows of the result go up together and ahead of everything else: an upload between two
+            # portions would wait for the first and leave the device idle while the next is launched (4000 tokens in two portions
+            # through four layers: 3429 us, and 3162 so).
+            parts = [(s0, min(self.max_chunk, n - s0)) for s0 in range(0, n, self.max_chunk)]
+            rows = [[k for k, w in enumerate(want) if s0 <= w < s0 + m] for s0, m in parts]
+            order = [k for r in rows for k in r]
+            places = [want[k] - s0 for (s0, _), r in zip(parts, rows) for k in r]
+            up = torch.from_numpy(np.concatenate([host, np.array(places + order, dtype=np.int64)])).to(self.dev, non_blocking=True)
+            ids, at, to = up[:n], up[n:n + len(order)], up[n + len(order):]
+            done, pieces = 0, []
+            for (s0, m), r in zip(parts, rows):
+                x = self._portion(ids[s0:s0 + m])
+                if r:
+                    pieces.append(self._logits_of(x[at[done:done + len(r)]]))
+                    done += len(r)
+            if not pieces:
+                return torch.empty(0, self.cfg.vocab_size, dtype=torch.float32, device=self.dev)
+            out = pieces[0] if len(pieces) == 1 else torch.cat(pieces)
+            if order != sorted(order):
+                out = torch.empty_like(out).index_copy_(0, to, out)
+            self.check_status()
         return out
 
     @torch.no_grad()

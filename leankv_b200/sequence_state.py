@@ -95,8 +95,8 @@ class SequenceState:
     def reset(self) -> None:
         """Give the sequence back. Rings and pooled blocks need no clearing: a position only ever reads
         slots that its own sequence has written."""
-        for t in self._carried:
-            t.zero_()
+        if self._carried:
+            torch._foreach_zero_(self._carried)          # one launch
 
     def bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in self._all)

@@ -252,3 +252,17 @@ def test_mixer_arguments_are_checked_before_any_launch():
     s = _native.StreamNorm(x_in=fake, x_out=fake, delta=fake, scale=fake, gain=fake, dtype=1, delta_dtype=2, rows=1,
                            width=8)
     assert lib.leankv_stream_norm(ctypes.byref(s), None) == -1                # in place
+
+
+def test_token_ids_of_every_kind_and_out_of_range():
+    import numpy as np
+
+    from leankv_b200.mixer_engine import _whole_numbers
+
+    for tokens in ([3, 1, 2], (3, 1, 2), range(3), torch.tensor([3, 1, 2]), np.array([3, 1, 2], dtype=np.int32), bytes([3, 1, 2]),
+                   [3.0, 1.0, 2.0], [np.int64(3), True, 2], [torch.tensor(3), 1, 2]):
+        want = torch.as_tensor(list(tokens), dtype=torch.int64)
+        got = _whole_numbers(tokens)
+        assert got.dtype == np.int64 and got.tolist() == want.tolist()
+    with pytest.raises(ValueError):
+        _whole_numbers([1 << 63])
