@@ -321,7 +321,7 @@ extern "C" int leankv_decode_end(const void* logits, int vocab, long long* token
                                  int history_cap, int32_t* state, void* stream) {
     if (!logits || !token || !history || !state || vocab <= 0 || history_cap < 0) return LEANKV_EINVAL;
     if (!aligned16(logits)) return LEANKV_EALIGN;
-    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<__half>, dim3(1), dim3(1024), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<__half>, dim3(kEndCtas), dim3(kEndThreads), 0, static_cast<cudaStream_t>(stream),
                                   static_cast<const __half*>(logits), vocab, token, history, history_cap,
                                   state + kPos, state + kStep, static_cast<int*>(nullptr)));
     return LEANKV_OK;
@@ -430,7 +430,7 @@ extern "C" int leankv_batch_decode_end(const void* logits, int vocab, int B, lon
     if (!logits || !tokens || !history || !pos || !steps || vocab <= 0 || B <= 0 || history_cap < 0)
         return LEANKV_EINVAL;
     if (!aligned16(logits) || vocab % 8 != 0) return LEANKV_EALIGN;
-    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<__half>, dim3(B), dim3(1024), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<__half>, dim3(B * kEndCtas), dim3(kEndThreads), 0, static_cast<cudaStream_t>(stream),
                                   static_cast<const __half*>(logits), vocab, tokens, history, history_cap, pos,
                                   steps, static_cast<int*>(nullptr)));
     return LEANKV_OK;

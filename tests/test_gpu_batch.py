@@ -107,6 +107,32 @@ def test_batch_decode_end_is_rowwise_argmax():
         assert int(hist[b, s]) == int(want[b])
 
 
+@pytest.mark.parametrize("vocab", [1, 7, 8, 31, 64, 4093, 32768, 50001])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_decode_end_over_the_shares_of_a_cluster(vocab, dtype):
+    """Best value in every share of the vocabulary and in the remainder, ties (the lowest index), NaN beside numbers, no number at all."""
+    lib = _native.lib() if dtype == torch.float16 else _native.mixers()
+    end = lib.leankv_decode_end if dtype == torch.float16 else lib.leankv_greedy_end
+    rows = []
+    for at in sorted({0, vocab // 2, vocab - 1, *(vocab * r // 8 for r in range(8))}):
+        row = torch.linspace(-1, 1, vocab).to(dtype)
+        row[at] = 5.0
+        rows.append(row.clone())
+        row[vocab - 1] = 5.0
+        row[vocab // 3] = float("nan") if vocab // 3 != at and vocab > 1 else row[vocab // 3]
+        rows.append(row)
+    rows.append(torch.full((vocab,), float("nan"), dtype=dtype))
+    for row in rows:
+        want = int(row.float().nan_to_num(nan=-10.0).argmax()) if not bool(row.isnan().all()) else 0
+        want = int((row == row[want]).nonzero()[0]) if not bool(row.isnan().all()) else 0
+        dev, token = row.to(_dev()), torch.full((1,), -1, dtype=torch.int64, device=_dev())
+        hist, state = torch.zeros(4, dtype=torch.int64, device=_dev()), torch.zeros(8, dtype=torch.int32, device=_dev())
+        state[:2] = torch.tensor([10, 2])
+        _native.check(end(dev.data_ptr(), vocab, token.data_ptr(), hist.data_ptr(), 4, state.data_ptr(), _st()), "end")
+        torch.cuda.synchronize()
+        assert int(token) == want == int(hist[2]) and state[:2].tolist() == [11, 3]
+
+
 def test_batch_qkv_post_is_bit_identical_to_single_sequence_kernel():
     """Same qkv rows, positions and pages through the batched launch and through one launch per sequence."""
     lib = _native.lib()
