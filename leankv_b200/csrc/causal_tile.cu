@@ -14,17 +14,13 @@
 #include <algorithm>
 
 #include "causal_attn.cuh"
+#include "tile_softmax.cuh"
 #include "tma.cuh"
 
 namespace leankv {
 namespace {
 
-constexpr int kTile = 128;                       // rows of a CTA
-constexpr int kKeys = 64;                        // keys of a tile
 constexpr int kThreads = 192;
-constexpr uint32_t kBlock = kTile * 128;         // 128 rows of 64 columns: 16 KB
-constexpr uint32_t kKeyBlock = kKeys * 128;      // 64 keys of 64 columns: 8 KB
-constexpr float kSlack = 8.f;
 
 struct TileArgs {
     CUtensorMap q, k, shared, v;
@@ -39,33 +35,6 @@ struct TileArgs {
     uint32_t q_box, tmem_cols;
     float c;                                     // scale * log2(e)
 };
-
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// Two floats at a time.
-struct Two { float x, y; };
-__device__ __forceinline__ Two fma2(Two a, Two b, Two c) {
-    Two d;
-    asm("{\n\t.reg .b64 a, b, c, d;\n\t"
-        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
-        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
-__device__ __forceinline__ Two add2(Two a, Two b) {
-    Two d;
-    asm("{\n\t.reg .b64 a, b, d;\n\t"
-        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
-        "add.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
 
 enum { kQ, kO, kKFull, kKFree = kKFull + 2, kVFull = kKFree + 2, kS = kVFull + 2, kP = kS + 2, kPV = kP + 2, kBars = kPV + 2 };
 
@@ -203,12 +172,7 @@ __global__ void __launch_bounds__(kThreads, 2) causal_tile_kernel(const __grid_c
                     for (int x = 0; x < 32; ++x)
                         if (c * 32 + x < k0 || c * 32 + x > k1) s[c][x] = 0xff800000u;      // -inf
             }
-            float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-#pragma unroll
-                for (int x = 0; x < 32; ++x) top[x & 3] = fmaxf(top[x & 3], __uint_as_float(s[c][x]));
-            const float best = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+            const float best = largest(s);
             const bool raise = best * p.c > m + kSlack;
             if (__any_sync(0xffffffffu, raise)) {
                 const float mn = raise ? best * p.c : m, f = ex2(m - mn);
@@ -218,35 +182,10 @@ __global__ void __launch_bounds__(kThreads, 2) causal_tile_kernel(const __grid_c
                     ok = __all_sync(0xffffffffu, wait(kPV, j - 1));      // nothing is being added to the outputs
                     if (!ok) break;
                     umma::fence_after_sync();
-#pragma unroll 1
-                    for (int c = 0; c < p.vdim_pad; c += 32) {
-                        uint32_t o[32];
-                        umma::ld32(o, tm_o, row0, c);
-#pragma unroll
-                        for (int x = 0; x < 32; ++x) o[x] = __float_as_uint(__uint_as_float(o[x]) * f);
-                        umma::st32(o, tm_o, row0, c);
-                    }
+                    scale_outputs(tm_o, row0, p.vdim_pad, f);
                 }
             }
-            Two sum[2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                uint32_t ph[16], pl[16];
-#pragma unroll
-                for (int x = 0; x < 32; x += 2) {
-                    Two w = fma2({__uint_as_float(s[c][x]), __uint_as_float(s[c][x + 1])}, {p.c, p.c}, {-m, -m});
-                    w.x = ex2(w.x);
-                    w.y = ex2(w.y);
-                    sum[(x >> 1) & 1] = add2(sum[(x >> 1) & 1], w);
-                    const uint32_t hi = pack_bf16(w.x, w.y);
-                    const Two left = add2(w, {-__uint_as_float(hi << 16), -__uint_as_float(hi & 0xffff0000u)});
-                    ph[x / 2] = hi;
-                    pl[x / 2] = pack_bf16(left.x, left.y);
-                }
-                umma::st16_async(ph, tm, row0, c * 32);
-                umma::st16_async(pl, tm, row0, c * 32 + 16);
-            }
-            l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+            l += put_weights(s, p.c, m, tm, row0);
             umma::stored();
             umma::fence_before_sync();
             umma::bar_arrive(bar(kP + (j & 1)));

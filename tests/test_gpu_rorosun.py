@@ -243,6 +243,20 @@ def test_window_pool_prompt_portions_and_steps_agree_with_plain(dtype, shape):
     assert rel(feed(steps, qkv, [1] * T), want) < tol(dtype)
 
 
+@pytest.mark.parametrize("shape", [(12, 4, 128, 128, 130, 1), (8, 2, 64, 96, 200, 3), (3, 1, 16, 32, 65, 2), (4, 4, 128, 128, 64, 64),
+                                   (16, 2, 48, 16, 100, 5), (6, 3, 112, 128, 1, 7)])
+def test_prompt_attention_by_key_tiles(shape):
+    """Tiles of 64 blocks or tokens with remainders, rings that wrap inside a tile, rows of CTAs that are not full, slots that nothing
+    has written (NaN), against float64. Values and outputs are bf16, weights 16 bits: 2^-8 a value bounds the difference."""
+    T = 400
+    win = Window(BF16, *shape, chunk=T, limit=T)
+    qkv = win.qkv(T)
+    want = win.expected(qkv)
+    assert rel(feed(win, qkv, [T]), want) < 3e-2
+    small = Window(BF16, *shape, chunk=150, limit=T)
+    assert rel(feed(small, qkv, [150, 2, 131, 1, 33, 83]), want) < 3e-2
+
+
 @pytest.mark.parametrize("shape", [(8, 2, 128, 128, 255, 16), (16, 4, 128, 128, 270, 16), (16, 16, 16, 32, 260, 8),
                                    (16, 2, 64, 48, 250, 300), (5, 1, 112, 16, 262, 7), (7, 7, 128, 128, 40, 3)])
 @pytest.mark.parametrize("normed,talk", [(True, True), (False, True), (True, False)])
