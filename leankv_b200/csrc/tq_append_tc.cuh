@@ -17,9 +17,11 @@
 // (sequence, head, K|V); CTAs are persistent over a contiguous range of tiles and keep the fp16 copies of Pi in
 // shared memory, reloading them only when their range crosses from K to V.
 //
-// A prompt chunk is one tile a CTA, so its time is the chain of a tile's phases, none of which fills the issue slots: with one
-// warp a page 512 tokens (8 heads) took 40 000 cycles (staging Pi 7 800, norms and division 6 500, products 4 700, codes 9 400,
-// exact chains 8 800, packing 1 300): 24 us; with two 13.
+// A prompt chunk is one tile a CTA, so its time is the chain of a tile's phases, none of which fills the issue slots. 512 tokens of 8
+// heads, cycles: indexes and positions 2000, staging Pi 2000 (3600 from HBM), norms 850, division 2100, band 650, products 3700 (the rate of
+// mma.sync), codes 2000, exact chains 2500, packing 1450: 11.0 us (13.1 with a rotation that is not in L2). With one warp a page
+// they took 24, with Pi staged by 8-byte loads, four in flight, 12.4 (16.4); 16 sequences of 2048 tokens 329, now 301 (tiles without a
+// token are left out, rows without one not divided).
 
 constexpr int kTcThreads = 256;
 constexpr int kTcTokens = 64;
@@ -119,51 +121,59 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
     unsigned long long n_exact = 0, n_coords = 0;
 
     for (long long tile = tile_lo; tile < tile_hi; ++tile) {
-        const int which = (int)(tile / per_which);
-        long long r = tile - (long long)which * per_which;
-        const int grp = (int)(r % tp.groups);
-        r /= tp.groups;
-        const int h = (int)(r % p.H), b = (int)(r / p.H);
+        const int which = tile < per_which ? 0 : 1;
+        const unsigned r = (unsigned)(tile - (which ? per_which : 0));       // the grid's tiles of a side fit 32 bits
+        const unsigned r2 = r / (unsigned)tp.groups, grp = r - r2 * (unsigned)tp.groups;
+        const int b = (int)(r2 / (unsigned)p.H), h = (int)(r2 - (unsigned)b * (unsigned)p.H);
         const float* Pi = which == 0 ? p.Pi_k : p.Pi_v;
 
+        const int pos0 = p.start_pos[b];
+        const int ord0 = pos0 / 16 + 4 * (int)grp;            // first page ordinal of this tile
+        const int pos_end = pos0 + p.T_new;
+        if (ord0 * 16 >= pos_end) continue;                   // one group more than needed where the start is a page's
+        const __half* src = append_source(p, which, b, h);
+
         __syncthreads();                 // the previous tile's readers of s_u / s_pi* are done
+        // the tile's vectors are asked for ahead of Pi, and Pi in two trips of eight 16-byte loads a thread
+        const int row = tid >> 2, qr = tid & 3;               // four threads per token, 32 coordinates each
+        const int pos = ord0 * 16 + row;
+        uint4 raw[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            raw[i] = pos >= pos0 && pos < pos_end
+                         ? __ldg(reinterpret_cast<const uint4*>(src + (size_t)(pos - pos0) * kDim + qr * 32) + i)
+                         : make_uint4(0, 0, 0, 0);
         const bool staged = which != loaded_which;
         if (staged) {
-            for (int i = tid; i < kDim * kDim / 2; i += kTcThreads) {
-                const int j = i >> 6, k2 = (i & 63) * 2;
-                const float2 v = __ldg(reinterpret_cast<const float2*>(Pi + j * kDim + k2));
-                uint32_t hi, lo;
-                split_h2(v.x, v.y, hi, lo);
-                *reinterpret_cast<uint32_t*>(&s_pih[j * kPiStride + k2]) = hi;
-                *reinterpret_cast<uint32_t*>(&s_pil[j * kPiStride + k2]) = lo;
+            constexpr int kTrip = 8;
+            static_assert(kDim * kDim / 4 == 2 * kTrip * kTcThreads, "two trips");
+#pragma unroll 1
+            for (int i0 = tid; i0 < kDim * kDim / 4; i0 += kTrip * kTcThreads) {
+                float4 v[kTrip];
+#pragma unroll
+                for (int x = 0; x < kTrip; ++x) v[x] = __ldg(reinterpret_cast<const float4*>(Pi) + i0 + x * kTcThreads);
+#pragma unroll
+                for (int x = 0; x < kTrip; ++x) {
+                    const int i = i0 + x * kTcThreads, at = (i >> 5) * kPiStride + (i & 31) * 4;
+                    uint2 hi, lo;
+                    split_h2(v[x].x, v[x].y, hi.x, lo.x);
+                    split_h2(v[x].z, v[x].w, hi.y, lo.y);
+                    *reinterpret_cast<uint2*>(&s_pih[at]) = hi;
+                    *reinterpret_cast<uint2*>(&s_pil[at]) = lo;
+                }
             }
             loaded_which = which;
         }
 
-        const int pos0 = p.start_pos[b];
-        const int ord0 = pos0 / 16 + 4 * grp;                 // first page ordinal of this tile
-        const int pos_end = pos0 + p.T_new;
-        const __half* src = append_source(p, which, b, h);
-
-        // ---- norms and unit vectors: four threads per token, 32 coordinates each. The norm is the contract's: the squares of
+        // ---- norms and unit vectors. The norm is the contract's: the squares of
         // each half one after another, so the second thread of a half goes on from the first one's sum ----
         {
-            const int row = tid >> 2, qr = tid & 3;
-            const int pos = ord0 * 16 + row;
-            const bool ok = pos >= pos0 && pos < pos_end;
             float xr[32];
-            if (ok) {
-                const uint4* s4 = reinterpret_cast<const uint4*>(src + (size_t)(pos - pos0) * kDim + qr * 32);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint4 w = __ldg(s4 + i);
-                    const float2 a = h2_to_f2(w.x), bb = h2_to_f2(w.y), c = h2_to_f2(w.z), d = h2_to_f2(w.w);
-                    xr[8 * i + 0] = a.x; xr[8 * i + 1] = a.y; xr[8 * i + 2] = bb.x; xr[8 * i + 3] = bb.y;
-                    xr[8 * i + 4] = c.x; xr[8 * i + 5] = c.y; xr[8 * i + 6] = d.x; xr[8 * i + 7] = d.y;
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) xr[i] = 0.f;
+            for (int i = 0; i < 4; ++i) {
+                const float2 a = h2_to_f2(raw[i].x), bb = h2_to_f2(raw[i].y), c = h2_to_f2(raw[i].z), d = h2_to_f2(raw[i].w);
+                xr[8 * i + 0] = a.x; xr[8 * i + 1] = a.y; xr[8 * i + 2] = bb.x; xr[8 * i + 3] = bb.y;
+                xr[8 * i + 4] = c.x; xr[8 * i + 5] = c.y; xr[8 * i + 6] = d.x; xr[8 * i + 7] = d.y;
             }
             double sum = 0.0;
 #pragma unroll
@@ -180,9 +190,15 @@ __global__ void __launch_bounds__(kTcThreads, 2) tq_pool_append_tc_kernel(const 
             const float denom = norm + 1e-10f;
             if (qr == 0) s_norm[row] = norm;
             float4* dst = reinterpret_cast<float4*>(&s_u[row * kUStride + qr * 32]);
+            if (norm > 0.f) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                dst[i] = make_float4(xr[4 * i] / denom, xr[4 * i + 1] / denom, xr[4 * i + 2] / denom, xr[4 * i + 3] / denom);
+                for (int i = 0; i < 8; ++i)
+                    dst[i] = make_float4(xr[4 * i] / denom, xr[4 * i + 1] / denom, xr[4 * i + 2] / denom, xr[4 * i + 3] / denom);
+            } else {      // no token or a zero vector (whose division by 1e-10 takes 9400 cycles a tile), or no numbers
+#pragma unroll
+                for (int i = 0; i < 8; ++i) dst[i] = norm == 0.f ? make_float4(xr[4 * i], xr[4 * i + 1], xr[4 * i + 2], xr[4 * i + 3])
+                                                                 : make_float4(norm, norm, norm, norm);
+            }
         }
         __syncthreads();
         if (staged) {
