@@ -818,7 +818,8 @@ def batched_decode_leg(dev, world, rank, K, W, small=False, attn_iters=20):
         "kv_bytes_per_sequence": eng.kv_bytes_per_sequence(ctx),
         "kv_bytes_per_sequence_fp16": 2 * cfg.num_layers * cfg.num_kv_heads * 128 * 2 * ctx,
         "parity_vs_sequences_served_alone": parity,
-        "prefill_s": prefill_s, "gpu_launches": eng.launches_per_step * K, "library_gemms": eng.gemms_per_step * K,
+        "prefill_s": prefill_s, "gpu_launches": (eng.launches_per_step + eng.own_gemms_per_step) * K,
+        "library_gemms": (eng.gemms_per_step - eng.own_gemms_per_step) * K,
         "bytes_per_step_per_gpu": {"weights": weight_bytes, "kv": kv_step},
         "step_gbs_per_gpu": (weight_bytes + kv_step) / (sec / K) / 1e9,
         "attn_kernel": {"us": t_attn * 1e6, "algorithmic_bytes": alg_attn, "gbs": alg_attn / t_attn / 1e9,

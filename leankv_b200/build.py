@@ -23,7 +23,7 @@ BUILD_DIR = os.path.join(PKG_DIR, "build")
 # library -> sources; capi.cu (status codes, device queries) is linked into each
 LIBRARIES = {
     "libleankv_b200.so": ["capi.cu", "teal_gemv.cu", "tq_quantize.cu", "tq_attn.cu", "decoder_ops.cu",
-                          "decode_fused.cu"],
+                          "decode_fused.cu", "skinny_gemm.cu"],
     "libleankv_mixers.so": ["capi.cu", "dense_gemv.cu", "stream_ops.cu", "window_pool.cu",
                             "window_pool_tile.cu", "window_pool_mma.cu", "time_mix.cu", "mixer_step.cu", "causal_rows.cu", "causal_tile.cu",
                             "causal_step.cu"],

@@ -133,6 +133,24 @@ def test_decode_end_over_the_shares_of_a_cluster(vocab, dtype):
         assert int(token) == want == int(hist[2]) and state[:2].tolist() == [11, 3]
 
 
+@pytest.mark.parametrize("rows", [1, 15, 17, 48, 80, 128])
+@pytest.mark.parametrize("k,n", [(8, 8), (64, 128), (72, 136), (1000, 520), (3584, 1024), (520, 8192), (128, 40000)])
+def test_skinny_gemm_edges(rows, k, n):
+    """Rows beyond a product's sixteen, K and N with remainders, one to eight CTAs a column block, more blocks than CTAs at once:
+    against float64. The sums are fp32 (below 1e-5 of the result), so the fp16 rounding of the outputs, 2^-11 a value, bounds it."""
+    lib = _native.lib()
+    g = torch.Generator(device=_dev()).manual_seed(rows + k)
+    x = torch.randn(rows, k, device=_dev(), generator=g).half()
+    w = (torch.randn(k, n, device=_dev(), generator=g) * k ** -0.5).half()
+    y = torch.full((rows + 1, n), 7.0, dtype=torch.float16, device=_dev())
+    want = x.double() @ w.double()
+    for early in (0, 1):
+        _native.check(lib.leankv_skinny_gemm_f16(x.data_ptr(), w.data_ptr(), y.data_ptr(), rows, k, n, early, _st()), "skinny_gemm")
+        torch.cuda.synchronize()
+        assert bool((y[rows] == 7.0).all())
+        assert float((y[:rows].double() - want).norm()) <= 2 ** -11 * float(want.norm())
+
+
 def test_batch_qkv_post_is_bit_identical_to_single_sequence_kernel():
     """Same qkv rows, positions and pages through the batched launch and through one launch per sequence."""
     lib = _native.lib()
