@@ -621,13 +621,11 @@ __global__ void __launch_bounds__(32 * warps_of(W), W == Walk::kWarps ? 2 : 1) c
     float* ml = p.ml + ((size_t)gb * p.clusters * C + rank) * kHeads * 2;
     const size_t ml_step = (size_t)C * kHeads * 2;
     if (tid < 2 * kHeads) ml[cluster * ml_step + tid] = top[tid];
-    __threadfence();
     __syncthreads();
     unsigned* ticket = p.tickets + gb * C + rank;
-    if (tid == 0) s_last = atomicAdd(ticket, 1u) == (unsigned)active - 1;
+    if (tid == 0) s_last = arrive(ticket) == (unsigned)active - 1;       // hands over what the CTA wrote, and takes the others'
     __syncthreads();
     if (!s_last) return;
-    __threadfence();
     if (tid == 0) *ticket = 0;
     for (int k = tid; k < n_mine; k += kThreads) {
         const int h = (rank * slice + k) / v4;

@@ -114,6 +114,15 @@ __device__ __forceinline__ float4 ld_cg_f32x4(const float* p) {
     return v;
 }
 
+// One arrival behind a CTA barrier: releases what the whole CTA has written, and acquires what the CTAs counted before it have (the
+// barriers on both sides make the one thread's order the CTA's). A fence by every thread in front of a relaxed atomic, and another one behind
+// it, do the same for some 0.6 us more.
+__device__ __forceinline__ unsigned arrive(unsigned* counter) {
+    unsigned before;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+    return before;
+}
+
 // Programmatic dependent launch: a kernel first lets the next kernel in the stream start
 // launching (its CTAs become resident and run up to their own pdl_wait), then waits until every
 // kernel before it has completed and its writes are visible. Nothing that depends on, or is read

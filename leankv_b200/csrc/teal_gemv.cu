@@ -413,9 +413,7 @@ __global__ void __launch_bounds__(kThreads, kSwiglu ? 3 : 4) sparse_gemv_kernel(
         if (kSwiglu) mine[npad] = sum2;
         __syncthreads();
         if (tid == 0) {
-            int prev;
-            asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(prev) : "l"(p.counters + slice) : "memory");
-            s_last = (prev == p.k_splits - 1);
+            s_last = arrive(reinterpret_cast<unsigned*>(p.counters + slice)) == (unsigned)p.k_splits - 1;
         }
         __syncthreads();
         if (!s_last) return;

@@ -462,14 +462,12 @@ __global__ void __launch_bounds__(kAttnThreads, kOcc) tq_decode_attn_kernel(cons
                 mine[kGroup * kDim + tid] = mh[tid];
                 mine[kGroup * kDim + kGroup + tid] = lh[tid];
             }
-            __threadfence();
             __syncthreads();
             const int c_first = cta_of(o_p), c_last = cta_of(o_p + n_b - 1);
             const int n_seg = c_last - c_first + 1;
             if (tid == 0) {
-                const int prev = atomicAdd(&p.counters[b * H + kvh], 1);
-                __threadfence();               // the other CTAs' partials are read after this point
-                s_last = (prev == n_seg - 1);
+                // hands over this CTA's partials and takes the others'
+                s_last = arrive(reinterpret_cast<unsigned*>(p.counters + b * H + kvh)) == (unsigned)n_seg - 1;
             }
             __syncthreads();
             if (s_last) {
