@@ -14,7 +14,9 @@
 // the last. That takes up to 128 registers, so sixteen warps an SM: 250 us a step of 295 MB of weights (width 1024) and
 // 239 of 560 MB (width 2048), where thirty-two warps of 64 registers that loaded after the wait took 274 and 258. Tried and slower:
 // rows through shared memory by bulk copies, 100 KB an SM (290, 304); 80 or 96 registers (spills; 284, 255 and
-// 289, 251); the next launch's weights asked into L2 as well (279, 278).
+// 289, 251); the next launch's weights asked into L2 as well (279, 278). For the same reason a normed x is read once and kept
+// (a step of six Rorosun layers 194.0 -> 188.0 us, when it was read again for the products), and the residual comes beside x
+// (187.1). The shift's vectors beside x too: 193.4, they delay x.
 
 #include <algorithm>
 #include <type_traits>
@@ -148,7 +150,12 @@ __global__ void __launch_bounds__(512, !kAhead && sizeof(T) == 2 ? 2 : 1) dense_
             if (a.delta != nullptr) load_x8(a.post_gain, k, cols, vec, pg[c]);
         }
     }
+    // what a residual sum needs, a row a thread: the scale now, the residual beside x
+    const int fin = lo + (int)threadIdx.x;
+    float fin_scale = 0.f, fin_residual = 0.f;
+    if (IN == Input::kPlain && a.residual != nullptr) fin_scale = __ldg(a.scale + min(fin, hi - 1));
     pdl_begin();
+    if (IN == Input::kPlain && a.residual != nullptr) fin_residual = ld_cg_f32(a.residual + min(fin, hi - 1));
     if (kAhead && !a.early_weights) load_rows(0, 0, n_rows - 1);
 
     float rs = 1.f;
@@ -326,7 +333,8 @@ __global__ void __launch_bounds__(512, !kAhead && sizeof(T) == 2 ? 2 : 1) dense_
             if (a.bias != nullptr && row < a.bias_rows) y += __ldg(a.bias + row);
         }
         if (a.softcap > 0.f) y = a.softcap * tanhf(y / a.softcap);
-        if (a.residual != nullptr) y = a.residual[row] + y * __ldg(a.scale + row);
+        if (a.residual != nullptr)
+            y = IN == Input::kPlain && i < (int)blockDim.x ? fin_residual + y * fin_scale : ld_cg_f32(a.residual + row) + y * __ldg(a.scale + row);
         a.y[row] = y;
     }
 }
@@ -392,7 +400,9 @@ extern "C" int leankv_dense_gemv(const leankv_dense_gemv_t* a, void* stream) {
     GemvParams p{};
     p.a = *a;
     p.vec = a->cols % 8 == 0 && (a->group_rows == 0 || a->group_stride % 4 == 0);
-    const bool staged = a->delta || (a->gain && a->gain_per_col);
+    // a branch that joins the stream or a norm: x is prepared once, in registers where one slab holds it, else in shared memory
+    // (a norm with one gain and several slabs reads x a second time instead)
+    const bool staged = a->delta || (a->gain && a->gain_per_col), prepared = staged || a->gain;
     // warps x slabs x CH column chunks of 256: the widest CTA that pads least
     const int chunks = (a->cols + 255) / 256;
     int warps = 1, per = 1;
@@ -412,7 +422,7 @@ extern "C" int leankv_dense_gemv(const leankv_dense_gemv_t* a, void* stream) {
             constexpr Input IN = decltype(in)::value;
             return per == 1 ? launch_gemv<T, 1, IN>(p, warps, st) : launch_gemv<T, 2, IN>(p, warps, st);
         };
-        if (staged && p.slabs == 1) return with(std::integral_constant<Input, Input::kJoined>{});
+        if (prepared && p.slabs == 1) return with(std::integral_constant<Input, Input::kJoined>{});
         if (staged) return with(std::integral_constant<Input, Input::kStaged>{});
         if (a->group_rows > 0) return with(std::integral_constant<Input, Input::kGrouped>{});
         return with(std::integral_constant<Input, Input::kPlain>{});
