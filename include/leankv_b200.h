@@ -320,6 +320,13 @@ int leankv_decode_qkv_post(const void* qkv, const float* inv_freq, const int32_t
                            const float* Pi_k_t, const float* Pi_v_t, const float* decision_boundaries,
                            void* pool, int n_pages, const int32_t* page_indices,
                            int n_q_heads, int n_kv_heads, float* q_rot, void* stream);
+/* The same with flags. LEANKV_POST_EARLY: position, page table and the page itself may be read while the launch ahead of this one still
+ * runs: that launch must write nothing that this one reads but qkv (in a decode loop it is the projection). */
+#define LEANKV_POST_EARLY 1
+int leankv_decode_qkv_post_flags(const void* qkv, const float* inv_freq, const int32_t* state,
+                                 const float* Pi_k_t, const float* Pi_v_t, const float* decision_boundaries,
+                                 void* pool, int n_pages, const int32_t* page_indices,
+                                 int n_q_heads, int n_kv_heads, float* q_rot, int flags, void* stream);
 /* *token = argmax(logits) (lowest index on ties); history[state[1]] = *token;
  * state[1] += 1; state[0] += 1. */
 int leankv_decode_end(const void* logits, int vocab, long long* token, long long* history,
@@ -406,6 +413,11 @@ int leankv_batch_qkv_post(const void* qkv, int B, const float* inv_freq, const i
                           const float* decision_boundaries, void* pool, int n_pages,
                           const int32_t* kv_page_indices, int n_q_heads, int n_kv_heads,
                           float* q_rot, void* stream);
+int leankv_batch_qkv_post_flags(const void* qkv, int B, const float* inv_freq, const int32_t* pos,
+                                const int32_t* kv_indptr, const float* Pi_k_t, const float* Pi_v_t,
+                                const float* decision_boundaries, void* pool, int n_pages,
+                                const int32_t* kv_page_indices, int n_q_heads, int n_kv_heads,
+                                float* q_rot, int flags, void* stream);
 /* y[rows][N] = x[rows][K] W[K][N], fp16 with fp32 sums, for up to 128 rows: the projections of a batched step. K % 8 == 0,
  * N % 8 == 0, everything 16-byte aligned. With early_weights W may be read while the launch ahead of this one still runs: that launch must
  * not write it. Where a wait inside the kernel runs out, the outputs are NaN. */

@@ -22,6 +22,7 @@ TQ_PAGE_TOKENS = 16
 TQ_DIM = 128
 TQ_CHUNK_BYTES = 800
 ATTN_EARLY_FETCH = 1
+POST_EARLY = 1
 
 
 class Segments(Structure):
@@ -92,6 +93,10 @@ SIGNATURES = {
                                               c_float, c_void_p, c_size_t, c_int, c_void_p]),
     "leankv_decode_qkv_post": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p]),
+    "leankv_decode_qkv_post_flags": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+                                             c_void_p, c_int, c_int, c_void_p, c_int, c_void_p]),
+    "leankv_batch_qkv_post_flags": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                            c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p]),
     "leankv_tq_decode_attn_status": (c_int, [c_void_p, POINTER(c_int)]),
     "leankv_tq_pool_append_strided": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                                               c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,

@@ -132,11 +132,11 @@ class BatchDecodeEngine(DecodeEngine):
         self._norm_rows(None, self.w["layers"][0]["ln1"])
         for l, lw in enumerate(self.w["layers"]):
             self._mm(self.x, lw["wqkv_t"], self.qkv)
-            _native.check(lib.leankv_batch_qkv_post(
+            _native.check(lib.leankv_batch_qkv_post_flags(
                 self.qkv.data_ptr(), B, self.inv_freq.data_ptr(), self.pos.data_ptr(), self.kv_indptr.data_ptr(),
                 self.Pi_k_t[l].data_ptr(), self.Pi_v_t[l].data_ptr(), self.bounds.data_ptr(),
                 self.pools[l].data_ptr(), self.max_pages, self.kv_page_indices.data_ptr(), self.nq, self.nkv,
-                self.q_rot.data_ptr(), st()), "batch_qkv_post")
+                self.q_rot.data_ptr(), _native.POST_EARLY, st()), "batch_qkv_post")
             _native.check(lib.leankv_tq_decode_attn_rotated(
                 self.q_rot.data_ptr(), self.attn.data_ptr(), B, self.nq, self.nkv, self.pools[l].data_ptr(),
                 self.max_pages, self.kv_indptr.data_ptr(), self.kv_page_indices.data_ptr(),

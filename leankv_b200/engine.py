@@ -342,11 +342,12 @@ class DecodeEngine(DecodeLoop):
         probe("qkv")
         if self.fused_post:
             # rope(q, k) + rotate/quantize/pack of k, v into the page + query rotation: one launch
-            _native.check(lib.leankv_decode_qkv_post(self.qkv.data_ptr(), self.inv_freq.data_ptr(), sp,
+            _native.check(lib.leankv_decode_qkv_post_flags(self.qkv.data_ptr(), self.inv_freq.data_ptr(), sp,
                                                      self.Pi_k_t[l].data_ptr(), self.Pi_v_t[l].data_ptr(),
                                                      self.bounds.data_ptr(), self.pools[l].data_ptr(),
                                                      self.max_pages, self.page_indices.data_ptr(), self.nq,
-                                                     self.nkv, self.q_rot.data_ptr(), st()), "decode_qkv_post")
+                                                     self.nkv, self.q_rot.data_ptr(), _native.POST_EARLY, st()),
+                          "decode_qkv_post")
             _native.check(lib.leankv_tq_decode_attn_rotated(
                 self.q_rot.data_ptr(), self.attn.data_ptr(), 1, self.nq, self.nkv, self.pools[l].data_ptr(),
                 self.max_pages, sp + 8, self.page_indices.data_ptr(), sp + 16, self.max_pages,
