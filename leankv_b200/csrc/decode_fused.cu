@@ -31,14 +31,14 @@ struct PostParams {
     const int32_t* page_indices;
     int nq, nkv;
     float* q_rot;             // [B][nq][128]
-    int early;                // positions, page table and pages may be read while the launch ahead still runs
 };
 
 // A CTA serves one head for kSeqs sequences at a time, its rotation column in registers. What bounds it is the chain of
 // one vector (the fp64 sum of 64 squares alone is 64 dependent steps), not any unit, so a batch takes four sequences
-// through the chain together: 32 sequences, 48 heads: 21.9 -> 12.6 us. With `early` position, page, shared word and rotary angles are there
-// when the projections are: four steps of 32 layers of one sequence 8577 us without this order, 8375 with it, 8210 with `early`.
-template <int kSeqs>
+// through the chain together: 32 sequences, 48 heads: 21.9 -> 12.6 us. With kEarly position, page, shared word and rotary angles are there
+// when the projections are: four steps of 32 layers of one sequence 8577 -> 8215 us; alone one sequence 3.5 -> 2.3, a batch of
+// 32 10.3 -> 9.5 without and 8.7 with kEarly, of 80 24.4 -> 22.5 and 23.5.
+template <int kSeqs, bool kEarly>
 __global__ void __launch_bounds__(kDim, kSeqs > 1 ? 3 : 1) decode_qkv_post_kernel(const PostParams p) {
     __shared__ float s_x[kSeqs][kDim];       // the head vectors (after rotary embedding, fp16 values)
     __shared__ __align__(16) float s_u[kSeqs][kDim];   // what gets rotated: x for q, x / (norm + 1e-10) for k and v
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kDim, kSeqs > 1 ? 3 : 1) decode_qkv_post_kerne
     const int row = (p.nq + 2 * p.nkv) * kDim;
     const int which = kind - 1;
     const int h = which == 0 ? head - p.nq : head - p.nq - p.nkv;
-    // Where the new tokens go, the word of V shared with the pair token, and the rotary angles: with `early` the first sequences' are there
+    // Where the new tokens go, the word of V shared with the pair token, and the rotary angles: with kEarly the first sequences' are there
     // when the projections are, else they are fetched beside the row, so that nothing trails the arithmetic.
     int slot[kSeqs];
     uint32_t* words[kSeqs];
@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(kDim, kSeqs > 1 ? 3 : 1) decode_qkv_post_kerne
     };
     // one sequence: the code of `locate` once, around the wait; a batch: ahead of it and in the loop
     const int first = blockIdx.y * kSeqs;
-    bool waited = kSeqs > 1 || !p.early;
-    if (kSeqs > 1 && p.early) locate(first);
+    bool waited = kSeqs > 1 || !kEarly;
+    if (kSeqs > 1 && kEarly) locate(first);
     if (waited) pdl_begin();
     for (int b0 = first; b0 < p.B; b0 += gridDim.y * kSeqs) {
         __half xr[kSeqs], other[kSeqs];
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kDim, kSeqs > 1 ? 3 : 1) decode_qkv_post_kerne
             }
         };
         if (waited) load_rows();
-        if (kSeqs == 1 || !p.early || b0 != first) locate(b0);
+        if (kSeqs == 1 || !kEarly || b0 != first) locate(b0);
         if (!waited) {
             pdl_begin();
             waited = true;
@@ -249,17 +249,18 @@ static int post_launch(const void* qkv, int B, const float* inv_freq, const int3
     p.nq = n_q_heads;
     p.nkv = n_kv_heads;
     p.q_rot = q_rot;
-    p.early = (flags & LEANKV_POST_EARLY) != 0;
     // One sequence alone keeps the kernel whose chain is its only work; a batch goes four at a time, over as many CTAs as are
     // resident at once (two or three an SM), each of which walks the rest of its head's sequences with the same column.
     const int heads = n_q_heads + 2 * n_kv_heads;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const bool early = (flags & LEANKV_POST_EARLY) != 0;
     if (B == 1) {
-        LEANKV_CUDA_TRY(launch_kernel_ex(true, decode_qkv_post_kernel<1>, dim3(heads, 1), dim3(kDim), 0, st, p));
+        LEANKV_CUDA_TRY(launch_kernel_ex(true, early ? decode_qkv_post_kernel<1, true> : decode_qkv_post_kernel<1, false>, dim3(heads, 1), dim3(kDim), 0, st, p));
     } else {
         constexpr int kSeqs = 4;
         const int gy = std::max(1, std::min((B + kSeqs - 1) / kSeqs, 3 * sm_count() / heads));
-        LEANKV_CUDA_TRY(launch_kernel_ex(true, decode_qkv_post_kernel<kSeqs>, dim3(heads, gy), dim3(kDim), 0, st, p));
+        LEANKV_CUDA_TRY(launch_kernel_ex(true, early ? decode_qkv_post_kernel<kSeqs, true> : decode_qkv_post_kernel<kSeqs, false>,
+                                         dim3(heads, gy), dim3(kDim), 0, st, p));
     }
     return LEANKV_OK;
 }
