@@ -426,6 +426,11 @@ int leankv_skinny_gemm_f16(const void* x, const void* w, void* y, int rows, int 
 int leankv_silu_mul_f16(const void* gate_up, void* out, int rows, int inter, void* stream);
 /* The same of two matrices fp16 [rows][inter]; out may be either of them. */
 int leankv_silu_mul_pair_f16(const void* gate, const void* up, void* out, int rows, int inter, void* stream);
+/* What the layers of a prompt chunk at positions start .. start + T - 1 share: cos, sin fp16 [T][128] for leankv_rope_split_f16 (of fp32
+ * angles position * inv_freq[64], halves equal), and indptr = {0, pages of start + T tokens}, *start_out = start for the append.
+ * inv_freq may be read while the launch ahead of this one still runs. */
+int leankv_prompt_begin_f16(const float* inv_freq, int T, int start, void* cos, void* sin, int32_t* indptr, int32_t* start_out,
+                            void* stream);
 /* A prompt chunk's projections, fp16 [T][n_q_heads + 2 n_kv_heads][128], apart: queries [T][n_q_heads][128] and keys
  * [n_kv_heads][T][128] with the rotary embedding (rotate_half form; cos, sin: fp16 [T][128]), values [n_kv_heads][T][128]. */
 int leankv_rope_split_f16(const void* qkv, const void* cos, const void* sin, void* q, void* k, void* v, int T,

@@ -65,8 +65,9 @@ class BatchDecodeEngine(DecodeEngine):
         self.centroids = self.centroids_host.to(dev)
         self.bounds = bounds[1:-1].float().contiguous().to(dev)
 
-        self.pools = [torch.zeros(self.max_pages, 2, self.nkv, _native.TQ_CHUNK_BYTES, dtype=torch.uint8,
-                                  device=dev) for _ in range(L)]
+        # one store, so that a prompt clears it in one launch
+        self._pool_store = torch.zeros(L, self.max_pages, 2, self.nkv, _native.TQ_CHUNK_BYTES, dtype=torch.uint8, device=dev)
+        self.pools = list(self._pool_store)
         # every sequence owns pps pages, scattered over the pool
         perm = torch.randperm(self.max_pages, generator=torch.Generator().manual_seed(tq_seed))
         self.block_table = perm.to(torch.int32).reshape(batch, self.pps).contiguous().to(dev)
@@ -199,8 +200,7 @@ class BatchDecodeEngine(DecodeEngine):
         if chunk < 1 or (attention == "dense" and chunk < T):
             raise ValueError("chunk must be positive; the dense route handles whole prompts only")
         with torch.cuda.device(self.dev):
-            for p in self.pools:
-                p.zero_()
+            self._pool_store.zero_()
             last = []
             for b in range(self.B):
                 for s0 in range(0, T, chunk):

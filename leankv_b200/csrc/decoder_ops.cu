@@ -277,6 +277,31 @@ __global__ void __launch_bounds__(256) rope_split_kernel(const __half* qkv, cons
     reinterpret_cast<uint4*>(dst)[c + 8] = hi;
 }
 
+// What the layers of a prompt chunk share: the rotary tables fp16 [T][128] of positions start .. start + T - 1 (halves equal; angles,
+// cosines and sines in fp32, as in rope_kernel), and the two small vectors that the append reads. As tensor operations and two uploads
+// this was eleven launches and a wait of the host for the device in front of every chunk. Here one launch: 40 tokens through two
+// layers of width 1024, where the launches are the time, 677 -> 586 us; 600 in three chunks through four of 2048, 2485 -> 2222.
+__global__ void __launch_bounds__(256) prompt_begin_kernel(const float* inv_freq, int T, int start, int n_pages, __half* cos_t,
+                                                           __half* sin_t, int32_t* indptr, int32_t* start_out) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    const int t = (int)(i >> 5), j = (int)(i & 31);                      // two neighbouring angles of a token
+    const float pos = (float)(start + min(t, T - 1));
+    const float2 rate = __ldg(reinterpret_cast<const float2*>(inv_freq) + j);
+    const float a = pos * rate.x, b = pos * rate.y;
+    const __half2 c = __floats2half2_rn(cosf(a), cosf(b)), s = __floats2half2_rn(sinf(a), sinf(b));
+    pdl_begin();
+    if (i == 0) {
+        indptr[0] = 0;
+        indptr[1] = n_pages;
+        *start_out = start;
+    }
+    if (t >= T) return;
+    __half2* ct = reinterpret_cast<__half2*>(cos_t + (size_t)t * 128) + j;
+    __half2* st = reinterpret_cast<__half2*>(sin_t + (size_t)t * 128) + j;
+    ct[0] = c; ct[32] = c;
+    st[0] = s; st[32] = s;
+}
+
 }  // namespace
 }  // namespace leankv
 
@@ -408,6 +433,18 @@ extern "C" int leankv_silu_mul_pair_f16(const void* gate, const void* up, void* 
     if (!gate || !up || !out || rows <= 0 || inter <= 0) return LEANKV_EINVAL;
     if (inter % 8 != 0 || !aligned16(gate) || !aligned16(up) || !aligned16(out)) return LEANKV_EALIGN;
     return launch_silu_mul(gate, up, (size_t)inter, out, rows, inter, stream);
+}
+
+extern "C" int leankv_prompt_begin_f16(const float* inv_freq, int T, int start, void* cos, void* sin, int32_t* indptr,
+                                       int32_t* start_out, void* stream) {
+    if (!inv_freq || !cos || !sin || !indptr || !start_out || T <= 0 || start < 0) return LEANKV_EINVAL;
+    if (start > 0x7fffffff - 15 - T) return LEANKV_ELIMIT;
+    if (!aligned16(inv_freq) || !aligned16(cos) || !aligned16(sin)) return LEANKV_EALIGN;
+    const long long blocks = ((long long)T * 32 + 255) / 256;
+    LEANKV_CUDA_TRY(launch_early(prompt_begin_kernel, dim3((unsigned)blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                 inv_freq, T, start, (start + T + 15) / 16, static_cast<__half*>(cos), static_cast<__half*>(sin),
+                                 indptr, start_out));
+    return LEANKV_OK;
 }
 
 extern "C" int leankv_rope_split_f16(const void* qkv, const void* cos, const void* sin, void* q, void* k, void* v, int T,

@@ -123,8 +123,9 @@ class DecodeEngine(DecodeLoop):
 
         # paged pool, one tensor per layer; the sequence's pages are assigned up front in a
         # shuffled order so that the page table is exercised
-        self.pools = [torch.zeros(self.max_pages, 2, self.nkv, _native.TQ_CHUNK_BYTES, dtype=torch.uint8,
-                                  device=dev) for _ in range(L)]
+        # one store, so that a prompt clears it in one launch
+        self._pool_store = torch.zeros(L, self.max_pages, 2, self.nkv, _native.TQ_CHUNK_BYTES, dtype=torch.uint8, device=dev)
+        self.pools = list(self._pool_store)
         perm = torch.randperm(self.max_pages, generator=torch.Generator().manual_seed(tq_seed))
         self.page_indices = perm.to(torch.int32).to(dev)
 
@@ -540,14 +541,12 @@ class DecodeEngine(DecodeLoop):
             if self._prefill_ws is None or self._prefill_ws.numel() < need:
                 self._prefill_ws = _native.grown_workspace(self._prefill_ws, need, self.dev, cleared=False)
             attn_out = torch.empty(T, self.nq, 128, dtype=torch.float16, device=self.dev)
-        pos = torch.arange(start_pos, start_pos + T, device=self.dev).float()
-        ang = torch.outer(pos, self.inv_freq)
-        emb = torch.cat((ang, ang), dim=-1)
-        cos, sin = emb.cos().half().unsqueeze(1), emb.sin().half().unsqueeze(1)
         h = self.w["embed"][ids]
-        n_pages = (start_pos + T + PAGE - 1) // PAGE
-        indptr = torch.tensor([0, n_pages], dtype=torch.int32, device=self.dev)
-        start = torch.full((1,), start_pos, dtype=torch.int32, device=self.dev)
+        cos, sin = torch.empty(2, T, 128, dtype=torch.float16, device=self.dev)
+        indptr = torch.empty(8, dtype=torch.int32, device=self.dev)
+        start = indptr[2:]
+        _native.check(self.lib.leankv_prompt_begin_f16(self.inv_freq.data_ptr(), T, start_pos, cos.data_ptr(), sin.data_ptr(),
+                                                       indptr.data_ptr(), start.data_ptr(), self._st()), "prompt_begin")
 
         def note(l, name, t):
             if collect is not None:
@@ -602,7 +601,7 @@ class DecodeEngine(DecodeLoop):
             note(l, "down_proj", m)
             d = m @ lw["wdown_t"]
             self._allreduce(d)
-        return _rmsnorm(h[-1] if d is None else h[-1] + d[-1], self.w["final_norm"], cfg.rms_eps)
+        return self._add_norm(h[-1:], None if d is None else d[-1:], self.w["final_norm"])[1][0]
 
     def _add_norm(self, h, delta, w):
         """(h + delta, its RMSNorm) of every row; h, which the prompt pass owns, is updated in place where the kernel takes
@@ -723,22 +722,23 @@ class DecodeEngine(DecodeLoop):
         if attention == "dense" and chunk < T:
             raise ValueError("the dense route handles whole prompts only")
         with torch.cuda.device(self.dev):
-            for p in self.pools:
-                p.zero_()
+            self._pool_store.zero_()
             for s0 in range(0, T, chunk):
                 x = self._dense_forward(ids[s0:s0 + chunk], write_cache=True, start_pos=s0,
                                         attention=attention)
-            if attention == "packed":
-                self._check_prefill_status()
-            logits = x @ self.w["lm_head_t"]
-            tok = torch.argmax(logits.float()).reshape(1)
-            self.token.copy_(tok)
             self.history.zero_()
-            self.history[0] = tok[0]
             self.state.zero_()
-            self.state[0], self.state[1] = T, 1
+            self.state[0].fill_(T)
+            self.state[1].fill_(1)
+            logits = x @ self.w["lm_head_t"]
+            tok = torch.argmax(logits).reshape(1)
+            self.token.copy_(tok)
+            self.history[:1].copy_(tok)
             self.prefill_logits = logits
-        return int(tok.item())
+            first = int(tok.item())
+            if attention == "packed":
+                self._check_prefill_status()      # behind the tail's launches: it waits for the device
+        return first
 
     def bytes_streamed(self) -> int:
         """Weight bytes the sparse GEMVs have streamed since the counter was last zeroed."""

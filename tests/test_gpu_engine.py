@@ -395,6 +395,23 @@ def test_prompt_pass_glue_kernels(T, n_q, n_kv, inter):
     assert ((gate - want).double().abs() <= want.double().abs() * 2.0 ** -10 + 2.0 ** -24)[finite].all()
 
 
+@pytest.mark.parametrize("T,start", [(1, 0), (1, 16383), (7, 9), (8, 8), (9, 100000), (257, 15), (2048, 4096)])
+def test_prompt_begin(T, start):
+    """The tables of the tensor operations: fp32 angle, cosine and sine of either are the same functions, so the same bits."""
+    from leankv_b200 import _native
+
+    dev = _dev()
+    inv_freq = (1.0 / (10000.0 ** (torch.arange(0, 128, 2).float() / 128))).to(dev)
+    tables = torch.full((2, T + 1, 128), 7.0, dtype=torch.float16, device=dev)       # a row behind each that stays
+    small = torch.full((8,), -1, dtype=torch.int32, device=dev)
+    _native.check(_native.lib().leankv_prompt_begin_f16(inv_freq.data_ptr(), T, start, tables[0].data_ptr(), tables[1].data_ptr(),
+                                                        small.data_ptr(), small[2:].data_ptr(), None), "prompt_begin")
+    ang = torch.outer(torch.arange(start, start + T, device=dev).float(), inv_freq)
+    for got, f in zip(tables, (torch.cos, torch.sin)):
+        assert torch.equal(got[:T], torch.cat([f(ang), f(ang)], -1).half()) and (got[T] == 7.0).all()
+    assert small.tolist() == [0, (start + T + 15) // 16, start, -1, -1, -1, -1, -1]
+
+
 def test_a_prompt_whose_first_chunk_failed_is_refused():
     """The status word is read once, after the last chunk: a chunk that needs a longer workspace may not drop it."""
     cfg = DecoderConfig(vocab_size=512, hidden_size=512, intermediate_size=1024, num_layers=1, num_q_heads=8, num_kv_heads=2)
