@@ -99,6 +99,9 @@ typedef struct leankv_stream_norm {
 
 int leankv_stream_norm(const leankv_stream_norm_t* args, void* stream);
 
+/* x[r] = row ids[r] (0 where it is outside the vocabulary) of table [vocab][width], as fp32; rows of x follow one another. */
+int leankv_embed_rows(const void* table, int dtype, const long long* ids, int rows, int width, int vocab, float* x, void* stream);
+
 /* out = silu(gate) * up; gate_up [rows][2 * inter], gate columns first. */
 int leankv_silu_mul(const void* gate_up, void* out, int dtype, int rows, int inter, void* stream);
 

@@ -243,6 +243,7 @@ class CausalStep(Structure):
 MIXER_SIGNATURES = {
     "leankv_dense_gemv": (c_int, [POINTER(DenseGemv), c_void_p]),
     "leankv_embed_begin": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p]),
+    "leankv_embed_rows": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
     "leankv_greedy_end": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
     "leankv_stream_norm": (c_int, [POINTER(StreamNorm), c_void_p]),
     "leankv_silu_mul": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),

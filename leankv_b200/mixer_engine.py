@@ -333,7 +333,9 @@ class MixerDecodeEngine(DecodeLoop):
     def _portion(self, ids: torch.Tensor) -> torch.Tensor:
         """Run the tokens ``ids`` at the current position; returns the fp32 stream [T][width] after the last layer."""
         T, W, dev = ids.numel(), self.cfg.hidden_size, self.dev
-        x = self.embed[ids].float()
+        x = torch.empty(T, W, dtype=torch.float32, device=dev)
+        _native.check(self.lib.leankv_embed_rows(self.embed.data_ptr(), dtype_code(self.dtype), ids.data_ptr(), T, W,
+                                                 self.cfg.vocab_size, x.data_ptr(), self._st()), "embed_rows", self.lib)
         h = torch.empty(T, W, dtype=self.dtype, device=dev)
         delta = join = None
         for l in self.layers:
@@ -351,8 +353,9 @@ class MixerDecodeEngine(DecodeLoop):
             self.stream_probe(x)
         self.pos += T
         self._parity ^= 1
-        self.state[0] = self.pos
-        self.state[_native.STATE_PARITY] = self._parity
+        # by kernels: an assignment uploads the number and waits for the whole portion
+        self.state[0].fill_(self.pos)
+        self.state[_native.STATE_PARITY].fill_(self._parity)
         return x
 
     def _logits_of(self, x: torch.Tensor) -> torch.Tensor:
@@ -443,5 +446,5 @@ class MixerDecodeEngine(DecodeLoop):
             self.token.copy_(tok)
             self.history.zero_()
             self.history[0] = tok[0]
-            self.state[1] = 1
+            self.state[1].fill_(1)
         return int(tok.item())

@@ -90,6 +90,20 @@ def test_gemv_row_groups_with_an_input_each(dtype, groups, n, cols, stride):
     assert rel(y, want) < 1e-5
 
 
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("rows,width", [(1, 8), (3, 1), (5, 2056), (7, 131), (2049, 64)])
+def test_embed_rows(dtype, rows, width):
+    """Whole trips, remainders and odd widths; a token outside the table reads row 0; nothing behind the last row is written."""
+    gen = torch.Generator().manual_seed(width)
+    table = torch.randn(19, width, generator=gen).to(dtype).cuda()
+    ids = torch.randint(0, 19, (rows,), generator=gen).cuda()
+    ids[-1], want = 19, table[ids.clamp(max=18)].float()
+    want[-1] = table[0].float()
+    x = torch.full((rows + 1, width), 5.0, device="cuda")
+    ok(_native.mixers().leankv_embed_rows(table.data_ptr(), CODE[dtype], ids.data_ptr(), rows, width, 19, x.data_ptr(), stream()))
+    assert torch.equal(x[:rows], want) and (x[rows] == 5.0).all()
+
+
 def test_softcap_in_the_head_and_on_rows():
     w, x = rnd(50, 24, seed=1, std=3.0), rnd(24, seed=2)
     wd, xd, y = w.to(DEV), x.to(DEV), torch.empty(50, device=DEV)
