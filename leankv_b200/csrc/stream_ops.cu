@@ -191,15 +191,14 @@ __global__ void __launch_bounds__(256) silu_mul_rows_kernel(const T* gate_up, T*
     }
 }
 
-// Eight elements per thread (inter % 8 == 0, aligned).
+// Eight elements per thread (inter % 8 == 0, aligned), a block for every 2048 columns of a row: with as many blocks as fit twice the
+// last round was nearly empty (2048 x 7168 in bf16: 17.9 us, so 15.9).
 template <typename T>
-__global__ void __launch_bounds__(256) silu_mul_vec_kernel(const T* gate_up, T* out, int inter, long long total8) {
+__global__ void __launch_bounds__(256) silu_mul_vec_kernel(const T* gate_up, T* out, int inter, int rows) {
     pdl_begin();
-    const int n8 = inter >> 3;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total8;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long r = i / n8;
-        const int c = (int)(i - r * n8) * 8;
+    const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
+    if (c >= inter) return;
+    for (long long r = blockIdx.y; r < rows; r += gridDim.y) {
         Raw8<T> rg, ru;
         load8(gate_up + r * 2 * inter + c, rg);
         load8(gate_up + r * 2 * inter + inter + c, ru);
@@ -349,12 +348,16 @@ extern "C" int leankv_silu_mul(const void* gate_up, void* out, int dtype, int ro
     if (!known(dtype)) return LEANKV_EUNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool vec = inter % 8 == 0 && aligned16(gate_up) && aligned16(out);
-    const long long total = (long long)rows * inter / (vec ? 8 : 1);
+    const long long total = (long long)rows * inter;
     const int grid = (int)std::min<long long>((total + 255) / 256, (long long)sm_count() * 16);
     auto go = [&](auto tag) -> int {
         using T = decltype(tag);
-        LEANKV_CUDA_TRY(launch_early(vec ? silu_mul_vec_kernel<T> : silu_mul_rows_kernel<T>, dim3(grid), dim3(256), 0,
-                                      st, static_cast<const T*>(gate_up), static_cast<T*>(out), inter, total));
+        if (vec)
+            LEANKV_CUDA_TRY(launch_early(silu_mul_vec_kernel<T>, dim3((inter / 8 + 255) / 256, std::min(rows, 65535)), dim3(256), 0, st,
+                                         static_cast<const T*>(gate_up), static_cast<T*>(out), inter, rows));
+        else
+            LEANKV_CUDA_TRY(launch_early(silu_mul_rows_kernel<T>, dim3(grid), dim3(256), 0, st, static_cast<const T*>(gate_up),
+                                         static_cast<T*>(out), inter, total));
         return LEANKV_OK;
     };
     return dtype == LEANKV_DT_BF16 ? go(bf16{}) : go(float{});

@@ -104,6 +104,25 @@ def test_embed_rows(dtype, rows, width):
     assert torch.equal(x[:rows], want) and (x[rows] == 5.0).all()
 
 
+@pytest.mark.parametrize("rows,inter", [(1, 2040), (2, 2048), (3, 2056), (65537, 8)])
+def test_silu_mul_by_rows(rows, inter):
+    """Blocks of 2048 columns, their remainders, and more rows than a grid has; fp32 against 64 bits, bf16 to one rounding."""
+    gu = rnd(rows, 2 * inter, seed=inter, std=3.0).cuda()
+    for dtype, bound in ((F32, 2e-6), (BF16, 2.0 ** -8)):
+        x = gu.to(dtype)
+        out = torch.full((rows + 1, inter), 5.0, dtype=dtype, device="cuda")
+        ok(_native.mixers().leankv_silu_mul(x.data_ptr(), out.data_ptr(), CODE[dtype], rows, inter, stream()))
+        g, u = x.double().split(inter, dim=1)
+        want = torch.nn.functional.silu(g) * u
+        assert ((out[:rows] - want).abs() <= bound * want.abs() + 1e-30).all() and (out[rows] == 5.0).all()
+    h = gu.clamp(-20, 20).half()
+    out = torch.full((rows + 1, inter), 5.0, dtype=torch.float16, device="cuda")
+    _native.check(_native.lib().leankv_silu_mul_f16(h.data_ptr(), out.data_ptr(), rows, inter, stream()), "silu_mul")
+    g, u = h.double().split(inter, dim=1)
+    want = torch.nn.functional.silu(g) * u           # two fp16 roundings, and silu's own may be subnormal
+    assert ((out[:rows] - want).abs() <= 2.0 ** -10 * want.abs() + 2.0 ** -24 * (1 + u.abs())).all() and (out[rows] == 5.0).all()
+
+
 def test_softcap_in_the_head_and_on_rows():
     w, x = rnd(50, 24, seed=1, std=3.0), rnd(24, seed=2)
     wd, xd, y = w.to(DEV), x.to(DEV), torch.empty(50, device=DEV)
