@@ -441,6 +441,9 @@ int leankv_batch_decode_end(const void* logits, int vocab, int B, long long* tok
                             long long* history, int history_cap, int32_t* pos, int32_t* steps,
                             void* stream);
 
+/* A new page table: words[0 .. zeros) = 0, the stack of free pages words[zeros + i] = i up to the word `top` behind it (at least
+ * zeros + max_pages), words[top] = max_pages, the stack's height. */
+int leankv_paged_table_begin(int32_t* words, int zeros, int max_pages, int top, void* stream);
 /* ------------------------------------------------------------------------- *
  * Page table of a paged cache, kept on the device. Replaces the host loops of
  * leankv/turboquant/paged_cache.py: _allocate_page (:96-103, LIFO free list), the page assignment

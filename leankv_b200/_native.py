@@ -129,6 +129,7 @@ SIGNATURES = {
                                           c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "leankv_batch_qkv_post": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                       c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p]),
+    "leankv_paged_table_begin": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p]),
     "leankv_paged_table_step": (c_int, [c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "leankv_skinny_gemm_f16": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),

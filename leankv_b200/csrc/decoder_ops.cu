@@ -481,6 +481,14 @@ namespace {
 
 constexpr int kTableThreads = 1024;
 
+// A new page table in one launch: `zeros` words of zero in front of the stack of free pages 0, 1, .., n - 1 and its height. As three
+// tensor operations: clearing a cache took the host 45 - 59 us, so 38 - 41; a prompt of 2048 tokens in four chunks 305 -> 291.
+__global__ void __launch_bounds__(256) paged_table_begin_kernel(int32_t* words, int zeros, int n, int top) {
+    pdl_begin();
+    for (long long i = blockIdx.x * 256 + threadIdx.x; i <= top; i += gridDim.x * 256)
+        words[i] = i < zeros ? 0 : i < top ? (int)i - zeros : n;
+}
+
 // One CTA. Sequence b grows by t_new tokens: it takes the pages it lacks from the top of the free
 // stack (sequence 0 first, as the reference's loop does), its length advances, and the flat
 // (kv_indptr, kv_page_indices, kv_last_page_len, start_pos) arrays of the append / attention calls are
@@ -558,6 +566,14 @@ __global__ void __launch_bounds__(kTableThreads) paged_table_step_kernel(
 
 }  // namespace
 }  // namespace leankv
+
+extern "C" int leankv_paged_table_begin(int32_t* words, int zeros, int max_pages, int top, void* stream) {
+    if (!words || zeros < 0 || max_pages <= 0 || top < zeros || top - zeros < max_pages) return LEANKV_EINVAL;
+    const int grid = std::min(top / 256 + 1, sm_count() * 8);
+    LEANKV_CUDA_TRY(launch_early(paged_table_begin_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream), words, zeros,
+                                 max_pages, top));
+    return LEANKV_OK;
+}
 
 extern "C" int leankv_paged_table_step(int t_new, int B, int32_t* seq_len, int32_t* block_table,
                                        int max_pages_per_seq, int32_t* free_stack, int32_t* free_top,

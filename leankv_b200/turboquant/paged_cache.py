@@ -100,17 +100,26 @@ class PagedKVCache:
         rows = max(batch_cap, 1)
         self._batch_cap = rows
         self._pps_cap = self.max_pages                       # a single sequence may take the whole pool
-        # one zeroed allocation, each array from a 16-byte boundary on
+        # one allocation, each array from a 16-byte boundary on
         sizes = [rows * self._pps_cap, rows, rows + 1, rows, rows]
         if old_table is None:
-            sizes += [self.max_pages, 1]
-        views = torch.zeros(sum(-(-n // 4) * 4 for n in sizes), dtype=i32, device=dev).split([-(-n // 4) * 4 for n in sizes])
+            sizes += [self.max_pages, 1, self.max_pages, 1]
+        padded = [-(-n // 4) * 4 for n in sizes]
+        new = old_table is None and dev.type == "cuda"
+        store = (torch.empty if new else torch.zeros)(sum(padded), dtype=i32, device=dev)
+        views = store.split(padded)
         self._block_table = views[0][:sizes[0]].view(rows, self._pps_cap)
         self._seq_len_dev, self._kv_indptr, self._kv_last, self._start_dev = (v[:n] for v, n in zip(views[1:5], sizes[1:5]))
         if old_table is None:
-            self._kv_page_indices, self._status = views[5][:self.max_pages], views[6][:1]
-            self._free_stack = torch.arange(self.max_pages, dtype=i32, device=dev)
-            self._free_top = torch.full((1,), self.max_pages, dtype=i32, device=dev)
+            self._kv_page_indices, self._status, self._free_stack, self._free_top = (v[:n] for v, n in zip(views[5:], sizes[5:]))
+            if new:
+                with _native.on_device(dev):
+                    rc = _native.lib().leankv_paged_table_begin(store.data_ptr(), sum(padded[:7]), self.max_pages, sum(padded[:8]),
+                                                                _native.current_stream())
+                _native.check(rc, "leankv_paged_table_begin")
+            else:
+                torch.arange(self.max_pages, out=self._free_stack)
+                self._free_top.fill_(self.max_pages)
         else:
             n = old_table.shape[0]
             self._block_table[:n] = old_table

@@ -523,6 +523,15 @@ def test_tensor_core_append_writes_the_same_pool_as_the_fp32_kernel_on_all_of_co
     assert out["fp32"][2] == 0
 
 
+@pytest.mark.parametrize("zeros,pages,top", [(0, 1, 1), (5, 3, 8), (251, 4, 256), (700000, 300001, 1000004)])
+def test_paged_table_begin(zeros, pages, top):
+    """Around a block and beyond one round of the grid; the word behind the height stays."""
+    words = torch.full((top + 2,), -7, dtype=torch.int32, device=_dev())
+    _native.check(_native.lib().leankv_paged_table_begin(words.data_ptr(), zeros, pages, top, None), "paged_table_begin")
+    assert not words[:zeros].any() and words[zeros:zeros + pages].tolist() == list(range(pages))
+    assert words[top:].tolist() == [pages, -7]
+
+
 def test_paged_cache_page_table_on_device_follows_the_reference_allocator():
     """Pages are handed out by the device kernel exactly as the reference's host loops would
     (LIFO free list, sequence 0 first, one shared table for all layers), including reuse after a
