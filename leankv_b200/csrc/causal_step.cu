@@ -133,6 +133,7 @@ __device__ __forceinline__ uint32_t transpose8(uint32_t x) {
 // The cluster waits for the CTA that makes the new row, so that CTA's chain is kept short: the row is asked for together with the
 // queries, the zeros behind it are written while the launch ahead drains, and the gates' logistic function is taken under the cluster
 // barrier. A step of four layers of width 2048 at 2100 positions 230.1 -> 224.3 us (its wait at the barrier 9400 -> 3700 cycles of 27 000).
+// Alone, 4 / 8 kv heads: 2184 keys 13.1 -> 11.6 and 14.1 -> 12.4 us; 32768 keys, where the stream is the time, 40.9 -> 40.0 and 38.6 -> 40.8.
 // NP: 16-column pieces of the values that a warp accumulates at most (tensor cores).
 template <Walk W, int NP>
 __global__ void __launch_bounds__(32 * warps_of(W), W == Walk::kWarps ? 2 : 1) causal_step_kernel(const __grid_constant__ StepArgs p) {

@@ -80,9 +80,11 @@ __device__ __forceinline__ void fetch4(const bf16* p, float (&v)[4]) {
 }
 
 // The same with 4-element accesses and rows in registers (width % 4 == 0, width <= kRowThreads * 4 * NV). A CTA
-// walks `per_cta` consecutive rows and keeps the row above, so only its first row is normed twice. A row's stream and branch are asked for
-// together and its two sums cost a barrier each (2048 x 2048 with a normed branch 13.2 us when the branch was read twice, now 12.0: 59 MB).
-template <typename T, typename D, int NV>
+// walks `per_cta` consecutive rows and keeps the row above, so only its first row is normed twice. With a normed branch (kPost) a
+// row's stream and branch are asked for together, and a sum costs one barrier: 2048 x 2048 13.2 us when the branch was read twice, now 12.0
+// (59 MB). A branch that joins as it is needs no sum of its own, so piece by piece takes fewer registers: with five shifted mixes
+// 1024 / 2048 / 4096 columns 9.6 / 24.8 / 47.5 us, in one trip 13.3 / 23.0 / 65.2; hence one trip at two pieces.
+template <typename T, typename D, int NV, bool kPost>
 __global__ void __launch_bounds__(kRowThreads) stream_norm_vec_kernel(const leankv_stream_norm_t a, int per_cta) {
     __shared__ float s_tmp[2][32];
     pdl_begin();
@@ -90,22 +92,25 @@ __global__ void __launch_bounds__(kRowThreads) stream_norm_vec_kernel(const lean
     const D* delta = static_cast<const D*>(a.delta);
     T* h = static_cast<T*>(a.h);
     T* mixed = static_cast<T*>(a.mixed);
-    const bool shift = a.n_mix > 0, post = a.post_gain != nullptr, per_col = a.gain_per_col != 0;
+    const bool shift = a.n_mix > 0, per_col = a.gain_per_col != 0;
     const float gain = a.gain == nullptr || per_col ? 1.f : __ldg(a.gain);
-    const float* scale = post ? a.post_gain : a.scale;
+    const float* scale = kPost ? a.post_gain : a.scale;
     float cur[NV][4], above[NV][4];
     int turn = 0;                 // sums take two buffers in turn, so that one barrier each is enough
     auto sum = [&](float v) { return cta_sum_once(v, s_tmp[turn ^= 1]); };
     auto load = [&](int row, bool store) -> float {       // the updated stream of `row` into cur; its norm factor
-        float dv[NV][4], ss = 0.f, f = 1.f;
+        constexpr bool kTrip = kPost || NV == 2;          // everything of the row in one trip
+        float dv[kTrip ? NV : 1][4], ss = 0.f, f = 1.f;
+        if constexpr (kTrip) {
 #pragma unroll
-        for (int n = 0; n < NV; ++n) {                    // everything of the row in one trip
-            const int i = (tid + n * kRowThreads) * 4;
-            if (i >= W) continue;
-            fetch4(a.x_in + (size_t)row * W + i, cur[n]);
-            if (delta != nullptr) fetch4(delta + (size_t)row * W + i, dv[n]);
+            for (int n = 0; n < NV; ++n) {
+                const int i = (tid + n * kRowThreads) * 4;
+                if (i >= W) continue;
+                fetch4(a.x_in + (size_t)row * W + i, cur[n]);
+                if (kPost || delta != nullptr) fetch4(delta + (size_t)row * W + i, dv[n]);
+            }
         }
-        if (post) {                                       // the branch is normed before it joins
+        if constexpr (kPost) {                            // the branch is normed before it joins
 #pragma unroll
             for (int n = 0; n < NV; ++n)
                 if ((tid + n * kRowThreads) * 4 < W)
@@ -118,11 +123,13 @@ __global__ void __launch_bounds__(kRowThreads) stream_norm_vec_kernel(const lean
         for (int n = 0; n < NV; ++n) {
             const int i = (tid + n * kRowThreads) * 4;
             if (i < W) {
-                if (delta != nullptr) {
+                if constexpr (!kTrip) fetch4(a.x_in + (size_t)row * W + i, cur[n]);
+                if (kPost || delta != nullptr) {
                     float sv[4];
+                    if constexpr (!kTrip) fetch4(delta + (size_t)row * W + i, dv[0]);
                     fetch4(scale + i, sv);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) cur[n][q] = fmaf(dv[n][q] * f, sv[q], cur[n][q]);
+                    for (int q = 0; q < 4; ++q) cur[n][q] = fmaf(dv[kTrip ? n : 0][q] * f, sv[q], cur[n][q]);
                     if (store) store4(a.x_out + (size_t)row * W + i, cur[n]);
                 }
 #pragma unroll
@@ -273,11 +280,17 @@ int launch_stream_norm(const leankv_stream_norm_t* a, cudaStream_t st) {
     const int per = a->n_mix > 0 && a->rows >= sm_count() * 8 ? 4 : 1;
     const dim3 grid((a->rows + per - 1) / per), block(kRowThreads);
     const int nv = (a->width + kRowThreads * 4 - 1) / (kRowThreads * 4);
-    if (nv <= 1) LEANKV_CUDA_TRY(launch_early(stream_norm_vec_kernel<T, D, 1>, grid, block, 0, st, *a, per));
-    else if (nv <= 2) LEANKV_CUDA_TRY(launch_early(stream_norm_vec_kernel<T, D, 2>, grid, block, 0, st, *a, per));
-    else if (nv <= 4) LEANKV_CUDA_TRY(launch_early(stream_norm_vec_kernel<T, D, 4>, grid, block, 0, st, *a, per));
-    else LEANKV_CUDA_TRY(launch_early(stream_norm_vec_kernel<T, D, 8>, grid, block, 0, st, *a, per));
-    return LEANKV_OK;
+    const bool post = a->post_gain != nullptr;
+    const auto go = [&](auto pieces) -> int {
+        constexpr int NV = decltype(pieces)::value;
+        LEANKV_CUDA_TRY(launch_early(post ? stream_norm_vec_kernel<T, D, NV, true> : stream_norm_vec_kernel<T, D, NV, false>, grid, block, 0,
+                                     st, *a, per));
+        return LEANKV_OK;
+    };
+    return nv <= 1   ? go(std::integral_constant<int, 1>{})
+           : nv <= 2 ? go(std::integral_constant<int, 2>{})
+           : nv <= 4 ? go(std::integral_constant<int, 4>{})
+                     : go(std::integral_constant<int, 8>{});
 }
 
 bool known(int dtype) { return dtype == LEANKV_DT_BF16 || dtype == LEANKV_DT_F32; }
