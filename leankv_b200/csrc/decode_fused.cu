@@ -35,9 +35,9 @@ struct PostParams {
 
 // A CTA serves one head for kSeqs sequences at a time, its rotation column in registers. What bounds it is the chain of
 // one vector (the fp64 sum of 64 squares alone is 64 dependent steps), not any unit, so a batch takes four sequences
-// through the chain together: 32 sequences, 48 heads: 21.9 -> 12.6 us. With kEarly position, page, shared word and rotary angles are there
-// when the projections are: four steps of 32 layers of one sequence 8577 -> 8215 us; alone one sequence 3.5 -> 2.3, a batch of
-// 32 10.3 -> 9.5 without and 8.7 with kEarly, of 80 24.4 -> 22.5 and 23.5.
+// through the chain together: 32 sequences, 48 heads: 21.9 -> 12.6 us. With kEarly position, page, shared word and rotary angles
+// are there when the projections are: four steps of 32 layers of one sequence 8577 -> 8215 us; alone one sequence 3.5 -> 2.3, a
+// batch of 32 10.3 -> 9.5 without and 8.7 with kEarly, of 80 24.4 -> 22.5 and 23.5 (hence without where a CTA walks several groups).
 template <int kSeqs, bool kEarly>
 __global__ void __launch_bounds__(kDim, kSeqs > 1 ? 3 : 1) decode_qkv_post_kernel(const PostParams p) {
     __shared__ float s_x[kSeqs][kDim];       // the head vectors (after rotary embedding, fp16 values)
@@ -253,12 +253,14 @@ static int post_launch(const void* qkv, int B, const float* inv_freq, const int3
     // resident at once (two or three an SM), each of which walks the rest of its head's sequences with the same column.
     const int heads = n_q_heads + 2 * n_kv_heads;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool early = (flags & LEANKV_POST_EARLY) != 0;
+    bool early = (flags & LEANKV_POST_EARLY) != 0;
     if (B == 1) {
-        LEANKV_CUDA_TRY(launch_kernel_ex(true, early ? decode_qkv_post_kernel<1, true> : decode_qkv_post_kernel<1, false>, dim3(heads, 1), dim3(kDim), 0, st, p));
+        LEANKV_CUDA_TRY(launch_kernel_ex(true, early ? decode_qkv_post_kernel<1, true> : decode_qkv_post_kernel<1, false>, dim3(heads, 1),
+                                         dim3(kDim), 0, st, p));
     } else {
         constexpr int kSeqs = 4;
-        const int gy = std::max(1, std::min((B + kSeqs - 1) / kSeqs, 3 * sm_count() / heads));
+        const int groups = (B + kSeqs - 1) / kSeqs, gy = std::max(1, std::min(groups, 3 * sm_count() / heads));
+        early = early && gy == groups;       // CTAs that walk several groups gain on the first only and pay on the others: 23.5 against 22.5
         LEANKV_CUDA_TRY(launch_kernel_ex(true, early ? decode_qkv_post_kernel<kSeqs, true> : decode_qkv_post_kernel<kSeqs, false>,
                                          dim3(heads, gy), dim3(kDim), 0, st, p));
     }
