@@ -419,9 +419,14 @@ int leankv_batch_qkv_post_flags(const void* qkv, int B, const float* inv_freq, c
                                 const int32_t* kv_page_indices, int n_q_heads, int n_kv_heads,
                                 float* q_rot, int flags, void* stream);
 /* y[rows][N] = x[rows][K] W[K][N], fp16 with fp32 sums, for up to 128 rows: the projections of a batched step. K % 8 == 0,
- * N % 8 == 0, everything 16-byte aligned. With early_weights W may be read while the launch ahead of this one still runs: that launch must
- * not write it. Where a wait inside the kernel runs out, the outputs are NaN. */
-int leankv_skinny_gemm_f16(const void* x, const void* w, void* y, int rows, int K, int N, int early_weights, void* stream);
+ * N % 8 == 0, everything 16-byte aligned. flags: 0 and 1 are safe behind any launch, apart from what the first flag says.
+ *   LEANKV_SKINNY_EARLY_WEIGHTS: W may be read while the launch ahead of this one still runs: that launch must not write it.
+ *   LEANKV_SKINNY_EARLY_TMEM: the launch ahead takes no tensor memory (it is no tensor-core kernel of this generation); this one may then
+ *     take its own while that one still runs. Behind a launch that does take some, both could wait for each other for good.
+ * Where a wait inside the kernel runs out, the outputs are NaN. */
+#define LEANKV_SKINNY_EARLY_WEIGHTS 1
+#define LEANKV_SKINNY_EARLY_TMEM 2
+int leankv_skinny_gemm_f16(const void* x, const void* w, void* y, int rows, int K, int N, int flags, void* stream);
 /* out[r][i] = fp16(silu(gate_up[r][i])) * gate_up[r][inter + i]  (LlamaMLP's act_fn(gate) * up). */
 int leankv_silu_mul_f16(const void* gate_up, void* out, int rows, int inter, void* stream);
 /* The same of two matrices fp16 [rows][inter]; out may be either of them. */

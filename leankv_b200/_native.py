@@ -23,6 +23,7 @@ TQ_DIM = 128
 TQ_CHUNK_BYTES = 800
 ATTN_EARLY_FETCH = 1
 POST_EARLY = 1
+SKINNY_EARLY_WEIGHTS, SKINNY_EARLY_TMEM = 1, 2
 
 
 class Segments(Structure):

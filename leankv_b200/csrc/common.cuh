@@ -79,8 +79,8 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
 }
 
 // A launch that may become resident while the one ahead drains: for kernels whose every thread begins with pdl_begin() (nothing
-// is left out by an early return before it) and that take no tensor memory. One that does could get it before a block of
-// the launch ahead has asked for its own, and both would wait. A prompt pass is a hundred launches with some 2 us between
+// is left out by an early return before it) and that take no tensor memory: one that took it before its wait could get it before a block
+// of the launch ahead has asked for its own, and both would wait (skinny_gemm.cu takes it between its wait and the next launch's start). A prompt pass is a hundred launches with some 2 us between
 // each and the one ahead: 2048 tokens through four Rorosun layers 3174 -> 3118 us, 4000 through four Pefitar layers 3460 -> 3400;
 // a generation's prompt and framing launches 14 310 -> 14 120 us (48 steps of six Rorosun layers).
 template <typename... KArgs, typename... Args>
@@ -127,15 +127,17 @@ __device__ __forceinline__ unsigned arrive(unsigned* counter) {
 // launching (its CTAs become resident and run up to their own pdl_wait), then waits until every
 // kernel before it has completed and its writes are visible. Nothing that depends on, or is read
 // by, an earlier kernel may be touched before pdl_wait(). Both are no-ops for a normal launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() {
 #ifdef LEANKV_PDL_TRIGGER_FIRST
-    asm volatile("griddepcontrol.launch_dependents;");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_launch();
+    pdl_wait();
 #else
     // wait first: when a dependent starts early, everything before its immediate predecessor is
     // complete and visible, and at most one kernel sits waiting behind the running one
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;");
+    pdl_wait();
+    pdl_launch();
 #endif
 }
 

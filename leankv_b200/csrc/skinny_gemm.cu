@@ -30,7 +30,7 @@ constexpr uint32_t kWBytes = kKStep * kCols * 2; // two blocks of 64 columns
 struct SkinnyArgs {
     CUtensorMap w, x;
     __half* y;
-    int rows, rows_pad, N, steps, stages, early;     // steps: of K
+    int rows, rows_pad, N, steps, stages, early, tmem_first;     // steps: of K
     uint32_t tmem_cols;
 };
 
@@ -62,13 +62,11 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_gemm_kernel(const __grid_c
         umma::bar_init_n(addr(&s_done), 1);
         s_fail = 0;
     }
-    // tensor memory is taken before later launches are let in: one of them could otherwise hold it while it waits for this one
-    if (warp == 1) umma::tmem_alloc_n(addr(&s_tmem), p.tmem_cols);
+    if (p.tmem_first && warp == 1) umma::tmem_alloc_n(addr(&s_tmem), p.tmem_cols);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
-    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
     const int split = blockIdx.y, n_split = gridDim.y, n0 = blockIdx.x * kCols;
     const int s0 = p.steps * split / n_split, n_steps = p.steps * (split + 1) / n_split - s0;
@@ -85,9 +83,9 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_gemm_kernel(const __grid_c
             load2(base + s * stage_bytes + kWBytes, &p.x, (s0 + j) * kKStep, 0, addr(&s_full[s]));
         };
         const int first = min(p.stages, n_steps);
-        if (!p.early) pdl_begin();
+        if (!p.early) pdl_wait();
         for (int j = 0; j < first; ++j) load_w(j);
-        if (p.early) pdl_begin();
+        if (p.early) pdl_wait();
         for (int j = 0; j < first; ++j) load_x(j);
         int j = first;
         for (; j < n_steps; ++j) {
@@ -99,7 +97,17 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_gemm_kernel(const __grid_c
         if (!ok)                                         // give up only once the copies in flight have landed
             for (int i = max(j - p.stages, 0); i < j; ++i) umma::bar_wait(addr(&s_full[i % p.stages]), (i / p.stages) & 1);
     } else if (warp == 1) {                              // ---- products ----
-        pdl_begin();
+        // Tensor memory is taken before later launches are let in: one of them could hold it while it waits for this one. And it is taken
+        // behind the wait, where no block of a launch ahead can still be asking for its own; only where the caller says that the
+        // launch ahead takes none it is taken while that one drains (two CTAs an SM ask one after the other: 2048 x 2048, 16 rows,
+        // launches of this kernel one behind the other 5.4 us so, 6.1 behind the wait; steps of two to four layers 1 to 5 us).
+        pdl_wait();
+        if (!p.tmem_first) umma::tmem_alloc_n(addr(&s_tmem), p.tmem_cols);
+        pdl_launch();
+        umma::fence_before_sync();
+        __syncwarp();
+        umma::fence_after_sync();
+        const uint32_t tmem = __shfl_sync(0xffffffffu, *static_cast<volatile uint32_t*>(&s_tmem), 0);
         const uint32_t idesc = idesc_f16_at(p.rows_pad);
         auto all = [&](bool done) { return __all_sync(0xffffffffu, done) != 0; };
         for (int j = 0; j < n_steps; ++j) {
@@ -119,13 +127,15 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_gemm_kernel(const __grid_c
         if (umma::elect()) umma::commit(addr(&s_done));
         __syncwarp();
     } else {
-        pdl_begin();
+        pdl_wait();
     }
     __syncwarp();                                        // no lane polls beside the copying one
     if (!umma::bar_wait(addr(&s_done), 0)) ok = false;
     if (!ok) s_fail = 1;
-    __syncwarp();
+    umma::fence_before_sync();
+    __syncthreads();                                     // the address of the tensor memory is there
     umma::fence_after_sync();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     // ---- this CTA's sums to shared memory, [row][column of W]: the stages are free ----
     float* sums = reinterpret_cast<float*>(raw + (base - addr(raw)));
 #pragma unroll 1
@@ -195,7 +205,8 @@ int make_map2(CUtensorMap* map, const void* base, cuuint64_t inner, cuuint64_t o
 
 using namespace leankv;
 
-extern "C" int leankv_skinny_gemm_f16(const void* x, const void* w, void* y, int rows, int K, int N, int early_weights, void* stream) {
+extern "C" int leankv_skinny_gemm_f16(const void* x, const void* w, void* y, int rows, int K, int N, int flags, void* stream) {
+    if ((flags & ~(LEANKV_SKINNY_EARLY_WEIGHTS | LEANKV_SKINNY_EARLY_TMEM)) != 0) return LEANKV_EINVAL;
     if (!x || !w || !y || rows <= 0 || K <= 0 || N <= 0) return LEANKV_EINVAL;
     if (rows > kMaxRows) return LEANKV_ELIMIT;
     if (K % 8 || N % 8 || !aligned16(x) || !aligned16(w) || !aligned16(y)) return LEANKV_EALIGN;
@@ -205,7 +216,8 @@ extern "C" int leankv_skinny_gemm_f16(const void* x, const void* w, void* y, int
     p.rows_pad = (rows + 15) / 16 * 16;
     p.N = N;
     p.steps = (K + kKStep - 1) / kKStep;
-    p.early = early_weights != 0;
+    p.early = (flags & LEANKV_SKINNY_EARLY_WEIGHTS) != 0;
+    p.tmem_first = (flags & LEANKV_SKINNY_EARLY_TMEM) != 0;
     p.tmem_cols = p.rows_pad <= 32 ? 32 : p.rows_pad <= 64 ? 64 : 128;
     const size_t x_bytes = ((size_t)p.rows_pad * 128 + 1023) / 1024 * 1024;
     p.stages = (int)std::min<size_t>(kMaxStages, (110 * 1024 - 1024) / (kWBytes + x_bytes));

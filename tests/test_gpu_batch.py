@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from conftest import rel_l2
+from gpu_util import RawPool
 from leankv_b200 import _native
 from leankv_b200.batch_engine import BatchDecodeEngine
 from leankv_b200.engine import DecodeEngine, DecoderConfig
@@ -149,6 +150,54 @@ def test_skinny_gemm_edges(rows, k, n):
         torch.cuda.synchronize()
         assert bool((y[rows] == 7.0).all())
         assert float((y[:rows].double() - want).norm()) <= 2 ** -11 * float(want.norm())
+
+
+@pytest.mark.parametrize("flags", [2, 3])
+def test_skinny_gemm_that_takes_its_tensor_memory_first(flags):
+    """Behind a launch of CUDA cores, in a row of both: the bits of a launch in plain order."""
+    lib, rows, k, n = _native.lib(), 33, 520, 2056
+    g = torch.Generator(device=_dev()).manual_seed(3)
+    x = torch.randn(rows, k, device=_dev(), generator=g).half()
+    w = (torch.randn(k, n, device=_dev(), generator=g) * k ** -0.5).half()
+    gain = torch.ones(k, dtype=torch.float16, device=_dev())
+    outs = [torch.empty(rows, n, dtype=torch.float16, device=_dev()) for _ in range(21)]
+    for i, y in enumerate(outs):
+        h = torch.empty_like(x)
+        _native.check(lib.leankv_rmsnorm_rows_f16(x.data_ptr(), None, gain.data_ptr(), h.data_ptr(), rows, k, 1e-5, _st()), "norm")
+        _native.check(lib.leankv_skinny_gemm_f16(h.data_ptr(), w.data_ptr(), y.data_ptr(), rows, k, n, flags if i else 0, _st()), "gemm")
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, outs[0]) for y in outs[1:])
+
+
+@pytest.mark.parametrize("early", [0, 1])
+def test_skinny_gemm_next_to_kernels_with_tensor_memory(early):
+    """Prompt attention holds all of an SM's tensor memory: a projection right behind it, and it right behind a projection, without the
+    host in between, give the bits that each gives alone."""
+    lib, T, H, rows, k, n = _native.lib(), 333, 2, 40, 1032, 1544
+    g = torch.Generator(device=_dev()).manual_seed(8)
+    rp = RawPool(64, H, _dev())
+    kv = [torch.randn(1, H, T, 128, device=_dev(), generator=g).half() for _ in range(2)]
+    rp.append(*kv, [0, 21], range(21), [0])
+    q = torch.randn(T, 4 * H, 128, device=_dev(), generator=g).half()
+    pages, attended = rp.i32(range(21)), rp.prefill_attention(q, range(21), 0)
+    x = torch.randn(rows, k, device=_dev(), generator=g).half()
+    w = (torch.randn(k, n, device=_dev(), generator=g) * k ** -0.5).half()
+    ws = torch.zeros(lib.leankv_tq_prefill_attn_workspace_bytes(T, 0, 4 * H, H), dtype=torch.uint8, device=_dev())
+    outs = [(torch.empty_like(q), torch.empty(rows, n, dtype=torch.float16, device=_dev())) for _ in range(20)]
+
+    def project(y):
+        _native.check(lib.leankv_skinny_gemm_f16(x.data_ptr(), w.data_ptr(), y.data_ptr(), rows, k, n, early, _st()), "skinny_gemm")
+
+    alone = torch.empty(rows, n, dtype=torch.float16, device=_dev())
+    project(alone)
+    torch.cuda.synchronize()
+    for out, y in outs:
+        _native.check(lib.leankv_tq_prefill_attn(q.data_ptr(), out.data_ptr(), T, 0, 4 * H, H, rp.pool.data_ptr(), rp.n_pages,
+                                                 pages.data_ptr(), rp.Pi_k.data_ptr(), rp.Pi_v.data_ptr(), rp.centroids_host.data_ptr(),
+                                                 128 ** -0.5, ws.data_ptr(), ws.numel(), _st()), "prefill_attn")
+        project(y)
+    torch.cuda.synchronize()
+    assert all(torch.equal(out, attended) and torch.equal(y, alone) for out, y in outs)
 
 
 def test_batch_qkv_post_is_bit_identical_to_single_sequence_kernel():
