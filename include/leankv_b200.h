@@ -423,10 +423,13 @@ int leankv_batch_qkv_post_flags(const void* qkv, int B, const float* inv_freq, c
  *   LEANKV_SKINNY_EARLY_WEIGHTS: W may be read while the launch ahead of this one still runs: that launch must not write it.
  *   LEANKV_SKINNY_EARLY_TMEM: the launch ahead takes no tensor memory (it is no tensor-core kernel of this generation); this one may then
  *     take its own while that one still runs. Behind a launch that does take some, both could wait for each other for good.
- * Where a wait inside the kernel runs out, the outputs are NaN. */
+ * Where a wait inside the kernel runs out, the outputs are NaN; the _status form also sets LEANKV_SKINNY_GAVE_UP in *status (device; NULL:
+ * nowhere). That bit is none of attention's, so one word may serve both. */
 #define LEANKV_SKINNY_EARLY_WEIGHTS 1
 #define LEANKV_SKINNY_EARLY_TMEM 2
+#define LEANKV_SKINNY_GAVE_UP 8
 int leankv_skinny_gemm_f16(const void* x, const void* w, void* y, int rows, int K, int N, int flags, void* stream);
+int leankv_skinny_gemm_f16_status(const void* x, const void* w, void* y, int rows, int K, int N, int flags, int32_t* status, void* stream);
 /* out[r][i] = fp16(silu(gate_up[r][i])) * gate_up[r][inter + i]  (LlamaMLP's act_fn(gate) * up). */
 int leankv_silu_mul_f16(const void* gate_up, void* out, int rows, int inter, void* stream);
 /* The same of two matrices fp16 [rows][inter]; out may be either of them. */

@@ -134,6 +134,7 @@ SIGNATURES = {
     "leankv_paged_table_step": (c_int, [c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "leankv_skinny_gemm_f16": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
+    "leankv_skinny_gemm_f16_status": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "leankv_silu_mul_f16": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "leankv_silu_mul_pair_f16": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "leankv_prompt_begin_f16": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),

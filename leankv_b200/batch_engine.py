@@ -108,9 +108,10 @@ class BatchDecodeEngine(DecodeEngine):
         library (gate / up 36.1 / 39.1 us alone)."""
         k, n = w.shape
         if a.shape[0] <= 48 and n <= 8192 and k % 8 == 0 and n % 8 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0:
-            _native.check(self.lib.leankv_skinny_gemm_f16(a.data_ptr(), w.data_ptr(), out.data_ptr(), a.shape[0], k, n,
-                                                          _native.SKINNY_EARLY_WEIGHTS | _native.SKINNY_EARLY_TMEM, self._st()),
-                          "skinny_gemm")               # behind norm, decode attention and SiLU: none takes tensor memory
+            # a wait that runs out sets a bit of attention's status word
+            _native.check(self.lib.leankv_skinny_gemm_f16_status(
+                a.data_ptr(), w.data_ptr(), out.data_ptr(), a.shape[0], k, n, _native.SKINNY_EARLY_WEIGHTS | _native.SKINNY_EARLY_TMEM,
+                self.ws_attn.data_ptr(), self._st()), "skinny_gemm")      # behind norm, decode attention and SiLU: none takes tensor memory
             self.own_gemms_per_step += 1
         else:
             torch.matmul(a, w, out=out)

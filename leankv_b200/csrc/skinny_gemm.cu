@@ -30,6 +30,7 @@ constexpr uint32_t kWBytes = kKStep * kCols * 2; // two blocks of 64 columns
 struct SkinnyArgs {
     CUtensorMap w, x;
     __half* y;
+    int* status;
     int rows, rows_pad, N, steps, stages, early, tmem_first;     // steps: of K
     uint32_t tmem_cols;
 };
@@ -152,8 +153,10 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_gemm_kernel(const __grid_c
         umma::fence_after_sync();
         umma::tmem_free_n(tmem, p.tmem_cols);
     }
-    if (s_fail)                                          // a wait ran out: no numbers
+    if (s_fail) {                                        // a wait ran out: no numbers
         for (int e = tid; e < p.rows * kCols; e += kThreads) sums[e] = __int_as_float(0x7fc00000);
+        if (tid == 0 && p.status != nullptr) atomicOr(p.status, LEANKV_SKINNY_GAVE_UP);
+    }
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     // ---- four columns a thread, this CTA's part of the rows ----
@@ -205,13 +208,15 @@ int make_map2(CUtensorMap* map, const void* base, cuuint64_t inner, cuuint64_t o
 
 using namespace leankv;
 
-extern "C" int leankv_skinny_gemm_f16(const void* x, const void* w, void* y, int rows, int K, int N, int flags, void* stream) {
+extern "C" int leankv_skinny_gemm_f16_status(const void* x, const void* w, void* y, int rows, int K, int N, int flags, int32_t* status,
+                                             void* stream) {
     if ((flags & ~(LEANKV_SKINNY_EARLY_WEIGHTS | LEANKV_SKINNY_EARLY_TMEM)) != 0) return LEANKV_EINVAL;
     if (!x || !w || !y || rows <= 0 || K <= 0 || N <= 0) return LEANKV_EINVAL;
     if (rows > kMaxRows) return LEANKV_ELIMIT;
     if (K % 8 || N % 8 || !aligned16(x) || !aligned16(w) || !aligned16(y)) return LEANKV_EALIGN;
     SkinnyArgs p{};
     p.y = static_cast<__half*>(y);
+    p.status = status;
     p.rows = rows;
     p.rows_pad = (rows + 15) / 16 * 16;
     p.N = N;
@@ -232,4 +237,8 @@ extern "C" int leankv_skinny_gemm_f16(const void* x, const void* w, void* y, int
     LEANKV_CUDA_TRY(launch_cluster_kernel_ex(true, dim3(1, split, 1), skinny_gemm_kernel, dim3(blocks, split), dim3(kThreads), smem,
                                              static_cast<cudaStream_t>(stream), p));
     return LEANKV_OK;
+}
+
+extern "C" int leankv_skinny_gemm_f16(const void* x, const void* w, void* y, int rows, int K, int N, int flags, void* stream) {
+    return leankv_skinny_gemm_f16_status(x, w, y, rows, K, N, flags, nullptr, stream);
 }

@@ -482,7 +482,7 @@ class DecodeEngine(DecodeLoop):
 
     def status_words(self) -> tuple[int, int]:
         """(exchange status, attention status) read from the device: non-zero once a bounded wait inside
-        the in-kernel all-reduce / the attention kernel's page copies has given up, or a page id was out
+        the in-kernel all-reduce / the attention kernel's page copies / a batched projection has given up, or a page id was out
         of range. Synchronises the device."""
         ex = int(self.xchg.status.item()) if self.xchg is not None else 0
         at = int(self.ws_attn[:4].view(torch.int32).item())
@@ -496,7 +496,7 @@ class DecodeEngine(DecodeLoop):
         if ex or at:
             raise RuntimeError(f"decode kernels reported a failure: exchange status {ex} "
                                f"(1 = a peer's partial sum never arrived), attention status {at} "
-                               f"(1 = page copy wait gave up, 2 = page id out of range)")
+                               f"(1 = page copy wait gave up, 2 = page id out of range, 8 = a projection's wait gave up)")
 
     def _queue_status(self) -> None:
         self._pinned_status[0:1].copy_(self.ws_attn[:4].view(torch.int32), non_blocking=True)

@@ -200,6 +200,19 @@ def test_skinny_gemm_next_to_kernels_with_tensor_memory(early):
     assert all(torch.equal(out, attended) and torch.equal(y, alone) for out, y in outs)
 
 
+def test_a_projection_that_gave_up_is_reported():
+    """The word that the kernels set is the one that the engine reads: untouched by steps that end well, an error once it is set."""
+    eng = BatchDecodeEngine.random_init(CFG, _dev(), 3, seed=1, max_seq_len=64)
+    prompts = torch.arange(3 * 20).reshape(3, 20)
+    eng.generate(prompts, 4)
+    assert eng.own_gemms_per_step > 0 and eng.status_words() == (0, 0)
+    eng.ws_attn[:4].view(torch.int32).fill_(8)
+    with pytest.raises(RuntimeError, match="projection"):
+        eng.check_status()
+    with pytest.raises(RuntimeError, match="projection"):
+        eng.generate(prompts, 4)
+
+
 def test_batch_qkv_post_is_bit_identical_to_single_sequence_kernel():
     """Same qkv rows, positions and pages through the batched launch and through one launch per sequence."""
     lib = _native.lib()

@@ -281,6 +281,7 @@ def test_argument_validation_of_the_decode_and_exchange_entry_points():
     assert lib.leankv_skinny_gemm_f16(fake, fake, fake, 4, 60, 64, 0, None) == -2
     assert lib.leankv_skinny_gemm_f16(fake, fake, odd, 4, 64, 64, 0, None) == -2
     assert lib.leankv_skinny_gemm_f16(fake, fake, fake, 4, 64, 64, 4, None) == -1          # no such flag
+    assert lib.leankv_skinny_gemm_f16_status(fake, None, fake, 4, 64, 64, 0, fake, None) == -1
     assert lib.leankv_skinny_gemm_f16(fake, fake, fake, 129, 64, 64, 0, None) == lib.leankv_sparse_gemv_f16_static(
         fake, fake, fake, 131072, 8, 0.1, None) < 0
     assert lib.leankv_batch_decode_end(fake, 32770, 2, fake, fake, 8, fake, fake, None) == -2   # vocab % 8
