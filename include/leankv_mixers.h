@@ -138,6 +138,9 @@ int leankv_window_pool_append(const leankv_window_pool_t* a, const float* qkv, i
 size_t leankv_window_pool_workspace_bytes(const leankv_window_pool_t* a, int rows, int max_pos);
 int leankv_window_pool_attend(const leankv_window_pool_t* a, const void* q, void* out, int out_ld, float out_scale,
                               int rows, int start, void* ws, size_t ws_bytes, void* stream);
+/* The same; status: int32 (device, may be NULL) set non-zero if a wait inside the kernel ran out (the rows are then NaN). */
+int leankv_window_pool_attend_status(const leankv_window_pool_t* a, const void* q, void* out, int out_ld, float out_scale,
+                                     int rows, int start, void* ws, size_t ws_bytes, int32_t* status, void* stream);
 
 /* Time mixing: per head o_t = (S + diag(u) k v^T)^T r, S = diag(w_t) S + k v^T, w = exp(-exp(z + w0)).
  * S fp32 [heads][dim key][dim value]. */

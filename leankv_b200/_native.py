@@ -257,6 +257,8 @@ MIXER_SIGNATURES = {
     "leankv_window_pool_workspace_bytes": (c_size_t, [POINTER(WindowPool), c_int, c_int]),
     "leankv_window_pool_attend": (c_int, [POINTER(WindowPool), c_void_p, c_void_p, c_int, c_float, c_int, c_int,
                                           c_void_p, c_size_t, c_void_p]),
+    "leankv_window_pool_attend_status": (c_int, [POINTER(WindowPool), c_void_p, c_void_p, c_int, c_float, c_int, c_int,
+                                                 c_void_p, c_size_t, c_void_p, c_void_p]),
     "leankv_time_mix_workspace_bytes": (c_size_t, [POINTER(TimeMix), c_int]),
     "leankv_time_mix_rows": (c_int, [POINTER(TimeMix), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                      c_int, c_float, c_int, c_void_p, c_size_t, c_void_p]),

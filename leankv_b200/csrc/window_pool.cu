@@ -229,15 +229,15 @@ extern "C" size_t leankv_window_pool_workspace_bytes(const leankv_window_pool_t*
     return pl.p_in_smem ? 0 : (size_t)rows * 2 * a->heads * pl.ldp * 4;
 }
 
-extern "C" int leankv_window_pool_attend(const leankv_window_pool_t* a, const void* q, void* out, int out_ld,
-                                         float out_scale, int rows, int start, void* ws, size_t ws_bytes,
-                                         void* stream) {
+extern "C" int leankv_window_pool_attend_status(const leankv_window_pool_t* a, const void* q, void* out, int out_ld,
+                                                float out_scale, int rows, int start, void* ws, size_t ws_bytes,
+                                                int32_t* status, void* stream) {
     const int rc = check_args(a);
     if (rc) return rc;
     if (!q || !out || rows <= 0 || start < 0 || out_ld < a->heads * a->vdim) return LEANKV_EINVAL;
     if (VisibleKeys(start + rows - 1, a->size, a->pool).n_blk > a->max_blocks) return LEANKV_ELIMIT;
     if (!aligned16(q)) return LEANKV_EALIGN;
-    const int mma = window_pool_mma_attend(*a, q, out, out_ld, out_scale, rows, start, static_cast<cudaStream_t>(stream));
+    const int mma = window_pool_mma_attend(*a, q, out, out_ld, out_scale, rows, start, status, static_cast<cudaStream_t>(stream));
     if (mma != LEANKV_EUNSUPPORTED) return mma;
     const int tiled = window_pool_tile_attend(*a, q, out, out_ld, out_scale, rows, start, static_cast<cudaStream_t>(stream));
     if (tiled != LEANKV_EUNSUPPORTED) return tiled;
@@ -246,4 +246,10 @@ extern "C" int leankv_window_pool_attend(const leankv_window_pool_t* a, const vo
     float* w = static_cast<float*>(ws);
     return a->dtype == LEANKV_DT_BF16 ? attend<bf16>(*a, q, out, out_ld, out_scale, rows, start, w, st)
                                       : attend<float>(*a, q, out, out_ld, out_scale, rows, start, w, st);
+}
+
+extern "C" int leankv_window_pool_attend(const leankv_window_pool_t* a, const void* q, void* out, int out_ld,
+                                         float out_scale, int rows, int start, void* ws, size_t ws_bytes,
+                                         void* stream) {
+    return leankv_window_pool_attend_status(a, q, out, out_ld, out_scale, rows, start, ws, ws_bytes, nullptr, stream);
 }

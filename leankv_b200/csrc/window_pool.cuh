@@ -31,7 +31,7 @@ int window_pool_tile_attend(const leankv_window_pool_t& a, const void* q, void* 
 
 // The tcgen05 route (window_pool_mma.cu), likewise.
 int window_pool_mma_attend(const leankv_window_pool_t& a, const void* q, void* out, int out_ld, float out_scale, int rows, int start,
-                           cudaStream_t st);
+                           int* status, cudaStream_t st);
 
 constexpr int kMaxCluster = 16;     // non-portable; 8 where the device does not place 16
 constexpr int kAttendHeads = 4;     // query heads a thread carries at once

@@ -34,6 +34,7 @@ struct MixArgs {
     CUtensorMap q, k, k_pool, v, v_pool;
     const float* talk;
     bf16* out;
+    int* status;
     int out_ld, rows, start, size, pool, ring;
     int heads, kv_heads, rep, tq;                // tq: tokens of a CTA
     int dim_pad, vdim, vdim_pad, nb, nbv, vec;   // nb, nbv: 64-column blocks
@@ -261,6 +262,7 @@ __global__ void __launch_bounds__(kThreads, 2) window_pool_mma_kernel(const __gr
         }
     }
     if (s_fail) {                                        // a wait ran out: the portion's rows are not numbers
+        if (tid == 0 && p.status != nullptr) atomicExch(p.status, 1);
         __syncthreads();
         for (int e = tid; e < used * ld; e += kThreads) rows[e] = __int_as_float(0x7fc00000);
     }
@@ -300,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, 2) window_pool_mma_kernel(const __gr
 }  // namespace
 
 int window_pool_mma_attend(const leankv_window_pool_t& a, const void* q, void* out, int out_ld, float out_scale, int rows, int start,
-                           cudaStream_t st) {
+                           int* status, cudaStream_t st) {
     const int rep = a.heads / a.kv_heads;
     if (a.dtype != LEANKV_DT_BF16 || a.talk == nullptr || a.k_pool == nullptr || a.v_pool == nullptr || !(a.scale > 0.f) || a.dim_pad > 128 || a.vdim_pad > 128 || rep > kMaxRep ||
         a.kv_heads > kMaxKvHeads || !aligned16(q) || !aligned16(a.k_ring) || !aligned16(a.v_ring) || !aligned16(a.k_pool) ||
@@ -309,6 +311,7 @@ int window_pool_mma_attend(const leankv_window_pool_t& a, const void* q, void* o
     MixArgs p{};
     p.talk = a.talk;
     p.out = static_cast<bf16*>(out);
+    p.status = status;
     p.out_ld = out_ld;
     p.rows = rows;
     p.start = start;

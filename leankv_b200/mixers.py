@@ -148,8 +148,8 @@ class WindowPoolAttention:
         _native.check(self.lib.leankv_window_pool_append(ref, qkv.data_ptr(), qkv.stride(0), bias.data_ptr(),
                                                          q.data_ptr(), T, start, st), "window_pool_append", self.lib)
         ws = scratch(self.lib.leankv_window_pool_workspace_bytes(ref, T, start + T))
-        _native.check(self.lib.leankv_window_pool_attend(ref, q.data_ptr(), out.data_ptr(), out.stride(0), out_scale,
-                                                         T, start, ws.data_ptr(), ws.numel(), st),
+        _native.check(self.lib.leankv_window_pool_attend_status(ref, q.data_ptr(), out.data_ptr(), out.stride(0), out_scale,
+                                                                T, start, ws.data_ptr(), ws.numel(), self.seq.status.data_ptr(), st),
                       "window_pool_attend", self.lib)
 
 

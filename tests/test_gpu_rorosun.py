@@ -486,6 +486,26 @@ def test_a_sequence_leaves_nothing_behind():
         assert torch.equal(eng.extend([t], [0]), r)
 
 
+def test_a_prompt_whose_attention_gave_up_is_refused(monkeypatch):
+    """The window kernel gets the engine's status word, and a portion during which that word is set ends with an error."""
+    cfg, _, eng = engine("wide", BF16)
+    lib, words = _native.mixers(), []
+    launch = lib.leankv_window_pool_attend_status
+
+    def gives_up(*args):
+        words.append(args[9])
+        eng.seq.status.fill_(1)
+        return launch(*args)
+
+    prompt = tokens(cfg, 40)
+    eng.extend(prompt, [39])
+    eng.reset()
+    monkeypatch.setattr(lib, "leankv_window_pool_attend_status", gives_up)
+    with pytest.raises(RuntimeError, match="gave up"):
+        eng.extend(prompt, [39])
+    assert words == [eng.seq.status.data_ptr()] * len(cfg["layers"])
+
+
 def test_long_decoding_past_windows_and_blocks():
     cfg, w, eng = engine("small", F32, limit=420)
     ids = tokens(cfg, 400, seed=4)

@@ -245,6 +245,7 @@ def test_mixer_arguments_are_checked_before_any_launch():
     attend = lambda rows, start: lib.leankv_window_pool_attend(ctypes.byref(w), fake, fake, 64, 1.0, rows, start, None,
                                                                0, None)
     assert attend(2, 20) == -6                                                # more blocks than there are
+    assert lib.leankv_window_pool_attend_status(ctypes.byref(w), fake, fake, 64, 1.0, 2, 20, None, 0, fake, None) == -6
     t = _native.TimeMix(dtype=1, heads=2, dim=8, S=fake, u=fake, w0=fake, norm=fake, eps=1e-5)
     args = [fake] * 6
     assert lib.leankv_time_mix_rows(ctypes.byref(t), *args, 16, 1.0, 4, None, 0, None) == -3
