@@ -726,6 +726,8 @@ class DecodeEngine(DecodeLoop):
             for s0 in range(0, T, chunk):
                 x = self._dense_forward(ids[s0:s0 + chunk], write_cache=True, start_pos=s0,
                                         attention=attention)
+            ready = (self.token, self.history, self.state)
+            before = [t.clone() for t in ready] if attention == "packed" else []
             self.history.zero_()
             self.state.zero_()
             self.state[0].fill_(T)
@@ -734,10 +736,15 @@ class DecodeEngine(DecodeLoop):
             tok = torch.argmax(logits).reshape(1)
             self.token.copy_(tok)
             self.history[:1].copy_(tok)
-            self.prefill_logits = logits
             first = int(tok.item())
             if attention == "packed":
-                self._check_prefill_status()      # behind the tail's launches: it waits for the device
+                try:
+                    self._check_prefill_status()      # behind the tail's launches: it waits for the device
+                except RuntimeError:
+                    for t, old in zip(ready, before):      # not ready for a step
+                        t.copy_(old)
+                    raise
+            self.prefill_logits = logits
         return first
 
     def bytes_streamed(self) -> int:

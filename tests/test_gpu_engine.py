@@ -431,3 +431,28 @@ def test_a_prompt_whose_first_chunk_failed_is_refused():
     with pytest.raises(RuntimeError, match="status 2"):
         eng.prefill([t % 512 for t in range(2900)], chunk=100)
     assert len(chunks) == 29
+
+
+@pytest.mark.parametrize("attention", ["packed", "dense"])
+def test_a_failed_prompt_leaves_no_engine_that_looks_ready(attention):
+    """Position, token, history and logits stay what they were before the prompt; a prompt that ends well replaces them."""
+    cfg = DecoderConfig(vocab_size=512, hidden_size=512, intermediate_size=1024, num_layers=1, num_q_heads=8, num_kv_heads=2)
+    eng = DecodeEngine.random_init(cfg, _dev(), seed=3, max_seq_len=400)
+    eng.generate(list(range(50)), 5)
+    ready = lambda: [t.clone() for t in (eng.state, eng.token, eng.history, eng.prefill_logits)]
+    old, forward = ready(), eng._dense_forward
+    if attention == "packed":
+        def failing(ids, **kw):
+            out = forward(ids, **kw)
+            eng._prefill_ws[:4].view(torch.int32).fill_(1)       # as if a wait had run out
+            return out
+
+        eng._dense_forward = failing
+        with pytest.raises(RuntimeError, match="status 1"):
+            eng.prefill(list(range(300)))
+        assert all(torch.equal(a, b) for a, b in zip(ready(), old))
+        eng._dense_forward = forward
+        eng._prefill_ws[:4].zero_()
+    first = eng.prefill(list(range(100, 400 - 1)), attention=attention)
+    assert eng.state[:2].tolist() == [299, 1] and int(eng.token) == first == int(eng.history[0]) and not eng.history[1:].any()
+    assert int(eng.prefill_logits.argmax()) == first
