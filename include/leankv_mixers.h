@@ -38,8 +38,8 @@ extern "C" {
  *   epilogue: y = acc + bias (first bias_rows rows);  gated: y = silu(acc_gate) * acc_up;
  *             softcap > 0: y = softcap * tanh(y / softcap);
  *             residual != NULL: y = residual + scale * acc (y may be residual; x may not be y).
- *   early_weights: the launch directly ahead on the stream does not write w (a decode step's weights); w may be read while
- *     it drains. */
+ *   early_weights: the launch directly ahead on the stream writes none of w, scale, gain and post_gain (a decode step's constants); they
+ *     may be read while it drains. */
 typedef struct leankv_dense_gemv {
     const void* w;
     const float* x;

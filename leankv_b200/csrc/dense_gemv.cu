@@ -94,14 +94,16 @@ template <int R>
 __device__ __forceinline__ int row_of_lane(int lane) { return (lane * R) >> 5; }
 
 // kJoined: a branch joins the stream first, or there is a gain per column; every thread prepares its columns in registers
-// (one slab). kStaged: the same in shared memory, any number of slabs. kGrouped: row groups with an input slice each.
-enum class Input { kPlain, kJoined, kStaged, kGrouped };
+// (one slab). kStaged: the same in shared memory, any number of slabs. kGrouped: row groups with an input slice each. kSum: a residual joins
+// the product (only of a plain input; beside the others it is read at the end).
+enum class Input { kPlain, kJoined, kStaged, kGrouped, kSum };
 // kAhead: the weights of the next rows are in registers before they are needed, sixteen warps an SM. Otherwise rows are asked for
 // when it is their turn, by twice as many warps (bf16) or twice as many rows a warp (fp32): more bytes in flight, for
 // ranges so long that their start does not count (see launch_gemv).
 template <typename T, int CH, Input IN, bool kAhead>
 __global__ void __launch_bounds__(512, !kAhead && sizeof(T) == 2 ? 2 : 1) dense_gemv_kernel(const GemvParams p) {
-    constexpr bool STAGED = IN == Input::kStaged, JOINED = IN == Input::kJoined, GROUPED = IN == Input::kGrouped;
+    constexpr bool STAGED = IN == Input::kStaged, JOINED = IN == Input::kJoined, GROUPED = IN == Input::kGrouped,
+                   SUM = IN == Input::kSum;
     constexpr int R = (sizeof(T) == 4 && kAhead ? 4 : 8) / CH;      // rows in flight: 128 bytes a lane (256 in fp32 without kAhead)
     extern __shared__ __align__(16) float s_dyn[];
     float* s_part = STAGED ? s_dyn + p.x_smem : s_dyn;      // [rows of this CTA (x2 if gated)][warps]
@@ -125,8 +127,8 @@ __global__ void __launch_bounds__(512, !kAhead && sizeof(T) == 2 ? 2 : 1) dense_
             asm volatile("prefetch.global.L2 [%0];" ::"l"(base + off));
         }
     }
-    // The first rows' weights into registers: ahead of the dependency wait where the caller says that the launch ahead does
-    // not write them, else beside the loads of x.
+    // The first rows' weights and the constants into registers: ahead of the dependency wait where the caller says that the launch ahead
+    // does not write them, else beside the loads of x.
     const int n_rows = (hi - lo) * mult;
     Raw8<T> raw[R][CH];
     auto load_rows = [&](int s, int v, int last) {
@@ -139,8 +141,8 @@ __global__ void __launch_bounds__(512, !kAhead && sizeof(T) == 2 ? 2 : 1) dense_
                 load_w8(W + row * cols, s * slab_cols + (c * warps + warp) * 256 + lane * 8, cols, vec, raw[r][c]);
         }
     };
-    if (kAhead && a.early_weights) load_rows(0, 0, n_rows - 1);
-    // kJoined: the gains do not depend on the launch ahead
+    if (!a.early_weights) pdl_begin();
+    if (kAhead) load_rows(0, 0, n_rows - 1);
     float gn[CH][8], pg[CH][8];
     if constexpr (JOINED) {
 #pragma unroll
@@ -153,10 +155,9 @@ __global__ void __launch_bounds__(512, !kAhead && sizeof(T) == 2 ? 2 : 1) dense_
     // what a residual sum needs, a row a thread: the scale now, the residual beside x
     const int fin = lo + (int)threadIdx.x;
     float fin_scale = 0.f, fin_residual = 0.f;
-    if (IN == Input::kPlain && a.residual != nullptr) fin_scale = __ldg(a.scale + min(fin, hi - 1));
-    pdl_begin();
-    if (IN == Input::kPlain && a.residual != nullptr) fin_residual = ld_cg_f32(a.residual + min(fin, hi - 1));
-    if (kAhead && !a.early_weights) load_rows(0, 0, n_rows - 1);
+    if constexpr (SUM) fin_scale = ld_cg_f32(a.scale + min(fin, hi - 1));
+    if (a.early_weights) pdl_begin();
+    if constexpr (SUM) fin_residual = ld_cg_f32(a.residual + min(fin, hi - 1));
 
     float rs = 1.f;
     float xj[CH][8];                // kJoined: this thread's columns of x'
@@ -334,7 +335,7 @@ __global__ void __launch_bounds__(512, !kAhead && sizeof(T) == 2 ? 2 : 1) dense_
         }
         if (a.softcap > 0.f) y = a.softcap * tanhf(y / a.softcap);
         if (a.residual != nullptr)
-            y = IN == Input::kPlain && i < (int)blockDim.x ? fin_residual + y * fin_scale : ld_cg_f32(a.residual + row) + y * __ldg(a.scale + row);
+            y = SUM && i < (int)blockDim.x ? fin_residual + y * fin_scale : ld_cg_f32(a.residual + row) + y * __ldg(a.scale + row);
         a.y[row] = y;
     }
 }
@@ -425,6 +426,7 @@ extern "C" int leankv_dense_gemv(const leankv_dense_gemv_t* a, void* stream) {
         if (prepared && p.slabs == 1) return with(std::integral_constant<Input, Input::kJoined>{});
         if (staged) return with(std::integral_constant<Input, Input::kStaged>{});
         if (a->group_rows > 0) return with(std::integral_constant<Input, Input::kGrouped>{});
+        if (a->residual && !a->gain) return with(std::integral_constant<Input, Input::kSum>{});
         return with(std::integral_constant<Input, Input::kPlain>{});
     };
     return a->dtype == LEANKV_DT_BF16 ? go(bf16{}) : go(float{});

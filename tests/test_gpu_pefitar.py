@@ -78,6 +78,32 @@ def test_gemv_gated_after_joined_branch(dtype):
     assert rel(y, v[:rows] * torch.sigmoid(v[:rows]) * v[rows:]) < 1e-5
 
 
+@pytest.mark.parametrize("form", ["scale", "gain", "post_gain"])
+def test_gemv_constants_that_the_launch_ahead_writes(form):
+    """Without early_weights nothing is read ahead of the wait: a long product in front writes the vector that this one needs."""
+    lib, n = _native.mixers(), 512
+    w1, x1, vec = rnd(n, 32768, seed=1, std=0.01).to(DEV), rnd(32768, seed=2).to(DEV), torch.empty(n, device=DEV)
+    ahead = _native.DenseGemv(w=w1.data_ptr(), x=x1.data_ptr(), y=vec.data_ptr(), dtype=CODE[F32], rows=n, cols=32768)
+    rows, cols = (n, 64) if form == "scale" else (96, n)
+    w, x, d, y = rnd(rows, cols, seed=3, std=cols ** -0.5).to(DEV), rnd(cols, seed=4).to(DEV), rnd(cols, seed=5).to(DEV), torch.empty(rows, device=DEV)
+    res, one, out = rnd(rows, seed=6).to(DEV), rnd(cols, seed=7, mean=1.0).to(DEV), torch.empty(cols, device=DEV)
+    more = {"scale": dict(scale=vec, residual=res), "gain": dict(gain=vec, gain_per_col=1, eps=1e-3),
+            "post_gain": dict(gain=one, gain_per_col=1, eps=1e-3, delta=d, post_gain=vec, post_mult=0.5, x_out=out)}[form]
+    a = _native.DenseGemv(**{k: v.data_ptr() if torch.is_tensor(v) else v
+                             for k, v in dict(w=w, x=x, y=y, dtype=CODE[F32], rows=rows, cols=cols, **more).items()})
+    _native.check(lib.leankv_dense_gemv(ctypes.byref(ahead), stream()), "product", lib)
+    v, xd = vec.double(), x.double()
+    want = {"scale": lambda: res.double() + v * (w.double() @ xd), "gain": lambda: w.double() @ plain.rms_norm(xd, v, 1e-3),
+            "post_gain": lambda: w.double() @ plain.rms_norm(xd + 0.5 * plain.rms_norm(d.double(), v, 1e-3), one.double(), 1e-3)}[form]()
+    for _ in range(10):
+        vec.fill_(50.0)
+        torch.cuda.synchronize()
+        for args in (ahead, a):
+            _native.check(lib.leankv_dense_gemv(ctypes.byref(args), stream()), "product", lib)
+        torch.cuda.synchronize()
+        assert rel(y, want) < 1e-5
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("groups,n,cols,stride", [(1, 5, 8, 8), (3, 28, 10, 16), (7, 33, 20, 27), (16, 512, 128, 192),
                                                   (32, 128, 512, 512), (5, 1, 300, 304)])
