@@ -362,15 +362,18 @@ int launch_gemv_as(const GemvParams& p, int warps, cudaStream_t st) {
 // 13.8, 4096 x 1024 (1) 3.8 / 5.2; eleven warps, bf16 2048 x 5632 (3.5) 7.4 / 6.3; eight warps, fp32 16384 x 128 (1.8) 5.9 / 5.2,
 // bf16 16384 x 128 (0.9) 4.6 / 4.9. With early weights a long range stays with kAhead: behind the other launches of a decode
 // step its first rows are there when these end, and a 32768 x 2048 head that starts as they drain cost the step 0.6 us more.
-template <typename T, int CH, Input IN>
-int launch_gemv(const GemvParams& p, int warps, cudaStream_t st) {
+template <typename T>
+bool looks_ahead(const GemvParams& p, int warps) {
     const int resident = std::min(std::max(1, kMaxWarps / warps), 8) * warps;
     const double bytes = (double)p.a.rows * (p.a.gated ? 2 : 1) * p.a.cols * sizeof(T);
     const double rounds = bytes / sm_count() / (4096.0 * resident);
     const bool thin = resident < (sizeof(T) == 2 ? 12 : 9);
     const bool deep = rounds >= 10.0 && !p.a.early_weights;
-    return deep || (thin && rounds > 1.5) ? launch_gemv_as<T, CH, IN, false>(p, warps, st)
-                                          : launch_gemv_as<T, CH, IN, true>(p, warps, st);
+    return !deep && !(thin && rounds > 1.5);
+}
+template <typename T, int CH, Input IN>
+int launch_gemv(const GemvParams& p, int warps, cudaStream_t st) {
+    return looks_ahead<T>(p, warps) ? launch_gemv_as<T, CH, IN, true>(p, warps, st) : launch_gemv_as<T, CH, IN, false>(p, warps, st);
 }
 
 }  // namespace
@@ -401,9 +404,10 @@ extern "C" int leankv_dense_gemv(const leankv_dense_gemv_t* a, void* stream) {
     GemvParams p{};
     p.a = *a;
     p.vec = a->cols % 8 == 0 && (a->group_rows == 0 || a->group_stride % 4 == 0);
-    // a branch that joins the stream or a norm: x is prepared once, in registers where one slab holds it, else in shared memory
-    // (a norm with one gain and several slabs reads x a second time instead)
-    const bool staged = a->delta || (a->gain && a->gain_per_col), prepared = staged || a->gain;
+    // A branch that joins the stream or a norm: x is prepared once, in registers where one slab holds it, else in shared memory. A norm with
+    // one gain reads x a second time instead where there are several slabs, or where its sixteen numbers a thread are registers that a
+    // kernel without kAhead wants for rows (us reading it again / once: 12288 x 5632 26.0 / 27.5, 1024 x 5632 6.6 / 7.2).
+    const bool staged = a->delta || (a->gain && a->gain_per_col);
     // warps x slabs x CH column chunks of 256: the widest CTA that pads least
     const int chunks = (a->cols + 255) / 256;
     int warps = 1, per = 1;
@@ -423,10 +427,10 @@ extern "C" int leankv_dense_gemv(const leankv_dense_gemv_t* a, void* stream) {
             constexpr Input IN = decltype(in)::value;
             return per == 1 ? launch_gemv<T, 1, IN>(p, warps, st) : launch_gemv<T, 2, IN>(p, warps, st);
         };
-        if (prepared && p.slabs == 1) return with(std::integral_constant<Input, Input::kJoined>{});
+        if ((staged || (a->gain && (per == 1 || looks_ahead<T>(p, warps)))) && p.slabs == 1) return with(std::integral_constant<Input, Input::kJoined>{});
         if (staged) return with(std::integral_constant<Input, Input::kStaged>{});
         if (a->group_rows > 0) return with(std::integral_constant<Input, Input::kGrouped>{});
-        if (a->residual && !a->gain) return with(std::integral_constant<Input, Input::kSum>{});
+        if (a->residual && !a->gain && looks_ahead<T>(p, warps)) return with(std::integral_constant<Input, Input::kSum>{});
         return with(std::integral_constant<Input, Input::kPlain>{});
     };
     return a->dtype == LEANKV_DT_BF16 ? go(bf16{}) : go(float{});

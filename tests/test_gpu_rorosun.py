@@ -105,6 +105,29 @@ def test_gemv_token_shift_segments_and_previous_token(dtype, ends, cols):
         h_prev = h
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("rows,cols", [(130, 2816), (1030, 2816), (600, 5632), (1100, 5632), (300, 5120), (7000, 8192)])
+def test_gemv_norms_and_sums_of_long_ranges(dtype, rows, cols):
+    """Either side of the lines between the kernels that look ahead and the others, with one and two pieces of x a thread, for a norm, a
+    shift and a residual. The sums are fp32."""
+    w, x = rnd(rows, cols, seed=1, std=cols ** -0.5).to(dtype).to(DEV), rnd(cols, seed=2, std=2.0).to(DEV)
+    g, s, r, mu = torch.tensor(1.3, device=DEV), rnd(rows, seed=3).to(DEV), rnd(rows, seed=4).to(DEV), rnd(cols, seed=5, mean=0.5).to(DEV)
+    prev, state, y = rnd(2, cols, seed=6).to(DEV), torch.zeros(8, dtype=torch.int32, device=DEV), torch.empty(rows, device=DEV)
+    h, wd = plain.scalar_norm(x.double(), g.double(), 1e-4), w.double()
+    above = prev[0].double().clone()
+    base = dict(w=w, x=x, y=y, dtype=CODE[dtype], rows=rows, cols=cols)
+    forms = [(dict(gain=g, eps=1e-4), wd @ h), (dict(scale=s, residual=r), r.double() + s.double() * (wd @ x.double())),
+             (dict(gain=g, eps=1e-4, scale=s, residual=r), r.double() + s.double() * (wd @ h)),
+             (dict(gain=g, eps=1e-4, n_mix=1, prev=prev, state=state), wd @ (h + (above - h) * mu.double()))]
+    for early in (0, 1):
+        for more, want in forms:
+            a = _native.DenseGemv(early_weights=early, **{k: v.data_ptr() if torch.is_tensor(v) else v for k, v in {**base, **more}.items()})
+            a.mix_end[0], a.mu[0] = rows, mu.data_ptr()
+            ok(_native.mixers().leankv_dense_gemv(ctypes.byref(a), stream()))
+            assert rel(y, want) < 1e-5
+        assert rel(prev[1], h) < 1e-6
+
+
 # ── row kernels of a portion ─────────────────────────────────────────────────────────────────
 
 @pytest.mark.parametrize("dtype", [F32, BF16])
