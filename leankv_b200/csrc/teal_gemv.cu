@@ -169,7 +169,8 @@ __device__ float sum_over_ranks(const GemvParams& p, int col, int npad, float su
     // meaningless, but no kernel hangs).
     const unsigned int ep = (unsigned int)*reinterpret_cast<const volatile int*>(p.xepoch);
     const unsigned long long word = ((unsigned long long)ep << 32) | (unsigned long long)__float_as_uint(sum);
-    // every rank starts with a different destination so that the ranks' stores do not all converge on
+    // Only columns that exist are sent and waited for: ranks whose shares of the input channels differ may run kernels with slices of
+    // different widths, whose paddings differ. Every rank starts with a different destination so that the ranks' stores do not all converge on
     // one GPU's links at the same moment
     for (int i = 0; i < p.xw; ++i) {
         int r = p.xrank + i;
@@ -474,8 +475,9 @@ __global__ void __launch_bounds__(kThreads, kSwiglu ? 3 : 4) sparse_gemv_kernel(
         if (tid == 0) p.counters[slice] = 0;   // leave the workspace ready for the next launch
     }
 
+    if (col >= p.N) return;
     if (!kSwiglu && p.xw > 0) sum = sum_over_ranks(p, col, npad, sum);
-    if (col < p.N) finish_column<kSwiglu>(p, col, sum, sum2);
+    finish_column<kSwiglu>(p, col, sum, sum2);
 }
 
 // One thread-block cluster a column slice: its CTAs take a share of the input channels each, and the split sums meet in the
@@ -697,8 +699,9 @@ __global__ void __launch_bounds__(kT, kT == 512 ? 2 : kSwiglu ? 3 : 4) sparse_ge
         if (kSwiglu) sum2 += s_part[r][kArrays - 1][tid];
     }
     const int col = slice * kCols + tid;
+    if (col >= p.N) return;
     if (!kSwiglu && p.xw > 0) sum = sum_over_ranks(p, col, (p.N + kColsPerCta - 1) / kColsPerCta * kColsPerCta, sum);
-    if (col < p.N) finish_column<kSwiglu>(p, col, sum, sum2);
+    finish_column<kSwiglu>(p, col, sum, sum2);
 }
 
 // Which matrices: those whose bytes take less time than a launch's chain. One array: up to 17 M elements (us before / here: 8192

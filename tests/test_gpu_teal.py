@@ -281,6 +281,34 @@ def test_allreduce_wait_gives_up_when_a_peer_never_arrives():
     torch.cuda.synchronize()
 
 
+@pytest.mark.parametrize("n,z", [(520, 512), (520, 8200), (200, 96)])
+def test_allreduce_needs_no_more_of_a_peer_than_its_columns(n, z):
+    """The peer's words are laid out beforehand, for columns that exist only: a rank whose shapes take a kernel of another slice width pads
+    differently. Nothing runs out, nothing is sent beyond them, and the result is the sum."""
+    lib, dev, world, cols = _native.lib(), _dev(), 2, 768
+    npad = (n + 255) // 256 * 256
+    recv = [torch.zeros(lib.leankv_xchg_recv_bytes(world, 1, cols), dtype=torch.uint8, device=dev) for _ in range(world)]
+    epoch, status = torch.full((1,), 5, dtype=torch.int32, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    xc = _native.Xchg()
+    xc.world, xc.rank, xc.n_slots, xc.max_cols, xc.max_wait_iters = world, 0, 1, cols, 2000
+    for r in range(world):
+        xc.recv[r] = recv[r].data_ptr()
+    xc.epoch, xc.status = epoch.data_ptr(), status.data_ptr()
+    gen = torch.Generator(device="cpu").manual_seed(n + z)
+    wt = (torch.randn(z, n, generator=gen) * 0.02).half().to(dev)
+    x, other = torch.randn(z, generator=gen).half().to(dev), torch.randn(n, generator=gen).to(dev)
+    mine = recv[0].view(torch.int32).reshape(-1, 2)
+    mine[npad:npad + n, 0] = other.view(torch.int32)
+    mine[npad:npad + n, 1] = 5
+    y = _allreduce_gemv(wt, x, 0.1, None, xc, 0)
+    assert int(status) == 0
+    live = torch.where(x.abs() > 0.1, x, torch.zeros_like(x)).double()
+    want = live @ wt.double() + other.double()
+    assert (y.double() - want).norm() <= 2 ** -11 * want.norm()
+    sent = recv[1].view(torch.int32).reshape(-1, 2)
+    assert (sent[:n, 1] == 5).all() and not sent[n:].any()
+
+
 def test_one_workspace_serves_projections_of_different_widths():
     """A decode step runs all its projections through one workspace. The widest (the output head: 128
     column slices at vocabulary 32768, 501 at 128256) must still find its arrival counters at zero after
