@@ -95,8 +95,11 @@ def _whole_numbers(tokens: Sequence[int]) -> np.ndarray:
         return np.frombuffer(array("q", list(tokens)), dtype=np.int64)
     except OverflowError:
         raise ValueError("token outside the vocabulary") from None
-    except TypeError:                      # floating-point numbers and whatever else a tensor takes
-        return torch.as_tensor(list(tokens), dtype=torch.int64).numpy()
+    except TypeError:                      # floating-point numbers and whatever else a tensor takes; rounded only if they are in range
+        values = list(tokens)
+        if min(values) < 0 or max(values) >= 1 << 63:
+            raise ValueError("token outside the vocabulary") from None
+        return torch.as_tensor(values, dtype=torch.int64).numpy()
 
 
 class _Sublayer:
@@ -410,7 +413,8 @@ class MixerDecodeEngine(DecodeLoop):
             rows = [[k for k, w in enumerate(want) if s0 <= w < s0 + m] for s0, m in parts]
             order = [k for r in rows for k in r]
             places = [want[k] - s0 for (s0, _), r in zip(parts, rows) for k in r]
-            up = torch.from_numpy(np.concatenate([host, np.array(places + order, dtype=np.int64)])).to(self.dev, non_blocking=True)
+            up = torch.from_numpy(np.concatenate([host, np.frombuffer(array("q", places + order), dtype=np.int64)])).to(
+                self.dev, non_blocking=True)           # array: places are whole numbers, or an error
             ids, at, to = up[:n], up[n:n + len(order)], up[n + len(order):]
             done, pieces = 0, []
             for (s0, m), r in zip(parts, rows):

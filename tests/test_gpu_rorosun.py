@@ -572,6 +572,15 @@ def test_window_and_block_longer_than_the_sequence():
     assert rel(torch.cat([eng.extend([t], [0]) for t in ids[50:]]), want[50:]) < MODEL_TOL[F32]
 
 
+def test_extend_takes_whole_places_and_tokens_in_range():
+    _, _, eng = engine("small", F32)
+    for tokens_, want in (([1, 2, 3], [0.5]), ([1, 2, 3], [1.0]), ([-0.5, 2], [1]), ([96.0, 97.0], [0])):
+        with pytest.raises((ValueError, TypeError, IndexError)):
+            eng.extend(tokens_, want)
+        assert eng.pos == 0
+    assert eng.extend([1.0, 2.0, 3.0], torch.tensor([2, 0])).shape == (2, 97)
+
+
 def test_engine_refuses_what_does_not_fit():
     cfg, w, eng = engine("small", F32, limit=10)
     with pytest.raises(ValueError):

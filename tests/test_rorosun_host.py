@@ -267,3 +267,6 @@ def test_token_ids_of_every_kind_and_out_of_range():
         assert got.dtype == np.int64 and got.tolist() == want.tolist()
     with pytest.raises(ValueError):
         _whole_numbers([1 << 63])
+    for outside in ([-0.5, 1], [2, -0.25], [1e30, 0.0], [float("inf")], [0.0, -float("inf")]):      # refused before they are rounded
+        with pytest.raises(ValueError):
+            _whole_numbers(outside)
