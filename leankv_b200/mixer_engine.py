@@ -416,18 +416,22 @@ class MixerDecodeEngine(DecodeLoop):
             up = torch.from_numpy(np.concatenate([host, np.frombuffer(array("q", places + order), dtype=np.int64)])).to(
                 self.dev, non_blocking=True)           # array: places are whole numbers, or an error
             ids, at, to = up[:n], up[n:n + len(order)], up[n + len(order):]
-            done, pieces = 0, []
+            # one portion's logits in order are the result; else they go into it portion by portion, never all of them twice
+            whole = sum(map(bool, rows)) == 1 and order == sorted(order)
+            out = None if whole else torch.empty(len(order), self.cfg.vocab_size, dtype=torch.float32, device=self.dev)
+            done = 0
             for (s0, m), r in zip(parts, rows):
                 x = self._portion(ids[s0:s0 + m])
-                if r:
-                    pieces.append(self._logits_of(x[at[done:done + len(r)]]))
-                    done += len(r)
-            if not pieces:
-                return torch.empty(0, self.cfg.vocab_size, dtype=torch.float32, device=self.dev)
-            out = pieces[0] if len(pieces) == 1 else torch.cat(pieces)
-            if order != sorted(order):
-                out = torch.empty_like(out).index_copy_(0, to, out)
-            self.check_status()
+                if not r:
+                    continue
+                z = self._logits_of(x[at[done:done + len(r)]])
+                if whole:
+                    out = z
+                else:
+                    out.index_copy_(0, to[done:done + len(r)], z)
+                done += len(r)
+            if order:
+                self.check_status()
         return out
 
     @torch.no_grad()

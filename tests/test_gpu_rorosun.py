@@ -572,6 +572,25 @@ def test_window_and_block_longer_than_the_sequence():
     assert rel(torch.cat([eng.extend([t], [0]) for t in ids[50:]]), want[50:]) < MODEL_TOL[F32]
 
 
+def test_logits_of_many_portions_are_held_once():
+    """All rows of ten portions wanted, in any order: beside the result there is room for a portion's logits, not for all once more."""
+    cfg = config(vocab=4099)
+    eng = MixerDecodeEngine(MixerModelConfig.from_dict(cfg), weights(cfg), DEV, max_seq_len=700, dtype=BF16, max_chunk=64)
+    ids, order = tokens(cfg, 640), torch.randperm(640, generator=gen(1)).tolist()
+    first = eng.extend(ids, range(640))
+    eng.reset()
+    torch.cuda.synchronize()
+    held = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    got = eng.extend(ids, order)
+    size = got.numel() * 4
+    assert torch.cuda.max_memory_allocated() - held < 1.5 * size
+    assert torch.equal(got, first[order])
+    eng.reset()
+    # one row through the head's product: the same bf16 numbers, fp32 sums in another order
+    assert rel(eng.extend(ids, [639]), first[639:]) < 1e-5 and eng.extend([1, 2]).shape == (0, 4099)
+
+
 def test_extend_takes_whole_places_and_tokens_in_range():
     _, _, eng = engine("small", F32)
     for tokens_, want in (([1, 2, 3], [0.5]), ([1, 2, 3], [1.0]), ([-0.5, 2], [1]), ([96.0, 97.0], [0])):
