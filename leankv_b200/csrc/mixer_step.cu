@@ -200,10 +200,11 @@ __device__ __forceinline__ uint32_t in_cta(uint32_t addr, int rank) {
     return r;
 }
 
-// 1 / sqrt(x): the approximation and a Newton step, without the subroutines of the exact division and root
+// 1 / sqrt(x): the approximation and a Newton step, without the subroutines of the exact division and root. Of a sum that is no longer
+// finite it is 0, as those have it.
 __device__ __forceinline__ float inv_sqrt(float x) {
     const float r = rsqrtf(x);
-    return r * fmaf(-0.5f * x * r, r, 1.5f);
+    return r > 0.f ? r * fmaf(-0.5f * x * r, r, 1.5f) : r;
 }
 
 // NT: blocks of eight heads. kTileVecs: float4s of the projection row a thread keeps. kSplit: half of the warps waits for the

@@ -293,6 +293,20 @@ def test_step_on_tensor_cores_around_whole_tiles(shape, normed, talk):
     assert rel(got[252:], win.expected(qkv)[252:]) < 3e-2
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+def test_step_with_queries_beyond_the_squares_of_fp32(dtype):
+    """Their norm factor is one over infinity: all keys count alike, as they do in every other kernel."""
+    T = 90
+    win = Window(dtype, 8, 2, 64, 64, 48, 8, chunk=T, limit=T)
+    qkv = win.qkv(T)
+    n = win.H * win.d
+    qkv[T - 1, :n] *= 1e25
+    none = qkv.clone()
+    none[T - 1, :n] = 0
+    got = feed(win, qkv, [T - 1, 1])
+    assert rel(got[T - 1:], win.expected(none)[T - 1:]) < (2e-5 if dtype == F32 else 3e-2)
+
+
 @pytest.mark.parametrize("normed,talk", [(False, True), (True, False), (False, False)])
 def test_window_pool_without_norm_or_mixing(normed, talk):
     win = Window(F32, 4, 2, 16, 24, 10, 3, chunk=60, limit=60, normed=normed, talk=talk)
