@@ -199,13 +199,15 @@ __global__ void __launch_bounds__(256) silu_mul_rows_kernel(const T* gate_up, T*
 }
 
 // Eight elements per thread (inter % 8 == 0, aligned), a block for every 2048 columns of a row: with as many blocks as fit twice the
-// last round was nearly empty (2048 x 7168 in bf16: 17.9 us, so 15.9).
+// last round was nearly empty (2048 x 7168 in bf16: 17.9 us, so 15.9). Blocks of short rows would be mostly idle: kShort walks over all pieces
+// (us by rows / so, bf16: 4096 x 256 4.6 / 3.0, 65536 x 64 68 / 5.8, 65536 x 768 69 / 62, but 4096 x 1792 8.2 / 8.9 and 512 x 256 1.7 / 1.8;
+// fp32: 4096 x 512 4.8 / 3.9, 65536 x 768 87 / 91).
 template <typename T>
+bool short_rows(int rows, int inter) { return rows > 1024 && inter < (sizeof(T) == 2 ? 1024 : 768); }
+template <typename T, bool kShort>
 __global__ void __launch_bounds__(256) silu_mul_vec_kernel(const T* gate_up, T* out, int inter, int rows) {
     pdl_begin();
-    const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
-    if (c >= inter) return;
-    for (long long r = blockIdx.y; r < rows; r += gridDim.y) {
+    const auto piece = [&](long long r, int c) {
         Raw8<T> rg, ru;
         load8(gate_up + r * 2 * inter + c, rg);
         load8(gate_up + r * 2 * inter + inter + c, ru);
@@ -217,6 +219,16 @@ __global__ void __launch_bounds__(256) silu_mul_vec_kernel(const T* gate_up, T* 
         for (int q = 0; q < 8; ++q) o[q] = from_f32<T>(g[q] * sigmoid_f32(g[q]) * u[q]);
         memcpy(&rg, o, sizeof(rg));
         *reinterpret_cast<Raw8<T>*>(out + r * inter + c) = rg;
+    };
+    if constexpr (kShort) {
+        const int n8 = inter >> 3;
+        const long long total = (long long)rows * n8;
+        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
+            piece(i / n8, (int)(i % n8) * 8);
+    } else {
+        const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
+        if (c >= inter) return;
+        for (long long r = blockIdx.y; r < rows; r += gridDim.y) piece(r, c);
     }
 }
 
@@ -362,11 +374,14 @@ extern "C" int leankv_silu_mul(const void* gate_up, void* out, int dtype, int ro
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool vec = inter % 8 == 0 && aligned16(gate_up) && aligned16(out);
     const long long total = (long long)rows * inter;
-    const int grid = (int)std::min<long long>((total + 255) / 256, (long long)sm_count() * 16);
+    const int grid = (int)std::min<long long>(((vec ? total / 8 : total) + 255) / 256, (long long)sm_count() * 16);
     auto go = [&](auto tag) -> int {
         using T = decltype(tag);
-        if (vec)
-            LEANKV_CUDA_TRY(launch_early(silu_mul_vec_kernel<T>, dim3((inter / 8 + 255) / 256, std::min(rows, 65535)), dim3(256), 0, st,
+        if (vec && short_rows<T>(rows, inter))
+            LEANKV_CUDA_TRY(launch_early(silu_mul_vec_kernel<T, true>, dim3(grid), dim3(256), 0, st, static_cast<const T*>(gate_up),
+                                         static_cast<T*>(out), inter, rows));
+        else if (vec)
+            LEANKV_CUDA_TRY(launch_early(silu_mul_vec_kernel<T, false>, dim3((inter / 8 + 255) / 256, std::min(rows, 65535)), dim3(256), 0, st,
                                          static_cast<const T*>(gate_up), static_cast<T*>(out), inter, rows));
         else
             LEANKV_CUDA_TRY(launch_early(silu_mul_rows_kernel<T>, dim3(grid), dim3(256), 0, st, static_cast<const T*>(gate_up),

@@ -130,7 +130,7 @@ def test_embed_rows(dtype, rows, width):
     assert torch.equal(x[:rows], want) and (x[rows] == 5.0).all()
 
 
-@pytest.mark.parametrize("rows,inter", [(1, 2040), (2, 2048), (3, 2056), (65537, 8)])
+@pytest.mark.parametrize("rows,inter", [(1, 2040), (2, 2048), (3, 2056), (65537, 8), (1025, 1016), (1025, 1024), (1024, 24), (1100, 760), (1100, 768), (300000, 16)])
 def test_silu_mul_by_rows(rows, inter):
     """Blocks of 2048 columns, their remainders, and more rows than a grid has; fp32 against 64 bits, bf16 to one rounding."""
     gu = rnd(rows, 2 * inter, seed=inter, std=3.0).cuda()
