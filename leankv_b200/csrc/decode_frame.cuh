@@ -48,18 +48,21 @@ __global__ void __launch_bounds__(256) decode_begin_kernel(const In* table, cons
 // Greedy next token (lowest index wins ties), appended to the history; advances the position.
 // One cluster of kEndCtas CTAs per sequence (pos / step are that sequence's words), each with a share of the vocabulary; the shares'
 // best meet in the first CTA's shared memory. One CTA alone read the row at the rate of one SM: 32768 fp32 logits 5.7 -> 2.8 us behind
-// the output head. `parity` (optional) is flipped.
-constexpr int kEndCtas = 8, kEndThreads = 512;
+// the output head. Where there are more sequences than the device holds clusters of eight at once, one larger CTA each: us by clusters / so,
+// 32000 logits, 48 sequences 4.1 / 4.6, 64 4.3 / 4.6, 80 5.3 / 4.6, 256 10.9 / 6.0; 4096 logits, 48 3.7 / 3.8, 64 4.2 / 3.8. `parity`
+// (optional) is flipped.
+constexpr int end_ctas(int sequences, int vocab) { return sequences <= (vocab >= 16384 ? 64 : 48) ? 8 : 1; }
+__host__ __device__ constexpr int end_threads(int ctas) { return ctas == 1 ? 1024 : 512; }
 
-template <typename L>
-__global__ void __cluster_dims__(kEndCtas, 1, 1) __launch_bounds__(kEndThreads)
+template <typename L, int kEndCtas>
+__global__ void __cluster_dims__(kEndCtas, 1, 1) __launch_bounds__(end_threads(kEndCtas))
     decode_end_kernel(const L* logits, int vocab, long long* token, long long* history, int history_cap, int* pos, int* step_ptr,
                       int* parity) {
-    constexpr int kWarps = kEndThreads / 32;
+    constexpr int kEndThreads = end_threads(kEndCtas), kWarps = kEndThreads / 32;
     __shared__ float s_v[kWarps], s_best[kEndCtas];
     __shared__ int s_i[kWarps], s_at[kEndCtas];
     const int rank = blockIdx.x % kEndCtas, seq = blockIdx.x / kEndCtas;
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    if constexpr (kEndCtas > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     pdl_begin();
     logits += (size_t)seq * vocab;
     float best = -INFINITY;
@@ -92,7 +95,7 @@ __global__ void __cluster_dims__(kEndCtas, 1, 1) __launch_bounds__(kEndThreads)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) { s_v[warp] = best; s_i[warp] = best_i; }
     __syncthreads();
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");        // every CTA of the cluster runs
+    if constexpr (kEndCtas > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");        // every CTA of the cluster runs
     if (warp == 0) {
         best = s_v[lane % kWarps];
         best_i = s_i[lane % kWarps];
@@ -111,8 +114,10 @@ __global__ void __cluster_dims__(kEndCtas, 1, 1) __launch_bounds__(kEndThreads)
         }
         __syncwarp();
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if constexpr (kEndCtas > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
     if (rank == 0 && threadIdx.x == 0) {
         best = s_best[0];
         best_i = s_at[0];

@@ -364,7 +364,7 @@ extern "C" int leankv_decode_end(const void* logits, int vocab, long long* token
                                  int history_cap, int32_t* state, void* stream) {
     if (!logits || !token || !history || !state || vocab <= 0 || history_cap < 0) return LEANKV_EINVAL;
     if (!aligned16(logits)) return LEANKV_EALIGN;
-    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<__half>, dim3(kEndCtas), dim3(kEndThreads), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<__half, 8>, dim3(8), dim3(end_threads(8)), 0, static_cast<cudaStream_t>(stream),
                                   static_cast<const __half*>(logits), vocab, token, history, history_cap,
                                   state + kPos, state + kStep, static_cast<int*>(nullptr)));
     return LEANKV_OK;
@@ -487,7 +487,8 @@ extern "C" int leankv_batch_decode_end(const void* logits, int vocab, int B, lon
     if (!logits || !tokens || !history || !pos || !steps || vocab <= 0 || B <= 0 || history_cap < 0)
         return LEANKV_EINVAL;
     if (!aligned16(logits) || vocab % 8 != 0) return LEANKV_EALIGN;
-    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<__half>, dim3(B * kEndCtas), dim3(kEndThreads), 0, static_cast<cudaStream_t>(stream),
+    const int ctas = end_ctas(B, vocab);
+    LEANKV_CUDA_TRY(launch_early(ctas == 1 ? decode_end_kernel<__half, 1> : decode_end_kernel<__half, 8>, dim3(B * ctas), dim3(end_threads(ctas)), 0, static_cast<cudaStream_t>(stream),
                                   static_cast<const __half*>(logits), vocab, tokens, history, history_cap, pos,
                                   steps, static_cast<int*>(nullptr)));
     return LEANKV_OK;

@@ -344,7 +344,7 @@ extern "C" int leankv_greedy_end(const float* logits, int vocab, long long* toke
                                  int history_cap, int32_t* state, void* stream) {
     if (!logits || !token || !history || !state || vocab <= 0 || history_cap < 0) return LEANKV_EINVAL;
     if (!aligned16(logits)) return LEANKV_EALIGN;
-    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<float>, dim3(kEndCtas), dim3(kEndThreads), 0, static_cast<cudaStream_t>(stream),
+    LEANKV_CUDA_TRY(launch_early(decode_end_kernel<float, 8>, dim3(8), dim3(end_threads(8)), 0, static_cast<cudaStream_t>(stream),
                                   logits, vocab, token, history, history_cap, state + kPos, state + kStep,
                                   state + kParity));
     return LEANKV_OK;

@@ -134,6 +134,26 @@ def test_decode_end_over_the_shares_of_a_cluster(vocab, dtype):
         assert int(token) == want == int(hist[2]) and state[:2].tolist() == [11, 3]
 
 
+@pytest.mark.parametrize("B", [1, 48, 49, 64, 65, 200])
+@pytest.mark.parametrize("vocab", [8, 4096, 32776])
+def test_batch_decode_end_of_few_and_many_sequences(B, vocab):
+    """Either side of the line between a cluster and a CTA for each: ties (the lowest index), rows of NaN, a full history."""
+    g = torch.Generator(device=_dev()).manual_seed(B)
+    logits = torch.randint(-40, 40, (B, vocab), device=_dev(), generator=g).half()
+    logits[B // 2, vocab // 2:] = float("nan")
+    logits[B - 1] = float("nan") if B > 1 else logits[B - 1]
+    tok, hist = torch.full((B,), -1, dtype=torch.int64, device=_dev()), torch.full((B, 3), -1, dtype=torch.int64, device=_dev())
+    pos, steps = torch.arange(B, dtype=torch.int32, device=_dev()), (torch.arange(B, device=_dev()) % 4).to(torch.int32)
+    p0, s0 = pos.clone(), steps.clone()
+    _native.check(_native.lib().leankv_batch_decode_end(logits.data_ptr(), vocab, B, tok.data_ptr(), hist.data_ptr(), 3, pos.data_ptr(),
+                                                        steps.data_ptr(), _st()), "end")
+    x = logits.float().nan_to_num(nan=-1e9)
+    want = (x == x.amax(1, keepdim=True)).int().argmax(1)
+    assert torch.equal(tok, want) and torch.equal(pos, p0 + 1) and torch.equal(steps, s0 + 1)
+    for b in range(B):
+        assert hist[b].tolist() == [int(want[b]) if s == int(s0[b]) else -1 for s in range(3)]
+
+
 @pytest.mark.parametrize("rows", [1, 15, 17, 48, 80, 128])
 @pytest.mark.parametrize("k,n", [(8, 8), (64, 128), (72, 136), (1000, 520), (3584, 1024), (520, 8192), (128, 40000)])
 def test_skinny_gemm_edges(rows, k, n):
