@@ -289,9 +289,13 @@ int launch_stream_norm(const leankv_stream_norm_t* a, cudaStream_t st) {
         LEANKV_CUDA_TRY(launch_early(stream_norm_kernel<T, D>, dim3(a->rows), dim3(kRowThreads), 0, st, *a));
         return LEANKV_OK;
     }
-    const int per = a->n_mix > 0 && a->rows >= sm_count() * 8 ? 4 : 1;
-    const dim3 grid((a->rows + per - 1) / per), block(kRowThreads);
+    // Rows of a CTA with a shift: more than one spares norming the row above, but leaves fewer CTAs. us, five mixes in bf16: 1200 x 1536 with
+    // four rows a CTA 10.3, with two 8.2, 2048 x 2048 16.3 and 14.2, 4000 x 2048 with a branch 41.4 and 35.8; one piece a thread, 600 x 1024 with
+    // one row 5.9, with two 4.9, 900 x 1024 6.0 and 5.4 (but 600 x 2048 6.1 and 7.1, and in fp32 900 x 1024 7.7 and 7.9).
     const int nv = (a->width + kRowThreads * 4 - 1) / (kRowThreads * 4);
+    const bool pairs = sizeof(T) == 2 && nv == 1 && a->rows >= sm_count() * 4;
+    const int per = a->n_mix == 0 ? 1 : a->rows >= sm_count() * 8 ? (nv == 2 ? 2 : 4) : pairs ? 2 : 1;
+    const dim3 grid((a->rows + per - 1) / per), block(kRowThreads);
     const bool post = a->post_gain != nullptr;
     const auto go = [&](auto pieces) -> int {
         constexpr int NV = decltype(pieces)::value;
