@@ -229,6 +229,22 @@ extern "C" size_t leankv_window_pool_workspace_bytes(const leankv_window_pool_t*
     return pl.p_in_smem ? 0 : (size_t)rows * 2 * a->heads * pl.ldp * 4;
 }
 
+// Whether a portion's queries see so few keys that the mma.sync kernel beats the tcgen05 one. That one gives every pair of kv heads a CTA, whose
+// start, exchange and last, mostly empty tiles do not shrink with the keys: with four kv heads (with three and many heads) and enough rows
+// to fill the device, the line is at some 220 keys that the middle row sees, with fewer heads or rows lower. us, mma.sync / tcgen05: 16 heads of
+// 4, 2048 rows, 184 keys 62.6 / 68.5, 244 keys 74.4 / 72.5; 1200 rows, 100 keys 27.7 / 42.4; 8 of 4, 1200 rows, 157 keys 25.4 / 30.9, 2048 rows, 79
+// keys 31.7 / 36.5, 124 keys 38.2 / 36.6; 4 of 4, 400 rows, 72 keys 15.2 / 17.7; 24 of 3, 2048 rows, 79 keys 60.6 / 64.7. With one or two
+// kv heads tcgen05 always wins.
+static bool few_keys(const leankv_window_pool_t& a, int rows, int start) {
+    if (a.kv_heads < 3 || a.kv_heads > 4) return false;
+    const int keys = VisibleKeys(start + rows / 2, a.size, a.pool).n;
+    const bool many = a.heads >= 16;
+    if (a.kv_heads == 3) return many && rows >= 800 && keys < 80;
+    if (rows >= 2000) return keys < (many ? 220 : a.heads >= 8 ? 100 : 0);
+    if (rows >= 800) return keys < (a.heads >= 8 ? 220 : 160);
+    return many ? rows >= 512 && keys < 80 : rows >= 300 && keys < (a.heads < 8 ? 100 : 50);
+}
+
 extern "C" int leankv_window_pool_attend_status(const leankv_window_pool_t* a, const void* q, void* out, int out_ld,
                                                 float out_scale, int rows, int start, void* ws, size_t ws_bytes,
                                                 int32_t* status, void* stream) {
@@ -237,10 +253,13 @@ extern "C" int leankv_window_pool_attend_status(const leankv_window_pool_t* a, c
     if (!q || !out || rows <= 0 || start < 0 || out_ld < a->heads * a->vdim) return LEANKV_EINVAL;
     if (VisibleKeys(start + rows - 1, a->size, a->pool).n_blk > a->max_blocks) return LEANKV_ELIMIT;
     if (!aligned16(q)) return LEANKV_EALIGN;
-    const int mma = window_pool_mma_attend(*a, q, out, out_ld, out_scale, rows, start, status, static_cast<cudaStream_t>(stream));
-    if (mma != LEANKV_EUNSUPPORTED) return mma;
-    const int tiled = window_pool_tile_attend(*a, q, out, out_ld, out_scale, rows, start, static_cast<cudaStream_t>(stream));
-    if (tiled != LEANKV_EUNSUPPORTED) return tiled;
+    const bool few = few_keys(*a, rows, start);
+    for (int turn = 0; turn < 2; ++turn) {               // the other one where the first does not take the call
+        const int rc = (turn == 0) != few
+            ? window_pool_mma_attend(*a, q, out, out_ld, out_scale, rows, start, status, static_cast<cudaStream_t>(stream))
+            : window_pool_tile_attend(*a, q, out, out_ld, out_scale, rows, start, static_cast<cudaStream_t>(stream));
+        if (rc != LEANKV_EUNSUPPORTED) return rc;
+    }
     if (leankv_window_pool_workspace_bytes(a, rows, start + rows) > (ws ? ws_bytes : 0)) return LEANKV_EWORKSPACE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     float* w = static_cast<float*>(ws);

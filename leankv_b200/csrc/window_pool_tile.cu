@@ -1,5 +1,6 @@
 // Window + pooled-block attention of a prompt portion on tensor cores (bf16): one CTA per eight queries, all heads. For what
-// window_pool_mma.cu does not take: more than four kv heads, more than eight query heads each, no mix across heads.
+// window_pool_mma.cu does not take: more than four kv heads, more than eight query heads each, no mix across heads; and for three or four
+// kv heads where queries see few keys (few_keys in window_pool.cu).
 //
 // The weights of all heads of a (query, key) pair meet in the mix across heads, so they have to be in one CTA,
 // normalised, before the mix. Pass 1 computes every head's softmax statistics, pass 2 the scores again and from

@@ -228,6 +228,30 @@ class Window:
             w = plain.talk(w, self.talk.double())
         return 0.5 * plain.apply_values(w, v.reshape(T, self.G, -1), self.pool).reshape(T, -1)
 
+    def exact(self, qkv, first, stepped):
+        """Rows first .. in float64 from what the kernels hold: keys, values and their block means in the storage type, and queries too, unless
+        the rows are steps (whose queries keep 16 bits or more)."""
+        T, n, H, G = qkv.shape[0], self.H * self.d, self.H, self.G
+        m = n + G * self.d
+        held = lambda x: x.to(self.dtype).double()
+        q, k, v = qkv[:, :n].double(), qkv[:, n:m].double(), qkv[:, m:].double()
+        if self.normed:
+            q, k = plain.rms(q, 1e-4) * self.qn.double(), plain.rms(k, 1e-4) * self.kn.double()
+        q = (q * self.scale if stepped else held(q) * self.scale).reshape(T, H, -1)[first:]
+        k, v = held(k).reshape(T, G, -1), held(v).reshape(T, G, -1)
+        nb = T // self.pool
+        mean = lambda x: held(x[:nb * self.pool].reshape(nb, self.pool, G, -1).mean(1))
+        k, v = torch.cat([mean(k), k]).to(DEV), torch.cat([mean(v), v]).to(DEV)
+        i, j = torch.arange(first, T)[:, None], torch.arange(T)[None]
+        seen = torch.cat([(torch.arange(nb)[None] + 1) * self.pool - 1 <= i - self.size, (j <= i) & (i - j < self.size)], 1).to(DEV)
+        rep = H // G
+        s = torch.einsum("tghd,kgd->ghtk", q.to(DEV).reshape(T - first, G, rep, -1), k).reshape(H, T - first, -1)
+        w = s.masked_fill(~seen, -math.inf).softmax(-1)
+        if self.talks:
+            w = torch.einsum("xh,htk->xtk", self.talk.double().to(DEV), w)
+        o = torch.einsum("ghtk,kgd->tghd", w.reshape(G, rep, T - first, -1), v)
+        return 0.5 * o.reshape(T - first, -1).cpu()
+
     def qkv(self, T, seed=7, std=1.0):
         return rnd(T, self.H * self.d + self.G * (self.d + self.dv), seed=seed, std=std)
 
@@ -278,6 +302,18 @@ def test_prompt_attention_by_key_tiles(shape):
     assert rel(feed(win, qkv, [T]), want) < 3e-2
     small = Window(BF16, *shape, chunk=150, limit=T)
     assert rel(feed(small, qkv, [150, 2, 131, 1, 33, 83]), want) < 3e-2
+
+
+@pytest.mark.parametrize("shape,T,start", [((16, 4, 64, 64, 64, 16), 800, 0), ((16, 4, 32, 48, 64, 16), 799, 0), ((16, 4, 32, 32, 100, 16), 600, 0),
+                                           ((8, 4, 64, 64, 60, 16), 820, 0), ((8, 4, 64, 64, 30, 16), 310, 0), ((4, 4, 128, 128, 64, 16), 300, 100),
+                                           ((18, 3, 48, 64, 20, 16), 800, 0), ((12, 3, 48, 64, 20, 16), 800, 0), ((5, 4 + 1, 16, 16, 20, 4), 400, 0)])
+def test_prompt_attention_with_few_keys(shape, T, start):
+    """Portions on either side of the lines between the two tensor-core kernels, against float64 of the bf16 numbers that they take. Outputs are
+    rounded to bf16, and in one of them mixed weights: 2^-8 a number each at most."""
+    win = Window(BF16, *shape, chunk=T, limit=T + start)
+    qkv = win.qkv(T + start)
+    got = feed(win, qkv, [start, T] if start else [T])
+    assert rel(got[start:], win.exact(qkv, start, False)) < 2 ** -7
 
 
 @pytest.mark.parametrize("shape", [(8, 2, 128, 128, 255, 16), (16, 4, 128, 128, 270, 16), (16, 16, 16, 32, 260, 8),
