@@ -102,12 +102,15 @@ class BatchDecodeEngine(DecodeEngine):
     # ── one step ─────────────────────────────────────────────────────────
 
     def _mm(self, a, w, out):
-        """out = a w. Up to 48 sequences and 8192 columns go through this library's kernel, which starts on the weights while the launch
-        ahead drains: steps of two 7B-shaped layers, library / so: 32 sequences of 4096 tokens 417.6 / 390.2 us, 8 of 1000 296.8 / 279.7,
-        16 of 500 at width 1024 130.7 / 124.6; 64 of 300 319.5 / 321.2. Gate / up and head, with one CTA a column block, stay with the
-        library (gate / up 36.1 / 39.1 us alone)."""
+        """out = a w, by this library's kernel or by the library. The kernel starts on the weights while the launch ahead drains, and its
+        clusters share a column block's rows of the weights; it wins up to 48 sequences where there are at least half as many rows as
+        columns, up to 8192 columns and 80 M weights (us of a step, library / so. All of q/k/v, o and down: width 4096, two layers, 2 / 8 / 16 / 32 / 48
+        sequences 272 / 246, 282 / 260, 270 / 257, 306 / 276, 293 / 290; width 1024, four layers 200 / 174, 207 / 185, 213 / 194, 232 / 227, 222 / 209;
+        64 sequences at 4096 319 / 321). Gate / up, with seven times as many columns as rows, is faster in the library at every width (512:
+        +0.3 to +1.2 us a layer, 1024: up to +1.2, 4096: up to +4.5), and so is down of width 8192, 235 M weights (+5 us)."""
         k, n = w.shape
-        if a.shape[0] <= 48 and n <= 8192 and k % 8 == 0 and n % 8 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0:
+        if (a.shape[0] <= 48 and n <= min(8192, 2 * k) and k * n <= 80_000_000 and k % 8 == 0 and n % 8 == 0 and w.is_contiguous()
+                and w.data_ptr() % 16 == 0):
             # a wait that runs out sets a bit of attention's status word
             _native.check(self.lib.leankv_skinny_gemm_f16_status(
                 a.data_ptr(), w.data_ptr(), out.data_ptr(), a.shape[0], k, n, _native.SKINNY_EARLY_WEIGHTS | _native.SKINNY_EARLY_TMEM,

@@ -220,6 +220,21 @@ def test_skinny_gemm_next_to_kernels_with_tensor_memory(early):
     assert all(torch.equal(out, attended) and torch.equal(y, alone) for out, y in outs)
 
 
+@pytest.mark.parametrize("rows,k,n,own", [(48, 512, 1024, True), (48, 512, 1032, False), (49, 512, 512, False), (3, 4096, 8192, True),
+                                          (3, 4200, 8200, False), (2, 20000, 4000, True), (2, 20000, 4008, False), (2, 516, 512, False)])
+def test_which_projections_are_this_library_s(rows, k, n, own):
+    """Either side of each line; both give the product to one fp16 rounding."""
+    eng = BatchDecodeEngine.random_init(CFG, _dev(), 2, seed=1, max_seq_len=64)
+    g = torch.Generator(device=_dev()).manual_seed(rows + n)
+    x = torch.randn(rows, k, device=_dev(), generator=g).half()
+    w = (torch.randn(k, n, device=_dev(), generator=g) * k ** -0.5).half()
+    y, before = torch.empty(rows, n, dtype=torch.float16, device=_dev()), eng.own_gemms_per_step
+    eng._mm(x, w, y)
+    assert eng.own_gemms_per_step - before == int(own)
+    want = x.double() @ w.double()
+    assert float((y.double() - want).norm()) <= 2 ** -11 * float(want.norm())
+
+
 def test_a_projection_that_gave_up_is_reported():
     """The word that the kernels set is the one that the engine reads: untouched by steps that end well, an error once it is set."""
     eng = BatchDecodeEngine.random_init(CFG, _dev(), 3, seed=1, max_seq_len=64)
