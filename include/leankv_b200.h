@@ -336,8 +336,8 @@ int leankv_decode_end(const void* logits, int vocab, long long* token, long long
  * Tensor-parallel row-split projections: GEMV + all-reduce in one kernel.
  * The reference has no multi-GPU path; this is the exchange step of the tensor-parallel
  * decode (one process per GPU). Rank r computes its partial y_r = Wt_r^T . mask(x_r) over
- * its slice of the input channels. Every thread of the CTA that finishes a 256-column tile
- * sends its column's fp32 value, tagged with the step's epoch in the same 64-bit store, into
+ * its slice of the input channels. Every thread that finishes a column
+ * sends its fp32 value, tagged with the step's epoch in the same 64-bit store, into
  * every rank's receive area through peer-mapped pointers (NVLink); it then polls its
  * column's words in the local area until all ranks' values of this epoch are there and adds
  * them in rank order (fp32, rounded once, then + residual). Every rank gets bit-identical y

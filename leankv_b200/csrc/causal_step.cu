@@ -133,7 +133,10 @@ __device__ __forceinline__ uint32_t transpose8(uint32_t x) {
 // The cluster waits for the CTA that makes the new row, so that CTA's chain is kept short: the row is asked for together with the
 // queries, the zeros behind it are written while the launch ahead drains, and the gates' logistic function is taken under the cluster
 // barrier. A step of four layers of width 2048 at 2100 positions 230.1 -> 224.3 us (its wait at the barrier 9400 -> 3700 cycles of 27 000).
-// Alone, 4 / 8 kv heads: 2184 keys 13.1 -> 11.6 and 14.1 -> 12.4 us; 32768 keys, where the stream is the time, 40.9 -> 40.0 and 38.6 -> 40.8.
+// Alone, 4 / 8 kv heads: 2184 keys 10.3 -> 9.0 and 11.5 -> 10.0 us; 32768 keys, where the stream is the time, 40.2 -> 39.5 and 38.0 -> 41 to 43: launches
+// of eight kv heads leave room for some CTAs of the next, and one right behind the other they share SMs less evenly. In a step, with
+// projections between, the shorter chain wins at every length (width 4096, 8 kv heads, 2000 / 16000 / 32000 keys 478.4 -> 473.7, 537.8 -> 535.0,
+// 590.9 -> 588.8 us), so it is taken at every length.
 // NP: 16-column pieces of the values that a warp accumulates at most (tensor cores).
 template <Walk W, int NP>
 __global__ void __launch_bounds__(32 * warps_of(W), W == Walk::kWarps ? 2 : 1) causal_step_kernel(const __grid_constant__ StepArgs p) {
@@ -222,7 +225,6 @@ __global__ void __launch_bounds__(32 * warps_of(W), W == Walk::kWarps ? 2 : 1) c
         return make_float2(d < dim ? __ldcg(x + d) : 0.f, d + 1 < dim ? __ldcg(x + d + 1) : 0.f);
     };
     auto turned = [&](float2 v, int d, int rot) { return d < rot ? turn(v.x, v.y, s_sin[d >> 1], s_cos[d >> 1]) : v; };
-    auto pair_at = [&](const float* x, int d, int dim, int rot) { return turned(pair_of(x, d, dim), d, rot); };
     constexpr int kBatch = 5;                             // loads in flight per thread
     float2 in[kBatch];
     auto load_queries = [&](int e0) {

@@ -285,6 +285,38 @@ def test_batch_qkv_post_is_bit_identical_to_single_sequence_kernel():
     assert not torch.equal(pool_a, base)
 
 
+@pytest.mark.parametrize("B,n_q,n_kv", [(1, 8, 2), (11, 8, 2), (48, 32, 8)])
+def test_qkv_post_with_the_early_flag_writes_the_same_bits(B, n_q, n_kv):
+    """One sequence, a CTA for every four sequences, and CTAs that walk several groups; behind a launch that writes the projections only."""
+    lib, g, pages = _native.lib(), torch.Generator(device=_dev()).manual_seed(B), 4
+    rp = RawPool(pages * B, n_kv, _dev())
+    n, Pk, Pv = (n_q + 2 * n_kv) * 128, rp.Pi_k.t().contiguous(), rp.Pi_v.t().contiguous()
+    src, qkv = torch.randn(B, n, device=_dev(), generator=g).half(), torch.empty(B, n, dtype=torch.float16, device=_dev())
+    ones, inv = torch.ones(n, dtype=torch.float16, device=_dev()), 10000.0 ** (-torch.arange(64, device=_dev()) / 64)
+    pos = torch.randint(0, 16 * pages, (B,), device=_dev(), generator=g).to(torch.int32)
+    state = torch.zeros(8, dtype=torch.int32, device=_dev())
+    state[0] = pos[0]
+    indptr, pages_of = rp.i32(range(0, pages * B + 1, pages)), rp.i32(reversed(range(pages * B)))
+    base = torch.randint(0, 256, rp.pool.shape, dtype=torch.uint8, device=_dev(), generator=g)
+    got = []
+    for flags in (0, _native.POST_EARLY):
+        for _ in range(5):
+            pool, q = base.clone(), torch.zeros(B, n_q, 128, device=_dev())
+            qkv.zero_()
+            _native.check(lib.leankv_rmsnorm_rows_f16(src.data_ptr(), None, ones.data_ptr(), qkv.data_ptr(), B, n, 1e-5, _st()), "norm")
+            rest = (Pk.data_ptr(), Pv.data_ptr(), rp.bounds.data_ptr(), pool.data_ptr(), rp.n_pages, pages_of.data_ptr(), n_q, n_kv,
+                    q.data_ptr(), flags, _st())
+            if B == 1:
+                rc = lib.leankv_decode_qkv_post_flags(qkv.data_ptr(), inv.data_ptr(), state.data_ptr(), *rest)
+            else:
+                rc = lib.leankv_batch_qkv_post_flags(qkv.data_ptr(), B, inv.data_ptr(), pos.data_ptr(), indptr.data_ptr(), *rest)
+            _native.check(rc, "post")
+            got.append((pool, q))
+    torch.cuda.synchronize()
+    assert not torch.equal(got[0][0], base) and got[0][1].abs().sum() > 0
+    assert all(torch.equal(p, got[0][0]) and torch.equal(q, got[0][1]) for p, q in got[1:])
+
+
 def test_batched_step_matches_single_sequence_engines():
     """Dense projections either way (no thresholds): library GEMM rows vs the GEMV kernel differ in
     summation order only, so logits agree to fp16 rounding while tokens are teacher-forced."""

@@ -155,6 +155,27 @@ def test_stream_norm_residual_shift(dtype, T, W):
 
 
 @pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("T,W", [(591, 1024), (592, 1024), (1184, 1024), (1183, 1028), (1185, 2048), (1187, 2052)])
+@pytest.mark.parametrize("branch", [False, True])
+def test_stream_norm_shift_by_rows_of_a_cta(dtype, T, W, branch):
+    """One, two and four rows a CTA, last CTAs that are not full: the row above is the same wherever it was normed."""
+    x, dlt, s, mu, first = (t.to(DEV) for t in (rnd(T, W, seed=1), rnd(T, W, seed=2), rnd(W, seed=3), rnd(2, W, seed=4, mean=0.5), rnd(W, seed=5)))
+    g, xo, h = torch.tensor(1.4, device=DEV), torch.empty(T, W, device=DEV), torch.empty(T, W, dtype=dtype, device=DEV)
+    mixed, last = torch.full((2, T, W), 7.0, dtype=dtype, device=DEV), torch.empty(W, device=DEV)
+    a = _native.StreamNorm(x_in=x.data_ptr(), gain=g.data_ptr(), h=h.data_ptr(), mixed=mixed.data_ptr(), prev_in=first.data_ptr(),
+                           prev_out=last.data_ptr(), dtype=CODE[dtype], delta_dtype=_native.DT_F32, rows=T, width=W, n_mix=2, eps=1e-3)
+    if branch:
+        a.x_out, a.delta, a.scale = xo.data_ptr(), dlt.data_ptr(), s.data_ptr()
+    a.mu[0], a.mu[1] = mu[0].data_ptr(), mu[1].data_ptr()
+    ok(_native.mixers().leankv_stream_norm(ctypes.byref(a), stream()))
+    hw = plain.scalar_norm(x.double() + (s.double() * dlt.double() if branch else 0), g.double(), 1e-3)
+    above, tol_ = torch.cat([first.double()[None], hw[:-1]]), 1e-5 if dtype == F32 else 4e-3
+    assert rel(h.float(), hw) < tol_ and rel(last, hw[-1]) < 1e-6
+    for i in range(2):
+        assert rel(mixed[i].float(), hw + (above - hw) * mu[i].double()) < tol_
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("T,n", [(3, 8), (2, 5), (17, 64)])
 def test_silu_mul_and_tanh_split(dtype, T, n):
     gu = rnd(T, 2 * n, seed=1, std=2.0).to(dtype)
@@ -176,6 +197,7 @@ class Window:
 
     def __init__(self, dtype, H, G, d, dv, size, pool, chunk, limit, scale=0.4, normed=True, talk=True, seed=0):
         self.H, self.G, self.d, self.dv, self.size, self.pool, self.scale, self.dtype = H, G, d, dv, size, pool, scale, dtype
+        self.early = 0
         ring = max(size, pool) + chunk - 1
         z = lambda n, w: torch.full((n, G, pad16(w)), float("nan"), dtype=dtype, device=DEV)
         self.buf = [z(ring, d), z(ring, dv), z(limit // pool + 1, d), z(limit // pool + 1, dv)]
@@ -212,7 +234,7 @@ class Window:
         state[0] = pos
         ws = torch.empty(max(16, lib.leankv_mixer_step_workspace_bytes(ref, self.limit)), dtype=torch.uint8, device=DEV)
         s = _native.MixerStep(y=y.data_ptr(), out=out.data_ptr(), left_scale=0.5, state=state.data_ptr(),
-                              max_pos=self.limit, ws=ws.data_ptr(), ws_bytes=ws.numel())
+                              max_pos=self.limit, ws=ws.data_ptr(), ws_bytes=ws.numel(), early_state=self.early)
         ok(lib.leankv_mixer_step(ref, None, ctypes.byref(s), stream()))
         return out.cpu()
 
@@ -238,10 +260,14 @@ class Window:
         if self.normed:
             q, k = plain.rms(q, 1e-4) * self.qn.double(), plain.rms(k, 1e-4) * self.kn.double()
         q = (q * self.scale if stepped else held(q) * self.scale).reshape(T, H, -1)[first:]
-        k, v = held(k).reshape(T, G, -1), held(v).reshape(T, G, -1)
         nb = T // self.pool
-        mean = lambda x: held(x[:nb * self.pool].reshape(nb, self.pool, G, -1).mean(1))
-        k, v = torch.cat([mean(k), k]).to(DEV), torch.cat([mean(v), v]).to(DEV)
+        if self.c.ring >= T:            # every token is still there: what the kernels have put, last bits and all
+            k, v = (torch.cat([p[:nb, :, :n], r[:T, :, :n]]).double() for p, r, n in ((self.buf[2], self.buf[0], self.d),
+                                                                                     (self.buf[3], self.buf[1], self.dv)))
+        else:
+            k, v = held(k).reshape(T, G, -1), held(v).reshape(T, G, -1)
+            mean = lambda x: held(x[:nb * self.pool].reshape(nb, self.pool, G, -1).mean(1))
+            k, v = torch.cat([mean(k), k]).to(DEV), torch.cat([mean(v), v]).to(DEV)
         i, j = torch.arange(first, T)[:, None], torch.arange(T)[None]
         seen = torch.cat([(torch.arange(nb)[None] + 1) * self.pool - 1 <= i - self.size, (j <= i) & (i - j < self.size)], 1).to(DEV)
         rep = H // G
@@ -294,14 +320,20 @@ def test_window_pool_prompt_portions_and_steps_agree_with_plain(dtype, shape):
                                    (16, 2, 48, 16, 100, 5), (6, 3, 112, 128, 1, 7)])
 def test_prompt_attention_by_key_tiles(shape):
     """Tiles of 64 blocks or tokens with remainders, rings that wrap inside a tile, rows of CTAs that are not full, slots that nothing
-    has written (NaN), against float64. Values and outputs are bf16, weights 16 bits: 2^-8 a value bounds the difference."""
+    has written (NaN), against float64 of the bf16 numbers that the kernel takes. Outputs are rounded to bf16, 2^-9 a value; weights keep 16
+    bits, sums 24: 2^-8 a row bounds the difference."""
     T = 400
     win = Window(BF16, *shape, chunk=T, limit=T)
     qkv = win.qkv(T)
     want = win.expected(qkv)
-    assert rel(feed(win, qkv, [T]), want) < 3e-2
+    got = feed(win, qkv, [T])
+    assert rel(got, want) < 3e-2 and rel(got, win.exact(qkv, 0, False)) < 2 ** -8
     small = Window(BF16, *shape, chunk=150, limit=T)
-    assert rel(feed(small, qkv, [150, 2, 131, 1, 33, 83]), want) < 3e-2
+    got = feed(small, qkv, [150, 2, 131, 1, 33, 83])
+    assert rel(got, want) < 3e-2
+    exact = small.exact(qkv, 0, False)
+    exact[283] = small.exact(qkv, 0, True)[283]              # the one step among them
+    assert rel(got, exact) < 2 ** -8
 
 
 @pytest.mark.parametrize("shape,T,start", [((16, 4, 64, 64, 64, 16), 800, 0), ((16, 4, 32, 48, 64, 16), 799, 0), ((16, 4, 32, 32, 100, 16), 600, 0),
@@ -321,12 +353,16 @@ def test_prompt_attention_with_few_keys(shape, T, start):
 @pytest.mark.parametrize("normed,talk", [(True, True), (False, True), (True, False)])
 def test_step_on_tensor_cores_around_whole_tiles(shape, normed, talk):
     """A CTA's share of the keys grows from 16 to 17 (255 .. 274 visible keys over 16 CTAs), the window moves past its first
-    token, blocks become visible and complete: against float64. The bound is the tests' own for bf16 keys and values."""
+    token, blocks become visible and complete: against float64 of the keys and values as they are stored. Queries keep 17 bits (two bf16
+    numbers), which moves a score of order ten by some 5e-5; exponentials keep 24, sums and outputs are fp32. With early_state the same bits."""
     T = 300
     win = Window(BF16, *shape, chunk=T, limit=T, normed=normed, talk=talk)
     qkv = win.qkv(T)
     got = feed(win, qkv, [252] + [1] * (T - 252))
     assert rel(got[252:], win.expected(qkv)[252:]) < 3e-2
+    assert rel(got[252:], win.exact(qkv, 252, True)) < 1.5e-4
+    win.early = 1
+    assert torch.equal(feed(win, qkv, [252] + [1] * (T - 252))[252:], got[252:])
 
 
 @pytest.mark.parametrize("dtype", [F32, BF16])
@@ -485,6 +521,16 @@ def test_time_mix_steps(dtype, H, d, rank):
         got.append(out.cpu().clone())
     assert rel(torch.stack(got), want) < 5e-5
     assert rel(m.S.reshape(1, -1), S.reshape(1, -1)) < 1e-5
+    # read ahead of the wait, behind launches that write none of it: the same bits
+    state_of = m.S.clone()
+    m.S.zero_()
+    for t in range(T):
+        yd = y[t].to(DEV)
+        s = _native.MixerStep(y=yd.data_ptr(), rkvg_off=0, w1_off=4 * N, rank=rank, w2=w2d.data_ptr(), out=out.data_ptr(),
+                              right_off=0, right_scale=0.7, state=state.data_ptr(), max_pos=T, early_state=1)
+        ok(_native.mixers().leankv_mixer_step(None, ctypes.byref(m.c), ctypes.byref(s), stream()))
+        assert torch.equal(out.cpu(), got[t])
+    assert torch.equal(m.S, state_of)
 
 
 # ── whole models ─────────────────────────────────────────────────────────────────────────────

@@ -339,6 +339,79 @@ def test_one_workspace_serves_projections_of_different_widths():
         assert torch.isfinite(g).all()
 
 
+def _written(ws):
+    """Whether partial sums were put behind the arrival counters (the first 16 KB, which end at zero): the kernel with the workspace ran."""
+    assert not ws[:16384].any()
+    return bool((ws[16384:] != 0x5A).any())
+
+
+def _near(got, want, roundings):
+    return bool((got.double() - want).norm() <= roundings * 2 ** -11 * want.norm() + 1e-6)
+
+
+def test_one_workspace_through_the_kernel_that_needs_it():
+    """Above the sizes of the cluster kernel: wide, long, ragged in both directions, a wide one with few splits. Segments with thresholds of their
+    own, bias and residual; a norm in front, with a residual and in the gated pair. One workspace serves all, twice over. Norm inputs are
+    half, one or two times a weight near one, so that no rounding decides what passes a threshold."""
+    lib, dev, st = _native.lib(), _dev(), torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device=dev).manual_seed(12)
+    shapes = [(6144, 4096), (14336, 2048), (4104, 8200), (512, 14336), (40008, 1032)]
+    need = max(lib.leankv_sparse_gemv_workspace_bytes(n, z) for n, z in shapes)
+    need = max(need, *(lib.leankv_sparse_swiglu_workspace_bytes(n, z) for n, z in shapes))
+    ws = torch.full((need,), 0x5A, dtype=torch.uint8, device=dev)
+    ws[:16384] = 0
+    rnd = lambda *s, std=1.0: (torch.randn(*s, device=dev, generator=gen) * std).half()
+    silu = lambda a: a / (1 + torch.exp(-a))
+    for turn in range(2):
+        for n, z in shapes:
+            w, x, bias, res = rnd(z, n, std=0.02), rnd(z), rnd(n), rnd(n)
+            segs = _native.Segments()
+            segs.n_segments = 3 if n > 512 else 2
+            ends, thr = (256, 512, n) if n > 512 else (256, n), (0.2, 0.9, 0.5)
+            for i, e in enumerate(ends):
+                segs.seg_end[i], segs.threshold[i] = e, thr[i]
+
+            def rows(v):
+                lo, out = 0, []
+                for e, t in zip(ends, thr):
+                    live = torch.where(v.abs() > torch.tensor(t).half(), v, torch.zeros_like(v)).double()
+                    out.append(live @ w[:, lo:e].double())
+                    lo = e
+                return torch.cat(out)
+
+            y = torch.full((n,), float("nan"), dtype=torch.float16, device=dev)
+            ws[16384:] = 0x5A
+            _native.check(lib.leankv_sparse_gemv_seg_f16(w.data_ptr(), x.data_ptr(), y.data_ptr(), n, z, ctypes.byref(segs), bias.data_ptr(),
+                                                         res.data_ptr(), ws.data_ptr(), ws.numel(), None, st), "seg")
+            assert _written(ws) and _near(y, rows(x) + bias.double() + res.double(), 3), (n, z, turn)
+
+            h = (torch.randint(0, 3, (z,), device=dev, generator=gen) - 1.0).exp2() * torch.randn(z, device=dev, generator=gen).sign()
+            h, nw = h.half(), (1 + 0.1 * torch.rand(z, device=dev, generator=gen)).half()
+            r = torch.rsqrt((h.float() ** 2).mean() + 1e-5)
+            normed = nw * (h.float() * r).half()
+            thr = [float(r) * f for f in (0.75, 1.5, 0.3)]
+            for i in range(segs.n_segments):
+                segs.threshold[i] = thr[i]
+            ws[16384:] = 0x5A
+            _native.check(lib.leankv_sparse_gemv_rmsnorm_f16(w.data_ptr(), h.data_ptr(), nw.data_ptr(), 1e-5, y.data_ptr(), n, z, ctypes.byref(segs),
+                                                             res.data_ptr(), ws.data_ptr(), ws.numel(), None, st), "normed")
+            assert _written(ws) and _near(y, rows(normed) + res.double(), 2), (n, z, turn)
+            if n * z < 20_000_000 and z <= 8192:
+                continue                                     # the pair of these is the cluster kernel's
+            w2 = rnd(z, n, std=0.02)
+            ws[16384:] = 0x5A
+            _native.check(lib.leankv_sparse_swiglu_rmsnorm_f16(w.data_ptr(), w2.data_ptr(), h.data_ptr(), nw.data_ptr(), 1e-5, y.data_ptr(), n, z,
+                                                               thr[0], thr[1], ws.data_ptr(), ws.numel(), None, st), "normed pair")
+            part = lambda m, t: torch.where(normed.abs() > torch.tensor(t).half(), normed, torch.zeros_like(normed)).double() @ m.double()
+            assert _written(ws) and _near(y, silu(part(w, thr[0])) * part(w2, thr[1]), 4), (n, z, turn)
+    for n, z in ((4096, 4096), (2048, 8192), (512, 512)):      # and these leave it alone
+        w, x, y = rnd(z, n, std=0.02), rnd(z), torch.empty(n, dtype=torch.float16, device=dev)
+        ws[16384:] = 0x5A
+        _native.check(lib.leankv_sparse_gemv_f16(w.data_ptr(), x.data_ptr(), y.data_ptr(), n, z, 0.5, None, None, ws.data_ptr(), ws.numel(),
+                                                 None, st), "gemv")
+        assert not _written(ws)
+
+
 _PREFETCH_SNIPPET = r"""
 import hashlib, sys, torch
 sys.path.insert(0, %(root)r)
