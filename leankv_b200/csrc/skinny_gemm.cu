@@ -4,7 +4,8 @@
 // W's columns are the 128 rows of a tcgen05 product and the batch its columns, so a tile of W goes from HBM by TMA into swizzled shared
 // memory and from there to the tensor core as it lies (MN-major operand): no register touches it. A CTA takes 128 columns of W and
 // a share of K; the shares of a column block are one cluster, whose CTAs add their sums through distributed shared memory, each a part
-// of the rows, in rank order. Five stages of 64 rows of W (16 KB) and two CTAs an SM keep about 160 KB an SM in flight.
+// of the rows, in rank order. Stages of 64 rows of W (16 KB) beside the batch's columns, as many as half an SM holds (six up to 16 rows, five up to 32,
+// four up to 64, three at 128), and two CTAs an SM keep 96 to 192 KB of W an SM in flight.
 //
 //   warp 0   copies: W's tiles, ahead of the dependency wait where the caller says that the launch ahead does not write them,
 //            and the batch's columns of the same K
@@ -186,23 +187,6 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_gemm_kernel(const __grid_c
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
-int make_map2(CUtensorMap* map, const void* base, cuuint64_t inner, cuuint64_t outer, cuuint32_t box_rows) {
-    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-    if (encode == nullptr) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        LEANKV_CUDA_TRY(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found));
-        if (found != cudaDriverEntryPointSuccess || fn == nullptr) return LEANKV_EUNSUPPORTED;
-        encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-    }
-    const cuuint64_t dims[2] = {inner, outer}, bytes[1] = {inner * 2};
-    const cuuint32_t box[2] = {64, box_rows}, step[2] = {1, 1};
-    const CUresult rc = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, bytes, box, step,
-                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return rc == CUDA_SUCCESS ? LEANKV_OK : LEANKV_EINVAL;
-}
-
 }  // namespace
 }  // namespace leankv
 
@@ -230,8 +214,13 @@ extern "C" int leankv_skinny_gemm_f16_status(const void* x, const void* w, void*
     const int blocks = (N + kCols - 1) / kCols;
     // as many CTAs as clusters of up to eight find room for (6144 columns, us by CTAs: 144 13.4, 192 12.1, 240 11.7, 288 18.1)
     const int split = std::max(1, std::min(std::min(kMaxSplit, 256 / blocks), p.steps / 2));
-    int rc = make_map2(&p.w, w, N, K, kKStep);
-    if (!rc) rc = make_map2(&p.x, x, K, rows, p.rows_pad);
+    const auto map = [](CUtensorMap* m, const void* base, cuuint64_t inner, cuuint64_t outer, cuuint32_t box_rows) {
+        const cuuint64_t dims[2] = {inner, outer}, strides[1] = {inner};
+        const cuuint32_t box[2] = {(cuuint32_t)tma::kBoxCols, box_rows};
+        return tma::make_map(m, base, 2, dims, strides, box, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    };
+    int rc = map(&p.w, w, N, K, kKStep);
+    if (!rc) rc = map(&p.x, x, K, rows, p.rows_pad);
     if (rc) return rc;
     LEANKV_CUDA_TRY(cudaFuncSetAttribute(skinny_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     LEANKV_CUDA_TRY(launch_cluster_kernel_ex(true, dim3(1, split, 1), skinny_gemm_kernel, dim3(blocks, split), dim3(kThreads), smem,

@@ -1,4 +1,4 @@
-// Tensor-map construction on the host and tiled copies (TMA) of bf16 operands into 128-byte-swizzled shared
+// Tensor-map construction on the host and tiled copies (TMA) of 16-bit operands into 128-byte-swizzled shared
 // memory, with the matching tcgen05 operand descriptors. A copied box is 64 elements (128 bytes) wide; its rows
 // follow one another, and every group of eight rows is one swizzle atom of 1024 bytes.
 #pragma once
@@ -13,9 +13,10 @@ namespace tma {
 
 constexpr int kBoxCols = 64;
 
-// Map of a row-major bf16 tensor of `rank` dimensions (innermost first); strides in elements of dimensions 1 .. .
+// Map of a row-major tensor of 16-bit numbers of `rank` dimensions (innermost first); strides in elements of dimensions 1 .. .
 inline int make_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
-                    const cuuint32_t* box) {
+                    const cuuint32_t* box, CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                    CUtensorMapL2promotion fetch = CU_TENSOR_MAP_L2_PROMOTION_L2_128B) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (encode == nullptr) {
         void* fn = nullptr;
@@ -27,9 +28,9 @@ inline int make_map(CUtensorMap* map, const void* base, int rank, const cuuint64
     cuuint64_t bytes[4];
     cuuint32_t step[5] = {1, 1, 1, 1, 1};
     for (int i = 0; i + 1 < rank; ++i) bytes[i] = strides[i] * 2;
-    const CUresult rc = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims, bytes,
+    const CUresult rc = encode(map, type, (cuuint32_t)rank, const_cast<void*>(base), dims, bytes,
                                box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                               fetch, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return rc == CUDA_SUCCESS ? LEANKV_OK : LEANKV_EINVAL;
 }
 
