@@ -361,10 +361,10 @@ class MixerDecodeEngine(DecodeLoop):
         self.state[_native.STATE_PARITY].fill_(self._parity)
         return x
 
-    def _logits_of(self, x: torch.Tensor) -> torch.Tensor:
+    def _logits_of(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         h = torch.empty(x.shape, dtype=self.dtype, device=self.dev)
         self._stream_norm(x, self.final_norm, h)
-        z = matmul(h, self.head)
+        z = matmul(h, self.head, out=out)
         if self.cfg.logit_softcap > 0:
             _native.check(self.lib.leankv_softcap(z.data_ptr(), z.numel(), self.cfg.logit_softcap, self._st()), "softcap",
                           self.lib)
@@ -416,19 +416,18 @@ class MixerDecodeEngine(DecodeLoop):
             up = torch.from_numpy(np.concatenate([host, np.frombuffer(array("q", places + order), dtype=np.int64)])).to(
                 self.dev, non_blocking=True)           # array: places are whole numbers, or an error
             ids, at, to = up[:n], up[n:n + len(order)], up[n + len(order):]
-            # one portion's logits in order are the result; else they go into it portion by portion, never all of them twice
-            whole = sum(map(bool, rows)) == 1 and order == sorted(order)
-            out = None if whole else torch.empty(len(order), self.cfg.vocab_size, dtype=torch.float32, device=self.dev)
+            # places in order: every portion's logits are written where they belong; else they are put there portion by portion
+            in_order = order == sorted(order)
+            out = torch.empty(len(order), self.cfg.vocab_size, dtype=torch.float32, device=self.dev)
             done = 0
             for (s0, m), r in zip(parts, rows):
                 x = self._portion(ids[s0:s0 + m])
                 if not r:
                     continue
-                z = self._logits_of(x[at[done:done + len(r)]])
-                if whole:
-                    out = z
-                else:
-                    out.index_copy_(0, to[done:done + len(r)], z)
+                mine = slice(done, done + len(r))
+                z = self._logits_of(x[at[mine]], out[mine] if in_order else None)
+                if not in_order:
+                    out.index_copy_(0, to[mine], z)
                 done += len(r)
             if order:
                 self.check_status()

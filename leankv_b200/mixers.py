@@ -30,11 +30,11 @@ def dtype_code(dtype: torch.dtype) -> int:
     return {torch.bfloat16: _native.DT_BF16, torch.float32: _native.DT_F32}[dtype]
 
 
-def matmul(a: torch.Tensor, w: torch.Tensor, exact_out: bool = True) -> torch.Tensor:
+def matmul(a: torch.Tensor, w: torch.Tensor, exact_out: bool = True, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """a [.., K] times w [N, K] transposed; fp32 result if ``exact_out``, else of a's type."""
     if exact_out and a.dtype != torch.float32:
-        return torch.mm(a, w.t(), out_dtype=torch.float32)
-    return torch.mm(a, w.t())
+        return torch.mm(a, w.t(), out_dtype=torch.float32, out=out)
+    return torch.mm(a, w.t(), out=out)
 
 
 def _step_gemv(**kw) -> _native.DenseGemv:

@@ -681,7 +681,7 @@ def test_logits_of_many_portions_are_held_once():
     got = eng.extend(ids, order)
     size = got.numel() * 4
     assert torch.cuda.max_memory_allocated() - held < 1.5 * size
-    assert torch.equal(got, first[order])
+    assert rel(got, first[order]) < 1e-5           # the head's product may go by another kernel: fp32 sums in another order
     eng.reset()
     # one row through the head's product: the same bf16 numbers, fp32 sums in another order
     assert rel(eng.extend(ids, [639]), first[639:]) < 1e-5 and eng.extend([1, 2]).shape == (0, 4099)
