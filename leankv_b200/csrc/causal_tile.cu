@@ -307,7 +307,7 @@ int causal_tile_attend(const leankv_causal_attn_t& a, const void* q, const float
     if (!rc && a.v) rc = map(&p.v, a.v, a.vdim_pad, G, a.k_rows, 1, kKeys);
     if (rc) return rc;
     LEANKV_CUDA_TRY(cudaFuncSetAttribute(causal_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    LEANKV_CUDA_TRY(launch_kernel(causal_tile_kernel, dim3((rows + p.tq - 1) / p.tq, a.kv_heads), dim3(kThreads), smem, st, p));
+    LEANKV_CUDA_TRY(launch_plain(causal_tile_kernel, dim3((rows + p.tq - 1) / p.tq, a.kv_heads), dim3(kThreads), smem, st, p));
     return LEANKV_OK;
 }
 

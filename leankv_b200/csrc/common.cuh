@@ -28,7 +28,7 @@ int sm_count();
 // Whether launches carry the programmatic-stream-serialization attribute (default on; the
 // environment variable LEANKV_PDL=0 turns it off).
 bool pdl_enabled();
-// LEANKV_PDL: 0 = never, 1 = every kernel may start early, 2 (default) = those whose launch says so: kernels that read
+// LEANKV_PDL: 0 = never, 1 = every kernel may start early but those of launch_plain, 2 (default) = those whose launch says so: kernels that read
 // constants ahead of the dependency wait (GEMVs, decode attention, the post kernel) and those of launch_early.
 int pdl_mode();
 
@@ -69,13 +69,25 @@ inline cudaError_t launch_cluster_kernel_ex(bool early_ok, dim3 cluster, void (*
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     const int mode = pdl_mode();
-    cfg.numAttrs = (mode == 1 || (mode == 2 && early_ok)) ? 2 : 1;
+    cfg.numAttrs = mode != 0 && early_ok ? 2 : 1;        // those that are not take tensor memory
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                  Args&&... args) {
     return launch_kernel_ex(false, kernel, grid, block, smem, st, static_cast<Args&&>(args)...);
+}
+
+// A launch behind the one ahead in any case: for kernels that take tensor memory ahead of their dependency wait, or let later launches in before
+// every block has its own (skinny_gemm.cu orders the three by itself).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_plain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 // A launch that may become resident while the one ahead drains: for kernels whose every thread begins with pdl_begin() (nothing

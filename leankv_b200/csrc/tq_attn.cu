@@ -694,10 +694,10 @@ extern "C" int leankv_tq_prefill_attn_strided(const void* q, long long q_token, 
         a.start_pos = start_pos;
         a.n_tiles = ep.k_tiles;
         a.status = e.status;
-        LEANKV_CUDA_TRY(launch_kernel(tq_prefill_tile_kernel, dim3(ep.q_tiles, n_kv_heads, ep.n_splits), dim3(kPtThreads),
+        LEANKV_CUDA_TRY(launch_plain(tq_prefill_tile_kernel, dim3(ep.q_tiles, n_kv_heads, ep.n_splits), dim3(kPtThreads),
                                       kPtSmemBytes, st, a));
         if (ep.n_splits > 1)
-            LEANKV_CUDA_TRY(launch_kernel(tq_rot_rows_kernel<false>, dim3(rot_grid), dim3(kRotThreads), kRotSmemBytes, st,
+            LEANKV_CUDA_TRY(launch_plain(tq_rot_rows_kernel<false>, dim3(rot_grid), dim3(kRotThreads), kRotSmemBytes, st,
                                           static_cast<const void*>(a.o_part), static_cast<const float*>(a.ml_part), ep.n_splits,
                                           Pi_v, out, n_vec, e.status));
         return LEANKV_OK;
@@ -707,7 +707,7 @@ extern "C" int leankv_tq_prefill_attn_strided(const void* q, long long q_token, 
     float* qprime = reinterpret_cast<float*>(ws + tp.off_qprime);
     float* o_part = reinterpret_cast<float*>(ws + tp.off_opart);
     float* ml_part = reinterpret_cast<float*>(ws + tp.off_ml);
-    LEANKV_CUDA_TRY(launch_kernel(tq_rot_rows_kernel<true>, dim3(rot_grid), dim3(kRotThreads), kRotSmemBytes, st, q,
+    LEANKV_CUDA_TRY(launch_plain(tq_rot_rows_kernel<true>, dim3(rot_grid), dim3(kRotThreads), kRotSmemBytes, st, q,
                                   static_cast<const float*>(nullptr), 0, Pi_k, static_cast<void*>(qprime), n_vec,
                                   reinterpret_cast<int*>(ws)));
     PrefillParams p{};
@@ -730,15 +730,15 @@ extern "C" int leankv_tq_prefill_attn_strided(const void* q, long long q_token, 
     p.inv_alpha = 1.0f / lut.alpha;
     p.status = reinterpret_cast<int*>(ws);
     if (prefill_mode() == 2)
-        LEANKV_CUDA_TRY(launch_kernel(tq_prefill_ws_kernel, dim3(tp.n_tiles, n_kv_heads, tp.n_splits),
+        LEANKV_CUDA_TRY(launch_plain(tq_prefill_ws_kernel, dim3(tp.n_tiles, n_kv_heads, tp.n_splits),
                                       dim3(kWsThreads), kWsSmemBytes, st, p));
     else if (prefill_mode() == 1)
-        LEANKV_CUDA_TRY(launch_kernel(tq_prefill_t5_kernel, dim3(tp.n_tiles, n_kv_heads, tp.n_splits),
+        LEANKV_CUDA_TRY(launch_plain(tq_prefill_t5_kernel, dim3(tp.n_tiles, n_kv_heads, tp.n_splits),
                                       dim3(kT5Threads), kT5SmemBytes, st, p));
     else
         LEANKV_CUDA_TRY(launch_kernel(tq_prefill_attn_kernel, dim3(tp.n_tiles, n_kv_heads, tp.n_splits),
                                       dim3(kAttnThreads), kPfSmemBytes, st, p));
-    LEANKV_CUDA_TRY(launch_kernel(tq_rot_rows_kernel<false>, dim3(rot_grid), dim3(kRotThreads), kRotSmemBytes, st,
+    LEANKV_CUDA_TRY(launch_plain(tq_rot_rows_kernel<false>, dim3(rot_grid), dim3(kRotThreads), kRotSmemBytes, st,
                                   static_cast<const void*>(o_part), static_cast<const float*>(ml_part), tp.n_splits,
                                   Pi_v, out, n_vec, reinterpret_cast<int*>(ws)));
     return LEANKV_OK;

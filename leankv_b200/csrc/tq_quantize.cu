@@ -390,7 +390,7 @@ extern "C" int leankv_tq_pool_append_strided(const void* k, const void* v, int B
             LEANKV_CUDA_TRY(cudaGetSymbolAddress(&st_word, g_append_status));
             const long long slots1 = sm_count();            // 148 KB of shared memory: one CTA per SM
             const int grid_t5 = (int)(tp.n_tiles < slots1 ? tp.n_tiles : slots1);
-            LEANKV_CUDA_TRY(launch_kernel(tq_pool_append_t5_kernel, dim3(grid_t5), dim3(kT5Threads), kT5SmemBytes,
+            LEANKV_CUDA_TRY(launch_plain(tq_pool_append_t5_kernel, dim3(grid_t5), dim3(kT5Threads), kT5SmemBytes,
                                           static_cast<cudaStream_t>(stream), tp, static_cast<int*>(st_word)));
             return LEANKV_OK;
         }

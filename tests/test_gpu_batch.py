@@ -364,3 +364,53 @@ def test_generate_returns_history_and_graph_equals_eager():
     torch.cuda.synchronize()
     assert torch.equal(toks, b.history[:, :8])
     assert a.kv_bytes_per_sequence(4096) == 256 * 2 * CFG.num_layers * CFG.num_kv_heads * 800
+
+
+_OVERLAP_SNIPPET = r"""
+import hashlib, sys, torch
+sys.path[:0] = [%(root)r, %(tests)r]
+from leankv_b200.batch_engine import BatchDecodeEngine
+from leankv_b200.engine import DecodeEngine, DecoderConfig
+from leankv_b200.mixer_engine import MixerDecodeEngine, MixerModelConfig
+from leankv_b200.turboquant.quantizer import TurboQuantMSE
+import pefitar_util, rorosun_util
+dev, out = torch.device("cuda:0"), []
+cfg = DecoderConfig(vocab_size=512, hidden_size=1024, intermediate_size=2048, num_layers=2, num_q_heads=8, num_kv_heads=2)
+one = DecodeEngine.random_init(cfg, dev, seed=1, max_seq_len=700)
+one.prefill([t %% 512 for t in range(600)], chunk=256)
+for _ in range(4):
+    one.step()
+out += [one.logits, one.prefill_logits]
+many = BatchDecodeEngine.random_init(cfg, dev, 5, seed=2, max_seq_len=128)
+out.append(many.generate(torch.arange(5 * 100).reshape(5, 100) %% 512, 6))
+for util in (rorosun_util, pefitar_util):
+    layers = ([util.layer(heads=8, kv_heads=2, dim=64, vdim=64, size=48, pool=8, r_heads=4, r_dim=64, ff=320)] * 2 if util is rorosun_util else
+              [util.attention(heads=8, kv_heads=2, dim=64, vdim=64, dims=64, ff=320), util.latent(heads=8, dim=64, rot_dim=64, vdim=64, q_rank=128, kv_rank=128, size=100)])
+    cfg = util.config(layers=layers, vocab=512, width=256, **({} if util is rorosun_util else {"loop": (0, 1, 2)}))
+    eng = MixerDecodeEngine(MixerModelConfig.from_dict(cfg), util.weights(cfg), dev, max_seq_len=600, dtype=torch.bfloat16, max_chunk=200)
+    out += [eng.extend([t %% 512 for t in range(450)], range(0, 450, 7)), torch.cat([eng.extend([t], [0]) for t in range(5)])]
+q = TurboQuantMSE(128, 3, dev)
+x = torch.randn(5000, 128, generator=torch.Generator().manual_seed(1)).half().to(dev)
+for _ in range(3):
+    out.append(q.dequantize(q.quantize(x)))
+torch.cuda.synchronize()
+print("OUT", hashlib.sha256(b"".join(t.float().cpu().numpy().tobytes() for t in out)).hexdigest())
+"""
+
+
+def test_no_form_of_overlap_changes_a_result():
+    """LEANKV_PDL: no launch before the one ahead has ended, every launch that may, those that gain by it. Kernels that hold tensor memory
+    follow one another in all of them."""
+    import os
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    code = _OVERLAP_SNIPPET % {"root": str(ROOT), "tests": os.path.join(str(ROOT), "tests")}
+    outs = []
+    for mode in "012":
+        run = subprocess.run([sys.executable, "-c", code], env={**os.environ, "LEANKV_PDL": mode}, capture_output=True, text=True, timeout=300)
+        assert run.returncode == 0, run.stderr[-2000:]
+        outs.append(next(l for l in run.stdout.splitlines() if l.startswith("OUT")))
+    assert len(set(outs)) == 1
