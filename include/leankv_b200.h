@@ -423,6 +423,7 @@ int leankv_batch_qkv_post_flags(const void* qkv, int B, const float* inv_freq, c
  *   LEANKV_SKINNY_EARLY_WEIGHTS: W may be read while the launch ahead of this one still runs: that launch must not write it.
  *   LEANKV_SKINNY_EARLY_TMEM: the launch ahead takes no tensor memory (it is no tensor-core kernel of this generation); this one may then
  *     take its own while that one still runs. Behind a launch that does take some, both could wait for each other for good.
+ * Only with both are the weights read early; either alone changes little.
  * Where a wait inside the kernel runs out, the outputs are NaN; the _status form also sets LEANKV_SKINNY_GAVE_UP in *status (device; NULL:
  * nowhere). That bit is none of attention's, so one word may serve both. */
 #define LEANKV_SKINNY_EARLY_WEIGHTS 1

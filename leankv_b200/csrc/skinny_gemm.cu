@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_gemm_kernel(const __grid_c
     } else if (warp == 1) {                              // ---- products ----
         // Tensor memory is taken before later launches are let in: one of them could hold it while it waits for this one. And it is taken
         // behind the wait, where no block of a launch ahead can still be asking for its own; only where the caller says that the
-        // launch ahead takes none it is taken while that one drains (two CTAs an SM ask one after the other: 2048 x 2048, 16 rows,
-        // launches of this kernel one behind the other 5.4 us so, 6.1 behind the wait; steps of two to four layers 1 to 5 us).
+        // launch ahead takes none it is taken while that one drains (2048 x 2048, 16 rows, launches of this kernel one behind the other
+        // 5.4 us so, 5.7 behind the wait; steps of two to four layers 1 to 5 us).
         pdl_wait();
         if (!p.tmem_first) umma::tmem_alloc_n(addr(&s_tmem), p.tmem_cols);
         pdl_launch();
@@ -205,8 +205,11 @@ extern "C" int leankv_skinny_gemm_f16_status(const void* x, const void* w, void*
     p.rows_pad = (rows + 15) / 16 * 16;
     p.N = N;
     p.steps = (K + kKStep - 1) / kKStep;
-    p.early = (flags & LEANKV_SKINNY_EARLY_WEIGHTS) != 0;
     p.tmem_first = (flags & LEANKV_SKINNY_EARLY_TMEM) != 0;
+    // Weights ahead of the wait pay only where the tensor memory is there, too: taken beside copies in flight it comes late (launches one behind the
+    // other, 16 rows, us with both early / only the weights / neither: 4096 x 6144 11.0 / 11.9 / 10.9, 2048 x 2048 5.4 / 6.1 / 5.7, 14336 x 4096
+    // 20.7 / 22.2 / 21.1; in steps of a batch both early is the best).
+    p.early = p.tmem_first && (flags & LEANKV_SKINNY_EARLY_WEIGHTS) != 0;
     p.tmem_cols = p.rows_pad <= 32 ? 32 : p.rows_pad <= 64 ? 64 : 128;
     const size_t x_bytes = ((size_t)p.rows_pad * 128 + 1023) / 1024 * 1024;
     p.stages = (int)std::min<size_t>(kMaxStages, (110 * 1024 - 1024) / (kWBytes + x_bytes));
